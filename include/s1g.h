@@ -468,20 +468,15 @@ int s1g_launch_count(int64_t* n);
  *              S1G_E_PACKET_LENGTH without a read)
  * Work is queued on `stream` (a cudaStream_t, or NULL for the default
  * stream); the call returns without waiting.  Nothing is allocated: the
- * decoder's scratch is a fixed 16 MiB device array inside the library (held
- * by every GPU that loads it until exit).  num_quads is at most 65535 (the
- * width of the num_quadratures field; S1G_E_INVALID_ARGUMENT beyond), which
- * needs 262 KB of scratch per packet, so the array holds at least 64 packets
- * at a time and longer packet runs are decoded in chunks of that many (696
- * packets per chunk at num_quads 6000).  S1G_E_SCRATCH_LIMIT is returned if
- * one packet's scratch cannot fit.  The first call on each device, with that device
- * current, resolves the scratch address and copies the 10 KB Huffman table in
- * with a synchronous cudaMemcpyToSymbol; make that first call before any
- * stream capture.  All calls share the one scratch array: calls that can
- * overlap on the GPU (different streams without ordering between them) race
- * and corrupt each other's results; calls on one stream are safe.  Nothing
- * in the scratch has to start at zero: every byte read was written earlier in
- * the same call. */
+ * decoder works in shared memory, one launch for any number of packets.
+ * num_quads is at most 65535 (the width of the num_quadratures field;
+ * S1G_E_INVALID_ARGUMENT beyond), whose symbols fit; S1G_E_SCRATCH_LIMIT is
+ * kept for builds with a smaller scratch and not returned.  The first call on
+ * each device, with that device current, copies the 2.5 KB Huffman table into
+ * a device array of the library with a synchronous cudaMemcpyToSymbol; make
+ * that first call before any stream capture.  Calls share nothing else: they
+ * may overlap on different streams.
+ */
 int s1g_decode_fdbaq_noalloc(const uint8_t* d_stream, int64_t nbytes, const int64_t* d_offsets, int64_t npackets,
                              int num_quads, void* d_out, int64_t out_pitch, int32_t* d_status, void* stream);
 

@@ -93,7 +93,6 @@ struct s1g_decoder {
     int abc_fields = 0;   // formats A/B/C: 0 = the reference's output, 1 = each sample from its own fields
     std::string err;
     IndexScratch isc;
-    DecodeScratch dsc;
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
     Buf bFdf, bKN, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
@@ -408,7 +407,7 @@ struct Pipe {
         cpx<R>* A = h->bA.as<cpx<R>>((size_t)npk * g.n_r);
         int* status = h->bStatus.as<int>(npk);
         if (any_d)
-            decode_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status, h->dsc, h->tabs, st);
+            decode_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status, h->tabs, st);
         if (any_fixed)
             decode_fixed_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status,
                                   h->abc_fields, st);
@@ -474,7 +473,7 @@ struct Pipe {
         int* status = h->bEccmSt.as<int>(npk);
         if (any_d)
             decode_burst<double>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, a64, g.n_r, status,
-                                 h->dsc, h->tabs, st);
+                                 h->tabs, st);
         if (any_fixed)
             decode_fixed_burst<double>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, a64, g.n_r,
                                        status, h->abc_fields, st);
@@ -2547,7 +2546,7 @@ struct BatchDecode {
     std::vector<int> pk;                 // packet index per job (for messages)
     std::vector<long long> raw_off;      // element offset of each burst in the raw array
     long long raw_elems = 0;
-    size_t sym_bytes = 0, blk_bytes = 0;
+    int nq_max = 0;
     DecodeJob* d_jobs = nullptr;
     int njobs = 0;
     bool any_d = false, any_fixed = false;
@@ -2559,12 +2558,12 @@ struct BatchDecode {
 static std::shared_ptr<BatchDecode> batch_decode_plan(s1g_decoder* h, const std::vector<const std::vector<int>*>& bl) {
     auto bd = std::make_shared<BatchDecode>();
     std::vector<DecodeJob> jobs;
-    long long sym = 0, blk = 0, out = 0;
+    long long out = 0;
     for (const auto* pkp : bl) {
         const std::vector<int>& pk = *pkp;
         const int nq = h->hdr[pk.front()].num_quads();
         const int n_r = 2 * nq;
-        const int nb = (2 * nq + 255) / 256;
+        bd->nq_max = std::max(bd->nq_max, nq);
         bd->raw_off.push_back(out);
         for (int i : pk) {
             const FormatKind k = format_kind(h->hdr[i]);
@@ -2573,19 +2572,13 @@ static std::shared_ptr<BatchDecode> batch_decode_plan(s1g_decoder* h, const std:
             DecodeJob j;
             j.pk = i;
             j.nq = nq;
-            j.sym = sym;
-            j.blk = blk;
             j.out = out;
             jobs.push_back(j);
             bd->pk.push_back(i);
-            sym += 4LL * sym_pitch(nq);
-            blk += nb;
             out += n_r;
         }
     }
     bd->raw_elems = out;
-    bd->sym_bytes = (size_t)sym;
-    bd->blk_bytes = (size_t)blk;
     bd->njobs = (int)jobs.size();
     check_cuda(cudaMalloc(&bd->d_jobs, sizeof(DecodeJob) * std::max<size_t>(jobs.size(), 1)), "decode jobs");
     check_cuda(cudaMemcpy(bd->d_jobs, jobs.data(), sizeof(DecodeJob) * jobs.size(), cudaMemcpyHostToDevice),
@@ -2641,8 +2634,8 @@ static const cf32* swath_cached_decode(s1g_decoder* h, const std::vector<int>& p
         cf32* raw = sd->raw.as<cf32>((size_t)std::max<long long>(sd->plan->raw_elems, 1));
         int* st = h->bDecStatus.as<int>((size_t)std::max(sd->plan->njobs, 1));
         if (sd->plan->any_d)
-            decode_jobs<float>(h->d_stream, h->nbytes, h->d_off, sd->plan->d_jobs, sd->plan->njobs,
-                               sd->plan->sym_bytes, sd->plan->blk_bytes, raw, st, h->dsc, h->tabs, h->stream);
+            decode_jobs(h->d_stream, h->nbytes, h->d_off, sd->plan->d_jobs, sd->plan->njobs, sd->plan->nq_max, raw,
+                        nullptr, st, h->tabs, h->stream);
         if (sd->plan->any_fixed)
             decode_fixed_jobs<float>(h->d_stream, h->nbytes, h->d_off, sd->plan->d_jobs, sd->plan->njobs, raw, st,
                                      h->abc_fields, h->stream);
@@ -2709,21 +2702,17 @@ static void enqueue_batch(s1g_decoder** hs, int n_streams, const char* swath, in
         br.dec[s] = bd;
         raw_all[s] = h->bRawAll.as<cf32>((size_t)bd->raw_elems);
         br.dec_status[s] = h->bDecStatus.as<int>((size_t)bd->njobs);
+        // the ECCM notch takes FP64 samples: both come from the one bit walk
+        if (h->use_eccm) raw64_all[s] = h->bRawAll64.as<cf64>((size_t)bd->raw_elems);
         if (bd->any_d)
-            decode_jobs<float>(h->d_stream, h->nbytes, h->d_off, bd->d_jobs, bd->njobs, bd->sym_bytes, bd->blk_bytes,
-                               raw_all[s], br.dec_status[s], h->dsc, h->tabs, h->stream);
+            decode_jobs(h->d_stream, h->nbytes, h->d_off, bd->d_jobs, bd->njobs, bd->nq_max, raw_all[s], raw64_all[s],
+                        br.dec_status[s], h->tabs, h->stream);
         if (bd->any_fixed)
             decode_fixed_jobs<float>(h->d_stream, h->nbytes, h->d_off, bd->d_jobs, bd->njobs, raw_all[s],
                                      br.dec_status[s], h->abc_fields, h->stream);
-        if (h->use_eccm) {
-            // FP64 samples for the notch from the same symbols (no second bit walk)
-            raw64_all[s] = h->bRawAll64.as<cf64>((size_t)bd->raw_elems);
-            if (bd->any_d) decode_jobs_values<double>(bd->d_jobs, bd->njobs, raw64_all[s], br.dec_status[s], h->dsc,
-                                                      h->stream);
-            if (bd->any_fixed)
-                decode_fixed_jobs<double>(h->d_stream, h->nbytes, h->d_off, bd->d_jobs, bd->njobs, raw64_all[s],
-                                          br.dec_status[s], h->abc_fields, h->stream);
-        }
+        if (h->use_eccm && bd->any_fixed)
+            decode_fixed_jobs<double>(h->d_stream, h->nbytes, h->d_off, bd->d_jobs, bd->njobs, raw64_all[s],
+                                      br.dec_status[s], h->abc_fields, h->stream);
     }
     // burst products, enqueued round-robin over the streams so that they overlap
     size_t nslots = 0;

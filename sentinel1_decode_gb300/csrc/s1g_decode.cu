@@ -9,15 +9,16 @@
 // sequentially only where it does not), and exclusive-scans the per-chunk
 // packet counts.  A last pass writes every packet offset at its global index.
 //
-// Decoder: one thread per packet reproduces the bitstream walk of
+// Decoder: one warp per packet reproduces the bitstream walk of
 // _set_quad_type_d / _get_h_code_type_d / huffman_decode (packet.cpp:755-818,
-// decoding_utils.cpp:44-77) with a 16-entry value-keyed lookup per BRC held
-// in shared memory and a 64-bit bit buffer, storing one byte (sign<<7|mcode)
-// per sample; a second, coalesced kernel applies the reconstruction of
-// _get_s_values_type_d (packet.cpp:678-693) and the IE/IO/QE/QO interleave of
-// _get_signal_type_d (packet.cpp:696-752).  Errors become per-packet status
-// codes instead of exceptions.
+// decoding_utils.cpp:44-77): the lanes walk short pieces of a block's bits
+// from guessed starts until the pieces fit together (see k_decode_fdbaq), and
+// the reconstruction of _get_s_values_type_d (packet.cpp:678-693) and the
+// IE/IO/QE/QO interleave of _get_signal_type_d (packet.cpp:696-752) happen in
+// the same kernel.  Errors become per-packet status codes instead of
+// exceptions.
 #include <cstring>
+#include <stdexcept>
 
 #include "s1g_kernels.h"
 
@@ -66,14 +67,14 @@ __constant__ double c_sf[256] = {
 __constant__ int c_brc_thidx[5] = {3, 3, 5, 6, 8};
 __constant__ int c_brc_mcode[5] = {3, 4, 6, 9, 15};
 
-// Huffman lookup: for BRC b and an 11-bit window w (MSB = next bit: the
-// sign, then the 10 bits the code can take), the value-keyed walk of
-// huffman_decode is resolved into the symbol byte sign<<7 | mcode (low byte)
-// and the bits the sample takes, 1 + code length (high byte; 0 = "Max bit
-// length exceeded").  The table is built on the host by running that walk on
-// every window.
-typedef uint16_t HuffEntry;
-constexpr int kHuffWindow = 2048;
+// Huffman lookup: for BRC b and the 9 bits w after a sample's sign bit (MSB =
+// next bit; no code is longer), the value-keyed walk of huffman_decode is
+// resolved into len<<4 | mcode, len = the bits the sample takes with its sign
+// (2..10).  The table is built on the host by running that walk on every
+// window; every window starts with a code, so "Max bit length exceeded"
+// cannot happen.
+typedef uint8_t HuffEntry;
+constexpr int kHuffWindow = 512;
 
 // ------------------------------------------------------------------ indexer
 constexpr uint32_t kSync = 0x352EF853u;
@@ -292,92 +293,6 @@ void gather_headers(const uint8_t* d_stream, long long n, const long long* d_off
 }
 
 // ------------------------------------------------------------------ decoder
-// Bit reader over one packet's user data: a 64-bit MSB-first buffer refilled
-// with big-endian 32-bit words.  The data's aligned 32-bit words stream
-// through an 8-slot ring in shared memory (one column per thread) by
-// asynchronous copies (cp.async): a refill assembles the next word from the
-// ring (funnel shift by the data's constant misalignment, byte swap) and
-// starts the copy of the word six ahead, so a copy has five refills to land
-// and no register ever waits on a global load.  Only aligned words that end
-// inside the data are copied (the first may start up to 3 bytes before u,
-// inside the packet header), and the words within 8 bytes of the end are
-// assembled byte by byte, bytes beyond `avail` read as zero: nothing past the
-// data is read, so a caller's unpadded buffer is safe.
-constexpr int kDecodeThreads = 128;
-constexpr int kRing = 8;
-
-struct BitBuf {
-    const uint8_t* u;
-    int avail;
-    int pos;                // byte position of the next word to enter buf
-    uint64_t buf;           // unread bits, MSB first
-    int nb;                 // number of valid bits in buf
-    int sh;                 // misalignment of u, in bits
-    int k;                  // aligned word holding byte pos (from wbase)
-    const uint32_t* wbase;  // aligned word holding byte 0
-    const uint32_t* ring;   // this thread's column: slot s at ring[s * kDecodeThreads]
-};
-
-__device__ __forceinline__ uint32_t load_be32(const uint8_t* u, long long pos, long long avail) {
-    uint32_t v = 0;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) v = (v << 8) | (pos + i < avail ? (uint32_t)u[pos + i] : 0u);
-    return v;
-}
-
-// start the copy of aligned word kw into its ring slot (one commit group per
-// word, empty past the end, so the group count stays one per word)
-__device__ __forceinline__ void bb_copy(const BitBuf& b, int kw) {
-    const uint32_t* g = b.wbase + kw;
-    if (reinterpret_cast<const uint8_t*>(g + 1) <= b.u + b.avail) {
-        const unsigned sa = (unsigned)__cvta_generic_to_shared(b.ring + (kw & (kRing - 1)) * kDecodeThreads);
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(g) : "memory");
-    }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-}
-
-__device__ __forceinline__ BitBuf bb_open(const uint8_t* u, int avail, const uint32_t* ring) {
-    BitBuf b;
-    b.u = u;
-    b.avail = avail;
-    b.pos = 0;
-    b.buf = 0ull;
-    b.nb = 0;
-    b.sh = (int)((uintptr_t)u & 3) * 8;
-    b.k = 0;
-    b.wbase = reinterpret_cast<const uint32_t*>((uintptr_t)u & ~(uintptr_t)3);
-    b.ring = ring;
-#pragma unroll
-    for (int kw = 0; kw < 6; ++kw) bb_copy(b, kw);
-    return b;
-}
-
-// at least 32 unread bits in buf afterwards
-__device__ __forceinline__ void bb_refill(BitBuf& b) {
-    if (b.nb <= 32) {
-        // words k and k + 1 are in: at most the four younger copies pending
-        asm volatile("cp.async.wait_group 4;" ::: "memory");
-        uint32_t nx;
-        if (b.pos + 8 <= b.avail) {
-            const uint32_t lo = b.ring[(b.k & (kRing - 1)) * kDecodeThreads];
-            const uint32_t hi = b.ring[((b.k + 1) & (kRing - 1)) * kDecodeThreads];
-            nx = __byte_perm(__funnelshift_r(lo, hi, b.sh), 0, 0x0123);
-        } else {
-            nx = load_be32(b.u, b.pos, b.avail);
-        }
-        b.buf |= (uint64_t)nx << (32 - b.nb);
-        b.pos += 4;
-        b.nb += 32;
-        bb_copy(b, b.k + 6);   // into the slot of word k - 2, already consumed
-        ++b.k;
-    }
-}
-__device__ __forceinline__ uint32_t bb_top32(const BitBuf& b) { return (uint32_t)(b.buf >> 32); }
-__device__ __forceinline__ void bb_skip(BitBuf& b, int k) {
-    b.buf <<= k;
-    b.nb -= k;
-}
-
 // Where packet j of a decode goes.  Job-table mode (jobs != nullptr): any mix
 // of bursts and row lengths in one launch.  Uniform mode: packets p0 + j (or
 // pk_idx[j]) of one burst, nq quads each, rows j * pitch.
@@ -395,197 +310,300 @@ __device__ __forceinline__ DecodeJob job_at(const DecodeSpec& d, int j) {
     DecodeJob o;
     o.pk = d.pk_idx ? d.pk_idx[j] : d.p0 + j;
     o.nq = d.nq;
-    const int nb = (2 * d.nq + 255) / 256;
-    o.sym = (long long)j * 4 * sym_pitch(d.nq);
-    o.blk = (long long)j * nb;
     o.out = (long long)j * d.pitch;
     return o;
 }
 
-// Symbols: one byte per sample, sign<<7 | mcode; rows ch = IE, IO, QE, QO of
-// sym_pitch(nq) bytes each at job.sym.  The walk reproduces _set_quad_type_d /
-// _get_h_code_type_d / huffman_decode (packet.cpp:755-818,
-// decoding_utils.cpp:44-77): per channel, blocks of 128 codes (IE blocks led
-// by the 3-bit BRC, QE blocks by the 8-bit THIDX), then a 16-bit alignment.
-__global__ void __launch_bounds__(kDecodeThreads) k_decode_symbols(const uint8_t* __restrict__ s, long long n,
+// ---- FDBAQ walk and reconstruction, one warp per packet
+//
+// A packet's codes are a serial chain (a code starts where the previous one
+// ends), and a thread that follows it takes ~170 cycles a code: 2.0 ms for
+// the 24000 codes of a 12000-sample packet, with 1500 such threads on a chip
+// that runs 300000.  Here a warp takes a block of 128 codes at a time: lane l
+// walks the piece of `seg` bits that starts at bit l * seg, first as if a code
+// began there, and hands the bit where its last code ended to lane l + 1 as
+// that lane's true start; lanes whose start changed walk again until none
+// does.  Lane 0's start is right, so after k rounds the first k + 1 lanes are,
+// and the codes resynchronise within a few codes: 2 to 4 rounds.  A prefix sum
+// over the lanes' code counts then places every symbol.  The pieces are short
+// enough for 8 codes (the shortest are 2 bits for BRC 0-2, 3 for BRC 3-4) and
+// 32 of them hold about one block: seg = 12, 14, 16, 20, 24 bits for BRC 0..4.
+// Where a block takes more than 32 pieces the rest of it follows the same way.
+//
+// The reconstruction runs as soon as a channel pair is there: the even
+// samples are (IE, QE) and the odd ones (IO, QO), so only the symbols of IE
+// and IO wait in shared memory (2 bytes a quad) and no symbol goes through
+// global memory.  Values come from a 16-entry table per block (the products
+// of the reconstruction level and the sigma factor, formed in FP64).
+//
+// Bound by the latency of this chain (one block: ~4800 cycles), with 10 warps
+// per SM in a 1500-packet burst of 12000 samples: 0.43 ms, where a thread per
+// packet and a second kernel for the values took 2.0 + 0.22 ms (6.2 ms through
+// the allocation-free call, in three chunks of a fixed scratch array).
+constexpr int kDecodeWarps = 2;
+constexpr int kRingWords = 256;      // the packet's words around the walk (1 KB per warp)
+constexpr int kMaxBlocks = 512;      // nq <= 65535
+
+// shared memory of one warp, before its 2 * sym_pitch(nq) symbol bytes
+struct DecodeWarp {
+    double tab64[16];
+    float tab32[16];
+    uint32_t ring[kRingWords];
+    uint8_t stage[128];
+    uint8_t brc[kMaxBlocks];
+    uint8_t thidx[kMaxBlocks];
+};
+struct DecodeShared {
+    double norm[5][16];
+    HuffEntry lut[5 * kHuffWindow];
+};
+static_assert(sizeof(DecodeWarp) % 16 == 0 && sizeof(DecodeShared) % 16 == 0, "16-byte rows");
+
+__host__ __device__ inline size_t decode_warp_bytes(int nq) {
+    return sizeof(DecodeWarp) + (((size_t)2 * sym_pitch(nq) + 15) & ~(size_t)15);
+}
+static size_t decode_smem(int nq, int warps) { return sizeof(DecodeShared) + warps * decode_warp_bytes(nq); }
+
+// a << k with 0 for k outside 0..31 (shl clamps)
+__device__ __forceinline__ uint32_t shl_clamp(uint32_t a, int k) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(k));
+    return r;
+}
+
+// The packet's user data as big-endian bits.  Bit positions count from the
+// aligned 32-bit word that holds the first byte.  Words stream into the ring
+// by cp.async, 32 per step and at least three steps ahead of the walk; only
+// aligned words that end inside the data are copied (the first may begin up
+// to 3 bytes before it, inside the packet header), the others are assembled
+// byte by byte with zeros past `avail`: nothing past the data is read.
+struct PacketBits {
+    const uint8_t* u;
+    int avail;
+    int mis;                 // bytes from the aligned word to u
+    const uint32_t* wbase;
+    uint32_t* ring;
+    int filled;              // words asked for so far
+
+    // make words [.., upto) readable by every lane
+    __device__ __forceinline__ void fill(int upto, int lane) {
+        __syncwarp();        // the slots written next have been read
+        while (filled < upto + 96) {
+            const int kw = filled + lane;
+            uint32_t* slot = ring + (kw & (kRingWords - 1));
+            const int end = 4 * kw + 4 - mis;   // bytes of u up to the end of word kw
+            if (end <= avail) {
+                const unsigned sa = (unsigned)__cvta_generic_to_shared(slot);
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(sa), "l"(wbase + kw) : "memory");
+            } else {
+                uint32_t v = 0;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int at = end - 4 + i;
+                    if (at >= 0 && at < avail) v |= (uint32_t)u[at] << (8 * i);
+                }
+                *slot = v;
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            filled += 32;
+        }
+        asm volatile("cp.async.wait_group 3;" ::: "memory");
+        __syncwarp();
+    }
+    __device__ __forceinline__ uint32_t word(int k) const {
+        return __byte_perm(ring[k & (kRingWords - 1)], 0, 0x0123);
+    }
+    __device__ __forceinline__ uint32_t top32(int bit) const {
+        return __funnelshift_l(word((bit >> 5) + 1), word(bit >> 5), bit & 31);
+    }
+};
+
+// Rows of out32 / out64 (either may be null): out[2k] = IE_k + i QE_k,
+// out[2k+1] = IO_k + i QO_k; a packet that failed gets a zero row.
+__global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_t* __restrict__ s, long long n,
                                                         const long long* __restrict__ offsets, DecodeSpec spec,
-                                                        uint8_t* __restrict__ sym, uint8_t* __restrict__ brc_out,
-                                                        uint8_t* __restrict__ thidx_out, int* __restrict__ status,
+                                                        cf32* __restrict__ out32, cf64* __restrict__ out64,
+                                                        int* __restrict__ status, int nq_max,
                                                         const HuffEntry* __restrict__ lut_g) {
-    __shared__ HuffEntry lut[5 * kHuffWindow];
-    __shared__ uint32_t ring[kRing * kDecodeThreads];
-    for (int i = threadIdx.x; i < 5 * kHuffWindow; i += blockDim.x) lut[i] = lut_g[i];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem_raw);
+    for (int i = threadIdx.x; i < 5 * kHuffWindow / 4; i += blockDim.x)
+        reinterpret_cast<uint32_t*>(sh.lut)[i] = reinterpret_cast<const uint32_t*>(lut_g)[i];
+    for (int i = threadIdx.x; i < 80; i += blockDim.x) sh.norm[i >> 4][i & 15] = c_norm[i >> 4][i & 15];
     __syncthreads();
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int j = blockIdx.x * (blockDim.x >> 5) + warp;
     if (j >= spec.njobs) return;
+    DecodeWarp& w = *reinterpret_cast<DecodeWarp*>(smem_raw + sizeof(DecodeShared) + warp * decode_warp_bytes(nq_max));
+    uint8_t* sym = reinterpret_cast<uint8_t*>(&w + 1);
     const DecodeJob jb = job_at(spec, j);
     const int nq = jb.nq;
     const long long off = offsets[jb.pk];
+    int st = 0;
     // the 68 header bytes must lie inside the stream before any is read
     // (offsets can come from the caller, not only from the indexer)
-    if (off < 0 || off > n - 68) {
-        status[j] = S1G_E_PACKET_LENGTH;
-        return;
+    const bool inside = off >= 0 && off <= n - 68;
+    const uint8_t* hdr = s + (inside ? off : 0);
+    long long ulen = -1;
+    if (inside) {
+        ulen = (((long long)hdr[4] << 8) | hdr[5]) + 1 - 62;
+        const int pnq = (hdr[6 + 59] << 8) | hdr[6 + 60];
+        if (ulen < 0) st = S1G_E_PACKET_LENGTH;
+        else if (pnq != nq) st = S1G_E_RAGGED_BURST;
+    } else {
+        st = S1G_E_PACKET_LENGTH;
     }
-    const uint8_t* hdr = s + off;
-    const long long pdl = ((long long)hdr[4] << 8) | hdr[5];
-    const long long ulen = pdl + 1 - 62;
-    // bytes actually present (a truncated last packet reads as zeros)
-    long long avail = n - (off + 68);
-    if (avail > ulen) avail = ulen;
-    if (avail < 0) avail = 0;
-    const int pnq = (hdr[6 + 59] << 8) | hdr[6 + 60];
-    int st = 0;
-    if (ulen < 0) st = S1G_E_PACKET_LENGTH;
-    else if (pnq != nq) st = S1G_E_RAGGED_BURST;
-    const int nb = (2 * nq + 255) / 256;
-    const int sp = sym_pitch(nq);
-    uint8_t* my_sym = sym + jb.sym;
-    uint8_t* my_brc = brc_out + jb.blk;
-    uint8_t* my_th = thidx_out + jb.blk;
-    BitBuf bb = bb_open(s + off + 68, (int)avail, ring + threadIdx.x);
-    int bit = 0;                               // user data: below 65536 bytes
-    const int ubits = (int)ulen * 8;
-    for (int ch = 0; ch < 4 && !st; ++ch) {
-        uint32_t* row = reinterpret_cast<uint32_t*>(my_sym + (long long)ch * sp);
-        // the BRCs of channels IO, QE, QO come back from the IE walk's stores,
-        // each read one block ahead of its use
-        int brc_next = ch > 0 ? my_brc[0] : 0;
-        for (int b = 0; b < nb && !st; ++b) {
-            bb_refill(bb);
-            int brc;
-            if (ch == 0) {
-                if (bit + 3 > ubits) { st = S1G_E_READ_PAST_END; break; }
-                const uint32_t v = bb_top32(bb) >> 29;
-                if (v > 4) { st = S1G_E_BAD_BRC; break; }
-                my_brc[b] = (uint8_t)v;
-                brc = (int)v;
-                bb_skip(bb, 3);
-                bit += 3;
-            } else {
-                brc = brc_next;
-                brc_next = my_brc[min(b + 1, nb - 1)];
-                if (ch == 2) {
-                    if (bit + 8 > ubits) { st = S1G_E_READ_PAST_END; break; }
-                    my_th[b] = (uint8_t)(bb_top32(bb) >> 24);
-                    bb_skip(bb, 8);
-                    bit += 8;
-                }
-            }
-            const HuffEntry* L = lut + brc * kHuffWindow;
-            const int cnt = (b == nb - 1) ? nq - 128 * (nb - 1) : 128;
-            uint32_t pack = 0;
-            int i = 0;
-            if (bit + 11 * cnt <= ubits) {
-                // every code of the block ends inside the user data: no
-                // per-sample bounds checks, and an invalid code (0 bits) is
-                // reported after the block.  Four samples per step with two
-                // refills: after a refill at least 32 bits are buffered, two
-                // samples take at most 22.
-                uint32_t ok = 1;
-                for (; i + 4 <= cnt; i += 4) {
-                    bb_refill(bb);
-                    const uint32_t e0 = L[bb_top32(bb) >> 21];
-                    bb_skip(bb, (int)(e0 >> 8));
-                    const uint32_t e1 = L[bb_top32(bb) >> 21];
-                    bb_skip(bb, (int)(e1 >> 8));
-                    bb_refill(bb);
-                    const uint32_t e2 = L[bb_top32(bb) >> 21];
-                    bb_skip(bb, (int)(e2 >> 8));
-                    const uint32_t e3 = L[bb_top32(bb) >> 21];
-                    bb_skip(bb, (int)(e3 >> 8));
-                    ok &= (uint32_t)((e0 >> 8) != 0) & (uint32_t)((e1 >> 8) != 0) & (uint32_t)((e2 >> 8) != 0) &
-                          (uint32_t)((e3 >> 8) != 0);
-                    bit += (int)((e0 >> 8) + (e1 >> 8) + (e2 >> 8) + (e3 >> 8));
-                    row[(128 * b + i) >> 2] = __byte_perm(__byte_perm(e0, e1, 0x0040), __byte_perm(e2, e3, 0x0040), 0x5410);
-                }
-                for (; i < cnt; ++i) {
-                    bb_refill(bb);
-                    const uint32_t e = L[bb_top32(bb) >> 21];
-                    bb_skip(bb, (int)(e >> 8));
-                    ok &= (uint32_t)((e >> 8) != 0);
-                    bit += (int)(e >> 8);
-                    pack |= (e & 0xffu) << (8 * (i & 3));
-                }
-                if (!ok) st = S1G_E_HUFFMAN;
-            } else {
-                for (; i < cnt; ++i) {
-                    bb_refill(bb);
-                    const uint32_t e = L[bb_top32(bb) >> 21];
-                    const int k = (int)(e >> 8);
-                    if (k == 0) { st = S1G_E_HUFFMAN; break; }
-                    // the reference reads the code's bits one width at a time, all
-                    // inside the user data (decoding_utils.cpp:107-119)
-                    if (bit + k > ubits) { st = S1G_E_READ_PAST_END; break; }
-                    pack |= (e & 0xffu) << (8 * (i & 3));
-                    if ((i & 3) == 3) {
-                        row[(128 * b + i) >> 2] = pack;
-                        pack = 0;
+    if (!st) {
+        const int nb = (2 * nq + 255) / 256;
+        const int sp = sym_pitch(nq);
+        PacketBits pb;
+        pb.u = hdr + 68;
+        // bytes actually present (a truncated last packet reads as zeros)
+        pb.avail = (int)max(0LL, min(ulen, n - (off + 68)));
+        pb.mis = (int)((uintptr_t)pb.u & 3);
+        pb.wbase = reinterpret_cast<const uint32_t*>((uintptr_t)pb.u & ~(uintptr_t)3);
+        pb.ring = w.ring;
+        pb.filled = 0;
+        const int bit0 = 8 * pb.mis;
+        const int uend = bit0 + (int)ulen * 8;   // user data: below 65536 bytes
+        int bit = bit0;
+        for (int ch = 0; ch < 4 && !st; ++ch) {
+            for (int b = 0; b < nb && !st; ++b) {
+                // the largest head (8 bits), 32 pieces of 24 bits and the window of the last one
+                pb.fill(((bit + 8 + 768) >> 5) + 4, lane);
+                int brc;
+                if (ch == 0) {
+                    if (bit + 3 > uend) { st = S1G_E_READ_PAST_END; break; }
+                    brc = (int)(pb.top32(bit) >> 29);
+                    if (brc > 4) { st = S1G_E_BAD_BRC; break; }
+                    if (lane == 0) w.brc[b] = (uint8_t)brc;
+                    bit += 3;
+                } else {
+                    brc = w.brc[b];
+                    if (ch == 2) {
+                        if (bit + 8 > uend) { st = S1G_E_READ_PAST_END; break; }
+                        if (lane == 0) w.thidx[b] = (uint8_t)(pb.top32(bit) >> 24);
+                        bit += 8;
                     }
-                    bb_skip(bb, k);
-                    bit += k;
                 }
+                const HuffEntry* L = sh.lut + brc * kHuffWindow;
+                const int seg = brc == 0 ? 12 : brc == 1 ? 14 : brc == 2 ? 16 : brc == 3 ? 20 : 24;
+                const int cnt = (b == nb - 1) ? nq - 128 * (nb - 1) : 128;
+                uint8_t* dst = ch < 2 ? sym + ch * sp + 128 * b : w.stage;
+                int done = 0;
+                while (done < cnt) {
+                    if (done) pb.fill(((bit + 768) >> 5) + 4, lane);
+                    const int p = bit + lane * seg;
+                    const uint32_t w0 = pb.word(p >> 5), w1 = pb.word((p >> 5) + 1), w2 = pb.word((p >> 5) + 2);
+                    const uint32_t hi = __funnelshift_l(w1, w0, p & 31), lo = __funnelshift_l(w2, w1, p & 31);
+                    // symbols and code ends of this piece, a byte each
+                    uint32_t sa = 0, sb = 0, ea = 0, eb = 0;
+                    int c = 0;
+                    auto walk = [&](int o) {
+                        sa = sb = ea = eb = 0;
+                        c = 0;
+                        while (o < seg) {
+                            const uint32_t win = __funnelshift_l(lo, hi, o);
+                            const uint32_t e = L[(win >> 22) & 511];
+                            o += (int)(e >> 4);
+                            const uint32_t y = (e & 15) | ((win >> 24) & 128);
+                            const int k = 8 * c;
+                            sa |= shl_clamp(y, k);
+                            sb |= shl_clamp(y, k - 32);
+                            ea |= shl_clamp((uint32_t)o, k);
+                            eb |= shl_clamp((uint32_t)o, k - 32);
+                            ++c;
+                        }
+                        return o - seg;
+                    };
+                    int start = 0;
+                    int left = walk(0);
+                    for (int round = 0; round < 32; ++round) {
+                        int ns = __shfl_up_sync(0xffffffffu, left, 1);
+                        if (lane == 0) ns = 0;
+                        const bool moved = ns != start;
+                        if (!__any_sync(0xffffffffu, moved)) break;
+                        if (moved) {
+                            start = ns;
+                            left = walk(ns);
+                        }
+                    }
+                    int incl = c;
+#pragma unroll
+                    for (int d = 1; d < 32; d <<= 1) {
+                        const int t = __shfl_up_sync(0xffffffffu, incl, d);
+                        if (lane >= d) incl += t;
+                    }
+                    const int total = __shfl_sync(0xffffffffu, incl, 31);
+                    const int rem = cnt - done;
+                    const int excl = incl - c;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        if (i < c && excl + i < rem) dst[done + excl + i] = (uint8_t)((i < 4 ? sa : sb) >> (8 * (i & 3)));
+                    if (total <= rem) {
+                        bit += 32 * seg + __shfl_sync(0xffffffffu, left, 31);
+                        done += total;
+                    } else {
+                        // the piece that holds the block's last code
+                        const unsigned own = __ballot_sync(0xffffffffu, excl < rem && rem <= incl);
+                        const int k = max(0, rem - 1 - excl) & 7;
+                        const int end = lane * seg + (int)(((k < 4 ? ea : eb) >> (8 * (k & 3))) & 255u);
+                        bit += __shfl_sync(0xffffffffu, end, __ffs(own) - 1);
+                        done = cnt;
+                    }
+                }
+                // the reference reads the codes one width at a time, all inside
+                // the user data (decoding_utils.cpp:107-119)
+                if (bit > uend) { st = S1G_E_READ_PAST_END; break; }
+                if (ch >= 2) {
+                    __syncwarp();
+                    const int th = w.thidx[b];
+                    if (lane < 16) {
+                        // m <= the BRC's comparison flag for every code of its tree
+                        double v;
+                        if (th <= c_brc_thidx[brc]) v = lane == c_brc_mcode[brc] ? c_simple[brc][th] : (double)lane;
+                        else v = sh.norm[brc][lane] * c_sf[th];
+                        if (out64) w.tab64[lane] = v;
+                        w.tab32[lane] = (float)v;
+                    }
+                    __syncwarp();
+                    const uint8_t* re = sym + (ch - 2) * sp + 128 * b;
+                    const long long at = jb.out + 256LL * b + (ch - 2);
+                    for (int q = lane; q < cnt; q += 32) {
+                        const int x = re[q], y = w.stage[q];
+                        if (out32) {
+                            const float a = w.tab32[x & 15], c = w.tab32[y & 15];
+                            out32[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
+                        }
+                        if (out64) {
+                            const double a = w.tab64[x & 15], c = w.tab64[y & 15];
+                            out64[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
+                        }
+                    }
+                }
+                __syncwarp();
             }
-            if (!st && (i & 3)) row[(128 * b + i) >> 2] = pack;   // tail word (row padded to 4 bytes)
+            bit += -(bit - bit0) & 15;   // channels end on 16-bit words
         }
-        const int r = (int)(bit & 15);
-        if (r) {
-            bb_refill(bb);
-            bb_skip(bb, 16 - r);
-            bit += 16 - r;
-        }
+        asm volatile("cp.async.wait_all;" ::: "memory");   // no copy outlives the walk
     }
-    asm volatile("cp.async.wait_all;" ::: "memory");   // no copy outlives the walk
-    status[j] = st;
+    if (st)
+        for (int k = lane; k < 2 * nq; k += 32) {
+            if (out32) out32[jb.out + k] = mk(0.f, 0.f);
+            if (out64) out64[jb.out + k] = mk(0.0, 0.0);
+        }
+    if (lane == 0) status[j] = st;
 }
 
-// Reconstruction + interleave, one block per packet: out[2k] = IE_k + i QE_k,
-// out[2k+1] = IO_k + i QO_k (_get_s_values_type_d / _get_signal_type_d,
-// packet.cpp:678-752).  A packet that failed (here or in the symbol walk)
-// gets a zero row.
-template <typename R>
-__global__ void __launch_bounds__(256) k_decode_values(const uint8_t* __restrict__ sym, const uint8_t* __restrict__ brc_g,
-                                                       const uint8_t* __restrict__ th_g, DecodeSpec spec,
-                                                       cpx<R>* __restrict__ out, int* __restrict__ status) {
-    __shared__ int bad;
-    const int j = blockIdx.x;
-    const DecodeJob jb = job_at(spec, j);
-    const int nq = jb.nq;
-    const int sp = sym_pitch(nq);
-    cpx<R>* row = out + jb.out;
-    if (threadIdx.x == 0) bad = status[j];
-    __syncthreads();
-    if (bad == 0) {
-        const uint8_t* sj = sym + jb.sym;
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            const int b = q >> 7;
-            const int brc = brc_g[jb.blk + b];
-            const int th = th_g[jb.blk + b];
-            double v[4];
-            bool err = false;
-#pragma unroll
-            for (int ch = 0; ch < 4; ++ch) {
-                const uint8_t c = sj[(long long)ch * sp + q];
-                const int m = c & 127;
-                const double sg = (c >> 7) ? -1.0 : 1.0;
-                if (th <= c_brc_thidx[brc]) {
-                    const int flag = c_brc_mcode[brc];
-                    if (m < flag) v[ch] = sg * (double)m;
-                    else if (m == flag) v[ch] = sg * c_simple[brc][th];
-                    else { v[ch] = 0.0; err = true; }
-                } else {
-                    v[ch] = sg * c_norm[brc][m] * c_sf[th];
-                }
-            }
-            if (err) atomicExch(&bad, S1G_E_MCODE);
-            row[2 * q] = mk((R)v[0], (R)v[2]);
-            row[2 * q + 1] = mk((R)v[1], (R)v[3]);
-        }
-        __syncthreads();
-        if (bad != 0 && threadIdx.x == 0) status[j] = bad;
-    }
-    if (bad != 0)
-        for (int k = threadIdx.x; k < 2 * nq; k += blockDim.x) row[k] = mk((R)0, (R)0);
+static void launch_fdbaq(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeSpec& spec,
+                         cf32* out32, cf64* out64, int* d_status, int nq_max, const void* d_lut, cudaStream_t st) {
+    // one warp per CTA where two packets' symbols do not fit (nq above ~53000)
+    const int warps = decode_smem(nq_max, kDecodeWarps) <= (size_t)kSmemBytes ? kDecodeWarps : 1;
+    const size_t smem = decode_smem(nq_max, warps);
+    if (smem > 48 * 1024)
+        check_cuda(cudaFuncSetAttribute(k_decode_fdbaq, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "attr");
+    note_launch(), k_decode_fdbaq<<<(spec.njobs + warps - 1) / warps, 32 * warps, smem, st>>>(
+        d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, (const HuffEntry*)d_lut);
 }
 
 // ------------------------------------------------------------------ formats A, B, C
@@ -740,31 +758,25 @@ static void build_lut(std::vector<HuffEntry>& lut) {
     static const int start[5] = {1, 1, 1, 2, 2};
     lut.assign(5 * kHuffWindow, 0);
     for (int brc = 0; brc < 5; ++brc) {
-        for (int w = 0; w < 1024; ++w) {
-            auto bits = [&](int len) { return (w >> (10 - len)) & ((1 << len) - 1); };
+        for (int w = 0; w < kHuffWindow; ++w) {
+            auto bits = [&](int len) { return (w >> (9 - len)) & ((1 << len) - 1); };
             int len = start[brc];
-            int mcode = 0, clen = 0;   // clen 0: no code within 10 bits
+            int mcode = 0, clen = 0;
             if (brc == 4 && bits(2) == 0) {
                 clen = 2;
             } else {
                 if (brc == 4) len += 1;
-                for (int i = 0; i < 10; ++i) {
+                for (; len <= 9 && !clen; ++len) {
                     const int v = bits(len);
-                    int m = -1;
                     for (int k = 0; k < nkeys[brc]; ++k)
-                        if (keys[brc][k][0] == v) m = keys[brc][k][1];
-                    if (m >= 0) {
-                        mcode = m;
-                        clen = len;
-                        break;
-                    }
-                    len += 1;
-                    if (len > 10) break;
+                        if (keys[brc][k][0] == v) {
+                            mcode = keys[brc][k][1];
+                            clen = len;
+                        }
                 }
             }
-            for (int sign = 0; sign < 2; ++sign)
-                lut[brc * kHuffWindow + (sign << 10) + w] =
-                    clen ? (HuffEntry)(((1 + clen) << 8) | (sign << 7) | mcode) : (HuffEntry)0;
+            if (!clen) throw std::runtime_error("FDBAQ table: a bit window without a code");
+            lut[brc * kHuffWindow + w] = (HuffEntry)(((1 + clen) << 4) | mcode);
         }
     }
 }
@@ -777,17 +789,12 @@ void huffman_lut_fill(void* host_dst) {
     memcpy(host_dst, h.data(), sizeof(HuffEntry) * h.size());
 }
 
-// Decode npk packets (offsets d_offsets[p0 .. p0+npk)) into FP32 rows using
-// caller-supplied scratch (sym: npk*4*sym_pitch(nq) bytes, brc/thidx: npk*nb
-// bytes) and a device copy of the Huffman table.  Used by the allocation-free
-// entry point.
-void decode_fp32_with_scratch(const uint8_t* d_stream, long long n, const long long* d_offsets, int p0, int npk,
-                              int nq, cf32* out, long long pitch, int* d_status, uint8_t* sym, uint8_t* brc,
-                              uint8_t* thidx, const void* d_lut, cudaStream_t st) {
-    const DecodeSpec spec{nullptr, npk, nullptr, p0, nq, pitch};
-    note_launch(), k_decode_symbols<<<(npk + kDecodeThreads - 1) / kDecodeThreads, kDecodeThreads, 0, st>>>(d_stream, n, d_offsets, spec, sym, brc, thidx,
-                                                                     d_status, (const HuffEntry*)d_lut);
-    note_launch(), k_decode_values<float><<<npk, 256, 0, st>>>(sym, brc, thidx, spec, out, d_status);
+// Decode npk packets (offsets d_offsets[0 .. npk)) into FP32 rows with a device
+// copy of the Huffman table; allocates nothing and uses no global scratch.
+void decode_fp32_uniform(const uint8_t* d_stream, long long n, const long long* d_offsets, int npk, int nq, cf32* out,
+                         long long pitch, int* d_status, const void* d_lut, cudaStream_t st) {
+    const DecodeSpec spec{nullptr, npk, nullptr, 0, nq, pitch};
+    launch_fdbaq(d_stream, n, d_offsets, spec, out, nullptr, d_status, nq, d_lut, st);
 }
 
 DecodeTables::~DecodeTables() {
@@ -804,40 +811,19 @@ void DecodeTables::init() {
 
 template <typename R>
 void decode_burst(const uint8_t* d_stream, long long n, const long long* d_offsets, const int* d_pkidx, int p0,
-                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, DecodeScratch& sc, const DecodeTables& tabs,
+                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, const DecodeTables& tabs,
                   cudaStream_t st) {
-    const int nb = (2 * nq + 255) / 256;
-    sc.reserve((size_t)npk * 4 * sym_pitch(nq), (size_t)npk * nb);
     const DecodeSpec spec{nullptr, npk, d_pkidx, p0, nq, pitch};
-    note_launch(), k_decode_symbols<<<(npk + kDecodeThreads - 1) / kDecodeThreads, kDecodeThreads, 0, st>>>(d_stream, n, d_offsets, spec, sc.sym, sc.brc,
-                                                                     sc.thidx, d_status, (const HuffEntry*)tabs.lut);
-    note_launch(), k_decode_values<R><<<npk, 256, 0, st>>>(sc.sym, sc.brc, sc.thidx, spec, out, d_status);
+    if constexpr (sizeof(R) == 4) launch_fdbaq(d_stream, n, d_offsets, spec, out, nullptr, d_status, nq, tabs.lut, st);
+    else launch_fdbaq(d_stream, n, d_offsets, spec, nullptr, out, d_status, nq, tabs.lut, st);
 }
 
-template <typename R>
 void decode_jobs(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeJob* d_jobs, int njobs,
-                 size_t sym_bytes, size_t blk_bytes, cpx<R>* out, int* d_status, DecodeScratch& sc,
-                 const DecodeTables& tabs, cudaStream_t st) {
-    if (njobs <= 0) return;
-    sc.reserve(sym_bytes, blk_bytes);
-    const DecodeSpec spec{d_jobs, njobs, nullptr, 0, 0, 0};
-    note_launch(), k_decode_symbols<<<(njobs + kDecodeThreads - 1) / kDecodeThreads, kDecodeThreads, 0, st>>>(d_stream, n, d_offsets, spec, sc.sym, sc.brc,
-                                                                       sc.thidx, d_status, (const HuffEntry*)tabs.lut);
-    note_launch(), k_decode_values<R><<<njobs, 256, 0, st>>>(sc.sym, sc.brc, sc.thidx, spec, out, d_status);
-}
-
-// The reconstruction (k_decode_values) of jobs whose symbols a decode_jobs
-// call just left in sc: e.g. FP64 samples of packets decoded for FP32 output,
-// without a second bit walk.  d_status must hold that walk's status.
-template <typename R>
-void decode_jobs_values(const DecodeJob* d_jobs, int njobs, cpx<R>* out, int* d_status, const DecodeScratch& sc,
-                        cudaStream_t st) {
+                 int nq_max, cf32* out32, cf64* out64, int* d_status, const DecodeTables& tabs, cudaStream_t st) {
     if (njobs <= 0) return;
     const DecodeSpec spec{d_jobs, njobs, nullptr, 0, 0, 0};
-    note_launch(), k_decode_values<R><<<njobs, 256, 0, st>>>(sc.sym, sc.brc, sc.thidx, spec, out, d_status);
+    launch_fdbaq(d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, tabs.lut, st);
 }
-template void decode_jobs_values<double>(const DecodeJob*, int, cpx<double>*, int*, const DecodeScratch&,
-                                         cudaStream_t);
 
 template <typename R>
 void decode_fixed_burst(const uint8_t* d_stream, long long n, const long long* d_offsets, const int* d_pkidx, int p0,
@@ -864,32 +850,9 @@ template void decode_fixed_jobs<float>(const uint8_t*, long long, const long lon
 template void decode_fixed_jobs<double>(const uint8_t*, long long, const long long*, const DecodeJob*, int,
                                         cpx<double>*, int*, int, cudaStream_t);
 
-void DecodeScratch::reserve(size_t sym_bytes, size_t blk_bytes) {
-    if (sym_bytes > sym_cap) {
-        if (sym) cudaFree(sym);
-        check_cuda(cudaMalloc(&sym, sym_bytes), "decode scratch");
-        sym_cap = sym_bytes;
-    }
-    if (blk_bytes > blk_cap) {
-        if (brc) cudaFree(brc);
-        if (thidx) cudaFree(thidx);
-        check_cuda(cudaMalloc(&brc, blk_bytes), "decode scratch");
-        check_cuda(cudaMalloc(&thidx, blk_bytes), "decode scratch");
-        blk_cap = blk_bytes;
-    }
-}
-
-DecodeScratch::~DecodeScratch() {
-    if (sym) cudaFree(sym);
-    if (brc) cudaFree(brc);
-    if (thidx) cudaFree(thidx);
-}
-
 template void decode_burst<float>(const uint8_t*, long long, const long long*, const int*, int, int, int, cpx<float>*,
-                                  long long, int*, DecodeScratch&, const DecodeTables&, cudaStream_t);
+                                  long long, int*, const DecodeTables&, cudaStream_t);
 template void decode_burst<double>(const uint8_t*, long long, const long long*, const int*, int, int, int,
-                                   cpx<double>*, long long, int*, DecodeScratch&, const DecodeTables&, cudaStream_t);
-template void decode_jobs<float>(const uint8_t*, long long, const long long*, const DecodeJob*, int, size_t, size_t,
-                                 cpx<float>*, int*, DecodeScratch&, const DecodeTables&, cudaStream_t);
+                                   cpx<double>*, long long, int*, const DecodeTables&, cudaStream_t);
 
 }  // namespace s1g

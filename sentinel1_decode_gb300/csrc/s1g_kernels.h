@@ -41,16 +41,7 @@ struct DecodeTables {
     ~DecodeTables();
 };
 
-struct DecodeScratch {
-    uint8_t* sym = nullptr;
-    uint8_t* brc = nullptr;
-    uint8_t* thidx = nullptr;
-    size_t sym_cap = 0, blk_cap = 0;
-    void reserve(size_t sym_bytes, size_t blk_bytes);
-    ~DecodeScratch();
-};
-
-// Symbol-row pitch (bytes) of one decoded channel: nq rounded up to 4.
+// Symbol-row pitch (bytes) of one decoded channel in shared memory: nq rounded up to 4.
 __host__ __device__ inline int sym_pitch(int nq) { return (nq + 3) & ~3; }
 
 // Short-time windows of the ECCM notch on a line of n_r samples (fft 128,
@@ -58,21 +49,17 @@ __host__ __device__ inline int sym_pitch(int nq) { return (nq + 3) & ~3; }
 inline int eccm_num_windows(int n_r) { return (int)floor(((double)n_r / 128.0) * (128.0 / 64.0)); }
 
 // One packet of a batched decode (any mix of bursts and row lengths): packet
-// index, quads, byte offset of its 4 symbol rows in the symbol scratch, index
-// of its first block code in the BRC/THIDX scratch, element offset of its
-// output row.
+// index, quads, element offset of its output row.
 struct DecodeJob {
     int pk;
     int nq;
-    long long sym;
-    long long blk;
     long long out;
 };
 
-template <typename R>
+// FDBAQ packets of a job table into FP32 rows, FP64 rows or both (null: not
+// wanted) from one walk; nq_max: the largest nq of the jobs.
 void decode_jobs(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeJob* d_jobs, int njobs,
-                 size_t sym_bytes, size_t blk_bytes, cpx<R>* out, int* d_status, DecodeScratch& sc,
-                 const DecodeTables& tabs, cudaStream_t st);
+                 int nq_max, cf32* out32, cf64* out64, int* d_status, const DecodeTables& tabs, cudaStream_t st);
 
 // Scaled float image of n complex samples (CF32 or CF64 `elem`), mode
 // S1G_SCALE_*; d_max: one device word for the max |x| of the norm modes.
@@ -87,8 +74,7 @@ int write_bigtiff(const char* path, const float* img, long long rows, long long 
 
 template <typename R>
 void decode_burst(const uint8_t* d_stream, long long n, const long long* d_offsets, const int* d_pkidx, int p0,
-                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, DecodeScratch& sc, const DecodeTables& tabs,
-                  cudaStream_t st);
+                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, const DecodeTables& tabs, cudaStream_t st);
 
 // Data formats A/B (bypass) and C (BAQ): rows of packets whose baq_mode is
 // 0 or 3..5 (FDBAQ rows are skipped).  fields = 0: the reference's output;
@@ -99,12 +85,6 @@ void decode_fixed_burst(const uint8_t* d_stream, long long n, const long long* d
 template <typename R>
 void decode_fixed_jobs(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeJob* d_jobs,
                        int njobs, cpx<R>* out, int* d_status, int fields, cudaStream_t st);
-// The reconstruction of jobs whose symbols decode_jobs just left in sc (the
-// FP64 samples of an FP32-decoded batch, for the FP64 ECCM notch).
-template <typename R>
-void decode_jobs_values(const DecodeJob* d_jobs, int njobs, cpx<R>* out, int* d_status, const DecodeScratch& sc,
-                        cudaStream_t st);
-
 // Differentiable azimuth chain (s1g_adjoint.cu): row factors, bulk RCMC
 // phase exp(i sign beta_k f_r), azimuth filter exp(i sign c4pl R_r omd_k),
 // image entropy sums / gradient, per-row sum_c w_c Im(conj(a) b) (w = colw,

@@ -8,13 +8,12 @@
 // and cudaFree imply.  Such a caller allocates its inputs and outputs itself,
 // once, and then decodes packets with this call, which allocates nothing.
 //
-// The decoder's working memory (one byte per decoded sample plus the
-// per-block BRC / THIDX codes) lives in the file-scope array below, 16 MiB,
-// which every GPU that loads the library keeps until the process exits.
-// Longer inputs are decoded in chunks that fit it.  Host code may not use the
+// The decoder's working memory is shared memory; only the Huffman table lives
+// in device memory, in the file-scope array below, which every GPU that loads
+// the library keeps until the process exits.  Host code may not use the
 // array's name as a device address (it is only a host-side stand-in), so the
 // address is looked up with cudaGetSymbolAddress once per device, with that
-// device current, and passed to the kernels.
+// device current, and passed to the kernel.
 #include <cstring>
 #include <mutex>
 #include <string>
@@ -25,38 +24,28 @@ namespace s1g {
 
 size_t huffman_lut_bytes();
 void huffman_lut_fill(void* host_dst);
-void decode_fp32_with_scratch(const uint8_t* d_stream, long long n, const long long* d_offsets, int p0, int npk,
-                              int nq, cf32* out, long long pitch, int* d_status, uint8_t* sym, uint8_t* brc,
-                              uint8_t* thidx, const void* d_lut, cudaStream_t st);
+void decode_fp32_uniform(const uint8_t* d_stream, long long n, const long long* d_offsets, int npk, int nq, cf32* out,
+                         long long pitch, int* d_status, const void* d_lut, cudaStream_t st);
 
-constexpr size_t kNoAllocScratchBytes = 16u << 20;   // 16 MiB
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) uint8_t g_noalloc_scratch[kNoAllocScratchBytes];
-static __device__ __align__(256) uint8_t g_noalloc_lut[5 * 2048 * 2];   // 11-bit windows x 5 BRCs, 2 bytes each
+static __device__ __align__(256) uint8_t g_noalloc_lut[5 * 512];   // 9-bit windows x 5 BRCs, one byte each
 
 struct NoAllocDevice {
     bool ready = false;
-    uint8_t* scratch = nullptr;
     uint8_t* lut = nullptr;
 };
 static NoAllocDevice g_dev[kMaxDevices];
 static std::mutex g_setup_mutex;
 
-// Once per device, with that device current: resolve the arrays' device
-// addresses and copy the Huffman table in (a synchronous copy, no allocation).
+// Once per device, with that device current: resolve the array's device
+// address and copy the Huffman table in (a synchronous copy, no allocation).
 static int setup_device(int dev, std::string& err) {
     std::lock_guard<std::mutex> lk(g_setup_mutex);
     NoAllocDevice& d = g_dev[dev];
     if (d.ready) return S1G_OK;
     void* p = nullptr;
-    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-    if (e != cudaSuccess) {
-        err = std::string("cudaGetSymbolAddress(scratch): ") + cudaGetErrorString(e);
-        return S1G_E_CUDA;
-    }
-    d.scratch = (uint8_t*)p;
-    e = cudaGetSymbolAddress(&p, g_noalloc_lut);
+    cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_lut);
     if (e != cudaSuccess) {
         err = std::string("cudaGetSymbolAddress(lut): ") + cudaGetErrorString(e);
         return S1G_E_CUDA;
@@ -88,27 +77,23 @@ int s1g_decode_fdbaq_noalloc(const uint8_t* d_stream, int64_t nbytes, const int6
     if (!d_stream || !d_offsets || !d_out || !d_status || npackets < 0 || nbytes < 0) return S1G_E_INVALID_ARGUMENT;
     // num_quadratures is a 16-bit packet field
     if (num_quads <= 0 || num_quads > 65535 || out_pitch < 2LL * num_quads) return S1G_E_INVALID_ARGUMENT;
-    const long long nb = (2LL * num_quads + 255) / 256;
-    const long long per_packet = 4LL * ((num_quads + 3LL) & ~3LL) + 2 * nb;   // symbol rows + BRC + THIDX
-    if (per_packet > (long long)kNoAllocScratchBytes) return S1G_E_SCRATCH_LIMIT;
     if (npackets == 0) return S1G_OK;
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return S1G_E_CUDA;
-    std::string err;
-    int rc = setup_device(dev, err);
-    if (rc != S1G_OK) return rc;
-    const NoAllocDevice& d = g_dev[dev];
     cudaStream_t st = (cudaStream_t)stream;
-    // chunks of packets that fit the scratch array; stream order keeps the
-    // chunks (and successive calls on one stream) from overlapping
-    const long long chunk = std::min<long long>(npackets, (long long)kNoAllocScratchBytes / per_packet);
-    for (long long p0 = 0; p0 < npackets; p0 += chunk) {
-        const int n = (int)std::min(chunk, npackets - p0);
-        uint8_t* sym = d.scratch;
-        uint8_t* brc = sym + (size_t)n * 4 * sym_pitch(num_quads);
-        uint8_t* th = brc + (size_t)n * nb;
-        decode_fp32_with_scratch(d_stream, nbytes, (const long long*)d_offsets, (int)p0, n, num_quads,
-                                 (cf32*)d_out + p0 * out_pitch, out_pitch, d_status + p0, sym, brc, th, d.lut, st);
+    try {
+        std::string err;
+        const int rc = setup_device(dev, err);
+        if (rc != S1G_OK) return rc;
+        const NoAllocDevice& d = g_dev[dev];
+        const int most = 1 << 30;   // packets of one launch
+        for (long long p0 = 0; p0 < npackets; p0 += most) {
+            const int n = (int)std::min<long long>(most, npackets - p0);
+            decode_fp32_uniform(d_stream, nbytes, (const long long*)d_offsets + p0, n, num_quads,
+                                (cf32*)d_out + p0 * out_pitch, out_pitch, d_status + p0, d.lut, st);
+        }
+    } catch (const std::exception&) {
+        return S1G_E_CUDA;
     }
     return cudaGetLastError() == cudaSuccess ? S1G_OK : S1G_E_CUDA;
 }
