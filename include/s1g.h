@@ -472,7 +472,7 @@ int s1g_launch_count(int64_t* n);
  * num_quads is at most 65535 (the width of the num_quadratures field;
  * S1G_E_INVALID_ARGUMENT beyond), whose symbols fit; S1G_E_SCRATCH_LIMIT is
  * kept for builds with a smaller scratch and not returned.  The first call on
- * each device, with that device current, copies the 2.5 KB Huffman table into
+ * each device, with that device current, copies the 10 KB Huffman table into
  * a device array of the library with a synchronous cudaMemcpyToSymbol; make
  * that first call before any stream capture.  Calls share nothing else: they
  * may overlap on different streams.

@@ -67,14 +67,14 @@ __constant__ double c_sf[256] = {
 __constant__ int c_brc_thidx[5] = {3, 3, 5, 6, 8};
 __constant__ int c_brc_mcode[5] = {3, 4, 6, 9, 15};
 
-// Huffman lookup: for BRC b and the 9 bits w after a sample's sign bit (MSB =
-// next bit; no code is longer), the value-keyed walk of huffman_decode is
-// resolved into len<<4 | mcode, len = the bits the sample takes with its sign
-// (2..10).  The table is built on the host by running that walk on every
-// window; every window starts with a code, so "Max bit length exceeded"
-// cannot happen.
-typedef uint8_t HuffEntry;
-constexpr int kHuffWindow = 512;
+// Huffman lookup: for BRC b and the next 10 bits w (MSB = next bit: the
+// sample's sign, then its code; no code is longer than 9 bits), the value-keyed
+// walk of huffman_decode is resolved into the symbol byte sign<<7 | mcode (low
+// byte) and the bits the sample takes with its sign, 2..10 (high byte).  The
+// table is built on the host by running that walk on every window; every
+// window starts with a code, so "Max bit length exceeded" cannot happen.
+typedef uint16_t HuffEntry;
+constexpr int kHuffWindow = 1024;
 
 // ------------------------------------------------------------------ indexer
 constexpr uint32_t kSync = 0x352EF853u;
@@ -320,15 +320,18 @@ __device__ __forceinline__ DecodeJob job_at(const DecodeSpec& d, int j) {
 // ends), and a thread that follows it takes ~170 cycles a code: 2.0 ms for
 // the 24000 codes of a 12000-sample packet, with 1500 such threads on a chip
 // that runs 300000.  Here a warp takes a block of 128 codes at a time: lane l
-// walks the piece of `seg` bits that starts at bit l * seg, first as if a code
-// began there, and hands the bit where its last code ended to lane l + 1 as
-// that lane's true start; lanes whose start changed walk again until none
-// does.  Lane 0's start is right, so after k rounds the first k + 1 lanes are,
-// and the codes resynchronise within a few codes: 2 to 4 rounds.  A prefix sum
-// over the lanes' code counts then places every symbol.  The pieces are short
-// enough for 8 codes (the shortest are 2 bits for BRC 0-2, 3 for BRC 3-4) and
-// 32 of them hold about one block: seg = 12, 14, 16, 20, 24 bits for BRC 0..4.
-// Where a block takes more than 32 pieces the rest of it follows the same way.
+// walks the piece of `seg` bits that starts at bit l * seg.  Codes
+// resynchronise within a few codes from a wrong start, so a lane first walks
+// the `pre` bits before its piece, from the block's start where that lies
+// inside them and else from an arbitrary bit, and takes the bit where it
+// arrives as its start.  Then every lane hands the bit where its last code
+// ended to the next, and lanes whose start was another walk again until none
+// is: lane 0 is right, so each round fixes at least one more lane, and 0.1
+// (BRC 0-2) to 2 (BRC 4) rounds are enough on average.  A prefix sum over the
+// lanes' code counts then places every symbol.  The pieces hold at most 7
+// codes (the shortest take 2 bits for BRC 0-2, 3 for BRC 3-4) and 32 of them
+// about one block: seg = 12, 12, 14, 16, 18 bits for BRC 0..4.  Where a block
+// takes more than 32 pieces the rest of it follows the same way.
 //
 // The reconstruction runs as soon as a channel pair is there: the even
 // samples are (IE, QE) and the odd ones (IO, QO), so only the symbols of IE
@@ -336,11 +339,15 @@ __device__ __forceinline__ DecodeJob job_at(const DecodeSpec& d, int j) {
 // global memory.  Values come from a 16-entry table per block (the products
 // of the reconstruction level and the sigma factor, formed in FP64).
 //
-// Bound by the latency of this chain (one block: ~4800 cycles), with 10 warps
-// per SM in a 1500-packet burst of 12000 samples: 0.43 ms, where a thread per
-// packet and a second kernel for the values took 2.0 + 0.22 ms (6.2 ms through
-// the allocation-free call, in three chunks of a fixed scratch array).
-constexpr int kDecodeWarps = 2;
+// Bound by the latency of this chain: ~520 instructions and ~3300 cycles a
+// block with 2.4 warps per scheduler in a 1500-packet burst.  1500 packets of
+// 12000 samples: 0.30 ms, where a thread per packet and a second kernel for
+// the values took 2.0 + 0.22 ms (6.2 ms through the allocation-free call, in
+// three chunks of a fixed scratch array).  The walk with branches in place of
+// selects took 0.39 ms, without the run-up 0.43, and a table of jumps over 16
+// codes from every bit (no guesses, but 250 shared-memory accesses a block)
+// 0.99.
+constexpr int kDecodeWarps = 4;
 constexpr int kRingWords = 256;      // the packet's words around the walk (1 KB per warp)
 constexpr int kMaxBlocks = 512;      // nq <= 65535
 
@@ -363,13 +370,6 @@ __host__ __device__ inline size_t decode_warp_bytes(int nq) {
     return sizeof(DecodeWarp) + (((size_t)2 * sym_pitch(nq) + 15) & ~(size_t)15);
 }
 static size_t decode_smem(int nq, int warps) { return sizeof(DecodeShared) + warps * decode_warp_bytes(nq); }
-
-// a << k with 0 for k outside 0..31 (shl clamps)
-__device__ __forceinline__ uint32_t shl_clamp(uint32_t a, int k) {
-    uint32_t r;
-    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(k));
-    return r;
-}
 
 // The packet's user data as big-endian bits.  Bit positions count from the
 // aligned 32-bit word that holds the first byte.  Words stream into the ring
@@ -418,8 +418,9 @@ struct PacketBits {
     }
 };
 
-// Rows of out32 / out64 (either may be null): out[2k] = IE_k + i QE_k,
+// Rows of out32 (F32) and out64 (F64): out[2k] = IE_k + i QE_k,
 // out[2k+1] = IO_k + i QO_k; a packet that failed gets a zero row.
+template <bool F32, bool F64>
 __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_t* __restrict__ s, long long n,
                                                         const long long* __restrict__ offsets, DecodeSpec spec,
                                                         cf32* __restrict__ out32, cf64* __restrict__ out64,
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
                                                         const HuffEntry* __restrict__ lut_g) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem_raw);
-    for (int i = threadIdx.x; i < 5 * kHuffWindow / 4; i += blockDim.x)
+    for (int i = threadIdx.x; i < 5 * kHuffWindow / 2; i += blockDim.x)
         reinterpret_cast<uint32_t*>(sh.lut)[i] = reinterpret_cast<const uint32_t*>(lut_g)[i];
     for (int i = threadIdx.x; i < 80; i += blockDim.x) sh.norm[i >> 4][i & 15] = c_norm[i >> 4][i & 15];
     __syncthreads();
@@ -469,8 +470,8 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
         int bit = bit0;
         for (int ch = 0; ch < 4 && !st; ++ch) {
             for (int b = 0; b < nb && !st; ++b) {
-                // the largest head (8 bits), 32 pieces of 24 bits and the window of the last one
-                pb.fill(((bit + 8 + 768) >> 5) + 4, lane);
+                // the largest head (8 bits), 32 pieces of 18 bits and the window of the last one
+                pb.fill(((bit + 8 + 32 * 18) >> 5) + 4, lane);
                 int brc;
                 if (ch == 0) {
                     if (bit + 3 > uend) { st = S1G_E_READ_PAST_END; break; }
@@ -487,70 +488,79 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
                     }
                 }
                 const HuffEntry* L = sh.lut + brc * kHuffWindow;
-                const int seg = brc == 0 ? 12 : brc == 1 ? 14 : brc == 2 ? 16 : brc == 3 ? 20 : 24;
+                const int seg = brc <= 1 ? 12 : brc == 2 ? 14 : brc == 3 ? 16 : 18;
+                const int pre = brc <= 2 ? seg : 24;
                 const int cnt = (b == nb - 1) ? nq - 128 * (nb - 1) : 128;
                 uint8_t* dst = ch < 2 ? sym + ch * sp + 128 * b : w.stage;
                 int done = 0;
                 while (done < cnt) {
-                    if (done) pb.fill(((bit + 768) >> 5) + 4, lane);
+                    if (done) pb.fill(((bit + 32 * 18) >> 5) + 4, lane);
                     const int p = bit + lane * seg;
                     const uint32_t w0 = pb.word(p >> 5), w1 = pb.word((p >> 5) + 1), w2 = pb.word((p >> 5) + 2);
                     const uint32_t hi = __funnelshift_l(w1, w0, p & 31), lo = __funnelshift_l(w2, w1, p & 31);
-                    // symbols and code ends of this piece, a byte each
+                    int start = 0;
+                    {
+                        // the bits before the piece; a lane whose run-up begins at
+                        // or before the block's first bit starts there
+                        const int r = p - pre;
+                        const uint32_t v0 = pb.word(r >> 5);
+                        const uint32_t v1 = (r >> 5) + 1 == (p >> 5) ? w0 : w1;
+                        const uint32_t v2 = (r >> 5) + 1 == (p >> 5) ? w1 : w2;
+                        const uint32_t ph = __funnelshift_l(v1, v0, r & 31), pl = __funnelshift_l(v2, v1, r & 31);
+                        int o = max(0, pre - lane * seg);
+#pragma unroll
+                        for (int i = 0; i < 8; ++i) {
+                            const int step = L[__funnelshift_l(pl, ph, o) >> 22] >> 8;
+                            o += o < pre ? step : 0;
+                        }
+                        start = lane == 0 ? 0 : o - pre;
+                    }
+                    // symbols and code ends of the piece, a byte each; what follows
+                    // its c codes is not used
                     uint32_t sa = 0, sb = 0, ea = 0, eb = 0;
-                    int c = 0;
+                    int c;
                     auto walk = [&](int o) {
-                        sa = sb = ea = eb = 0;
                         c = 0;
-                        while (o < seg) {
-                            const uint32_t win = __funnelshift_l(lo, hi, o);
-                            const uint32_t e = L[(win >> 22) & 511];
-                            o += (int)(e >> 4);
-                            const uint32_t y = (e & 15) | ((win >> 24) & 128);
-                            const int k = 8 * c;
-                            sa |= shl_clamp(y, k);
-                            sb |= shl_clamp(y, k - 32);
-                            ea |= shl_clamp((uint32_t)o, k);
-                            eb |= shl_clamp((uint32_t)o, k - 32);
-                            ++c;
+#pragma unroll
+                        for (int i = 0; i < 7; ++i) {
+                            const uint32_t e = L[__funnelshift_l(lo, hi, o) >> 22];
+                            const bool on = o < seg;
+                            o += on ? (int)(e >> 8) : 0;
+                            c += on ? 1 : 0;
+                            // byte i & 3 of the pair of words
+                            const int at = 4 * (i & 3);
+                            const int sel = (0x3210 & ~(15 << at)) | (4 << at);
+                            uint32_t& sy = i < 4 ? sa : sb;
+                            uint32_t& en = i < 4 ? ea : eb;
+                            sy = __byte_perm(sy, e, sel);
+                            en = __byte_perm(en, (uint32_t)o, sel);
                         }
                         return o - seg;
                     };
-                    int start = 0;
-                    int left = walk(0);
+                    int left = walk(start);
                     for (int round = 0; round < 32; ++round) {
                         int ns = __shfl_up_sync(0xffffffffu, left, 1);
                         if (lane == 0) ns = 0;
-                        const bool moved = ns != start;
-                        if (!__any_sync(0xffffffffu, moved)) break;
-                        if (moved) {
-                            start = ns;
-                            left = walk(ns);
-                        }
+                        if (__all_sync(0xffffffffu, ns == start)) break;
+                        start = ns;
+                        left = walk(ns);
                     }
-                    int incl = c;
-#pragma unroll
-                    for (int d = 1; d < 32; d <<= 1) {
-                        const int t = __shfl_up_sync(0xffffffffu, incl, d);
-                        if (lane >= d) incl += t;
-                    }
-                    const int total = __shfl_sync(0xffffffffu, incl, 31);
+                    // codes before the piece and in all of them (1 to 7 each: three bits)
+                    const unsigned c0 = __ballot_sync(0xffffffffu, c & 1), c1 = __ballot_sync(0xffffffffu, c & 2),
+                                   c2 = __ballot_sync(0xffffffffu, c & 4), lt = (1u << lane) - 1;
+                    const int excl = __popc(c0 & lt) + 2 * __popc(c1 & lt) + 4 * __popc(c2 & lt);
+                    const int total = __popc(c0) + 2 * __popc(c1) + 4 * __popc(c2);
                     const int rem = cnt - done;
-                    const int excl = incl - c;
+                    const int lim = min(c, rem - excl);   // codes of this piece that belong to the block
+                    uint8_t* to = dst + done + excl;
 #pragma unroll
-                    for (int i = 0; i < 8; ++i)
-                        if (i < c && excl + i < rem) dst[done + excl + i] = (uint8_t)((i < 4 ? sa : sb) >> (8 * (i & 3)));
-                    if (total <= rem) {
-                        bit += 32 * seg + __shfl_sync(0xffffffffu, left, 31);
-                        done += total;
-                    } else {
-                        // the piece that holds the block's last code
-                        const unsigned own = __ballot_sync(0xffffffffu, excl < rem && rem <= incl);
-                        const int k = max(0, rem - 1 - excl) & 7;
-                        const int end = lane * seg + (int)(((k < 4 ? ea : eb) >> (8 * (k & 3))) & 255u);
-                        bit += __shfl_sync(0xffffffffu, end, __ffs(own) - 1);
-                        done = cnt;
-                    }
+                    for (int i = 0; i < 7; ++i)
+                        if (i < lim) to[i] = (uint8_t)((i < 4 ? sa : sb) >> (8 * (i & 3)));
+                    // the bit behind the last of them
+                    const int k = max(lim - 1, 0);
+                    const int end = lane * seg + (int)(((k < 4 ? ea : eb) >> (8 * (k & 3))) & 255u);
+                    bit += __reduce_max_sync(0xffffffffu, lim > 0 ? end : 0);
+                    done += min(total, rem);
                 }
                 // the reference reads the codes one width at a time, all inside
                 // the user data (decoding_utils.cpp:107-119)
@@ -563,21 +573,25 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
                         double v;
                         if (th <= c_brc_thidx[brc]) v = lane == c_brc_mcode[brc] ? c_simple[brc][th] : (double)lane;
                         else v = sh.norm[brc][lane] * c_sf[th];
-                        if (out64) w.tab64[lane] = v;
-                        w.tab32[lane] = (float)v;
+                        if (F64) w.tab64[lane] = v;
+                        if (F32) w.tab32[lane] = (float)v;
                     }
                     __syncwarp();
                     const uint8_t* re = sym + (ch - 2) * sp + 128 * b;
                     const long long at = jb.out + 256LL * b + (ch - 2);
-                    for (int q = lane; q < cnt; q += 32) {
-                        const int x = re[q], y = w.stage[q];
-                        if (out32) {
-                            const float a = w.tab32[x & 15], c = w.tab32[y & 15];
-                            out32[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
-                        }
-                        if (out64) {
-                            const double a = w.tab64[x & 15], c = w.tab64[y & 15];
-                            out64[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int q = lane + 32 * i;
+                        if (q < cnt) {
+                            const int x = re[q], y = w.stage[q];
+                            if (F32) {
+                                const float a = w.tab32[x & 15], c = w.tab32[y & 15];
+                                out32[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
+                            }
+                            if (F64) {
+                                const double a = w.tab64[x & 15], c = w.tab64[y & 15];
+                                out64[at + 2 * q] = mk(x & 128 ? -a : a, y & 128 ? -c : c);
+                            }
                         }
                     }
                 }
@@ -589,21 +603,26 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
     }
     if (st)
         for (int k = lane; k < 2 * nq; k += 32) {
-            if (out32) out32[jb.out + k] = mk(0.f, 0.f);
-            if (out64) out64[jb.out + k] = mk(0.0, 0.0);
+            if (F32) out32[jb.out + k] = mk(0.f, 0.f);
+            if (F64) out64[jb.out + k] = mk(0.0, 0.0);
         }
     if (lane == 0) status[j] = st;
 }
 
 static void launch_fdbaq(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeSpec& spec,
                          cf32* out32, cf64* out64, int* d_status, int nq_max, const void* d_lut, cudaStream_t st) {
-    // one warp per CTA where two packets' symbols do not fit (nq above ~53000)
+    // one warp per CTA where two packets' symbols do not fit (nq above ~25000)
     const int warps = decode_smem(nq_max, kDecodeWarps) <= (size_t)kSmemBytes ? kDecodeWarps : 1;
     const size_t smem = decode_smem(nq_max, warps);
-    if (smem > 48 * 1024)
-        check_cuda(cudaFuncSetAttribute(k_decode_fdbaq, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "attr");
-    note_launch(), k_decode_fdbaq<<<(spec.njobs + warps - 1) / warps, 32 * warps, smem, st>>>(
-        d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, (const HuffEntry*)d_lut);
+    auto go = [&](auto kernel) {
+        if (smem > 48 * 1024)
+            check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "attr");
+        note_launch(), kernel<<<(spec.njobs + warps - 1) / warps, 32 * warps, smem, st>>>(
+            d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, (const HuffEntry*)d_lut);
+    };
+    if (out32 && out64) go(k_decode_fdbaq<true, true>);
+    else if (out64) go(k_decode_fdbaq<false, true>);
+    else go(k_decode_fdbaq<true, false>);
 }
 
 // ------------------------------------------------------------------ formats A, B, C
@@ -758,7 +777,7 @@ static void build_lut(std::vector<HuffEntry>& lut) {
     static const int start[5] = {1, 1, 1, 2, 2};
     lut.assign(5 * kHuffWindow, 0);
     for (int brc = 0; brc < 5; ++brc) {
-        for (int w = 0; w < kHuffWindow; ++w) {
+        for (int w = 0; w < kHuffWindow / 2; ++w) {
             auto bits = [&](int len) { return (w >> (9 - len)) & ((1 << len) - 1); };
             int len = start[brc];
             int mcode = 0, clen = 0;
@@ -776,7 +795,8 @@ static void build_lut(std::vector<HuffEntry>& lut) {
                 }
             }
             if (!clen) throw std::runtime_error("FDBAQ table: a bit window without a code");
-            lut[brc * kHuffWindow + w] = (HuffEntry)(((1 + clen) << 4) | mcode);
+            for (int sign = 0; sign < 2; ++sign)
+                lut[brc * kHuffWindow + (sign << 9) + w] = (HuffEntry)(((1 + clen) << 8) | (sign << 7) | mcode);
         }
     }
 }

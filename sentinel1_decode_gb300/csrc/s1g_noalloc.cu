@@ -29,7 +29,7 @@ void decode_fp32_uniform(const uint8_t* d_stream, long long n, const long long* 
 
 constexpr int kMaxDevices = 64;
 
-static __device__ __align__(256) uint8_t g_noalloc_lut[5 * 512];   // 9-bit windows x 5 BRCs, one byte each
+static __device__ __align__(256) uint8_t g_noalloc_lut[5 * 1024 * 2];   // 10-bit windows x 5 BRCs, 2 bytes each
 
 struct NoAllocDevice {
     bool ready = false;
