@@ -96,6 +96,7 @@ struct s1g_decoder {
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
     Buf bFdf, bKN, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
+    Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
     Buf bTuD, bTuG, bTuI, bTuW, bTuR, bKa0;   // time-unfolding per-burst tables
     Buf bImgIn, bImgOut, bImgMax;        // image epilogue
     Buf bJ0, bJ1, bJ2, bJ3, bJ4, bJ5, bJe, bJd;   // differentiable azimuth chains
@@ -1087,7 +1088,7 @@ struct CztTables {
 struct FastBurst {          // per-burst tables of the fast path
     s1g::BurstGeom g;
     int M = 0;
-    s1g::Fft3Desc dM;
+    s1g::Fft4Desc dM;
     s1g::cf32* ref = nullptr;
     // TOPS azimuth
     double rate = 0, nrep = 0, time_delta = 0;
@@ -1099,7 +1100,7 @@ struct FastBurst {          // per-burst tables of the fast path
     s1g::CfftDesc dcDesc;
     float4 *dcH = nullptr, *dcG = nullptr;
     int na_smooth = 0, nr_smooth = 0;
-    s1g::Fft3Desc dna, dnr;
+    s1g::Fft4Desc dna, dnr;
     s1g::CztDev cna, cnr, cf, ci, cS;
     s1g::RowDf* rows_df = nullptr;
     s1g::RowParam* rows64 = nullptr;
@@ -1142,15 +1143,22 @@ static inline cpx<double> chirp_at(long long n, long long P, int sign) {
 // within the shared-memory budget.
 static int fused_cap() { return smem_capacity<float>() * 31 / 32 - 512; }
 
+// Plan of a transform of at least minlen points, minlen within fused_cap().
+static std::shared_ptr<Fft4Plan> fused_plan(s1g_decoder* h, long long minlen, const char* what) {
+    const long long m = minlen <= fused_cap() ? h->fft->tuned_len(minlen) : -1;
+    if (m < 0) throw S1Error(S1G_E_GEOMETRY, std::string(what) + " " + std::to_string(minlen) + " too long");
+    return h->fft->plan4((int)m);
+}
+
 // Chirp-z tables for X[k] = sum_{s<nin} x[s] exp(-2 pi i s k / P), k < nout.
 static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     auto key = std::make_tuple(P, nin, nout);
     auto it = h->czts.find(key);
     if (it != h->czts.end()) return it->second->dev;
     auto t = std::make_shared<CztTables>();
-    const int m = (int)h->fft->tuned_len((long long)nin + nout - 1, fused_cap());
-    if (m > fused_cap()) throw S1Error(S1G_E_GEOMETRY, "chirp-z length " + std::to_string(m) + " too long");
-    t->dev.dm = h->fft->desc3(m);
+    const auto plan = fused_plan(h, (long long)nin + nout - 1, "chirp-z length");
+    const int m = plan->d.n;
+    t->dev.dm = plan->d;
     t->dev.nin = nin;
     t->dev.nout = nout;
     const int nw = std::max(nin, nout);
@@ -1178,7 +1186,7 @@ static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     check_cuda(cudaMemcpy(B.data(), db, sizeof(cpx<double>) * m, cudaMemcpyDeviceToHost), "czt down");
     cudaFree(db);
     std::vector<cf32> K(m);
-    for (int q = 0; q < m; ++q) K[q] = mk((float)(B[q].x / m), (float)(B[q].y / m));
+    for (int q = 0; q < m; ++q) K[plan->mid[q]] = mk((float)(B[q].x / m), (float)(B[q].y / m));
     check_cuda(cudaMemcpy(dk, K.data(), sizeof(cf32) * m, cudaMemcpyHostToDevice), "czt up");
     t->dev.chirp = (const cf32*)dw;
     t->dev.kern = (const cf32*)dk;
@@ -1230,7 +1238,12 @@ struct FastPipe {
         const int mid = down / 2;
         fb.s0 = mid - output_shape / 2;
         fb.n_out = (mid + output_shape / 2) - fb.s0;
-        fb.m_nu = (int)h->fft->tuned_len((5LL * fb.bw_max + 3) / 4, fused_cap());
+        // 1.4 x the band (1.25 where that is too long): the kernel's aliases take
+        // energy from outside the band, which the deramped line has plenty of.
+        // SLC of a 1500 x 12000 burst against FP64: 1.3e-5 at 1.27 x, 4.3e-6 at
+        // 1.42 x, where other errors lead.
+        const long long wide = (7LL * fb.bw_max + 4) / 5;
+        fb.m_nu = fused_plan(h, wide <= fused_cap() ? wide : (5LL * fb.bw_max + 3) / 4, "time unfolding grid")->d.n;
     }
 
     // Gauss-Legendre nodes and weights on [-1, 1] (Newton iteration on the
@@ -1266,9 +1279,9 @@ struct FastPipe {
         fb->g = make_geom(h->hdr, pk);
         const BurstGeom& g = fb->g;
         // range compression: correlation length M and reference spectrum
-        fb->M = (int)fft.tuned_len((long long)g.n_r + g.L, fused_cap());
-        if (fb->M > fused_cap()) throw S1Error(S1G_E_GEOMETRY, "range line too long for the fused kernel");
-        fb->dM = fft.desc3(fb->M);
+        const auto planM = fused_plan(h, (long long)g.n_r + g.L, "range line too long for the fused kernel:");
+        fb->dM = planM->d;
+        fb->M = fb->dM.n;
         {
             Pipe<float> plain(h);
             const int M = fb->M;
@@ -1283,7 +1296,7 @@ struct FastPipe {
             check_cuda(cudaStreamSynchronize(st), "ref sync");
             std::vector<cf32> ref(M);
             const double s = 1.0 / (g.energy * (double)M);
-            for (int k = 0; k < M; ++k) ref[k] = mk((float)(spec[k].x * s), (float)(-spec[k].y * s));
+            for (int k = 0; k < M; ++k) ref[planM->mid[k]] = mk((float)(spec[k].x * s), (float)(-spec[k].y * s));
             fb->ref = fb->up(ref, st);
         }
         const int n_a = g.n_a, n_r = g.n_r;
@@ -1358,7 +1371,7 @@ struct FastPipe {
             fb->dfwd = fb->up(dfwd, st);
             fb->reramp = fb->up(rer, st);
             fb->na_smooth = is_smooth7(n_a) && n_a <= fused_cap();
-            if (fb->na_smooth) fb->dna = fft.desc3(n_a);
+            if (fb->na_smooth) fb->dna = fft.plan4(n_a)->d;
             else fb->cna = get_czt(h, n_a, n_a, n_a);
             fb->cf = get_czt(h, S, S, fb->bw);
             fb->ci = get_czt(h, S, fb->bw, S);
@@ -1412,7 +1425,7 @@ struct FastPipe {
         fb->slant = fb->up(g.slant, st);
         fb->zero_df = fb->up(std::vector<df>(n_r, df_make(0.f, 0.f)), st);
         fb->nr_smooth = is_smooth7(n_r) && n_r <= fused_cap();
-        if (fb->nr_smooth) fb->dnr = fft.desc3(n_r);
+        if (fb->nr_smooth) fb->dnr = fft.plan4(n_r)->d;
         else fb->cnr = get_czt(h, n_r, n_r, n_r);
         h->fast_bursts[key] = fb;
         return fb;
@@ -1476,6 +1489,13 @@ struct FastPipe {
         const double wl = kC_ / kCF_;
         ra.lam2_4 = df_from(std::pow(wl, 2.0) / 4.0);
         ra.post = 1;
+        if (ra.smooth && tops) {
+            float4* src = h->bSrc.as<float4>(fb.g.n_r);
+            float* lo = h->bSrcLo.as<float>(fb.g.n_r);
+            rowpass_src_table(ra.cols, fdc, ra.d.mid, ra.n_r, src, lo, st);
+            ra.src = src;
+            ra.src_lo = lo;
+        }
         return ra;
     }
 
@@ -1598,7 +1618,7 @@ struct FastPipe {
         ta.S = S;
         ta.n_r = n_r;
         ta.P = dP;
-        ta.dnu = fft.desc3(fb.m_nu);
+        ta.dnu = fft.plan4(fb.m_nu)->d;
         ta.rows = fb.rows_df;
         ta.cols = fb.cols;
         ta.fdc = fdc_df;

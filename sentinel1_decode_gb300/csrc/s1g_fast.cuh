@@ -2,18 +2,18 @@
 #pragma once
 
 #include "s1g_df.cuh"
-#include "s1g_fft3.cuh"
+#include "s1g_fft4.cuh"
 #include "s1g_kernels.h"
 
 namespace s1g {
 
 // Chirp-z transform X[k] = sum_{s<nin} x[s] exp(dir 2 pi i s k / period),
-// k < nout, computed as a circular convolution of length m (7-smooth,
-// m >= nin + nout - 1) in shared memory (Bluestein's identity).
+// k < nout, computed as a circular convolution of length m (m >= nin + nout - 1)
+// in shared memory (Bluestein's identity).
 struct CztDev {
-    Fft3Desc dm;           // length m
+    Fft4Desc dm;           // length m
     const cf32* chirp;     // w[n] = exp(-i pi n^2 / period), n < max(nin, nout)
-    const cf32* kern;      // FFT_m of b[n] = conj(w[n]), n in (-nin, nout), scaled by 1/m
+    const cf32* kern;      // FFT_m of b[n] = conj(w[n]), n in (-nin, nout), scaled by 1/m, at dm.mid
     int nin, nout;
 };
 
@@ -44,9 +44,9 @@ struct FufrArgs {
     const cf32* rcT;        // [n_r][n_a]
     int n_a, n_r;
     int na_smooth;
-    Fft3Desc dna;           // n_a (smooth case)
+    Fft4Desc dna;           // n_a (smooth case)
     CztDev cna;             // n_a-point DFT (otherwise)
-    CztDev cf, ci;          // band CZT forward (nin=S, nout=bw) and inverse (nin=bw, nout=S)
+    CztDev cf, ci;          // band CZT forward (nin=S, nout=bw) and inverse (nin=bw, nout=S), of one length
     const cf32* dfwd;       // deramp * exp(-2 pi i s start / S), S
     const cf32* reramp;     // re-ramp / S, S
     int S, tile_len, bw;
@@ -59,9 +59,11 @@ struct RowArgs {
     const ColDf* cols;
     const df* fdc;
     int smooth;
-    Fft3Desc d;              // n_r (smooth)
+    Fft4Desc d;              // n_r (smooth)
     CztDev cz;               // n_r-point DFT (non-smooth)
     df lam2_4;               // lambda^2 / 4
+    const float4* src;       // smooth, tops: {R^2 hi, R^2 lo, csrc, f_dc hi} of every range frequency at d.mid
+    const float* src_lo;     // and f_dc lo (rowpass_src_table)
     int post;                // 1: multiply by the scale / RCMC / azimuth-filter factor; 0: store the range IFFT
 };
 // Range cell migration correction by sinc interpolation (the S1G_RCMC_SINC
@@ -102,7 +104,7 @@ constexpr int kNuQuad = 128;   // Gauss-Legendre nodes of the kernel's Fourier t
 
 // Per-burst tables of the time unfolding that do not depend on the range bin
 // (k_tufr_tables, from the device-side parameters):
-//   band[p], p < M       band mask / Phi(p / M)^2 on the grid (p in FFT order)
+//   band[p], p < M       band mask / Phi(p / M)^2 of grid bin f at dnu.mid[f]
 //   nu_l0[p], p < n_out  first grid point of the interpolation window
 //   nu_w[j][p]           interpolation weights (complex), tap-major
 //   rer[p]               {knot index (int bits), fraction, tau hi, tau lo} of the re-ramp
@@ -120,7 +122,7 @@ struct TufrArgs {
     const cf32* in;          // [n_r][S], row pass output transposed
     int S, n_r;
     const TufrDev* P;
-    Fft3Desc dnu;            // grid FFT of both non-uniform FFTs (length M)
+    Fft4Desc dnu;            // grid FFT of both non-uniform FFTs (length M)
     const RowDf* rows;       // S knots
     const ColDf* cols;
     const df* fdc;
@@ -136,11 +138,14 @@ struct TufrArgs {
     TufrTables tab;
 };
 
-void rc_fused(const cf32* raw, cf32* rc, int n_a, int n_r, int h, const Fft3Desc& d, const cf32* ref,
+void rc_fused(const cf32* raw, cf32* rc, int n_a, int n_r, int h, const Fft4Desc& d, const cf32* ref,
               cudaStream_t st);
 void fufr_fused(const FufrArgs& a, cudaStream_t st);
 // Doppler centroid polynomial from nchunk partial lag-1 sums [nchunk][n_r]
 void dc_fit_fast(const cf64* part, int nchunk, const DcFitArgs& a, double* f_dc, df* f_dc_df, cudaStream_t st);
+// src / src_lo of a smooth TOPS row pass (n_r entries each) from cols and fdc
+void rowpass_src_table(const ColDf* cols, const df* fdc, const int* mid, int n_r, float4* src, float* src_lo,
+                       cudaStream_t st);
 void rowpass_fused(const RowArgs& a, cudaStream_t st);
 // ka0: device scratch of S doubles
 void tufr_params_fast(const RowParam* rows, const double* slant, const double* f_dc, int S, int n_r, double rate,

@@ -3,6 +3,7 @@
 #include "s1g_tma.h"
 
 #include <algorithm>
+#include <iterator>
 #include <atomic>
 #include <cmath>
 #include <cstdio>
@@ -33,42 +34,97 @@ long long next_smooth7(long long n) {
     return n;
 }
 
-static void radices3_for(long long n, std::vector<int>& out) {
-    int c2 = 0, c3 = 0, c5 = 0, c7 = 0;
-    while (n % 2 == 0) { n /= 2; ++c2; }
-    while (n % 3 == 0) { n /= 3; ++c3; }
-    while (n % 5 == 0) { n /= 5; ++c5; }
-    while (n % 7 == 0) { n /= 7; ++c7; }
-    while (c2 >= 4) { out.push_back(16); c2 -= 4; }
-    if (c2 == 3) out.push_back(8);
-    if (c2 == 2) out.push_back(4);
-    if (c2 == 1) out.push_back(2);
-    for (int i = 0; i < c5; ++i) out.push_back(5);
-    for (int i = 0; i < c3; ++i) out.push_back(3);
-    for (int i = 0; i < c7; ++i) out.push_back(7);
+// Modelled instructions per point of a pass of the fused kernels' core.
+static double pass_cost(int r) {
+    switch (r) {
+        case 2: return 9;
+        case 3: return 11;
+        case 4: return 11;
+        case 5: return 14;
+        case 6: return 15;
+        case 7: return 19;
+        case 8: return 13.5;
+        case 9: return 18;
+        case 10: return 18;
+        case 12: return 17;
+        case 15: return 24;
+        default: return 16;
+    }
 }
 
-int fft3_passes(long long n) {
-    std::vector<int> r;
-    radices3_for(n, r);
-    return (int)r.size();
+static const int kRadices[] = {16, 15, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+
+// factorisations of n into the radices (largest first), at most `left` of them
+static void factorisations(long long n, size_t first, int left, std::vector<int>& cur,
+                           std::vector<std::vector<int>>& out) {
+    if (n == 1) {
+        out.push_back(cur);
+        return;
+    }
+    if (left == 0) return;
+    for (size_t i = first; i < sizeof(kRadices) / sizeof(int); ++i)
+        if (n % kRadices[i] == 0) {
+            cur.push_back(kRadices[i]);
+            factorisations(n / kRadices[i], i, left - 1, cur, out);
+            cur.pop_back();
+        }
 }
 
-long long fast_len(long long minlen, long long cap) {
-    long long best = -1;
-    double bc = 0;
-    const long long hi = std::max(minlen, (long long)(minlen * 1.25) + 1);
-    for (long long m = std::max(1LL, minlen); m <= hi; ++m) {
-        if (m > cap) break;
-        if (!is_smooth7(m)) continue;
-        const double c = (double)m * (double)fft3_passes(m);
-        if (best < 0 || c < bc) {
-            best = m;
-            bc = c;
+static double order_cost(const std::vector<int>& r) {
+    double c = 0;
+    for (int x : r) c += pass_cost(x);
+    // the last inverse pass reads 32 bytes of twiddles per butterfly
+    return c + 8.0 / r.front();
+}
+
+std::vector<std::vector<int>> fft4_orders(long long n, size_t most) {
+    std::vector<std::pair<double, std::vector<int>>> c;
+    std::vector<std::vector<int>> f;
+    std::vector<int> cur;
+    if (n < 2 || !is_smooth7(n)) return {};
+    if (n % 16 == 0) {
+        // affine: radix 16 last, a radix of the functor passes first
+        factorisations(n / 16, 0, kFft4Passes - 1, cur, f);
+        for (auto v : f) {
+            if (v.empty()) continue;
+            std::sort(v.begin(), v.end());
+            do {
+                if (!fft4_end_radix(v[0])) continue;
+                std::vector<int> o = v;
+                o.push_back(16);
+                c.push_back({order_cost(o), o});
+            } while (std::next_permutation(v.begin(), v.end()));
         }
     }
-    if (best < 0) best = next_smooth7(minlen);
-    return best;
+    if (c.empty()) {
+        f.clear();
+        factorisations(n, 0, kFft4Passes, cur, f);
+        for (auto& v : f) c.push_back({order_cost(v), v});
+    }
+    std::stable_sort(c.begin(), c.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+    std::vector<std::vector<int>> out;
+    for (size_t i = 0; i < c.size() && out.size() < most; ++i) out.push_back(c[i].second);
+    return out;
+}
+
+std::vector<long long> fft4_lengths(long long minlen, size_t most) {
+    std::vector<std::pair<double, long long>> c;
+    const long long hi = std::max(64LL, (long long)(minlen * 1.25) + 16);
+    for (long long m = std::max(64LL, (minlen + 15) / 16 * 16); m <= hi; m += 16) {
+        if ((long long)sizeof(cf32) * padded16_len((int)m) > kFft4SmemBytes) break;
+        const auto o = fft4_orders(m, 1);
+        if (o.empty() || o[0].back() != 16 || !fft4_end_radix(o[0][0])) continue;
+        c.push_back({(double)m * (order_cost(o[0]) + 12.0), m});
+    }
+    std::stable_sort(c.begin(), c.end(), [](const auto& a, const auto& b) { return a.first < b.first; });
+    std::vector<long long> out;
+    for (size_t i = 0; i < c.size() && out.size() < most; ++i) out.push_back(c[i].second);
+    return out;
+}
+
+long long fast_len(long long minlen) {
+    const auto c = fft4_lengths(minlen, 1);
+    return c.empty() ? -1 : c[0];
 }
 
 DeviceArena::~DeviceArena() {
@@ -398,72 +454,88 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     return p;
 }
 
-Fft3Plan::~Fft3Plan() {
+Fft4Plan::~Fft4Plan() {
     for (void* p : owned) cudaFree(p);
 }
 
-std::vector<int> default_radices3(long long n) {
-    std::vector<int> r;
-    radices3_for(n, r);
-    return r;
+// w, w^2, w^4, w^8 of w = exp(sign 2 pi i num / den)
+static void twiddle_entry(std::vector<float4>& out, long long num, long long den, int sign) {
+    double c[4], s[4];
+    for (int b = 0; b < 4; ++b) unit_root(num * (1 << b), den, c[b], s[b]);
+    const double g = sign > 0 ? -1.0 : 1.0;   // unit_root gives exp(-)
+    out.push_back(make_float4((float)c[0], (float)(g * s[0]), (float)c[1], (float)(g * s[1])));
+    out.push_back(make_float4((float)c[2], (float)(g * s[2]), (float)c[3], (float)(g * s[3])));
 }
 
-std::shared_ptr<Fft3Plan> build_plan3(int n, const std::vector<int>& rad) {
-    if (!is_smooth7(n) || n > smem_capacity<float>()) throw std::runtime_error("desc3: length not smooth/small");
-    if ((int)rad.size() > kMaxStages) throw std::runtime_error("desc3: too many stages");
+std::shared_ptr<Fft4Plan> build_plan4(int n, const std::vector<int>& rad) {
+    if (rad.empty() || (int)rad.size() > kFft4Passes || sizeof(cf32) * padded16_len(n) > (size_t)kFft4SmemBytes)
+        throw std::runtime_error("plan4: length " + std::to_string(n) + " not smooth/small");
     long long prod = 1;
-    for (int r : rad) prod *= r;
-    if (prod != n) throw std::runtime_error("desc3: radices do not multiply to the length");
-    auto p = std::make_shared<Fft3Plan>();
-    Fft3Desc& d = p->d;
+    for (int r : rad) {
+        if (std::find(std::begin(kRadices), std::end(kRadices), r) == std::end(kRadices))
+            throw std::runtime_error("plan4: radix");
+        prod *= r;
+    }
+    if (prod != n) throw std::runtime_error("plan4: radices do not multiply to the length");
+    auto p = std::make_shared<Fft4Plan>();
+    Fft4Desc& d = p->d;
     d.n = n;
-    d.nstages = (int)rad.size();
-    for (size_t i = 0; i < rad.size(); ++i) d.radix[i] = (int8_t)rad[i];
-    const int nhi = fft3_nhi(n);
-    std::vector<cf32> tw(fft3_tw_len(n));
-    for (int q = 0; q < nhi; ++q) {
-        double c, s;
-        unit_root(64LL * q, n, c, s);
-        tw[q] = mk((float)c, (float)s);
+    d.np = (int)rad.size();
+    d.affine = d.np >= 2 && rad.back() == 16 && fft4_end_radix(rad[0]);
+    // block g of a pass holds the input modulo x^len - exp(-2 pi i F[g] / N)
+    std::vector<long long> F{0};
+    std::vector<float4> tab;
+    size_t fo[kFft4Passes], io[kFft4Passes];
+    long long N = 1;
+    int Ns = n;
+    for (int q = 0; q < d.np; ++q) {
+        const int R = rad[q];
+        d.radix[q] = R;
+        Ns /= R;
+        fo[q] = tab.size();
+        for (long long f : F) twiddle_entry(tab, f, N * R, -1);
+        io[q] = tab.size();
+        for (int k = 0; k < Ns; ++k) twiddle_entry(tab, k, (long long)Ns * R, +1);
+        std::vector<long long> G;
+        G.reserve(F.size() * R);
+        for (long long f : F)
+            for (int j = 0; j < R; ++j) G.push_back(f + j * N);
+        F.swap(G);
+        N *= R;
     }
-    for (int q = 0; q < 64; ++q) {
-        double c, s;
-        unit_root(q, n, c, s);
-        tw[nhi + q] = mk((float)c, (float)s);
+    std::vector<int> pos(n);
+    p->mid.resize(n);
+    const int R = rad.back();
+    for (int i = 0; i < n; ++i) {
+        pos[F[i]] = i;
+        p->mid[F[i]] = (i % R) * (n / R) + i / R;
     }
-    std::vector<int> perm(n);
-    for (int j = 0; j < n; ++j) {
-        int jj = j, size = n, pos = 0;
-        for (int st = d.nstages - 1; st >= 0; --st) {
-            const int r = jj % rad[st];
-            jj /= rad[st];
-            size /= rad[st];
-            pos += r * size;
-        }
-        perm[j] = pos;
+    auto up = [&](const void* src, size_t bytes) {
+        void* v = nullptr;
+        check_cuda(cudaMalloc(&v, bytes), "plan4 table");
+        p->owned.push_back(v);
+        check_cuda(cudaMemcpy(v, src, bytes, cudaMemcpyHostToDevice), "plan4 upload");
+        return v;
+    };
+    const float4* t = (const float4*)up(tab.data(), sizeof(float4) * tab.size());
+    for (int q = 0; q < d.np; ++q) {
+        d.fw[q] = t + fo[q];
+        d.iv[q] = t + io[q];
     }
-    void *dt = nullptr, *dp = nullptr;
-    check_cuda(cudaMalloc(&dt, sizeof(cf32) * tw.size()), "desc3 tw");
-    p->owned.push_back(dt);
-    check_cuda(cudaMalloc(&dp, sizeof(int) * n), "desc3 perm");
-    p->owned.push_back(dp);
-    check_cuda(cudaMemcpy(dt, tw.data(), sizeof(cf32) * tw.size(), cudaMemcpyHostToDevice), "desc3 tw up");
-    check_cuda(cudaMemcpy(dp, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "desc3 perm up");
-    d.tw = (const cf32*)dt;
-    d.perm = (const int*)dp;
+    d.pos = (const int*)up(pos.data(), sizeof(int) * n);
+    d.mid = (const int*)up(p->mid.data(), sizeof(int) * n);
     return p;
 }
 
-Fft3Desc FftEngine::desc3(int n) {
-    auto it = plans3.find(n);
-    if (it != plans3.end()) return it->second->d;
-    const std::vector<int> rad = tuned_radices(n, stream);
-    auto p = build_plan3(n, rad);
-    plans3[n] = p;
-    return p->d;
+std::shared_ptr<Fft4Plan> FftEngine::plan4(int n) {
+    auto it = plans4.find(n);
+    if (it != plans4.end()) return it->second;
+    auto p = build_plan4(n, tuned_radices(n, stream));
+    plans4[n] = p;
+    return p;
 }
 
-long long FftEngine::tuned_len(long long minlen, long long cap) { return tuned_length(minlen, cap, stream); }
+long long FftEngine::tuned_len(long long minlen) { return tuned_length(minlen, stream); }
 
 template <typename R>
 FftDesc<R> FftEngine::smem_desc(int n) {

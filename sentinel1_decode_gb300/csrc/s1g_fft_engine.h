@@ -17,7 +17,7 @@
 #include <vector>
 
 #include "s1g_fft.cuh"
-#include "s1g_fft3.cuh"
+#include "s1g_fft4.cuh"
 
 namespace s1g {
 
@@ -28,11 +28,12 @@ constexpr int kSmemBytes = 220 * 1024;
 
 bool is_smooth7(long long n);
 long long next_smooth7(long long n);
-// Transform length >= minlen for the radix-16 core: the 7-smooth length in
-// [minlen, 1.25 minlen] (and <= cap) of least length x passes.
-long long fast_len(long long minlen, long long cap);
-// Shared-memory passes of the radix-16 core for length n.
-int fft3_passes(long long n);
+// Shared memory of the fused kernels (the most a CTA can have).
+constexpr int kFft4SmemBytes = 227 * 1024;
+// Transform length >= minlen for the fused kernels' core: the affine length
+// (16 x radices, s1g_fft4.cuh) in [minlen, 1.25 minlen] of least modelled
+// cost that fits shared memory, -1 if there is none.
+long long fast_len(long long minlen);
 template <typename R>
 inline int smem_capacity() { return kSmemBytes / (int)sizeof(cpx<R>); }
 
@@ -59,11 +60,12 @@ struct FftPlan {
     ~FftPlan();
 };
 
-// Device tables of the radix-16 core for one length.
-struct Fft3Plan {
-    Fft3Desc d;
+// Device tables of the fused kernels' core (s1g_fft4.cuh) for one length.
+struct Fft4Plan {
+    Fft4Desc d;
+    std::vector<int> mid;         // host copy of d.mid
     std::vector<void*> owned;
-    ~Fft3Plan();
+    ~Fft4Plan();
 };
 
 // One per processing context (device + stream).
@@ -73,7 +75,7 @@ struct FftEngine {
     cudaStream_t stream;
     std::map<int, std::shared_ptr<FftPlan<float>>> plans32;
     std::map<int, std::shared_ptr<FftPlan<double>>> plans64;
-    std::map<int, std::shared_ptr<Fft3Plan>> plans3;
+    std::map<int, std::shared_ptr<Fft4Plan>> plans4;
     DeviceArena scratch_a, scratch_b, scratch_c;
 
     template <typename R>
@@ -90,23 +92,26 @@ struct FftEngine {
     template <typename R>
     FftDesc<R> smem_desc(int n);
 
-    // Radix-16 core descriptor (n 7-smooth, fits shared memory); the radix
-    // order comes from the autotuner (s1g_tune.cu) when it is on.
-    Fft3Desc desc3(int n);
-    // Transform length >= minlen (<= cap) for the fused kernels: the
-    // autotuner's pick among the cheapest 7-smooth candidates, or fast_len.
-    long long tuned_len(long long minlen, long long cap);
+    // Plan of the fused kernels' core (n 7-smooth, fits shared memory); the
+    // radix order comes from the autotuner (s1g_tune.cu) when it is on.
+    std::shared_ptr<Fft4Plan> plan4(int n);
+    // Transform length >= minlen for the fused kernels: the autotuner's pick
+    // among the cheapest candidates, or fast_len.
+    long long tuned_len(long long minlen);
 };
 
-// Radix-16 plans and their autotuner (s1g_tune.cu).
-std::vector<int> default_radices3(long long n);
-std::shared_ptr<Fft3Plan> build_plan3(int n, const std::vector<int>& radices);
+// Radix orders for length n in the order of their modelled cost (at most
+// `most`; affine ones where there are any); empty if n is not 7-smooth.
+std::vector<std::vector<int>> fft4_orders(long long n, size_t most);
+// The cheapest affine lengths >= minlen that fit shared memory.
+std::vector<long long> fft4_lengths(long long minlen, size_t most);
+std::shared_ptr<Fft4Plan> build_plan4(int n, const std::vector<int>& radices);
 // Radix order for length n: the fastest measured candidate when tuning is on
-// (S1G_AUTOTUNE unset or not "0"), else default_radices3.  Measurements run
-// on `st` (skipped while st is being captured) and persist in a text file
+// (S1G_AUTOTUNE unset or not "0"), else the model's.  Measurements run on
+// `st` (skipped while st is being captured) and persist in a text file
 // (S1G_FFT_TUNE_FILE, default fft_tune.txt beside the library).
 std::vector<int> tuned_radices(int n, cudaStream_t st);
-long long tuned_length(long long minlen, long long cap, cudaStream_t st);
+long long tuned_length(long long minlen, cudaStream_t st);
 // "n:r1.r2..;..." of the radix orders and "minlen>M;..." of the lengths
 // chosen so far in this process.
 std::string tuning_report();
