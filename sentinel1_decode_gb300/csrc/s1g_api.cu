@@ -95,9 +95,9 @@ struct s1g_decoder {
     IndexScratch isc;
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
-    Buf bFdf, bKN, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
+    Buf bFdf, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
     Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
-    Buf bTuD, bTuG, bTuI, bTuW, bTuR, bKa0;   // time-unfolding per-burst tables
+    Buf bTuD, bTuG, bTuI, bTuW, bTuR, bTuWt, bTuRamp, bKa0;   // time-unfolding per-burst tables and grids
     Buf bImgIn, bImgOut, bImgMax;        // image epilogue
     Buf bJ0, bJ1, bJ2, bJ3, bJ4, bJ5, bJe, bJd;   // differentiable azimuth chains
     Buf bRawW;                               // decoded rows after the FP64 ECCM notch (FP32 paths)
@@ -115,7 +115,6 @@ struct s1g_decoder {
     // FP32 calls (built on the first such call, dropped when the stream
     // content or the A/B/C decode mode changes)
     std::map<std::string, std::shared_ptr<struct SwathDecode>> swath_decodes;
-    int num_sms = 0;
     Result last;
     double last_ms = 0;
     std::string stage_text;
@@ -1413,7 +1412,7 @@ struct FastPipe {
             cols[j].tau2pi = df_from((2.0 * kPIref_) * g.tcorr[j]);
             const double a0 = std::fmod(k4r, 2.0 * M_PI);
             cols[j].az0 = mk((float)std::cos(a0), (float)std::sin(a0));
-            cols[j].rscale = (float)g.rscale[j];
+            cols[j].rscale = (float)(1.0 / g.rscale[j]);
             const double fr = g.range_freq[j];
             cols[j].csrc = (float)(kPIref_ * fr * fr * kC_ * R / (2.0 * c3));
             cols[j].crcmc = (float)((4.0 * kPIref_) * fr * R / kC_);
@@ -1599,13 +1598,9 @@ struct FastPipe {
         cf32* ufrT2 = h->bD.as<cf32>((size_t)n_r * S);
         transpose_batched<float>(ufr, n_r, 0, ufrT2, S, 0, S, n_r, 1, st);
         TufrDev* dP = h->bTd.as<TufrDev>(1);
+        const TufrLaunch tl = tufr_launch(S, fb.t_hi, fb.m_nu);
         tufr_params_fast(fb.rows64, fb.slant, fdc, S, n_r, fb.rate, g.T, g.prf, bd, g.swath_number,
-                         h->bKa0.as<double>(S), dP, st);
-        if (h->num_sms == 0) {
-            int dev = 0;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&h->num_sms, cudaDevAttrMultiProcessorCount, dev);
-        }
+                         h->bKa0.as<double>(S), fb.m_nu, tl.ycap, fb.t_hi, dP, st);
         h->mark("azimuth_ifft");
         // azimuth IFFT (length S, 1/S) of every range bin, s1_decoder.cpp:682
         cf32* Aaz = h->bC.as<cf32>((size_t)n_r * S);
@@ -1625,16 +1620,19 @@ struct FastPipe {
         ta.inv_lamR = fb.inv_lamR;
         const double wl = kC_ / kCF_;
         ta.lam2_4 = df_from(std::pow(wl, 2.0) / 4.0);
-        ta.rate = df_from(fb.rate);
+        ta.inv_rate = df_from(1.0 / fb.rate);
         ta.pi_ = df_from(kPIref_);
         ta.two_pi_ = df_from(2.0 * kPIref_);
-        ta.tmax = fb.t_hi;
         ta.bwmax = fb.bw_max;
         ta.s0 = fb.s0;
         ta.n_out = fb.n_out;
-        const int grid = std::max(1, h->num_sms * tufr_ctas_per_sm(ta));
-        ta.KN = h->bKN.as<float>((size_t)grid * kTufrGroup * 4 * S);
-        ta.G = h->bTuG.as<cf32>((size_t)grid * kTufrGroup * fb.m_nu);
+        ta.ycap = tl.ycap;
+        // the row pass output (bD) and the unfolded burst (bA) are done with
+        ta.poly = h->bD.as<uint2>((size_t)n_r * S);
+        ta.curv = h->bA.as<float>((size_t)n_r * S);
+        ta.ramp = h->bTuRamp.as<cf32>((size_t)n_r * ta.n_out);
+        ta.G = h->bTuG.as<cf32>((size_t)n_r * fb.m_nu);
+        ta.tab.wt = h->bTuWt.as<float4>((size_t)tl.weights);
         ta.tab.band = h->bTuD.as<float>((size_t)fb.m_nu);
         ta.tab.nu_l0 = h->bTuI.as<int>((size_t)ta.n_out);
         ta.tab.nu_w = h->bTuW.as<cf32>((size_t)ta.n_out * kNuTaps);
@@ -1647,7 +1645,7 @@ struct FastPipe {
         int* stat = tufr_status ? tufr_status : h->bTstat.as<int>(1);
         if (!tufr_status) check_cuda(cudaMemsetAsync(stat, 0, sizeof(int), st), "tstat");
         ta.status = stat;
-        tufr_fused(ta, grid, st);
+        tufr_fused(ta, tl, st);
         h->mark("corner_turn");
         cf32* O = final_out ? final_out : h->bA.as<cf32>((size_t)ta.n_out * n_r);
         transpose_batched<float>(outT, ta.n_out, 0, O, n_r, 0, n_r, ta.n_out, 1, st);

@@ -115,6 +115,48 @@ __device__ __forceinline__ df df_sqrt(df a) {
     const float corr = r.hi * (0.5f * df_rcp_approx(s));
     return quick_two_sum(s, corr);
 }
+// Double-float sum without the second error term (Hida-Li-Bailey's "sloppy"
+// add): its error is below 2^-46 of the larger operand, the absolute
+// accuracy the phases need, at half the operations of df_add.
+__device__ __forceinline__ df df_add_abs(df a, df b) {
+    df s = two_sum(a.hi, b.hi);
+    s.lo = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
+    return quick_two_sum(s.hi, s.lo);
+}
+// a / b from two quotient digits, the second from the exact remainder of the
+// first (relative error ~2^-44: the digits' own are 2^-22): 7 operations where
+// df_div takes ~60.
+__device__ __forceinline__ df df_div2(df a, df b) {
+    const float rb = df_rcp_approx(b.hi);
+    const float q1 = __fmul_rn(a.hi, rb);
+    const float r = __fadd_rn(__fmaf_rn(-q1, b.hi, a.hi), __fmaf_rn(-q1, b.lo, a.lo));
+    return quick_two_sum(q1, __fmul_rn(r, rb));
+}
+// 1 - sqrt(1 - x) of a small x >= 0 (the cosine of the squint): its Taylor
+// series below 2e-3 (truncation below 1e-18), x and x^2 in double-float and
+// the rest, below 6e-10, in float; else through df_sqrt.
+__device__ __forceinline__ df df_one_minus_sqrt1m(df x) {
+    if (x.hi < 2e-3f) {
+        const df x2 = df_mul(x, x);
+        const float h = x.hi;
+        const float rest = x2.hi * h * fmaf(h, fmaf(h, 7.0f / 256.0f, 5.0f / 128.0f), 1.0f / 16.0f);
+        return df_add_f(df_add_abs(df_make(0.5f * x.hi, 0.5f * x.lo), df_make(0.125f * x2.hi, 0.125f * x2.lo)), rest);
+    }
+    const df D = df_sqrt(df_sub(df_make(1.f, 0.f), x));
+    return df_div(x, df_add_f(D, 1.0f));
+}
+// (1 - x)^(3/2) of the same x: 1 - 3/2 x in double-float plus the series'
+// rest (below 1.5e-6) in float.
+__device__ __forceinline__ df df_pow32_1m(df x) {
+    if (x.hi < 2e-3f) {
+        const float h = x.hi;
+        const float rest = h * h * fmaf(h, fmaf(h, 3.0f / 128.0f, 1.0f / 16.0f), 3.0f / 8.0f);
+        const df c = df_mul_f(x, 1.5f);
+        return df_add_f(df_add_abs(df_make(1.f, 0.f), df_neg(c)), rest);
+    }
+    const df D = df_sqrt(df_sub(df_make(1.f, 0.f), x));
+    return df_mul(D, df_mul(D, D));
+}
 // 2*pi as a float pair and its reciprocal.
 __device__ __forceinline__ df df_two_pi() { return df_make(6.28318548202514648f, -1.74845553e-7f); }
 

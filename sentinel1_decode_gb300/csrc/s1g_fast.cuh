@@ -30,7 +30,7 @@ struct ColDf {
     df k4r;          // 4 pi R / lambda
     df tau2pi;       // 2 pi * timing correction (packet.cpp:322-342)
     cf32 az0;        // exp(i (4 pi R / lambda mod 2 pi))
-    float rscale;    // sqrt((R_ref / R)^3)
+    float rscale;    // 1 / sqrt((R_ref / R)^3)
     float csrc;      // pi f_r^2 c R / (2 f_c^3)   (SRC phase = -csrc F^2 / (v_rel^2 D^2))
     float crcmc;     // 4 pi f_r R / c             (RCMC phase = -crcmc (1-D)/D)
     float rmig;      // 2 R f_s / c                (range migration in samples = rmig (1-D)/D)
@@ -38,6 +38,12 @@ struct ColDf {
 
 struct TufrDev {       // device-side time unfolding parameters (from k_tufr_params_fast)
     TufrParams q;
+    int ok;             // parameters valid and inside the kernels' limits
+    int lc, kw, chunks; // spreading: grid points per CTA, samples per thread, runs of lc (tufr_split)
+    unsigned long long ks64;   // band shift per sample, 2^64 to the turn
+    df tau0, dtau, dt;  // azimuth times: first, step, sample spacing
+    float gk, rt;       // knots per sample, samples per knot
+    int perm;           // spreading: distance of adjacent lanes' grid-point groups
 };
 
 struct FufrArgs {
@@ -98,19 +104,21 @@ void rcmc_sinc(const RcmcArgs& a, cudaStream_t st);
 // Phi is the kernel's Fourier transform (Gauss-Legendre quadrature); each
 // end has relative error ~1e-8 in FP64, below the FP32 FFT noise.
 constexpr int kNuW = 13;
-constexpr int kTufrGroup = 2;   // range bins spread together (one kernel weight for both lines)
+constexpr int kTufrGroup = 4;   // range bins spread together (one kernel weight for all)
 constexpr int kNuTaps = kNuW + 2;
 constexpr int kNuQuad = 128;   // Gauss-Legendre nodes of the kernel's Fourier transform
 
 // Per-burst tables of the time unfolding that do not depend on the range bin
 // (k_tufr_tables, from the device-side parameters):
 //   band[p], p < M       band mask / Phi(p / M)^2 of grid bin f at dnu.mid[f]
+//   wt                   spreading weights (k_tufr_weights)
 //   nu_l0[p], p < n_out  first grid point of the interpolation window
 //   nu_w[j][p]           interpolation weights (complex), tap-major
 //   rer[p]               {knot index (int bits), fraction, tau hi, tau lo} of the re-ramp
 //   gl_x, gl_w           Gauss-Legendre nodes and weights on [-1, 1] (kNuQuad)
 struct TufrTables {
     float* band;
+    float4* wt;
     int* nu_l0;
     cf32* nu_w;
     float4* rer;
@@ -127,11 +135,13 @@ struct TufrArgs {
     const ColDf* cols;
     const df* fdc;
     const df* inv_lamR;      // 1 / (lambda R), per range bin
-    df lam2_4, rate, pi_, two_pi_;
-    float* KN;               // per-CTA scratch: kTufrGroup * 4 * S (pi K_t and -f_dc/K_a as float pairs)
-    cf32* G;                 // per-CTA scratch: kTufrGroup * M (spread grids)
-    int tmax, bwmax;
-    int ychunk;              // shared-memory samples of a spreading pass (all kTufrGroup range bins)
+    df lam2_4, inv_rate, pi_, two_pi_;
+    uint2* poly;             // [n_r][S] deramp polynomials (base, slope) of the knot intervals
+    float* curv;             // [n_r][S] and their curvature
+    cf32* ramp;              // [n_r][n_out] exp(i re-ramp phase)
+    cf32* G;                 // [n_r][M] spread grids
+    int bwmax;
+    int ycap;                // samples a spreading CTA holds
     cf32* out;               // [n_r][n_out]
     int n_out, s0;           // cropped output rows: [s0, s0 + n_out)
     int* status;             // set to 1 if the burst falls outside the launch plan
@@ -149,10 +159,32 @@ void rowpass_src_table(const ColDf* cols, const df* fdc, const int* mid, int n_r
 void rowpass_fused(const RowArgs& a, cudaStream_t st);
 // ka0: device scratch of S doubles
 void tufr_params_fast(const RowParam* rows, const double* slant, const double* f_dc, int S, int n_r, double rate,
-                      double T, double prf, double bd, int swath_number, double* ka0, TufrDev* out, cudaStream_t st);
-// CTAs per SM the time-unfolding kernel runs with (its grid is this times the SM count)
-int tufr_ctas_per_sm(const TufrArgs& a);
-void tufr_fused(const TufrArgs& a, int grid, cudaStream_t st);
+                      double T, double prf, double bd, int swath_number, double* ka0, int M, int ycap, int tmax,
+                      TufrDev* out, cudaStream_t st);
+// How the grid is split for spreading: a thread takes 4 adjacent grid points
+// and reads the kw samples that can lie in their joint window of
+// (W + 3) TS / M; a CTA of up to 128 threads takes lc points whose samples fit
+// ycap (lc < 4: none do).
+struct TufrSplit {
+    int lc, kw, chunks;
+};
+__host__ __device__ inline TufrSplit tufr_split(long long TS, int M, int ycap) {
+    TufrSplit s;
+    const double r = (double)TS / (double)M;
+    s.kw = (int)((kNuW + 3) * r) + 2;
+    // samples of a run: (lc - 4) r + 1 up to the last group's first, then kw
+    const double lc = ((double)ycap - 2.0 - s.kw) / r + 4.0;
+    s.lc = lc < 4.0 ? 0 : lc > 512.0 ? 512 : (int)lc / 4 * 4;
+    s.chunks = s.lc >= 4 ? (M + s.lc - 1) / s.lc : 0;
+    return s;
+}
+// Bounds of the spreading launch for any tile count up to tmax.
+struct TufrLaunch {
+    int ycap, chunks;
+    long long weights;       // entries of TufrTables::wt
+};
+TufrLaunch tufr_launch(int S, int tmax, int M);
+void tufr_fused(const TufrArgs& a, const TufrLaunch& L, cudaStream_t st);
 // Fill a.tab for the burst whose parameters are at a.P (tables sized for a.tmax tiles).
 void tufr_tables(const TufrArgs& a, cudaStream_t st);
 void czt_rows(const cf32* in, long long ip, cf32* out, long long op, long long rows, const CztDev& c, int dir,

@@ -15,22 +15,18 @@ __device__ __forceinline__ float src_phase(const RowDf& r, df Q, float csrc, df 
     const float F = r.fa.hi + fdc.hi + (r.fa.lo + fdc.lo);
     const float vq = r.P.hi * ((r.A.hi - Q.hi) + (r.A.lo - Q.lo));
     const float F2 = F * F;
-    const float D2 = 1.0f - lam2_4 * F2 / vq;
-    return -csrc * F2 / (vq * D2);
+    return -csrc * F2 / (vq - lam2_4 * F2);   // v^2 D^2 = v^2 - lambda^2 F^2 / 4
 }
 
 // Scale, RCMC and azimuth filter factor (s1_decoder.cpp:643-676).
 __device__ __forceinline__ cf32 post_factor(const RowDf& r, const ColDf& c, df fdc, df lam2_4, int tops) {
-    const df F = df_add(r.fa, fdc);
-    const df vq = df_mul(r.P, df_sub(r.A, c.Q));
-    const df x = df_div(df_mul(lam2_4, df_mul(F, F)), vq);
-    const df D = df_sqrt(df_sub(df_make(1.f, 0.f), x));
-    const df omd = df_div(x, df_add_f(D, 1.0f));   // 1 - D
-    const df th = df_add(df_neg(df_mul(c.k4r, omd)), df_mul(c.tau2pi, F));
+    const df F = df_add_abs(r.fa, fdc);
+    const df vq = df_mul(r.P, df_add_abs(r.A, df_neg(c.Q)));
+    const df omd = df_one_minus_sqrt1m(df_div2(df_mul(lam2_4, df_mul(F, F)), vq));   // 1 - D
+    const df th = df_add_abs(df_neg(df_mul(c.k4r, omd)), df_mul(c.tau2pi, F));
     float theta = df_wrap(th);
-    if (tops) theta -= c.crcmc * (omd.hi / D.hi);
-    const cf32 f = cexpf_fast(theta) * c.az0;
-    return f * (1.0f / c.rscale);
+    if (tops) theta -= c.crcmc * __fdividef(omd.hi, 1.0f - omd.hi);
+    return cexpf_fast(theta) * c.az0 * c.rscale;
 }
 
 // What the SRC phase takes of the range columns, in the order of the
@@ -124,12 +120,10 @@ __global__ void __launch_bounds__(256) k_rcmc_sinc(RcmcArgs a) {
     const int jj = act ? j : a.n_r - 1;
     const ColDf c = a.cols[jj];
     const df fdc = a.fdc[jj];
-    const df F = df_add(rp.fa, fdc);
-    const df vq = df_mul(rp.P, df_sub(rp.A, c.Q));
-    const df x = df_div(df_mul(a.lam2_4, df_mul(F, F)), vq);
-    const df D = df_sqrt(df_sub(df_make(1.f, 0.f), x));
-    const df omd = df_div(x, df_add_f(D, 1.0f));   // 1 - D
-    const double t = (double)j + (double)(c.rmig * (omd.hi / D.hi));
+    const df F = df_add_abs(rp.fa, fdc);
+    const df vq = df_mul(rp.P, df_add_abs(rp.A, df_neg(c.Q)));
+    const df omd = df_one_minus_sqrt1m(df_div2(df_mul(a.lam2_4, df_mul(F, F)), vq));   // 1 - D
+    const double t = (double)j + (double)(c.rmig * (omd.hi / (1.0f - omd.hi)));
     const cf32 v = sinc_warp<float>(a.in + (long long)i * a.n_r, a.n_r, t, a.L, act);
     if (act) a.out[(long long)i * a.n_r + j] = v * post_factor(rp, c, fdc, a.lam2_4, 0);
 }

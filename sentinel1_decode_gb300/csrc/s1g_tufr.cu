@@ -13,37 +13,44 @@ namespace s1g {
 
 // ------------------------------------------------------------------ time unfolding
 
-// Knot of the deramp / re-ramp phase: pi K_t and the deramp time -f_dc/K_a,
-// as float pairs (one float4 per knot).
-__device__ __forceinline__ void load_knot(const float4* KN, int i, df& pkt, df& dct) {
-    const float4 v = KN[i];
-    pkt = df_make(v.x, v.y);
-    dct = df_make(v.z, v.w);
+// Knot of the deramp / re-ramp phase at azimuth row rw of a range bin:
+// pi K_t and the deramp time -f_dc/K_a.
+struct Knot {
+    df pkt, dct;
+};
+__device__ __forceinline__ Knot knot_at(const RowDf& rw, df Q, df fdc, df ilr, const TufrArgs& a) {
+    const df F = df_add_abs(rw.fa, fdc);
+    const df vq = df_mul(rw.P, df_add_abs(rw.A, df_neg(Q)));
+    const df x = df_div2(df_mul(a.lam2_4, df_mul(F, F)), vq);
+    // 1 / K_a with K_a = -2 v^2 D^3 / (lambda R), D = sqrt(1 - x); then
+    // K_t = -K_a r / (r - K_a) = 1 / (1 / r - 1 / K_a)
+    const df w = df_mul(df_mul(vq, df_pow32_1m(x)), ilr);
+    const df iu = df_div2(df_make(-0.5f, 0.f), w);
+    Knot k;
+    k.dct = df_neg(df_mul(fdc, iu));                          // -f_dc / K_a
+    k.pkt = df_div2(a.pi_, df_add_abs(a.inv_rate, df_neg(iu)));
+    return k;
 }
 
-// Deramp (sgn -1) / re-ramp (sgn +1) phase of azimuth_time_ufr
-// (image_formation.cpp:305-313, 365-373) at time tau between knots i and i+1
-// (fraction al).  With t = dct + tau and K_a dct = -f_dc the reference's
-//   -pi kt t^2 + 2 pi (kt + K_a) dct t
-// equals -[pi kt (tau^2 - dct^2) + 2 pi f_dc (tau + dct)], evaluated here as
-// -(tau + dct) [pi kt (tau - dct) + 2 pi f_dc].
-__device__ __forceinline__ float tufr_phase(const float4* KN, int i, float al, df tau, int sgn, df tpf) {
-    df p0, d0, p1, d1;
-    load_knot(KN, i, p0, d0);
-    load_knot(KN, i + 1, p1, d1);
-    const df pkt = df_add_f(p0, ((p1.hi - p0.hi) + (p1.lo - p0.lo)) * al);
-    const df dct = df_add_f(d0, ((d1.hi - d0.hi) + (d1.lo - d0.lo)) * al);
-    const df a = df_add(tau, dct);
-    const df b = df_sub(tau, dct);
-    const df th = df_mul(a, df_add(df_mul(pkt, b), tpf));
-    return sgn < 0 ? -df_wrap(th) : df_wrap(th);
+// Re-ramp phase of azimuth_time_ufr (image_formation.cpp:365-373) at time tau
+// between two knots (fraction al).  With t = dct + tau and K_a dct = -f_dc
+// the reference's pi kt t^2 - 2 pi (kt + K_a) dct t equals
+// pi kt (tau^2 - dct^2) + 2 pi f_dc (tau + dct), evaluated here as
+// (tau + dct) [pi kt (tau - dct) + 2 pi f_dc]; the deramp phase
+// (image_formation.cpp:305-313) is its negative (DerampPoly).
+__device__ __forceinline__ float reramp_phase(Knot k0, Knot k1, float al, df tau, df tpf) {
+    const df pkt = df_add_f(k0.pkt, ((k1.pkt.hi - k0.pkt.hi) + (k1.pkt.lo - k0.pkt.lo)) * al);
+    const df dct = df_add_f(k0.dct, ((k1.dct.hi - k0.dct.hi) + (k1.dct.lo - k0.dct.lo)) * al);
+    const df a = df_add_abs(tau, dct);
+    const df b = df_add_abs(tau, df_neg(dct));
+    return df_wrap(df_mul(a, df_add_abs(df_mul(pkt, b), tpf)));
 }
 
 // ---- deramp phase of a knot interval as a polynomial in the sample step
 // Over the samples n = n_a + d of one knot interval iv (K_a resampled from
 // knots iv, iv + 1, fraction al = al_a + d (S - 1) / (TS - 1)), pi K_t and
 // -f_dc/K_a are linear in d and so is az_time, and the deramp argument
-// th = (tau + dct) [pi kt (tau - dct) + 2 pi f_dc] (tufr_phase) is the cubic
+// th = (tau + dct) [pi kt (tau - dct) + 2 pi f_dc] (reramp_phase) is the cubic
 //   th(d) = H0 + G1 d + G2 d^2 + (A1 C2 d^3, below 1e-8 rad over an interval)
 // H0 and G1 in double-float, reduced to fractions of a turn in 32-bit fixed
 // point; the phase -th / (2 pi) - n k_s / TS then wraps by integer overflow.
@@ -60,24 +67,11 @@ __device__ __forceinline__ unsigned int turns_fx(df x, df i2p) {
     return (unsigned int)__float2int_rn((t.hi - k) * 4294967296.0f) + (unsigned int)__float2int_rn(t.lo * 4294967296.0f);
 }
 
-// Double-float sum without the second error term (Hida-Li-Bailey's "sloppy"
-// add): its error is below 2^-46 of the larger operand, the absolute
-// accuracy the phases need, at half the operations of df_add.
-__device__ __forceinline__ df df_add_abs(df a, df b) {
-    df s = two_sum(a.hi, b.hi);
-    s.lo = __fadd_rn(s.lo, __fadd_rn(a.lo, b.lo));
-    return quick_two_sum(s.hi, s.lo);
-}
-
-__device__ __forceinline__ DerampPoly deramp_poly(const float4* KN, int iv, float al, df tau, df tpf, df dt, float gk,
-                                                  df i2p) {
-    df p0, d0, p1, d1;
-    load_knot(KN, iv, p0, d0);
-    load_knot(KN, iv + 1, p1, d1);
-    const float dpk = (p1.hi - p0.hi) + (p1.lo - p0.lo);
-    const float ddc = (d1.hi - d0.hi) + (d1.lo - d0.lo);
-    const df P = df_add_f(p0, dpk * al);
-    const df D = df_add_f(d0, ddc * al);
+__device__ __forceinline__ DerampPoly deramp_poly(Knot k0, Knot k1, float al, df tau, df tpf, df dt, float gk, df i2p) {
+    const float dpk = (k1.pkt.hi - k0.pkt.hi) + (k1.pkt.lo - k0.pkt.lo);
+    const float ddc = (k1.dct.hi - k0.dct.hi) + (k1.dct.lo - k0.dct.lo);
+    const df P = df_add_f(k0.pkt, dpk * al);
+    const df D = df_add_f(k0.dct, ddc * al);
     const float Pd = dpk * gk, Dd = ddc * gk;   // per-sample steps of P and D
     const df A0 = df_add_abs(tau, D), B0 = df_add_abs(tau, df_neg(D));
     const df C0 = df_add_abs(df_mul(P, B0), tpf);
@@ -101,28 +95,39 @@ __device__ __forceinline__ DerampPoly deramp_poly(const float4* KN, int iv, floa
 }
 
 // exp(i 2 pi (phase in turns)) at step d of the interval, band shift pm
-__device__ __forceinline__ cf32 deramp_rot(const DerampPoly& p, int d, float d2, unsigned int pm) {
-    const unsigned int ph = p.base + p.slope * (unsigned int)d + (unsigned int)__float2int_rn(p.curv * d2) - pm;
+__device__ __forceinline__ cf32 deramp_rot(unsigned int base, unsigned int slope, float curv, int d, float d2,
+                                           unsigned int pm) {
+    const unsigned int ph = base + slope * (unsigned int)d + (unsigned int)__float2int_rn(curv * d2) - pm;
     float sn, cs;
     __sincosf((float)(int)ph * 1.46291807926715968e-9f, &sn, &cs);   // 2 pi / 2^32
     return mk(cs, sn);
 }
 
-__host__ __device__ __forceinline__ long long floor_div_ll(long long a, long long b) {
-    return a >= 0 ? a / b : -((-a + b - 1) / b);
-}
 // Knot intervals of the TS-point deramp axis (K_a resampled S -> TS,
 // linear_resample): sample u lies in interval floor(u (S - 1) / (TS - 1))
 // (the last sample in interval S - 2), and interval iv starts at
 // ceil(iv (TS - 1) / (S - 1)).  Both from float estimates (within one of the
 // answer for TS < 2^24) corrected with exact integer products, which keeps
 // 64-bit divisions off the sample path.
-__device__ __forceinline__ int knot_of_near(int u, int S, long long TS, float gk) {
+// The interval of sample u and its step from the interval's first sample.
+// The remainder num = u (S - 1) - q (TS - 1) is below 2 TS in magnitude, so
+// 32-bit products that wrap give it exactly; the step is floor(num / (S - 1)).
+__device__ __forceinline__ int knot_of_near(int u, int S, int TS, float gk, float inv_s1, int& d) {
     int q = __float2int_rz((float)u * gk);
-    const long long num = (long long)u * (S - 1);
-    if ((long long)q * (TS - 1) > num) --q;
-    else if ((long long)(q + 1) * (TS - 1) <= num) ++q;
-    return min(q, S - 2);
+    int num = (int)((unsigned int)u * (unsigned int)(S - 1) - (unsigned int)q * (unsigned int)(TS - 1));
+    if (num < 0) {
+        --q;
+        num += TS - 1;
+    } else if (num >= TS - 1) {
+        ++q;
+        num -= TS - 1;
+    }
+    if (q > S - 2) {
+        q = S - 2;
+        num += TS - 1;
+    }
+    d = __float2int_rz(((float)num + 0.5f) * inv_s1);
+    return q;
 }
 __device__ __forceinline__ int knot_first_near(int iv, int S, long long TS, float rt) {
     const long long num = (long long)iv * (TS - 1);
@@ -132,29 +137,53 @@ __device__ __forceinline__ int knot_first_near(int iv, int S, long long TS, floa
     return n;
 }
 
-// Shared memory: one region that holds either the deramped samples of a
-// spreading pass (ychunk, kTufrGroup range bins interleaved) or the grid
-// (padded M) of one range bin's transforms, behind the group's 2 pi f_dc.
-struct TufrLayout {
-    static constexpr int head = 8;   // kTufrGroup double-floats; the region starts 16-byte aligned (read as float4)
-    int grid;
-    __host__ __device__ explicit TufrLayout(const TufrArgs& a) : grid(padded16_len(a.dnu.n)) {}
-    __host__ __device__ size_t floats(const TufrArgs& a) const {
-        return (size_t)head + (size_t)(grid > a.ychunk ? grid : a.ychunk);
-    }
-};
-
-// ex2.approx / sqrt.approx (relative error ~2^-22): the spreading weights
-// need ~1e-6, far looser than the special-function paths would give.
-__device__ __forceinline__ float ex2_approx(float x) {
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+// Deramp polynomials of every knot interval and range bin: a warp forms 32
+// adjacent knots of a bin, each lane the interval to the next one.  Bound by
+// instruction issue (86 % of it; double-float arithmetic, 430 instructions a
+// knot): 1.06 ms for 12000 bins of 6900 knots, 1.67 with df_div / df_sqrt
+// instead of two-digit quotients and series, about 2.4 inside the spreading
+// kernel, between its barriers.
+__global__ void __launch_bounds__(256) k_tufr_knots(TufrArgs a) {
+    if (!a.P->ok) return;
+    const int S = a.S;
+    const int TS = a.P->q.num_tiles * S;
+    const int lane = threadIdx.x & 31;
+    const int iv0 = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 31;
+    if (iv0 >= S - 1) return;
+    const int j = blockIdx.y;
+    const int iv = iv0 + lane;
+    const df fdc = a.fdc[j];
+    const Knot k0 = knot_at(a.rows[min(iv, S - 1)], a.cols[j].Q, fdc, a.inv_lamR[j], a);
+    Knot k1;
+    k1.pkt = df_make(__shfl_down_sync(0xffffffffu, k0.pkt.hi, 1), __shfl_down_sync(0xffffffffu, k0.pkt.lo, 1));
+    k1.dct = df_make(__shfl_down_sync(0xffffffffu, k0.dct.hi, 1), __shfl_down_sync(0xffffffffu, k0.dct.lo, 1));
+    if (lane == 31 || iv >= S - 1) return;
+    const df dt = a.P->dt, dtau = a.P->dtau, tau0 = a.P->tau0;
+    const float gk = a.P->gk;
+    const df i2p = df_from(0.15915494309189533577);
+    const int na = knot_first_near(iv, S, TS, a.P->rt);
+    // knot fraction and az_time of the anchor, as the reference's
+    // linear_resample and linspace give them
+    const float al = (float)(int)((long long)na * (S - 1) - (long long)iv * (TS - 1)) / (float)(TS - 1);
+    const df tau = df_add_abs(tau0, df_mul_f(dtau, (float)na));
+    const DerampPoly p = deramp_poly(k0, k1, al, tau, df_mul(a.two_pi_, fdc), dt, gk, i2p);
+    const long long o = (long long)j * S + iv;
+    a.poly[o] = make_uint2(p.base, p.slope);
+    a.curv[o] = p.curv;
 }
-__device__ __forceinline__ float sqrt_approx(float x) {
-    float y;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
+
+// exp(i re-ramp phase) of every output row and range bin (image_formation.cpp:355-378).
+__global__ void __launch_bounds__(256) k_tufr_ramp(TufrArgs a) {
+    if (!a.P->ok) return;
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= a.n_out) return;
+    const int j = blockIdx.y;
+    const float4 rr = __ldg(a.tab.rer + p);
+    const int ir = __float_as_int(rr.x);
+    const df fdc = a.fdc[j], Q = a.cols[j].Q, ilr = a.inv_lamR[j];
+    const Knot k0 = knot_at(a.rows[ir], Q, fdc, ilr, a), k1 = knot_at(a.rows[ir + 1], Q, fdc, ilr, a);
+    a.ramp[(long long)j * a.n_out + p] =
+        cexpf_fast(reramp_phase(k0, k1, rr.y, df_make(rr.z, rr.w), df_mul(a.two_pi_, fdc)));
 }
 
 // Smallest n with m2 n >= A, and largest n with m2 n <= B (m2 > 0), for
@@ -168,260 +197,198 @@ __device__ __forceinline__ int first_at_or_above(int a, int TS, int m2, float in
     while ((long long)m2 * (n - 1) >= A) --n;
     return n;
 }
-__device__ __forceinline__ int last_at_or_below(int b, int TS, int m2, float inv_m2) {
-    const long long B = (long long)b * TS;
-    int n = (int)floorf((float)b * (float)TS * inv_m2);
-    while ((long long)m2 * n > B) --n;
-    while ((long long)m2 * (n + 1) <= B) ++n;
-    return n;
-}
 
-template <int NT>
-__global__ void __launch_bounds__(NT, NT <= 512 ? 2 : 1) k_tufr_fused(TufrArgs a) {
+// Band of the length-TS DFT (image_formation.cpp:315-333), type-1 non-uniform
+// FFT: spread y[n] exp(-2 pi i n k_s / TS), the deramped tiled line
+// y[s + S t] = A[s] exp(-i deramp(s + S t)), onto the grid (grid point l
+// gathers the samples within W/2 of x_n = n M / TS; n is taken modulo TS).
+//
+// A CTA takes kTufrGroup = 4 range bins and a run of lc grid points: it stages
+// the deramped samples around them in shared memory (two float4 planes, two
+// bins each), then each thread gathers 4 adjacent grid points of all four
+// bins: per sample two 16-byte shared loads, one 16-byte load of the four
+// weights and 32 FMAs.  The weights do not depend on the range bin: a table
+// per burst in the order the threads read it (2.7 MB, from L2).  The threads
+// of a warp take point groups `perm` apart, which puts the 8 lanes of a
+// quarter-warp load on different banks for the sample spacing at hand
+// (perm = 1 put all 8 on one where 4 TS / M is near a multiple of 8).
+// Three CTAs of 128 threads per SM, so one's staging (latency of L2 loads)
+// runs under another's gather (FMA).
+//
+// 12000 bins of 41400 samples onto 10240 points: 2.09 ms (2.72 with one or two
+// samples' loads in flight in the staging instead of three).  The kernel
+// before took two bins and two points per thread, formed each weight from its
+// square root and exponential (special-function bound), and spread,
+// transformed and evaluated in one CTA: 8.75 ms, now 4.37 for the four kernels.
+constexpr int kSpreadThreads = 128;
+
+__global__ void __launch_bounds__(kSpreadThreads, 3) k_tufr_spread(TufrArgs a, int launch_chunks) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int R = kTufrGroup;
-    static_assert(R == 2, "the staged samples are range-bin pairs (16 bytes per sample)");
-    const TufrParams q = a.P->q;
-    const int S = a.S;
+    static_assert(kTufrGroup == 4, "two planes of range-bin pairs");
+    const TufrDev& dev = *a.P;
+    const TufrParams q = dev.q;
     const int T = q.num_tiles;
-    const int M = a.dnu.n;
+    const int S = a.S, M = a.dnu.n;
     const int bw = q.end - q.start;
-    const long long TS = (long long)T * S;
-    // grid points per spreading pass: their samples (at most (L - 1 + W) TS / M + 1
-    // per range bin) fit the staged chunk; two per thread of the block when possible
-    const int cap = a.ychunk / R;
-    const long long lmax = (T >= 1 ? ((long long)(cap - 2) * M) / TS : 0) - kNuW + 1;
-    const int Lc = (int)(lmax >= 2 * NT ? (lmax / (2 * NT)) * (2 * NT) : lmax);   // two grid points per thread
     // outside the launch plan (tile count, band, chunk): flag, do nothing
-    if (!q.ok || T < 1 || T > a.tmax || S < 8 || bw > a.bwmax || 4 * bw > 5 * M || lmax < 1 || TS >= (1LL << 24)) {
+    if (!dev.ok || bw > a.bwmax || dev.chunks > launch_chunks) {
         if (blockIdx.x == 0 && threadIdx.x == 0) *a.status = 1;
         return;
     }
-    const TufrLayout L(a);
-    df* s_tpf = reinterpret_cast<df*>(smem_raw);
-    cf32* big = reinterpret_cast<cf32*>(smem_raw) + L.head;   // grid of one range bin (padded M) ...
-    cf32* ych = big;                       // ... or the staged samples of a pass, range-bin
-                                           // pairs (16 bytes per sample)
-    const int K0 = bw / 2;
-    const long long ks = q.start + K0;     // band centre bin
-    // spreading kernel phi(z) = exp(beta (sqrt(1 - z^2) - 1)), z = 2 (x_n - l) / W
-    const double sigma = (double)M / (double)bw;
-    const float bl2 = (float)(0.97 * 3.141592653589793 * kNuW * (1.0 - 1.0 / (2.0 * sigma)) * 1.4426950408889634);
-    const float zs = (float)(2.0 / ((double)kNuW * (double)TS));
+    const int chunk = blockIdx.x % launch_chunks;
+    if (chunk >= dev.chunks) return;
+    const int j0 = (int)(blockIdx.x / launch_chunks) * kTufrGroup;
+    const int rc = min(kTufrGroup, a.n_r - j0);
+    const int TS = T * S;
     const int m2 = 2 * M;
     const float inv_m2 = 1.0f / (float)m2;
-    // deramp: sample spacing of az_times (linspace over TS), knot-position
-    // step per sample, 1 / (2 pi), and the band shift k_s / TS as a 64-bit
-    // fraction of a turn (floor(2^64 (k_s mod TS) / TS))
-    const df dt = df_from(q.focused_time / (double)(TS - 1));
-    const float gk = (float)((double)(S - 1) / (double)(TS - 1));
-    const df i2p = df_from(0.15915494309189533577);
-    const float inv_s = 1.0f / (float)S;
-    const float rt = (float)((double)(TS - 1) / (double)(S - 1));
-    const double ft = q.focused_time;
-    const double dtau = (ft / 2 - (-ft / 2)) / (double)(TS - 1);   // az_times = linspace(-ft/2, ft/2, TS)
-    const df tau0 = df_from(-ft / 2), dtau_df = df_from(dtau);
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned long long KS64;
+    const int lc = dev.lc, kw = dev.kw;
+    const int l0 = chunk * lc;
+    const int l1 = min(M, l0 + lc);
+    float4* pa = reinterpret_cast<float4*>(smem_raw);
+    float4* pb = pa + a.ycap;
+    // samples nA .. nA + len of the windows of groups l0 .. l1 - 4
+    const int nA = first_at_or_above(2 * l0 - kNuW, TS, m2, inv_m2);
+    const int len = first_at_or_above(2 * (l1 - 4) - kNuW, TS, m2, inv_m2) + kw - nA;
     {
-        const unsigned long long kk = (unsigned long long)(((ks % TS) + TS) % TS);
-        const unsigned long long hi = (kk << 32) / (unsigned long long)TS;
-        const unsigned long long rem = (kk << 32) - hi * (unsigned long long)TS;
-        KS64 = (hi << 32) | ((rem << 32) / (unsigned long long)TS);
-    }
-    float4* KNg = reinterpret_cast<float4*>(a.KN) + (long long)blockIdx.x * R * S;
-    cf32* Gg = a.G + (long long)blockIdx.x * R * M;
-    for (int j0 = blockIdx.x * R; j0 < a.n_r; j0 += gridDim.x * R) {
-        const int rc = min(R, a.n_r - j0);
-        // 1. the azimuth IFFT (length S, 1/S, s1_decoder.cpp:682) ran in k_czt_rows
-        // 2. knots: pi K_t and -f_dc/K_a at the S azimuth rows of each range bin
-        for (int r = 0; r < rc; ++r) {
-            const int j = j0 + r;
-            const ColDf cj = a.cols[j];
-            const df fdc = a.fdc[j];
-            const df ilr = a.inv_lamR[j];
-            float4* KN = KNg + (long long)r * S;
-            for (int s = threadIdx.x; s < S; s += blockDim.x) {
-                const RowDf rw = a.rows[s];
-                const df F = df_add(rw.fa, fdc);
-                const df vq = df_mul(rw.P, df_sub(rw.A, cj.Q));
-                const df x = df_div(df_mul(a.lam2_4, df_mul(F, F)), vq);
-                const df D = df_sqrt(df_sub(df_make(1.f, 0.f), x));
-                const df D3 = df_mul(D, df_mul(D, D));
-                const df u = df_neg(df_mul(df_mul(df_mul(df_make(2.f, 0.f), vq), D3), ilr));   // K_a = -2 v^2 D^3/(lambda R)
-                const df kt = df_neg(df_div(df_mul(u, a.rate), df_sub(a.rate, u)));              // -K_a r / (r - K_a)
-                const df dct = df_neg(df_div(fdc, u));                                          // -f_dc / K_a
-                const df pkt = df_mul(a.pi_, kt);
-                KN[s] = make_float4(pkt.hi, pkt.lo, dct.hi, dct.lo);
-            }
-            if (threadIdx.x == 0) s_tpf[r] = df_mul(a.two_pi_, fdc);
-        }
-        __syncthreads();
-        // 3. band of the length-TS DFT (image_formation.cpp:315-333), type-1
-        //    non-uniform FFT: spread y[n] exp(-2 pi i n k_s / TS), the deramped
-        //    tiled line y[s + S t] = A[s] exp(-i deramp(s + S t)), onto the grid
-        //    (grid point l gathers the samples within W/2 of x_n = n M / TS;
-        //    n is taken modulo TS), in passes of Lc grid points, R range bins
-        //    per pass sharing each kernel weight
-        for (int l0 = 0; l0 < M; l0 += Lc) {
-            const int l1 = min(M, l0 + Lc);
-            const int nA = first_at_or_above(2 * l0 - kNuW, (int)TS, m2, inv_m2);
-            const int nB = last_at_or_below(2 * (l1 - 1) + kNuW, (int)TS, m2, inv_m2);
-            // Deramped samples of the pass.  The deramp phase is a cubic in
-            // the sample step over each knot interval (the ~T consecutive
-            // samples whose K_a comes from knots iv, iv + 1): a warp takes a
-            // share of the samples, each lane anchors one interval in
-            // double-float (deramp_poly), and the lanes then take the samples
-            // in runs of 32 (coalesced loads and stores), fetching their
-            // interval's anchor by shuffle and evaluating the phase in 32-bit
-            // fixed-point turns; the band shift n k_s / TS in 64-bit fixed point.
-            for (long long k = floor_div_ll(nA, TS); k <= floor_div_ll(nB, TS); ++k) {
-                const int u0 = (int)max((long long)nA - k * TS, 0LL);
-                const int u1 = (int)min((long long)nB - k * TS, TS - 1);
-                const int posoff = (int)(k * TS - nA);   // staged position of sample u: u + posoff
-                const int len = u1 - u0 + 1;
-                const int wlo = u0 + (int)((long long)len * warp / (NT / 32));
-                const int whi = u0 + (int)((long long)len * (warp + 1) / (NT / 32)) - 1;
-                int nstart = wlo;
-                int ivw = knot_of_near(wlo, S, TS, gk);
-                const int ivlast = knot_of_near(whi, S, TS, gk);
-                const cf32* in0 = a.in + (long long)j0 * S;
-                const cf32* in1 = in0 + (rc > 1 ? S : 0);
-                while (nstart <= whi) {   // warp-uniform: up to 32 intervals per round
-                    const int ive = min(ivw + 31, ivlast);
-                    const int nend = min(whi, ive == S - 2 ? (int)TS - 1 : knot_first_near(ive + 1, S, TS, rt) - 1);
-                    // the first run's samples are loaded before the anchors
-                    int n = min(nstart + lane, nend);
-                    int si = n - S * __float2int_rz((float)n * inv_s);
-                    if (si < 0) si += S;
-                    else if (si >= S) si -= S;
-                    cf32 v0 = in0[si], v1 = in1[si];
-                    const int iv = ivw + lane;
-                    int na = nstart;
-                    DerampPoly p0 = {0u, 0u, 0.f}, p1 = {0u, 0u, 0.f};
-                    if (iv <= ive) {
-                        na = max(nstart, knot_first_near(iv, S, TS, rt));
-                        // knot fraction and az_time of the anchor, as the
-                        // reference's linear_resample and linspace give them
-                        const float al = (float)(int)((long long)na * (S - 1) - (long long)iv * (TS - 1)) / (float)(TS - 1);
-                        const df taua = df_add(tau0, df_mul_f(dtau_df, (float)na));
-                        p0 = deramp_poly(KNg, iv, al, taua, s_tpf[0], dt, gk, i2p);
-                        if (rc > 1) p1 = deramp_poly(KNg + S, iv, al, taua, s_tpf[1], dt, gk, i2p);
-                    }
-                    for (int n0 = nstart; n0 <= nend; n0 += 32) {
-                        // next run's samples in flight while this one is evaluated
-                        const int nn = min(n0 + 32 + lane, nend);
-                        int sn = nn - S * __float2int_rz((float)nn * inv_s);
-                        if (sn < 0) sn += S;
-                        else if (sn >= S) sn -= S;
-                        cf32 w0 = mk(0.f, 0.f), w1 = w0;
-                        if (n0 + 32 <= nend) {
-                            w0 = in0[sn];
-                            w1 = in1[sn];
-                        }
-                        const int src = knot_of_near(n, S, TS, gk) - ivw;
-                        const unsigned int b0 = __shfl_sync(0xffffffffu, p0.base, src);
-                        const unsigned int s0 = __shfl_sync(0xffffffffu, p0.slope, src);
-                        const float c0 = __shfl_sync(0xffffffffu, p0.curv, src);
-                        const unsigned int b1 = __shfl_sync(0xffffffffu, p1.base, src);
-                        const unsigned int s1 = __shfl_sync(0xffffffffu, p1.slope, src);
-                        const float c1 = __shfl_sync(0xffffffffu, p1.curv, src);
-                        const int d = n - __shfl_sync(0xffffffffu, na, src);
-                        if (n0 + lane <= nend) {
-                            const unsigned int pm = (unsigned int)(((unsigned long long)n * KS64) >> 32);
-                            const float d2 = (float)(d * d);
-                            const cf32 e0 = deramp_rot({b0, s0, c0}, d, d2, pm);
-                            float4 o;
-                            o.x = v0.x * e0.x - v0.y * e0.y;
-                            o.y = v0.x * e0.y + v0.y * e0.x;
-                            o.z = 0.f;
-                            o.w = 0.f;
-                            if (rc > 1) {
-                                const cf32 e1 = deramp_rot({b1, s1, c1}, d, d2, pm);
-                                o.z = v1.x * e1.x - v1.y * e1.y;
-                                o.w = v1.x * e1.y + v1.y * e1.x;
-                            }
-                            reinterpret_cast<float4*>(ych)[n + posoff] = o;
-                        }
-                        n = nn;
-                        v0 = w0;
-                        v1 = w1;
-                    }
-                    nstart = nend + 1;
-                    ivw = ive + 1;
-                }
-            }
-            __syncthreads();
-            // a thread takes two adjacent grid points and reads each sample of
-            // their joint window once (16 bytes: both range bins); lanes'
-            // windows start ~2 TS / M samples apart, so a quarter-warp's loads
-            // fall in distinct bank quads
-            const float4* y01 = reinterpret_cast<const float4*>(ych);
-            for (int pi = threadIdx.x; 2 * pi < l1 - l0; pi += NT) {
-                const int l = l0 + 2 * pi;
-                const bool two = l + 1 < l1;
-                const int lo = first_at_or_above(2 * l - kNuW, (int)TS, m2, inv_m2);
-                const int hi = last_at_or_below(2 * (two ? l + 1 : l) + kNuW, (int)TS, m2, inv_m2);
-                int num = (int)((long long)lo * M - (long long)l * TS);   // (x_n - l) TS, |.| <= W TS / 2 + TS
-                const float4* p01 = y01 + (lo - nA);
-                float4 aa = make_float4(0.f, 0.f, 0.f, 0.f), ab = aa;
-                for (int n = 0; n <= hi - lo; ++n) {
-                    const float za = (float)num * zs;
-                    const float zb = (float)(num - (int)TS) * zs;
-                    // outside the support (|z| >= 1) the weight is exp(-beta)
-                    // (~4e-11 of the peak) instead of 0: a few window-edge samples
-                    const float wa = ex2_approx(fmaf(bl2, sqrt_approx(fmaxf(fmaf(-za, za, 1.0f), 0.f)), -bl2));
-                    const float wb = ex2_approx(fmaf(bl2, sqrt_approx(fmaxf(fmaf(-zb, zb, 1.0f), 0.f)), -bl2));
-                    const float4 v = p01[n];
-                    aa.x = fmaf(wa, v.x, aa.x);
-                    aa.y = fmaf(wa, v.y, aa.y);
-                    aa.z = fmaf(wa, v.z, aa.z);
-                    aa.w = fmaf(wa, v.w, aa.w);
-                    ab.x = fmaf(wb, v.x, ab.x);
-                    ab.y = fmaf(wb, v.y, ab.y);
-                    ab.z = fmaf(wb, v.z, ab.z);
-                    ab.w = fmaf(wb, v.w, ab.w);
-                    num += M;
-                }
-                Gg[l] = mk(aa.x, aa.y);
-                if (rc > 1) Gg[M + l] = mk(aa.z, aa.w);
-                if (two) {
-                    Gg[l + 1] = mk(ab.x, ab.y);
-                    if (rc > 1) Gg[M + l + 1] = mk(ab.z, ab.w);
-                }
-            }
-            __syncthreads();
-        }
-        for (int r = 0; r < rc; ++r) {
-            const float4* KN = KNg + (long long)r * S;
-            const df tpf = s_tpf[r];
-            // grid FFT; bin p holds Z[K0 + p] Phi(p / M) on the band.
-            // 4. band mask and both deconvolutions, then the inverse grid FFT of
-            //    the type-2 evaluation, back into the grid
-            const cf32* G = Gg + (long long)r * M;
-            fft4_head(big, a.dnu, [&](int l) { return G[l]; });
-            fft4_mid(big, a.dnu, [&](int m, cf32 v) { return v * __ldg(a.tab.band + m); });
-            fft4_tail(big, a.dnu, [&](int l, cf32 v) { big[pad16(l)] = v; });
-            __syncthreads();
-            // 5. kNuTaps-tap interpolation (weights fold the Lagrange stencil, the
-            //    centring phase and 1/TS), re-ramp (image_formation.cpp:355-378),
-            //    store the cropped rows
-            cf32* out = a.out + (long long)(j0 + r) * a.n_out;
-            for (int p = threadIdx.x; p < a.n_out; p += blockDim.x) {
-                int l = __ldg(a.tab.nu_l0 + p) % M;
-                if (l < 0) l += M;
-                const cf32* w = a.tab.nu_w + p;   // tap t at w[t n_out]: lanes read consecutive words
-                cf32 acc = mk(0.f, 0.f);
+        const float gk = dev.gk;
+        const float inv_s = 1.0f / (float)S, inv_s1 = 1.0f / (float)(S - 1);
+        const unsigned long long KS64 = dev.ks64;
+        const cf32* in[kTufrGroup];
+        const uint2* po[kTufrGroup];
+        const float* cu[kTufrGroup];
 #pragma unroll
-                for (int t = 0; t < kNuTaps; ++t) {
-                    acc = acc + big[pad16(l)] * ldg(w + (long long)t * a.n_out);
-                    if (++l == M) l = 0;
-                }
-                const float4 rr = __ldg(a.tab.rer + p);
-                out[p] = acc * cexpf_fast(tufr_phase(KN, __float_as_int(rr.x), rr.y, df_make(rr.z, rr.w), +1, tpf));
-            }
-            __syncthreads();
+        for (int r = 0; r < kTufrGroup; ++r) {
+            const long long o = (long long)(j0 + min(r, rc - 1)) * S;
+            in[r] = a.in + o;
+            po[r] = a.poly + o;
+            cu[r] = a.curv + o;
         }
+        // kBatch samples' loads in flight before the first is used
+        constexpr int kBatch = 3;
+        for (int i0 = threadIdx.x; i0 < len; i0 += kBatch * kSpreadThreads) {
+            cf32 v[kBatch][kTufrGroup];
+            uint2 p[kBatch][kTufrGroup];
+            float c[kBatch][kTufrGroup];
+            unsigned int pm[kBatch];
+            int d[kBatch];
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                int u = nA + min(i0 + b * kSpreadThreads, len - 1);
+                while (u < 0) u += TS;
+                while (u >= TS) u -= TS;
+                int si = u - S * __float2int_rz((float)u * inv_s);
+                if (si < 0) si += S;
+                else if (si >= S) si -= S;
+                const unsigned int iv = knot_of_near(u, S, TS, gk, inv_s1, d[b]);
+                pm[b] = (unsigned int)(((unsigned long long)u * KS64) >> 32);
+#pragma unroll
+                for (int r = 0; r < kTufrGroup; ++r) {
+                    v[b][r] = ldg(in[r] + (unsigned int)si);
+                    p[b][r] = __ldg(po[r] + iv);
+                    c[b][r] = __ldg(cu[r] + iv);
+                }
+            }
+#pragma unroll
+            for (int b = 0; b < kBatch; ++b) {
+                const int i = i0 + b * kSpreadThreads;
+                const float d2 = (float)(d[b] * d[b]);
+                cf32 o[kTufrGroup];
+#pragma unroll
+                for (int r = 0; r < kTufrGroup; ++r)
+                    o[r] = v[b][r] * deramp_rot(p[b][r].x, p[b][r].y, c[b][r], d[b], d2, pm[b]);
+                if (i < len) {
+                    pa[i] = make_float4(o[0].x, o[0].y, o[1].x, o[1].y);
+                    pb[i] = make_float4(o[2].x, o[2].y, o[3].x, o[3].y);
+                }
+            }
+        }
+    }
+    __syncthreads();
+    const int ng = lc >> 2;
+    const int l = l0 + 4 * (int)((unsigned int)(threadIdx.x * dev.perm) % (unsigned int)ng);
+    if (threadIdx.x >= ng || l >= M) return;
+    const int lo = first_at_or_above(2 * l - kNuW, TS, m2, inv_m2) - nA;
+    const float4* wt = a.tab.wt + (long long)chunk * kw * kSpreadThreads + threadIdx.x;
+    float4 g[4][2];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) g[c][0] = g[c][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto step = [&](int k, float4 w) {
+        const float4 x = pa[lo + k], y = pb[lo + k];
+        const float wc[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            g[c][0].x = fmaf(wc[c], x.x, g[c][0].x);
+            g[c][0].y = fmaf(wc[c], x.y, g[c][0].y);
+            g[c][0].z = fmaf(wc[c], x.z, g[c][0].z);
+            g[c][0].w = fmaf(wc[c], x.w, g[c][0].w);
+            g[c][1].x = fmaf(wc[c], y.x, g[c][1].x);
+            g[c][1].y = fmaf(wc[c], y.y, g[c][1].y);
+            g[c][1].z = fmaf(wc[c], y.z, g[c][1].z);
+            g[c][1].w = fmaf(wc[c], y.w, g[c][1].w);
+        }
+    };
+    // the next four weights are on their way while four are used (the table
+    // is four entries of a row longer than it is read)
+    float4 w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __ldg(wt + i * kSpreadThreads);
+    int k = 0;
+    for (; k + 4 <= kw; k += 4) {
+        float4 nx[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) nx[i] = __ldg(wt + (k + 4 + i) * kSpreadThreads);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) step(k + i, w[i]);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = nx[i];
+    }
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (k + i < kw) step(k + i, w[i]);
+#pragma unroll
+    for (int r = 0; r < kTufrGroup; ++r) {
+        if (r >= rc) break;
+        float4* o = reinterpret_cast<float4*>(a.G + (long long)(j0 + r) * M + l);
+        const int h = r >> 1;
+        if (r & 1) {
+            o[0] = make_float4(g[0][h].z, g[0][h].w, g[1][h].z, g[1][h].w);
+            o[1] = make_float4(g[2][h].z, g[2][h].w, g[3][h].z, g[3][h].w);
+        } else {
+            o[0] = make_float4(g[0][h].x, g[0][h].y, g[1][h].x, g[1][h].y);
+            o[1] = make_float4(g[2][h].x, g[2][h].y, g[3][h].x, g[3][h].y);
+        }
+    }
+}
+
+// Grid FFT of a range bin (bin p then holds Z[K0 + p] Phi(p / M) on the band),
+// band mask and both deconvolutions, inverse grid FFT of the type-2
+// evaluation, kNuTaps-tap interpolation at the output rows (weights fold the
+// Lagrange stencil, the centring phase and 1/TS) and the re-ramp.
+template <int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_tufr_grid(TufrArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (!a.P->ok) return;
+    cf32* buf = reinterpret_cast<cf32*>(smem_raw);
+    const int M = a.dnu.n;
+    const cf32* G = a.G + (long long)blockIdx.x * M;
+    fft4_head(buf, a.dnu, [&](int l) { return ldg(G + l); });
+    fft4_mid(buf, a.dnu, [&](int m, cf32 v) { return v * __ldg(a.tab.band + m); });
+    fft4_tail(buf, a.dnu, [&](int l, cf32 v) { buf[pad16(l)] = v; });
+    __syncthreads();
+    cf32* out = a.out + (long long)blockIdx.x * a.n_out;
+    const cf32* ramp = a.ramp + (long long)blockIdx.x * a.n_out;
+    for (int p = threadIdx.x; p < a.n_out; p += NT) {
+        int l = __ldg(a.tab.nu_l0 + p) % M;
+        if (l < 0) l += M;
+        const cf32* w = a.tab.nu_w + p;   // tap t at w[t n_out]: lanes read consecutive words
+        cf32 acc = mk(0.f, 0.f);
+#pragma unroll
+        for (int t = 0; t < kNuTaps; ++t) {
+            acc = acc + buf[pad16(l)] * ldg(w + (long long)t * a.n_out);
+            if (++l == M) l = 0;
+        }
+        out[p] = acc * ldg(ramp + p);
     }
 }
 
@@ -442,11 +409,39 @@ __device__ double nu_kernel_ft(double xi, double beta, const double* gx, const d
 }
 
 // Per-burst tables of the time unfolding (see TufrTables), one thread per entry.
-__global__ void k_tufr_tables(const TufrDev* __restrict__ P, int S, int n_out, int s0, int M,
-                              const int* __restrict__ mid, TufrTables t) {
+// Band mask / Phi(p / M)^2 at the grid bins, a warp per bin: Phi by the
+// Gauss-Legendre rule, whose nodes come in pairs +-x (two pairs per lane).
+__global__ void __launch_bounds__(256) k_tufr_band(const TufrDev* __restrict__ P, int M, const int* __restrict__ mid,
+                                                   TufrTables t) {
+    if (!P->ok) return;
+    const int p = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (p >= M) return;
+    const int bw = P->q.end - P->q.start;
+    const int K0 = bw / 2;
+    if (!(p < bw - K0 || p >= M - K0)) {
+        if (lane == 0) t.band[mid[p]] = 0.0f;
+        return;
+    }
+    // oversampling M / bw >= 1.25 and the kernel's beta for it
+    const double sigma = (double)M / (double)bw;
+    const double beta = 0.97 * 3.141592653589793 * kNuW * (1.0 - 1.0 / (2.0 * sigma));
+    const double xi = (double)(p < bw - K0 ? p : p - M) / (double)M;
+    double acc = 0.0;
+    for (int q = lane; q < kNuQuad / 2; q += 32) {
+        const double tq = 0.5 * kNuW * t.gl_x[q];
+        acc += 2.0 * t.gl_w[q] * nu_kernel(tq, beta) * cospi(2.0 * xi * tq);
+    }
+    for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+    if (lane == 0) {
+        const double inv_phi = 1.0 / (0.5 * kNuW * acc);
+        t.band[mid[p]] = (float)(inv_phi * inv_phi);
+    }
+}
+
+__global__ void k_tufr_tables(const TufrDev* __restrict__ P, int S, int n_out, int s0, int M, TufrTables t) {
     const TufrParams q = P->q;
     const int T = q.num_tiles;
-    if (!q.ok || T < 1) return;
+    if (!P->ok) return;
     const long long TS = (long long)T * S;
     const double ft = q.focused_time;
     const int bw = q.end - q.start;
@@ -456,27 +451,6 @@ __global__ void k_tufr_tables(const TufrDev* __restrict__ P, int S, int n_out, i
     const double beta = 0.97 * 3.141592653589793 * kNuW * (1.0 - 1.0 / (2.0 * sigma));
     const long long stride = (long long)gridDim.x * blockDim.x;
     const long long tid = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    // band mask / Phi(p / M)^2 at the grid bins (FFT order), Phi by the
-    // Gauss-Legendre rule of nu_kernel_ft with the kernel values at the nodes
-    // (which do not depend on the bin) formed once per block
-    __shared__ double kq[kNuQuad], tq[kNuQuad];
-    for (int q = threadIdx.x; q < kNuQuad; q += blockDim.x) {
-        tq[q] = 0.5 * kNuW * t.gl_x[q];
-        kq[q] = t.gl_w[q] * nu_kernel(tq[q], beta);
-    }
-    __syncthreads();
-    for (long long p = tid; p < M; p += stride) {
-        const bool in_band = p < bw - K0 || p >= M - K0;
-        if (!in_band) {
-            t.band[mid[p]] = 0.0f;
-            continue;
-        }
-        const double xi = (double)(p < bw - K0 ? p : p - M) / (double)M;
-        double acc = 0.0;
-        for (int q = 0; q < kNuQuad; ++q) acc += kq[q] * cospi(2.0 * xi * tq[q]);
-        const double inv_phi = 1.0 / (0.5 * kNuW * acc);
-        t.band[mid[p]] = (float)(inv_phi * inv_phi);
-    }
     for (long long p = tid; p < n_out; p += stride) {
         const long long qo = s0 + p;
         // quadratic resampling TS -> down: stencil n = i-1, i, i+1 (signal_processing.cpp:109-155)
@@ -523,74 +497,85 @@ __global__ void k_tufr_tables(const TufrDev* __restrict__ P, int S, int n_out, i
     }
 }
 
-void tufr_tables(const TufrArgs& a, cudaStream_t st) {
-    const long long n = std::max<long long>((long long)a.tmax * a.S, a.dnu.n);
-    const int grid = (int)std::min<long long>((n + 255) / 256, 152 * 8);
-    note_launch(), k_tufr_tables<<<grid, 256, 0, st>>>(a.P, a.S, a.n_out, a.s0, a.dnu.n, a.dnu.mid, a.tab);
-}
 
-// Staged-sample region (kTufrGroup range bins interleaved): what is left of
-// two CTAs' shared memory per SM after the head and twiddles, when that also
-// holds the grid and at least 1024 samples per range bin (checked with the
-// occupancy calculator), else of one CTA's.
-template <class K>
-static bool fits_two(K kernel, int threads, size_t smem) {
-    allow_smem(kernel);
-    int nb = 0;
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, threads, smem) == cudaSuccess && nb >= 2;
-}
-
-// Two CTAs of 384 threads per SM (85 registers a thread; 512-thread CTAs at
-// 64 registers spilled and ran 4 % slower), else one of 1024.
-constexpr int kTufrThreads = 384;
-
-static int tufr_chunk(const TufrArgs& a, bool& two) {
-    TufrArgs b = a;
-    b.ychunk = 0;
-    const TufrLayout L(b);
-    static std::mutex mu;
-    static std::map<int, std::pair<int, bool>> memo;   // grid length -> (chunk, two per SM)
-    std::lock_guard<std::mutex> lk(mu);
-    auto it = memo.find(a.dnu.n);
-    if (it != memo.end()) {
-        two = it->second.second;
-        return it->second.first;
-    }
-    const long long fixed = L.head;
-    long long cap = (114LL * 1024 - 1024) / (long long)sizeof(cf32) - fixed;
-    cap -= cap % 16;
-    two = false;
-    for (; cap >= L.grid && cap >= 1024LL * kTufrGroup; cap -= 16)
-        if (fits_two(k_tufr_fused<kTufrThreads>, kTufrThreads, sizeof(cf32) * (size_t)(fixed + cap))) {
-            two = true;
-            break;
+// Spreading weights in the order k_tufr_spread reads them: entry
+// [chunk][k][thread] holds the weights of the thread's sample k for its four
+// grid points (0 outside the kernel's support).
+__global__ void k_tufr_weights(const TufrDev* __restrict__ P, int S, int M, float4* __restrict__ wt) {
+    const TufrDev& dev = *P;
+    if (!dev.ok) return;
+    const long long TS = (long long)dev.q.num_tiles * S;
+    const double sigma = (double)M / (double)(dev.q.end - dev.q.start);
+    const double beta = 0.97 * 3.141592653589793 * kNuW * (1.0 - 1.0 / (2.0 * sigma));
+    const int ng = dev.lc >> 2;
+    const double zs = 2.0 / ((double)kNuW * (double)TS);
+    const long long total = (long long)dev.chunks * dev.kw * kSpreadThreads;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < total; e += (long long)gridDim.x * blockDim.x) {
+        const int t = (int)(e % kSpreadThreads);
+        const int k = (int)(e / kSpreadThreads % dev.kw);
+        const int chunk = (int)(e / kSpreadThreads / dev.kw);
+        const long long l = (long long)chunk * dev.lc + 4 * (int)((unsigned int)(t * dev.perm) % (unsigned int)ng);
+        const long long num0 = (2 * l - kNuW) * TS, den = 2LL * M;
+        const long long lo = num0 >= 0 ? (num0 + den - 1) / den : -((-num0) / den);   // ceil
+        float w[4];
+        for (int c = 0; c < 4; ++c) {
+            const double z = (double)((lo + k) * M - (l + c) * TS) * zs;
+            w[c] = fabs(z) < 1.0 ? (float)exp(beta * (sqrt(1.0 - z * z) - 1.0)) : 0.0f;
         }
-    if (!two) cap = (long long)kFft4SmemBytes / (long long)sizeof(cf32) - fixed;
-    if (cap < L.grid || cap < 512LL * kTufrGroup) throw std::runtime_error("time unfolding: shared memory");
-    const int chunk = (int)(cap / 2 * 2);
-    memo[a.dnu.n] = {chunk, two};
-    return chunk;
-}
-
-int tufr_ctas_per_sm(const TufrArgs& a) {
-    bool two = false;
-    tufr_chunk(a, two);
-    return two ? 2 : 1;
-}
-
-void tufr_fused(const TufrArgs& args, int grid, cudaStream_t st) {
-    TufrArgs a = args;
-    bool two = false;
-    a.ychunk = tufr_chunk(a, two);
-    const size_t smem = sizeof(cf32) * TufrLayout(a).floats(a);
-    if (smem > (size_t)kFft4SmemBytes) throw std::runtime_error("time unfolding: shared memory");
-    if (two) {
-        allow_smem(k_tufr_fused<kTufrThreads>);
-        note_launch(), k_tufr_fused<kTufrThreads><<<grid, kTufrThreads, smem, st>>>(a);
-    } else {
-        allow_smem(k_tufr_fused<1024>);
-        note_launch(), k_tufr_fused<1024><<<grid, 1024, smem, st>>>(a);
+        wt[e] = make_float4(w[0], w[1], w[2], w[3]);
     }
+}
+
+// Samples a spreading CTA can hold (two float4 each) with three CTAs per SM;
+// where a group of four grid points alone spans more (tile counts far above
+// the band's, no burst of the IW geometry), what one CTA can.
+static int spread_cap(int S, int tmax, int M) {
+    const double ratio = (double)tmax * S / M;
+    return (kNuW + 3) * ratio * 4 < 2392 ? 2392 : (kFft4SmemBytes - 1024) / 32;
+}
+// Upper bounds of the chunk count and of the weight table for any tile count
+// up to tmax (the device picks the chunk length from its own).
+static int spread_chunks(int S, int tmax, int M, int cap) {
+    int most = 0;
+    for (int T = 1; T <= tmax; ++T) {
+        const TufrSplit sp = tufr_split((long long)T * S, M, cap);
+        most = std::max(most, sp.lc >= 4 ? sp.chunks : 0);
+    }
+    return std::max(most, 1);
+}
+TufrLaunch tufr_launch(int S, int tmax, int M) {
+    TufrLaunch L;
+    L.ycap = spread_cap(S, tmax, M);
+    L.chunks = spread_chunks(S, tmax, M, L.ycap);
+    L.weights = 0;
+    for (int T = 1; T <= tmax; ++T) {
+        const TufrSplit sp = tufr_split((long long)T * S, M, L.ycap);
+        if (sp.lc >= 4) L.weights = std::max<long long>(L.weights, (long long)sp.chunks * sp.kw * kSpreadThreads);
+    }
+    L.weights = std::max<long long>(L.weights, 1) + 8 * kSpreadThreads;   // read ahead
+    return L;
+}
+
+void tufr_tables(const TufrArgs& a, cudaStream_t st) {
+    note_launch(), k_tufr_band<<<(a.dnu.n + 7) / 8, 256, 0, st>>>(a.P, a.dnu.n, a.dnu.mid, a.tab);
+    note_launch(), k_tufr_tables<<<(a.n_out + 63) / 64, 64, 0, st>>>(a.P, a.S, a.n_out, a.s0, a.dnu.n, a.tab);
+    note_launch(), k_tufr_weights<<<152 * 8, 256, 0, st>>>(a.P, a.S, a.dnu.n, a.tab.wt);
+}
+
+void tufr_fused(const TufrArgs& a, const TufrLaunch& L, cudaStream_t st) {
+    const dim3 gk((a.S - 1 + 31 * 8 - 1) / (31 * 8), a.n_r);
+    note_launch(), k_tufr_knots<<<gk, 256, 0, st>>>(a);
+    note_launch(), k_tufr_ramp<<<dim3((a.n_out + 255) / 256, a.n_r), 256, 0, st>>>(a);
+    const size_t sm = sizeof(float4) * 2 * (size_t)L.ycap;
+    allow_smem(k_tufr_spread);
+    const long long blocks = (long long)((a.n_r + kTufrGroup - 1) / kTufrGroup) * L.chunks;
+    note_launch(), k_tufr_spread<<<(unsigned)blocks, kSpreadThreads, sm, st>>>(a, L.chunks);
+    const size_t smem = fft4_smem(a.dnu.n);
+    fft4_launch(smem, [&](auto nt, auto mb) {
+        auto kernel = k_tufr_grid<decltype(nt)::value, decltype(mb)::value>;
+        allow_smem(kernel);
+        note_launch(), kernel<<<a.n_r, decltype(nt)::value, smem, st>>>(a);
+    });
 }
 
 // Scalars of azimuth_time_ufr (tile count, band, output crop), FP64, one block.
@@ -618,7 +603,7 @@ __global__ void k_ka_row0(const RowParam* rows, const double* slant, const doubl
 
 __global__ void k_tufr_params_fast(const RowParam* rows, const double* slant, const double* f_dc, int S, int n_r,
                                    double rate, double T, double prf, double bd, int swath_number,
-                                   const double* ka0, TufrDev* out) {
+                                   const double* ka0, int M, int ycap, int tmax, TufrDev* out) {
     __shared__ double part[256];
     // ordered blocked sum of K_a over the first range bin (contiguous runs per thread)
     const int per = (S + blockDim.x - 1) / blockDim.x;
@@ -654,14 +639,62 @@ __global__ void k_tufr_params_fast(const RowParam* rows, const double* slant, co
     q.start = (int)(mid - q.bandwidth / 2);
     q.end = (int)(mid + q.bandwidth / 2);
     q.ok = (q.num_tiles >= 1 && q.num_tiles <= 64 && q.start >= 0 && q.end <= q.shape && q.down >= 3) ? 1 : 0;
+    // spreading split and the checks of the launch plan that need the tile count
+    d.ok = 0;
+    const long long TS = (long long)q.num_tiles * S;
+    const int bw = q.end - q.start;
+    if (q.ok && q.num_tiles <= tmax && S >= 8 && TS < (1LL << 24) && 5LL * bw <= 4LL * M) {
+        const TufrSplit sp = tufr_split(TS, M, ycap);
+        d.lc = sp.lc;
+        d.kw = sp.kw;
+        d.chunks = sp.chunks;
+        d.perm = 1;
+        // az_times = linspace(-ft/2, ft/2, TS): first time, step, sample
+        // spacing; knot positions per sample and samples per knot
+        const double f = q.focused_time;
+        d.tau0 = df_from(-f / 2);
+        d.dtau = df_from((f / 2 - (-f / 2)) / (double)(TS - 1));
+        d.dt = df_from(f / (double)(TS - 1));
+        d.gk = (float)((double)(S - 1) / (double)(TS - 1));
+        d.rt = (float)((double)(TS - 1) / (double)(S - 1));
+        // band shift k_s / TS (k_s the band centre bin) as a 64-bit fraction of a turn
+        const unsigned long long kk = (unsigned long long)((((long long)q.start + bw / 2) % TS + TS) % TS);
+        const unsigned long long hi = (kk << 32) / (unsigned long long)TS;
+        const unsigned long long rem = (kk << 32) - hi * (unsigned long long)TS;
+        d.ks64 = (hi << 32) | ((rem << 32) / (unsigned long long)TS);
+        if (sp.lc >= 4) {
+            d.ok = 1;
+            // groups this far apart put the 16-byte loads of 8 lanes on
+            // different bank quads, as far as their sample spacing allows
+            const double step = 4.0 * (double)TS / (double)M;
+            const int ng = sp.lc / 4;
+            int best = 1 << 30;
+            for (int D = 1; D < 16; ++D) {
+                int x = D, y = ng;
+                while (y) { const int r = x % y; x = y; y = r; }
+                if (x != 1) continue;
+                int cost = 0;
+                for (int f = 0; f < 4; ++f) {
+                    int hit[8] = {0, 0, 0, 0, 0, 0, 0, 0}, worst = 0;
+                    for (int i = 0; i < 8; ++i) worst = max(worst, ++hit[(long long)(step * D * i + 0.25 * f) & 7]);
+                    cost += worst;
+                }
+                if (cost < best) {
+                    best = cost;
+                    d.perm = D;
+                }
+            }
+        }
+    }
     *out = d;
 }
 
 void tufr_params_fast(const RowParam* rows, const double* slant, const double* f_dc, int S, int n_r, double rate,
-                      double T, double prf, double bd, int swath_number, double* ka0, TufrDev* out, cudaStream_t st) {
+                      double T, double prf, double bd, int swath_number, double* ka0, int M, int ycap, int tmax,
+                      TufrDev* out, cudaStream_t st) {
     note_launch(), k_ka_row0<<<(S + 127) / 128, 128, 0, st>>>(rows, slant, f_dc, S, ka0);
     note_launch(), k_tufr_params_fast<<<1, 256, 0, st>>>(rows, slant, f_dc, S, n_r, rate, T, prf, bd, swath_number,
-                                                        ka0, out);
+                                                        ka0, M, ycap, tmax, out);
 }
 
 }  // namespace s1g
