@@ -95,7 +95,7 @@ struct s1g_decoder {
     IndexScratch isc;
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
-    Buf bFdf, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
+    Buf bFdf, bFit, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
     Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
     Buf bTuD, bTuG, bTuI, bTuW, bTuR, bTuWt, bTuRamp, bKa0;   // time-unfolding per-burst tables and grids
     Buf bImgIn, bImgOut, bImgMax;        // image epilogue
@@ -597,7 +597,7 @@ struct Pipe {
         fa.near = g.near;
         fa.far = g.far;
         double* fdc = h->bCols.as<double>(n_r);
-        dc_fit(sums, fa, fdc, st);
+        dc_fit(sums, 1, fa, h->bFit.as<double>(3), fdc, nullptr, st);
         return fdc;
     }
 
@@ -614,7 +614,8 @@ struct Pipe {
         if (tops) {
             rate = dc_rate(g);
             h->mark("doppler");
-            fdc = doppler(A, g, rate);
+            // FP32: formed from FP64 lines before this burst's own (run)
+            fdc = sizeof(R) == 4 ? (double*)h->bCols.p : doppler(A, g, rate);
             h->mark("freq_unfold");
             // azimuth_frequency_ufr (image_formation.cpp:125-219)
             nrep = std::abs(rate * g.T / g.prf);
@@ -730,6 +731,16 @@ struct Pipe {
             throw S1Error(S1G_E_UNSUPPORTED, "sinc RCMC: only the FP32 precision (S1G_PREC_FP32) has it");
         const BurstGeom g = make_geom(h->hdr, pk);
         cur_pk = &pk;
+        if constexpr (sizeof(R) == 4) {
+            // The rounding of FP32 range-compressed lines (2e-7) moves the
+            // Doppler centroid by up to 1e-5 Hz and the SLC by up to 1.3e-4:
+            // the lag-1 sums take FP64 lines.
+            if (level == S1G_AZIMUTH_COMPRESSED && tops) {
+                h->mark("doppler");
+                Pipe<double> p64(h);
+                p64.doppler(p64.range_compress(p64.decode(pk, g), g, false), g, dc_rate(g));
+            }
+        }
         h->mark("decode");
         cpx<R>* A = decode(pk, g);
         h->mark("range_compress");
@@ -1569,7 +1580,7 @@ struct FastPipe {
         dfa.far = g.far;
         double* fdc = h->bCols.as<double>(n_r);
         df* fdc_df = h->bFdf.as<df>(n_r);
-        dc_fit_fast(da.part, nchunk, dfa, fdc, fdc_df, st);
+        dc_fit(da.part, nchunk, dfa, h->bFit.as<double>(3), fdc, fdc_df, st);
         h->mark("row_pass");
         cf32* ufr = h->bA.as<cf32>((size_t)S * n_r);
         transpose_batched<float>(ufrT, S, 0, ufr, n_r, 0, n_r, S, 1, st);

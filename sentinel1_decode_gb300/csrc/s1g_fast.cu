@@ -132,40 +132,58 @@ void fufr_fused(const FufrArgs& a, cudaStream_t st) {
     });
 }
 
-// ------------------------------------------------------------------ Doppler fit (parallel DFT)
+// ------------------------------------------------------------------ Doppler fit
+// FP64 on one pipe-bound SM: what can be spread over threads or blocks is.
 constexpr double kPIref = 3.14159265358979;
+constexpr int kFitBlocks = 64;    // num_blocks at most
 
-__global__ void k_dc_fit_fast(const cf64* part, int nchunk, DcFitArgs a, double* f_dc, df* f_dc_df) {
-    __shared__ double fine[64];
-    __shared__ double fval[64];
-    __shared__ double mag2[512];
-    __shared__ double fre[512], fim[512];
-    __shared__ double poly[3];
-    const int n = a.n_rng, nb = a.num_blocks;
-    (void)part;
-    (void)nchunk;
-    // f_dc holds the wrapped per-bin estimates (k_dc_wrapped)
+// Wrapped per-bin centroid -prf arg(sum) / (2 pi) (doppler.cpp:4-39), all bins in parallel.
+__global__ void k_dc_wrapped(const cf64* __restrict__ part, int nchunk, int n, double prf, double* __restrict__ f_dc) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= n) return;
+    double sr = 0.0, si = 0.0;
+    for (int c = 0; c < nchunk; ++c) {
+        sr += part[(long long)c * n + j].x;
+        si += part[(long long)c * n + j].y;
+    }
+    f_dc[j] = -prf * atan2(si, sr) / (2 * kPIref);
+}
+
+// Block means, unwrap (doppler.cpp:42-95) and the quadratic fit's three
+// coefficients: a warp per block mean, a thread per bin of the dense DFT (its
+// roots from a table: one SM does 1.9 FP64 operations a clock) and per block
+// of the unwrap.  20 us, where 256 threads with serial means and one thread
+// for the unwrap took 288 (and the FP64 pipeline's all-serial fit 19.8 ms).
+__global__ void __launch_bounds__(1024) k_dc_fit(const double* __restrict__ f_dc, DcFitArgs a, double* __restrict__ poly) {
+    __shared__ double fine[kFitBlocks], fval[kFitBlocks], un[kFitBlocks];
+    __shared__ double mag2[8 * kFitBlocks], fre[8 * kFitBlocks], fim[8 * kFitBlocks];
+    __shared__ double wre[8 * kFitBlocks], wim[8 * kFitBlocks];
+    __shared__ double line[2];
+    const int n = a.n_rng, nb = a.num_blocks, m = nb * 8;
     const int bs = n / nb;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int b = warp; b < nb; b += (int)(blockDim.x >> 5)) {
         const int s = b * bs;
         const int e = (s + bs < n) ? s + bs : n - 1;
         double acc = 0.0;
-        for (int j = s; j < e; ++j) acc += f_dc[j];
-        fine[b] = acc / ((double)e - (double)s);
-        double sn, cs;
-        sincos((2.0 * kPIref) * fine[b] / a.prf, &sn, &cs);
-        fval[b] = floor(hypot(cs, sn));
+        for (int j = s + lane; j < e; j += 32) acc += f_dc[j];
+        for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+        if (lane == 0) {
+            fine[b] = acc / ((double)e - (double)s);
+            double sn, cs;
+            sincos((2.0 * kPIref) * fine[b] / a.prf, &sn, &cs);
+            fval[b] = floor(hypot(cs, sn));
+        }
     }
+    for (int k = threadIdx.x; k < m; k += blockDim.x) sincospi(-2.0 * (double)k / (double)m, &wim[k], &wre[k]);
     __syncthreads();
-    const int m = nb * 8;
     for (int k = threadIdx.x; k < m; k += blockDim.x) {
         double re = 0.0, im = 0.0;
         for (int j = 0; j < nb; ++j) {
             if (fval[j] == 0.0) continue;
-            double ws, wc;
-            sincospi(-2.0 * (double)((long long)j * k % m) / (double)m, &ws, &wc);
-            re += fval[j] * wc;
-            im += fval[j] * ws;
+            const int q = (int)((long long)j * k % m);
+            re += fval[j] * wre[q];
+            im += fval[j] * wim[q];
         }
         const double mg = hypot(re, im);
         mag2[k] = mg * mg;
@@ -181,80 +199,79 @@ __global__ void k_dc_fit_fast(const cf64* part, int nchunk, DcFitArgs a, double*
         const double val = 1.0 / (m * (double)dt);
         const int N = (m - 1) / 2 + 1;
         const double v = bi < N ? bi * val : (bi - m) * val;
-        const double aa = v / (double)dt;
-        const double bb = atan2(fim[bi], fre[bi]) / (2.0 * kPIref);
-        double un[64];
-        for (int j = 0; j < nb; ++j) {
-            double s1, c1, s2, c2;
-            sincos((2.0 * kPIref) * fine[j] / a.prf, &s1, &c1);
-            sincos(-1.0 * (aa * a.rt[j] + bb), &s2, &c2);
-            const double pr = c1 * c2 - s1 * s2, pi_ = c1 * s2 + s1 * c2;
-            un[j] = (aa * a.rt[j] + bb + atan2(pi_, pr) / (2.0 * kPIref)) * a.prf;
-        }
-        double Sx[5] = {0, 0, 0, 0, 0}, Sy[3] = {0, 0, 0};
-        for (int i = 0; i < nb; ++i) {
-            double xi = 1.0;
-            for (int jj = 0; jj <= 4; ++jj) {
-                if (jj <= 2) Sy[jj] += xi * un[i];
-                Sx[jj] += xi;
-                xi *= a.rt[i];
-            }
-        }
-        double A[3][3] = {{Sx[0], Sx[1], Sx[2]}, {Sx[1], Sx[2], Sx[3]}, {Sx[2], Sx[3], Sx[4]}};
-        double B[3] = {Sy[0], Sy[1], Sy[2]};
-        for (int i = 0; i < 3; ++i) {
-            for (int k = i + 1; k < 3; ++k)
-                if (fabs(A[k][i]) > fabs(A[i][i])) {
-                    for (int jj = 0; jj < 3; ++jj) {
-                        const double t = A[i][jj];
-                        A[i][jj] = A[k][jj];
-                        A[k][jj] = t;
-                    }
-                    const double t = B[i];
-                    B[i] = B[k];
-                    B[k] = t;
-                }
-            for (int k = i + 1; k < 3; ++k) {
-                const double f = A[k][i] / A[i][i];
-                for (int jj = i; jj < 3; ++jj) A[k][jj] -= f * A[i][jj];
-                B[k] -= f * B[i];
-            }
-        }
-        double c[3];
-        for (int i = 2; i >= 0; --i) {
-            c[i] = B[i];
-            for (int jj = i + 1; jj < 3; ++jj) c[i] -= A[i][jj] * c[jj];
-            c[i] /= A[i][i];
-        }
-        poly[0] = c[0];
-        poly[1] = c[1];
-        poly[2] = c[2];
+        line[0] = v / (double)dt;
+        line[1] = atan2(fim[bi], fre[bi]) / (2.0 * kPIref);
     }
     __syncthreads();
-    const double step = (a.far - a.near) / (n - 1);
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double t = (a.near + j * step) - a.near;
-        const double v = (poly[0] + poly[1] * t + poly[2] * t * t);
-        f_dc[j] = v;
-        f_dc_df[j] = df_from(v);
+    if (threadIdx.x < nb) {
+        const int j = threadIdx.x;
+        const double aa = line[0], bb = line[1];
+        double s1, c1, s2, c2;
+        sincos((2.0 * kPIref) * fine[j] / a.prf, &s1, &c1);
+        sincos(-1.0 * (aa * a.rt[j] + bb), &s2, &c2);
+        const double pr = c1 * c2 - s1 * s2, pi_ = c1 * s2 + s1 * c2;
+        un[j] = (aa * a.rt[j] + bb + atan2(pi_, pr) / (2.0 * kPIref)) * a.prf;
     }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    // polyfit, degree 2 (signal_processing.cpp:159-214)
+    double Sx[5] = {0, 0, 0, 0, 0}, Sy[3] = {0, 0, 0};
+    for (int i = 0; i < nb; ++i) {
+        double xi = 1.0;
+        for (int jj = 0; jj <= 4; ++jj) {
+            if (jj <= 2) Sy[jj] += xi * un[i];
+            Sx[jj] += xi;
+            xi *= a.rt[i];
+        }
+    }
+    double A[3][3] = {{Sx[0], Sx[1], Sx[2]}, {Sx[1], Sx[2], Sx[3]}, {Sx[2], Sx[3], Sx[4]}};
+    double B[3] = {Sy[0], Sy[1], Sy[2]};
+    for (int i = 0; i < 3; ++i) {
+        for (int k = i + 1; k < 3; ++k)
+            if (fabs(A[k][i]) > fabs(A[i][i])) {
+                for (int jj = 0; jj < 3; ++jj) {
+                    const double t = A[i][jj];
+                    A[i][jj] = A[k][jj];
+                    A[k][jj] = t;
+                }
+                const double t = B[i];
+                B[i] = B[k];
+                B[k] = t;
+            }
+        for (int k = i + 1; k < 3; ++k) {
+            const double f = A[k][i] / A[i][i];
+            for (int jj = i; jj < 3; ++jj) A[k][jj] -= f * A[i][jj];
+            B[k] -= f * B[i];
+        }
+    }
+    double c[3];
+    for (int i = 2; i >= 0; --i) {
+        c[i] = B[i];
+        for (int jj = i + 1; jj < 3; ++jj) c[i] -= A[i][jj] * c[jj];
+        c[i] /= A[i][i];
+    }
+    poly[0] = c[0];
+    poly[1] = c[1];
+    poly[2] = c[2];
 }
 
-// Wrapped per-bin centroid -prf arg(sum) / (2 pi) (doppler.cpp:4-39), all bins in parallel.
-__global__ void k_dc_wrapped(const cf64* __restrict__ part, int nchunk, int n, double prf, double* __restrict__ f_dc) {
+// The fitted centroid of every range bin (f_dc_df may be null).
+__global__ void k_dc_eval(const double* __restrict__ poly, DcFitArgs a, double* __restrict__ f_dc, df* __restrict__ f_dc_df) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    double sr = 0.0, si = 0.0;
-    for (int c = 0; c < nchunk; ++c) {
-        sr += part[(long long)c * n + j].x;
-        si += part[(long long)c * n + j].y;
-    }
-    f_dc[j] = -prf * atan2(si, sr) / (2 * kPIref);
+    if (j >= a.n_rng) return;
+    const double step = (a.far - a.near) / (a.n_rng - 1);
+    const double t = (a.near + j * step) - a.near;
+    const double v = (poly[0] + poly[1] * t + poly[2] * t * t);
+    f_dc[j] = v;
+    if (f_dc_df) f_dc_df[j] = df_from(v);
 }
 
-void dc_fit_fast(const cf64* part, int nchunk, const DcFitArgs& a, double* f_dc, df* f_dc_df, cudaStream_t st) {
-    note_launch(), k_dc_wrapped<<<(a.n_rng + 127) / 128, 128, 0, st>>>(part, nchunk, a.n_rng, a.prf, f_dc);
-    note_launch(), k_dc_fit_fast<<<1, 256, 0, st>>>(part, nchunk, a, f_dc, f_dc_df);
+void dc_fit(const cf64* part, int nchunk, const DcFitArgs& a, double* poly, double* f_dc, df* f_dc_df, cudaStream_t st) {
+    if (a.num_blocks > kFitBlocks) throw std::runtime_error("Doppler fit: too many blocks");
+    const int grid = (a.n_rng + 127) / 128;
+    note_launch(), k_dc_wrapped<<<grid, 128, 0, st>>>(part, nchunk, a.n_rng, a.prf, f_dc);
+    note_launch(), k_dc_fit<<<1, 1024, 0, st>>>(f_dc, a, poly);
+    note_launch(), k_dc_eval<<<grid, 128, 0, st>>>(poly, a, f_dc, f_dc_df);
 }
 
 }  // namespace s1g

@@ -151,8 +151,10 @@ struct TufrArgs {
 void rc_fused(const cf32* raw, cf32* rc, int n_a, int n_r, int h, const Fft4Desc& d, const cf32* ref,
               cudaStream_t st);
 void fufr_fused(const FufrArgs& a, cudaStream_t st);
-// Doppler centroid polynomial from nchunk partial lag-1 sums [nchunk][n_r]
-void dc_fit_fast(const cf64* part, int nchunk, const DcFitArgs& a, double* f_dc, df* f_dc_df, cudaStream_t st);
+// Doppler centroid of every range bin (f_dc, and as float pairs in f_dc_df
+// unless it is null) from nchunk partial lag-1 sums [nchunk][n_r]; poly: device
+// scratch of 3 doubles
+void dc_fit(const cf64* part, int nchunk, const DcFitArgs& a, double* poly, double* f_dc, df* f_dc_df, cudaStream_t st);
 // src / src_lo of a smooth TOPS row pass (n_r entries each) from cols and fdc
 void rowpass_src_table(const ColDf* cols, const df* fdc, const int* mid, int n_r, float4* src, float* src_lo,
                        cudaStream_t st);

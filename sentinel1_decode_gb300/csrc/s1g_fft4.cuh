@@ -1,4 +1,5 @@
-// FP32 shared-memory FFT core of the fused kernels: forward transform,
+// Shared-memory FFT core of the fused kernels (FP32) and of the row engine
+// (FP32 and FP64): forward transform,
 // pointwise factor, inverse transform, with the ends of the chain in
 // registers.
 //
@@ -17,8 +18,8 @@
 // forward / inverse pair of P passes sweeps shared memory 2 P - 2 times,
 // with as many barriers.
 //
-// Twiddles: w, w^2, w^4, w^8 of each block or position as 32 bytes in global
-// memory, rounded from FP64 (read through L1 / L2, coalesced where they
+// Twiddles: w, w^2, w^4, w^8 of each block or position as one entry in global
+// memory (32 bytes in FP32), rounded from FP64 (read through L1 / L2, coalesced where they
 // differ from lane to lane); other powers are products of at most three.
 //
 // Layout: one element of padding per 16.  With Ns a multiple of 16 (a plan
@@ -49,16 +50,31 @@ inline void fft4_launch(size_t smem, F f) {
     else f(integral_constant<int, 768>(), integral_constant<int, 1>());
 }
 
-struct Fft4Desc {
+template <typename R>
+struct alignas(16) Tw4 {
+    cpx<R> w1, w2, w4, w8;
+};
+
+template <typename R>
+struct Fft4DescT {
     int n = 0;
     int np = 0;
-    int affine = 0;                    // last radix 16 and a first radix of the fused kernels' set
+    int affine = 0;                    // last radix 16 and a first radix of the fused kernels' set (FP32 only)
     int radix[kFft4Passes] = {};
-    const float4* fw[kFft4Passes] = {};   // forward pass p: 2 float4 per block
-    const float4* iv[kFft4Passes] = {};   // inverse pass p: 2 float4 per position
+    const Tw4<R>* fw[kFft4Passes] = {};   // forward pass p: an entry per block
+    const Tw4<R>* iv[kFft4Passes] = {};   // inverse pass p: an entry per position
     const int* pos = nullptr;          // digit-reversed position of frequency f
     const int* mid = nullptr;          // where the factor of frequency f lies: j (n / R) + g
 };
+using Fft4Desc = Fft4DescT<float>;
+
+__device__ __forceinline__ Tw4<float> ldg_tw(const Tw4<float>* p) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    return Tw4<float>{mk(a.x, a.y), mk(a.z, a.w), mk(b.x, b.y), mk(b.z, b.w)};
+}
+__device__ __forceinline__ Tw4<double> ldg_tw(const Tw4<double>* p) {
+    return Tw4<double>{ldg(&p->w1), ldg(&p->w2), ldg(&p->w4), ldg(&p->w8)};
+}
 
 __host__ __device__ inline int pad16(int i) { return i + (i >> 4); }
 __host__ __device__ inline int padded16_len(int n) { return n + (n >> 4) + 1; }
@@ -77,48 +93,52 @@ __device__ __forceinline__ void split4(int t, int ns, float inv_ns, int& g, int&
 }
 
 // ---------------------------------------------------------------- butterflies
+__device__ __forceinline__ float fma_(float a, float b, float c) { return fmaf(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return fma(a, b, c); }
 // x, y -> x + w y, x - w y
-__device__ __forceinline__ void pm4(cf32& x, cf32& y, cf32 w) {
-    const cf32 s = mk(fmaf(w.x, y.x, fmaf(-w.y, y.y, x.x)), fmaf(w.x, y.y, fmaf(w.y, y.x, x.y)));
-    y = mk(fmaf(2.0f, x.x, -s.x), fmaf(2.0f, x.y, -s.y));
+template <typename T>
+__device__ __forceinline__ void pm4(cpx<T>& x, cpx<T>& y, cpx<T> w) {
+    const cpx<T> s = mk(fma_(w.x, y.x, fma_(-w.y, y.y, x.x)), fma_(w.x, y.y, fma_(w.y, y.x, x.y)));
+    y = mk(fma_((T)2, x.x, -s.x), fma_((T)2, x.y, -s.y));
     x = s;
 }
-__device__ __forceinline__ cf32 cmul4(cf32 a, cf32 b) {
-    return mk(fmaf(a.x, b.x, -a.y * b.y), fmaf(a.x, b.y, a.y * b.x));
+template <typename T>
+__device__ __forceinline__ cpx<T> cmul4(cpx<T> a, cpx<T> b) {
+    return mk(fma_(a.x, b.x, -a.y * b.y), fma_(a.x, b.y, a.y * b.x));
 }
 // times exp(DIR i pi m / 8) for m = 0..3
-template <int DIR, int M>
-__device__ __forceinline__ cf32 rot16(cf32 w) {
-    constexpr float c[4] = {1.0f, 0.92387953251128675613f, 0.70710678118654752440f, 0.38268343236508977173f};
-    constexpr float s[4] = {0.0f, 0.38268343236508977173f, 0.70710678118654752440f, 0.92387953251128675613f};
+template <int DIR, int M, typename T>
+__device__ __forceinline__ cpx<T> rot16(cpx<T> w) {
+    constexpr T c[4] = {(T)1.0, (T)0.92387953251128675613, (T)0.70710678118654752440, (T)0.38268343236508977173};
+    constexpr T s[4] = {(T)0.0, (T)0.38268343236508977173, (T)0.70710678118654752440, (T)0.92387953251128675613};
     if (M == 0) return w;
-    return mk(fmaf(c[M], w.x, -DIR * s[M] * w.y), fmaf(c[M], w.y, DIR * s[M] * w.x));
+    return mk(fma_(c[M], w.x, -DIR * s[M] * w.y), fma_(c[M], w.y, DIR * s[M] * w.x));
 }
-template <int DIR>
-__device__ __forceinline__ cf32 muli4(cf32 w) { return DIR > 0 ? mk(-w.y, w.x) : mk(w.y, -w.x); }
+template <int DIR, typename T>
+__device__ __forceinline__ cpx<T> muli4(cpx<T> w) { return DIR > 0 ? mk(-w.y, w.x) : mk(w.y, -w.x); }
 
 // out[j] = sum_r a[r] w^r exp(DIR 2 pi i r j / R), R = 2, 4, 8, 16 with the
 // powers w1 = w, w2 = w^2, w4, w8; out[j] lies at a[slot(j)].
-template <int R, int DIR>
+template <typename T, int R, int DIR>
 struct Tw2 {
     // a[slot]: out index of slot s is the bit reversal of s
-    static __device__ __forceinline__ void run(cf32* a, cf32 w1, cf32 w2, cf32 w4, cf32 w8) {
+    static __device__ __forceinline__ void run(cpx<T>* a, cpx<T> w1, cpx<T> w2, cpx<T> w4, cpx<T> w8) {
         if (R == 16) {
 #pragma unroll
             for (int r = 0; r < 8; ++r) pm4(a[r], a[r + 8], w8);
         }
         if (R >= 8) {
-            const cf32 u = muli4<DIR>(w4);
+            const cpx<T> u = muli4<DIR>(w4);
 #pragma unroll
             for (int b = 0; b < R / 8; ++b)
 #pragma unroll
                 for (int r = 0; r < 4; ++r) pm4(a[8 * b + r], a[8 * b + r + 4], b ? u : w4);
         }
         if (R >= 4) {
-            const cf32 v1 = R >= 16 ? rot16<DIR, 2>(w2) : w2;   // w2 exp(DIR i pi / 4): only with 16
-            const cf32 i0 = muli4<DIR>(w2), i1 = muli4<DIR>(v1);
+            const cpx<T> v1 = R >= 16 ? rot16<DIR, 2>(w2) : w2;   // w2 exp(DIR i pi / 4): only with 16
+            const cpx<T> i0 = muli4<DIR>(w2), i1 = muli4<DIR>(v1);
             // out index bits so far of block b (bit-reversed): R = 16: 0, 2, 1, 3; R = 8: 0, 1; R = 4: 0
-            const cf32 w[4] = {w2, i0, v1, i1};
+            const cpx<T> w[4] = {w2, i0, v1, i1};
 #pragma unroll
             for (int b = 0; b < R / 4; ++b)
 #pragma unroll
@@ -126,9 +146,9 @@ struct Tw2 {
         }
         {
             // factors exp(DIR 2 pi i j / R) of the out index bits of block b
-            const cf32 e1 = R >= 16 ? rot16<DIR, 1>(w1) : w1, e3 = R >= 16 ? rot16<DIR, 3>(w1) : w1;
-            const cf32 e2 = R >= 8 ? rot16<DIR, 2>(w1) : w1;
-            const cf32 f[8] = {w1, muli4<DIR>(w1), e2, muli4<DIR>(e2), e1, muli4<DIR>(e1), e3, muli4<DIR>(e3)};
+            const cpx<T> e1 = R >= 16 ? rot16<DIR, 1>(w1) : w1, e3 = R >= 16 ? rot16<DIR, 3>(w1) : w1;
+            const cpx<T> e2 = R >= 8 ? rot16<DIR, 2>(w1) : w1;
+            const cpx<T> f[8] = {w1, muli4<DIR>(w1), e2, muli4<DIR>(e2), e1, muli4<DIR>(e1), e3, muli4<DIR>(e3)};
 #pragma unroll
             for (int b = 0; b < R / 2; ++b) pm4(a[2 * b], a[2 * b + 1], f[b]);
         }
@@ -142,27 +162,27 @@ struct Tw2 {
 };
 
 // plain DFTs of the other radices, out[j] at a[j]
-template <int R, int DIR>
+template <typename T, int R, int DIR>
 struct Dft {
-    static __device__ __forceinline__ void run(cf32* a) { Bfly<float, R>::run(a, DIR); }
+    static __device__ __forceinline__ void run(cpx<T>* a) { Bfly<T, R>::run(a, DIR); }
 };
-template <int DIR>
-struct Dft<2, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) {
-        const cf32 t = a[0];
+template <typename T, int DIR>
+struct Dft<T, 2, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) {
+        const cpx<T> t = a[0];
         a[0] = t + a[1];
         a[1] = t - a[1];
     }
 };
-template <int DIR>
-struct Dft<16, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) {
+template <typename T, int DIR>
+struct Dft<T, 16, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) {
         // r = r0 + 4 r1, j = j0 + 4 j1, inner twiddles exp(DIR 2 pi i r0 j0 / 16)
-        cf32 b[4][4];
+        cpx<T> b[4][4];
 #pragma unroll
         for (int r0 = 0; r0 < 4; ++r0) {
-            cf32 v[4] = {a[r0], a[r0 + 4], a[r0 + 8], a[r0 + 12]};
-            Bfly<float, 4>::run(v, DIR);
+            cpx<T> v[4] = {a[r0], a[r0 + 4], a[r0 + 8], a[r0 + 12]};
+            Bfly<T, 4>::run(v, DIR);
 #pragma unroll
             for (int j0 = 0; j0 < 4; ++j0) b[r0][j0] = v[j0];
         }
@@ -177,8 +197,8 @@ struct Dft<16, DIR> {
         b[3][3] = muli4<DIR>(muli4<DIR>(rot16<DIR, 1>(b[3][3])));
 #pragma unroll
         for (int j0 = 0; j0 < 4; ++j0) {
-            cf32 v[4] = {b[0][j0], b[1][j0], b[2][j0], b[3][j0]};
-            Bfly<float, 4>::run(v, DIR);
+            cpx<T> v[4] = {b[0][j0], b[1][j0], b[2][j0], b[3][j0]};
+            Bfly<T, 4>::run(v, DIR);
 #pragma unroll
             for (int j1 = 0; j1 < 4; ++j1) a[j0 + 4 * j1] = v[j1];
         }
@@ -186,22 +206,22 @@ struct Dft<16, DIR> {
 };
 // coprime factors A x B (Good-Thomas): r = (B r1 + A r2) mod R, and the out
 // index j with j = j1 mod A, j = j2 mod B
-template <int A, int B, int DIR>
-__device__ __forceinline__ void good_thomas(cf32* a) {
+template <int A, int B, int DIR, typename T>
+__device__ __forceinline__ void good_thomas(cpx<T>* a) {
     constexpr int R = A * B;
-    cf32 t[A][B];
+    cpx<T> t[A][B];
 #pragma unroll
     for (int r1 = 0; r1 < A; ++r1)
 #pragma unroll
         for (int r2 = 0; r2 < B; ++r2) t[r1][r2] = a[(B * r1 + A * r2) % R];
 #pragma unroll
-    for (int r1 = 0; r1 < A; ++r1) Dft<B, DIR>::run(t[r1]);
+    for (int r1 = 0; r1 < A; ++r1) Dft<T, B, DIR>::run(t[r1]);
 #pragma unroll
     for (int r2 = 0; r2 < B; ++r2) {
-        cf32 c[A];
+        cpx<T> c[A];
 #pragma unroll
         for (int r1 = 0; r1 < A; ++r1) c[r1] = t[r1][r2];
-        Dft<A, DIR>::run(c);
+        Dft<T, A, DIR>::run(c);
 #pragma unroll
         for (int j1 = 0; j1 < A; ++j1) {
             // (B r1 + A r2) j / R = r1 j / A + r2 j / B
@@ -211,34 +231,34 @@ __device__ __forceinline__ void good_thomas(cf32* a) {
         }
     }
 }
-template <int DIR>
-struct Dft<6, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) { good_thomas<2, 3, DIR>(a); }
+template <typename T, int DIR>
+struct Dft<T, 6, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) { good_thomas<2, 3, DIR>(a); }
 };
-template <int DIR>
-struct Dft<10, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) { good_thomas<2, 5, DIR>(a); }
+template <typename T, int DIR>
+struct Dft<T, 10, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) { good_thomas<2, 5, DIR>(a); }
 };
-template <int DIR>
-struct Dft<12, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) { good_thomas<4, 3, DIR>(a); }
+template <typename T, int DIR>
+struct Dft<T, 12, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) { good_thomas<4, 3, DIR>(a); }
 };
-template <int DIR>
-struct Dft<15, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) { good_thomas<3, 5, DIR>(a); }
+template <typename T, int DIR>
+struct Dft<T, 15, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) { good_thomas<3, 5, DIR>(a); }
 };
-template <int DIR>
-struct Dft<9, DIR> {
-    static __device__ __forceinline__ void run(cf32* a) {
+template <typename T, int DIR>
+struct Dft<T, 9, DIR> {
+    static __device__ __forceinline__ void run(cpx<T>* a) {
         // r = 3 r1 + r2, j = j1 + 3 j2, inner twiddles exp(DIR 2 pi i r2 j1 / 9)
-        constexpr float c1 = 0.76604444311897803520f, s1 = 0.64278760968653932632f;
-        constexpr float c2 = 0.17364817766693034885f, s2 = 0.98480775301220805937f;
-        constexpr float c4 = -0.93969262078590838405f, s4 = 0.34202014332566873304f;
-        cf32 t[3][3];
+        constexpr T c1 = (T)0.76604444311897803520, s1 = (T)0.64278760968653932632;
+        constexpr T c2 = (T)0.17364817766693034885, s2 = (T)0.98480775301220805937;
+        constexpr T c4 = (T)-0.93969262078590838405, s4 = (T)0.34202014332566873304;
+        cpx<T> t[3][3];
 #pragma unroll
         for (int r2 = 0; r2 < 3; ++r2) {
-            cf32 v[3] = {a[r2], a[3 + r2], a[6 + r2]};
-            Dft<3, DIR>::run(v);
+            cpx<T> v[3] = {a[r2], a[3 + r2], a[6 + r2]};
+            Dft<T, 3, DIR>::run(v);
             for (int j1 = 0; j1 < 3; ++j1) t[r2][j1] = v[j1];
         }
         t[1][1] = cmul4(t[1][1], mk(c1, DIR * s1));
@@ -247,8 +267,8 @@ struct Dft<9, DIR> {
         t[2][2] = cmul4(t[2][2], mk(c4, DIR * s4));
 #pragma unroll
         for (int j1 = 0; j1 < 3; ++j1) {
-            cf32 v[3] = {t[0][j1], t[1][j1], t[2][j1]};
-            Dft<3, DIR>::run(v);
+            cpx<T> v[3] = {t[0][j1], t[1][j1], t[2][j1]};
+            Dft<T, 3, DIR>::run(v);
             for (int j2 = 0; j2 < 3; ++j2) a[j1 + 3 * j2] = v[j2];
         }
     }
@@ -256,23 +276,21 @@ struct Dft<9, DIR> {
 
 __host__ __device__ constexpr bool pow2r(int r) { return r == 2 || r == 4 || r == 8 || r == 16; }
 
-// a[r] <- sum_r a[r] w^r exp(DIR 2 pi i r j / R) at a[j] for the twiddle entry
-// (w, w^2) (w^4, w^8)
-template <int R, int DIR>
-__device__ __forceinline__ void bfly4_tw(cf32* a, float4 p, float4 q) {
-    const cf32 w1 = mk(p.x, p.y), w2 = mk(p.z, p.w), w4 = mk(q.x, q.y), w8 = mk(q.z, q.w);
+// a[r] <- sum_r a[r] w^r exp(DIR 2 pi i r j / R) at a[j]
+template <int R, int DIR, typename T>
+__device__ __forceinline__ void bfly4_tw(cpx<T>* a, const Tw4<T>& e) {
     if constexpr (pow2r(R)) {
-        Tw2<R, DIR>::run(a, w1, w2, w4, w8);
-        cf32 t[R];
+        Tw2<T, R, DIR>::run(a, e.w1, e.w2, e.w4, e.w8);
+        cpx<T> t[R];
 #pragma unroll
-        for (int s = 0; s < R; ++s) t[Tw2<R, DIR>::out_of(s)] = a[s];
+        for (int s = 0; s < R; ++s) t[Tw2<T, R, DIR>::out_of(s)] = a[s];
 #pragma unroll
         for (int s = 0; s < R; ++s) a[s] = t[s];
     } else {
-        const cf32 w[4] = {w1, w2, w4, w8};
+        const cpx<T> w[4] = {e.w1, e.w2, e.w4, e.w8};
 #pragma unroll
         for (int r = 1; r < R; ++r) {
-            cf32 f = mk(1.f, 0.f);
+            cpx<T> f = mk((T)1, (T)0);
             bool first = true;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
@@ -282,12 +300,12 @@ __device__ __forceinline__ void bfly4_tw(cf32* a, float4 p, float4 q) {
                 }
             a[r] = cmul4(a[r], f);
         }
-        Dft<R, DIR>::run(a);
+        Dft<T, R, DIR>::run(a);
     }
 }
-template <int R, int DIR>
-__device__ __forceinline__ void bfly4(cf32* a) {
-    Dft<R, DIR>::run(a);
+template <int R, int DIR, typename T>
+__device__ __forceinline__ void bfly4(cpx<T>* a) {
+    Dft<T, R, DIR>::run(a);
 }
 
 // ---------------------------------------------------------------- passes
@@ -299,29 +317,28 @@ struct At4 {
     __device__ __forceinline__ int operator()(int r) const { return AFF ? b + r * s : pad16(b + r * s); }
 };
 
-template <int R, int DIR, bool AFF>
-__device__ __forceinline__ void pass4_r(cf32* buf, int n, int Ns, const float4* __restrict__ tw) {
+template <int R, int DIR, bool AFF, typename T>
+__device__ __forceinline__ void pass4_r(cpx<T>* buf, int n, int Ns, const Tw4<T>* __restrict__ tw) {
     const int nb = n / R;
     const float inv = 1.0f / (float)Ns;
     for (int t = threadIdx.x; t < nb; t += blockDim.x) {
         int g, k;
         split4(t, Ns, inv, g, k);
         // forward: the block's entry; inverse: the position's
-        const int e = DIR < 0 ? g : k;
-        const float4 p = __ldg(tw + 2 * e), q = __ldg(tw + 2 * e + 1);
+        const Tw4<T> e = ldg_tw(tw + (DIR < 0 ? g : k));
         const At4<AFF> at(g * Ns * R + k, Ns);
-        cf32 a[R];
+        cpx<T> a[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = buf[at(r)];
-        bfly4_tw<R, DIR>(a, p, q);
+        bfly4_tw<R, DIR>(a, e);
 #pragma unroll
         for (int r = 0; r < R; ++r) buf[at(r)] = a[r];
     }
 }
 
 // One pass with twiddles over shared memory (caller synchronises).
-template <int DIR, bool AFF>
-__device__ __noinline__ void pass4(cf32* buf, int R, int n, int Ns, const float4* tw) {
+template <int DIR, bool AFF, typename T>
+__device__ __noinline__ void pass4(cpx<T>* buf, int R, int n, int Ns, const Tw4<T>* tw) {
     switch (R) {
         case 2: pass4_r<2, DIR, AFF>(buf, n, Ns, tw); break;
         case 3: pass4_r<3, DIR, AFF>(buf, n, Ns, tw); break;
@@ -330,20 +347,37 @@ __device__ __noinline__ void pass4(cf32* buf, int R, int n, int Ns, const float4
         case 6: pass4_r<6, DIR, AFF>(buf, n, Ns, tw); break;
         case 7: pass4_r<7, DIR, AFF>(buf, n, Ns, tw); break;
         case 8: pass4_r<8, DIR, AFF>(buf, n, Ns, tw); break;
-        case 9: pass4_r<9, DIR, AFF>(buf, n, Ns, tw); break;
-        case 10: pass4_r<10, DIR, AFF>(buf, n, Ns, tw); break;
-        case 12: pass4_r<12, DIR, AFF>(buf, n, Ns, tw); break;
-        case 15: pass4_r<15, DIR, AFF>(buf, n, Ns, tw); break;
-        default: pass4_r<16, DIR, AFF>(buf, n, Ns, tw); break;
+        default:
+            // FP64 plans stop at radix 8 (registers)
+            if constexpr (sizeof(T) == 4) {
+                switch (R) {
+                    case 9: pass4_r<9, DIR, AFF>(buf, n, Ns, tw); break;
+                    case 10: pass4_r<10, DIR, AFF>(buf, n, Ns, tw); break;
+                    case 12: pass4_r<12, DIR, AFF>(buf, n, Ns, tw); break;
+                    case 15: pass4_r<15, DIR, AFF>(buf, n, Ns, tw); break;
+                    default: pass4_r<16, DIR, AFF>(buf, n, Ns, tw); break;
+                }
+            }
     }
 }
 
-template <int R, class LoadF>
-__device__ __forceinline__ void first4_r(cf32* buf, int n, LoadF load) {
+template <int DIR, typename T>
+__device__ __forceinline__ void pass4_any(cpx<T>* buf, const Fft4DescT<T>& d, int R, int Ns, const Tw4<T>* tw) {
+    if constexpr (sizeof(T) == 4) {
+        if (d.affine) {
+            pass4<DIR, true>(buf, R, d.n, Ns, tw);
+            return;
+        }
+    }
+    pass4<DIR, false>(buf, R, d.n, Ns, tw);
+}
+
+template <int R, typename T, class LoadF>
+__device__ __forceinline__ void first4_r(cpx<T>* buf, int n, LoadF load) {
     const int Ns = n / R;
     for (int t = threadIdx.x; t < Ns; t += blockDim.x) {
         const At4<true> at(t, Ns);
-        cf32 a[R];
+        cpx<T> a[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = load(t + r * Ns);
         bfly4<R, -1>(a);
@@ -353,16 +387,16 @@ __device__ __forceinline__ void first4_r(cf32* buf, int n, LoadF load) {
 }
 // ROLL: the outputs go back to the thread's own slots and to the functor from
 // a loop, for functors too long to be unrolled R times.
-template <int R, bool ROLL, class StoreF>
-__device__ __forceinline__ void last4_r(cf32* buf, int n, const float4* __restrict__ tw, StoreF store) {
+template <int R, bool ROLL, typename T, class StoreF>
+__device__ __forceinline__ void last4_r(cpx<T>* buf, int n, const Tw4<T>* __restrict__ tw, StoreF store) {
     const int Ns = n / R;
     for (int t = threadIdx.x; t < Ns; t += blockDim.x) {
-        const float4 p = __ldg(tw + 2 * t), q = __ldg(tw + 2 * t + 1);
+        const Tw4<T> e = ldg_tw(tw + t);
         const At4<true> at(t, Ns);
-        cf32 a[R];
+        cpx<T> a[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = buf[at(r)];
-        bfly4_tw<R, +1>(a, p, q);
+        bfly4_tw<R, +1>(a, e);
         if (ROLL) {
 #pragma unroll
             for (int r = 0; r < R; ++r) buf[at(r)] = a[r];
@@ -382,11 +416,13 @@ __host__ __device__ constexpr bool fft4_end_radix(int r) {
 
 // Forward passes of d up to the last: load(i) gives input i.  Ends with a
 // barrier; buf may be read by other threads until the call.
-template <class LoadF>
-__device__ __forceinline__ void fft4_head(cf32* buf, const Fft4Desc& d, LoadF load) {
+template <typename T, class LoadF>
+__device__ __forceinline__ void fft4_head(cpx<T>* buf, const Fft4DescT<T>& d, LoadF load) {
     int Ns = d.n;
     int p = 0;
-    if (d.affine) {
+    bool done = false;
+    if constexpr (sizeof(T) == 4) if (d.affine) {
+        done = true;
         switch (d.radix[0]) {
             case 6: first4_r<6>(buf, d.n, load); break;
             case 8: first4_r<8>(buf, d.n, load); break;
@@ -396,31 +432,31 @@ __device__ __forceinline__ void fft4_head(cf32* buf, const Fft4Desc& d, LoadF lo
         }
         Ns /= d.radix[0];
         p = 1;
-    } else {
+    }
+    if (!done) {
         for (int i = threadIdx.x; i < d.n; i += blockDim.x) buf[pad16(i)] = load(i);
     }
     __syncthreads();
     for (; p + 1 < d.np; ++p) {
         Ns /= d.radix[p];
-        if (d.affine) pass4<-1, true>(buf, d.radix[p], d.n, Ns, d.fw[p]);
-        else pass4<-1, false>(buf, d.radix[p], d.n, Ns, d.fw[p]);
+        pass4_any<-1>(buf, d, d.radix[p], Ns, d.fw[p]);
         __syncthreads();
     }
 }
 
 // The last forward pass (Ns = 1), mid(m, v) at every frequency with m its
 // place in the factor table, and the first inverse pass.  Barrier at the end.
-template <int R, bool AFF, class MidF>
-__device__ __forceinline__ void mid4_r(cf32* buf, const Fft4Desc& d, MidF mid) {
+template <int R, bool AFF, typename T, class MidF>
+__device__ __forceinline__ void mid4_r(cpx<T>* buf, const Fft4DescT<T>& d, MidF mid) {
     const int nb = d.n / R;
-    const float4* __restrict__ tw = d.fw[d.np - 1];
+    const Tw4<T>* __restrict__ tw = d.fw[d.np - 1];
     for (int g = threadIdx.x; g < nb; g += blockDim.x) {
-        const float4 p = __ldg(tw + 2 * g), q = __ldg(tw + 2 * g + 1);
-        cf32 a[R];
+        const Tw4<T> e = ldg_tw(tw + g);
+        cpx<T> a[R];
         const int b = AFF ? 17 * g : R * g;
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = buf[AFF ? b + r : pad16(b + r)];
-        bfly4_tw<R, -1>(a, p, q);
+        bfly4_tw<R, -1>(a, e);
 #pragma unroll
         for (int j = 0; j < R; ++j) a[j] = mid(j * nb + g, a[j]);
         bfly4<R, +1>(a);
@@ -428,11 +464,14 @@ __device__ __forceinline__ void mid4_r(cf32* buf, const Fft4Desc& d, MidF mid) {
         for (int r = 0; r < R; ++r) buf[AFF ? b + r : pad16(b + r)] = a[r];
     }
 }
-template <class MidF>
-__device__ __forceinline__ void fft4_mid(cf32* buf, const Fft4Desc& d, MidF mid) {
-    if (d.affine) {
+template <typename T, class MidF>
+__device__ __forceinline__ void fft4_mid(cpx<T>* buf, const Fft4DescT<T>& d, MidF mid) {
+    bool done = false;
+    if constexpr (sizeof(T) == 4) if (d.affine) {
+        done = true;
         mid4_r<16, true>(buf, d, mid);
-    } else {
+    }
+    if (!done) {
         // the last pass, the factor and the first inverse pass (no twiddles) apart
         const int R = d.radix[d.np - 1], nb = d.n / R;
         pass4<-1, false>(buf, R, d.n, 1, d.fw[d.np - 1]);
@@ -448,21 +487,23 @@ __device__ __forceinline__ void fft4_mid(cf32* buf, const Fft4Desc& d, MidF mid)
 }
 
 // The remaining inverse passes but the last (functor) one.
-__device__ __forceinline__ void fft4_back(cf32* buf, const Fft4Desc& d) {
+template <typename T>
+__device__ __forceinline__ void fft4_back(cpx<T>* buf, const Fft4DescT<T>& d) {
     int Ns = d.radix[d.np - 1];
-    for (int p = d.np - 2; p >= (d.affine ? 1 : 0); --p) {
-        if (d.affine) pass4<+1, true>(buf, d.radix[p], d.n, Ns, d.iv[p]);
-        else pass4<+1, false>(buf, d.radix[p], d.n, Ns, d.iv[p]);
+    for (int p = d.np - 2; p >= (sizeof(T) == 4 && d.affine ? 1 : 0); --p) {
+        pass4_any<+1>(buf, d, d.radix[p], Ns, d.iv[p]);
         Ns *= d.radix[p];
         __syncthreads();
     }
 }
 
 // The other inverse passes: store(i, v) gets output i.  No barrier at the end.
-template <bool ROLL = false, class StoreF>
-__device__ __forceinline__ void fft4_tail(cf32* buf, const Fft4Desc& d, StoreF store) {
+template <bool ROLL = false, typename T, class StoreF>
+__device__ __forceinline__ void fft4_tail(cpx<T>* buf, const Fft4DescT<T>& d, StoreF store) {
     fft4_back(buf, d);
-    if (d.affine) {
+    bool done = false;
+    if constexpr (sizeof(T) == 4) if (d.affine) {
+        done = true;
         switch (d.radix[0]) {
             case 6: last4_r<6, ROLL>(buf, d.n, d.iv[0], store); break;
             case 8: last4_r<8, ROLL>(buf, d.n, d.iv[0], store); break;
@@ -470,7 +511,8 @@ __device__ __forceinline__ void fft4_tail(cf32* buf, const Fft4Desc& d, StoreF s
             case 12: last4_r<12, ROLL>(buf, d.n, d.iv[0], store); break;
             default: last4_r<16, ROLL>(buf, d.n, d.iv[0], store); break;
         }
-    } else {
+    }
+    if (!done) {
         for (int i = threadIdx.x; i < d.n; i += blockDim.x) store(i, buf[pad16(i)]);
     }
 }
@@ -479,16 +521,16 @@ __device__ __forceinline__ void fft4_tail(cf32* buf, const Fft4Desc& d, StoreF s
 // f(i, v) takes output i to input i of the next (in registers: the last
 // inverse and the first forward pass have the same butterflies).  Ends with a
 // barrier, as fft4_head.
-template <int R, class JoinF>
-__device__ __forceinline__ void join4_r(cf32* buf, int n, const float4* __restrict__ tw, JoinF f) {
+template <int R, typename T, class JoinF>
+__device__ __forceinline__ void join4_r(cpx<T>* buf, int n, const Tw4<T>* __restrict__ tw, JoinF f) {
     const int Ns = n / R;
     for (int t = threadIdx.x; t < Ns; t += blockDim.x) {
-        const float4 p = __ldg(tw + 2 * t), q = __ldg(tw + 2 * t + 1);
+        const Tw4<T> e = ldg_tw(tw + t);
         const At4<true> at(t, Ns);
-        cf32 a[R];
+        cpx<T> a[R];
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = buf[at(r)];
-        bfly4_tw<R, +1>(a, p, q);
+        bfly4_tw<R, +1>(a, e);
 #pragma unroll
         for (int r = 0; r < R; ++r) a[r] = f(t + r * Ns, a[r]);
         bfly4<R, -1>(a);
@@ -496,11 +538,13 @@ __device__ __forceinline__ void join4_r(cf32* buf, int n, const float4* __restri
         for (int r = 0; r < R; ++r) buf[at(r)] = a[r];
     }
 }
-template <class JoinF>
-__device__ __forceinline__ void fft4_join(cf32* buf, const Fft4Desc& d, JoinF f) {
+template <typename T, class JoinF>
+__device__ __forceinline__ void fft4_join(cpx<T>* buf, const Fft4DescT<T>& d, JoinF f) {
     fft4_back(buf, d);
     int Ns = d.n, p = 0;
-    if (d.affine) {
+    bool done = false;
+    if constexpr (sizeof(T) == 4) if (d.affine) {
+        done = true;
         switch (d.radix[0]) {
             case 6: join4_r<6>(buf, d.n, d.iv[0], f); break;
             case 8: join4_r<8>(buf, d.n, d.iv[0], f); break;
@@ -510,23 +554,23 @@ __device__ __forceinline__ void fft4_join(cf32* buf, const Fft4Desc& d, JoinF f)
         }
         Ns /= d.radix[0];
         p = 1;
-    } else {
+    }
+    if (!done) {
         for (int i = threadIdx.x; i < d.n; i += blockDim.x) buf[pad16(i)] = f(i, buf[pad16(i)]);
     }
     __syncthreads();
     for (; p + 1 < d.np; ++p) {
         Ns /= d.radix[p];
-        if (d.affine) pass4<-1, true>(buf, d.radix[p], d.n, Ns, d.fw[p]);
-        else pass4<-1, false>(buf, d.radix[p], d.n, Ns, d.fw[p]);
+        pass4_any<-1>(buf, d, d.radix[p], Ns, d.fw[p]);
         __syncthreads();
     }
 }
 
 // The last forward pass alone: frequency f then lies at buf[pad16(d.pos[f])].
 // Barrier at the end.
-__device__ __forceinline__ void fft4_spectrum(cf32* buf, const Fft4Desc& d) {
-    if (d.affine) pass4<-1, true>(buf, 16, d.n, 1, d.fw[d.np - 1]);
-    else pass4<-1, false>(buf, d.radix[d.np - 1], d.n, 1, d.fw[d.np - 1]);
+template <typename T>
+__device__ __forceinline__ void fft4_spectrum(cpx<T>* buf, const Fft4DescT<T>& d) {
+    pass4_any<-1>(buf, d, d.radix[d.np - 1], 1, d.fw[d.np - 1]);
     __syncthreads();
 }
 

@@ -107,6 +107,28 @@ std::vector<std::vector<int>> fft4_orders(long long n, size_t most) {
     return out;
 }
 
+std::vector<int> fft4_order64(long long n) {
+    // FP64 instructions per point of a pass with its twiddles
+    static const std::pair<int, double> cost[] = {{8, 9.4}, {7, 20}, {6, 13.5}, {5, 11}, {4, 6.3}, {3, 7.5}, {2, 3.2}};
+    std::vector<std::vector<int>> f;
+    std::vector<int> cur;
+    if (n < 2 || !is_smooth7(n)) return {};
+    factorisations(n, 5, kFft4Passes, cur, f);   // radices from 8 down
+    std::vector<int> best;
+    double bc = 1e30;
+    for (const auto& v : f) {
+        double c = 0.3 * v.size();
+        for (int r : v)
+            for (const auto& k : cost)
+                if (k.first == r) c += k.second;
+        if (c < bc) {
+            bc = c;
+            best = v;
+        }
+    }
+    return best;
+}
+
 std::vector<long long> fft4_lengths(long long minlen, size_t most) {
     std::vector<std::pair<double, long long>> c;
     const long long hi = std::max(64LL, (long long)(minlen * 1.25) + 16);
@@ -146,58 +168,115 @@ void* DeviceArena::get(size_t bytes) {
 }
 
 // ------------------------------------------------------------------ kernels
-constexpr int kFftThreads = 512;
-
-template <typename R>
-__global__ void __launch_bounds__(kFftThreads) k_fft_smem(const cpx<R>* __restrict__ in, long long in_pitch,
-                                                         cpx<R>* __restrict__ out, long long out_pitch,
-                                                         FftDesc<R> d, int dir) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cpx<R>* buf = reinterpret_cast<cpx<R>*>(smem_raw);
-    const long long row = blockIdx.x;
-    const cpx<R>* x = in + row * in_pitch;
-    for (int j = threadIdx.x; j < d.n; j += blockDim.x) buf[__ldg(d.perm + j)] = x[j];
-    __syncthreads();
-    fft_dit(buf, d, dir);
-    cpx<R>* y = out + row * out_pitch;
-    for (int k = threadIdx.x; k < d.n; k += blockDim.x) y[k] = buf[k];
+// Launch shape of the row kernels.  FP64 is bound by its pipe (1.9 FMAs per
+// clock and SM): a few warps keep it busy, and 256 threads leave radix 8 its
+// registers.
+template <typename R, class F>
+static void rows4_launch(size_t smem, F f) {
+    using std::integral_constant;
+    if constexpr (sizeof(R) == 4) {
+        fft4_launch(smem, f);
+    } else {
+        if (2 * (smem + 1024) <= 228 * 1024) f(integral_constant<int, 256>(), integral_constant<int, 2>());
+        else f(integral_constant<int, 256>(), integral_constant<int, 1>());
+    }
 }
 
+// Where the rows of a launch lie.  Split rows: row r takes every a-th element
+// of line r / a from element r % a on, and its output k is multiplied by
+// exp(dir 2 pi i (r % a) k / n) (tw, n entries).
 template <typename R>
-struct BlueArgs {
-    int n;
-    FftDesc<R> dm;          // length m
-    const cpx<R>* chirp;    // n
-    const cpx<R>* kern;     // m
+struct RowsIo {
+    const cpx<R>* in;
+    long long ip;
+    cpx<R>* out;
+    long long op;
+    int a;               // 1: plain rows
+    const cpx<R>* tw;
+    int dir;
 };
-
 template <typename R>
-__global__ void __launch_bounds__(kFftThreads) k_fft_blue(const cpx<R>* __restrict__ in, long long in_pitch,
-                                                         cpx<R>* __restrict__ out, long long out_pitch,
-                                                         BlueArgs<R> b, int dir) {
+__device__ __forceinline__ void rows_put(const RowsIo<R>& io, cpx<R>* y, int k, int off, cpx<R> v) {
+    if (io.dir > 0) v = conj(v);
+    if (io.a > 1) {
+        cpx<R> w = ldg(io.tw + (long long)off * k);
+        if (io.dir > 0) w = conj(w);
+        v = cmul4(v, w);
+    }
+    y[k] = v;
+}
+
+// Rows of a 7-smooth length: out[k] = sum_j in[j] exp(dir 2 pi i j k / n).
+// The core transforms forward; dir = +1 conjugates both ends.
+template <typename R, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_rows_smooth(RowsIo<R> io, Fft4DescT<R> d) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cpx<R>* buf = reinterpret_cast<cpx<R>*>(smem_raw);
-    const long long row = blockIdx.x;
-    const cpx<R>* x = in + row * in_pitch;
-    const int m = b.dm.n;
-    for (int q = threadIdx.x; q < m; q += blockDim.x) {
-        cpx<R> v = mk((R)0, (R)0);
-        if (q < b.n) {
-            cpx<R> xv = x[q];
-            if (dir > 0) xv = conj(xv);
-            v = xv * ldg(b.chirp + q);
-        }
-        buf[__ldg(b.dm.perm + q)] = v;
-    }
-    __syncthreads();
-    fft_dit(buf, b.dm, -1);
-    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = buf[q] * ldg(b.kern + q);
-    __syncthreads();
-    fft_dif(buf, b.dm, +1);
-    cpx<R>* y = out + row * out_pitch;
-    for (int k = threadIdx.x; k < b.n; k += blockDim.x) {
-        cpx<R> v = ldg(b.chirp + k) * buf[__ldg(b.dm.perm + k)];
-        y[k] = dir > 0 ? conj(v) : v;
+    const long long line = blockIdx.x / io.a;
+    const int off = (int)(blockIdx.x - line * io.a);
+    const cpx<R>* x = io.in + line * io.ip + off;
+    cpx<R>* y = io.out + (long long)blockIdx.x * io.op;
+    fft4_head(buf, d, [&](int j) {
+        const cpx<R> v = x[(long long)j * io.a];
+        return io.dir > 0 ? conj(v) : v;
+    });
+    fft4_spectrum(buf, d);
+    for (int k = threadIdx.x; k < d.n; k += NT) rows_put(io, y, k, off, buf[pad16(__ldg(d.pos + k))]);
+}
+
+// Rows of any length n by Bluestein's identity over a convolution of d.n.
+template <typename R, int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_rows_blue(RowsIo<R> io, Fft4DescT<R> d, int n,
+                                                      const cpx<R>* __restrict__ chirp,
+                                                      const cpx<R>* __restrict__ kern) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cpx<R>* buf = reinterpret_cast<cpx<R>*>(smem_raw);
+    const long long line = blockIdx.x / io.a;
+    const int off = (int)(blockIdx.x - line * io.a);
+    const cpx<R>* x = io.in + line * io.ip + off;
+    cpx<R>* y = io.out + (long long)blockIdx.x * io.op;
+    fft4_head(buf, d, [&](int j) {
+        if (j >= n) return mk((R)0, (R)0);
+        const cpx<R> v = x[(long long)j * io.a];
+        return cmul4(io.dir > 0 ? conj(v) : v, ldg(chirp + j));
+    });
+    fft4_mid(buf, d, [&](int m, cpx<R> v) { return cmul4(v, ldg(kern + m)); });
+    fft4_tail(buf, d, [&](int k, cpx<R> v) {
+        if (k < n) rows_put(io, y, k, off, cmul4(v, ldg(chirp + k)));
+    });
+}
+
+// a-point transforms across the a split rows of a line: out[k + b k1].
+template <typename R, int A>
+__device__ __forceinline__ void split_out(const cpx<R>* y, cpx<R>* out, int b, int k, int dir) {
+    cpx<R> v[A];
+#pragma unroll
+    for (int r = 0; r < A; ++r) v[r] = y[(long long)r * b + k];
+    if (dir > 0) Dft<R, A, +1>::run(v);
+    else Dft<R, A, -1>::run(v);
+#pragma unroll
+    for (int j = 0; j < A; ++j) out[k + (long long)j * b] = v[j];
+}
+template <typename R>
+__global__ void __launch_bounds__(256) k_split_out(const cpx<R>* __restrict__ y, cpx<R>* __restrict__ out,
+                                                   long long op, int a, int b, int dir) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= b) return;
+    y += (long long)blockIdx.y * a * b;
+    out += (long long)blockIdx.y * op;
+    switch (a) {
+        case 2: split_out<R, 2>(y, out, b, k, dir); break;
+        case 3: split_out<R, 3>(y, out, b, k, dir); break;
+        case 4: split_out<R, 4>(y, out, b, k, dir); break;
+        case 5: split_out<R, 5>(y, out, b, k, dir); break;
+        case 6: split_out<R, 6>(y, out, b, k, dir); break;
+        case 7: split_out<R, 7>(y, out, b, k, dir); break;
+        case 8: split_out<R, 8>(y, out, b, k, dir); break;
+        case 9: split_out<R, 9>(y, out, b, k, dir); break;
+        case 10: split_out<R, 10>(y, out, b, k, dir); break;
+        case 12: split_out<R, 12>(y, out, b, k, dir); break;
+        case 15: split_out<R, 15>(y, out, b, k, dir); break;
+        default: split_out<R, 16>(y, out, b, k, dir); break;
     }
 }
 
@@ -274,10 +353,12 @@ __global__ void k_blue_post(const cpx<R>* __restrict__ a, int m, cpx<R>* __restr
     }
 }
 
+// out[at[i]] = in[i] scale (at null: out[i])
 template <typename R>
-__global__ void k_cvt64(const cpx<double>* __restrict__ in, cpx<R>* __restrict__ out, long long n, double scale) {
+__global__ void k_cvt64(const cpx<double>* __restrict__ in, cpx<R>* __restrict__ out, long long n, double scale,
+                        const int* __restrict__ at) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
-        out[i] = mk((R)(in[i].x * scale), (R)(in[i].y * scale));
+        out[at ? at[i] : i] = mk((R)(in[i].x * scale), (R)(in[i].y * scale));
 }
 
 static int grid_for(long long total, int threads = 256) {
@@ -325,8 +406,12 @@ static inline void unit_root(long long num, long long den, double& c, double& s)
     s = -std::sin(a);
 }
 
+FftDescTables::~FftDescTables() {
+    for (void* p : owned) cudaFree(p);
+}
+
 template <typename R>
-static void fill_desc(FftPlan<R>& p, FftDesc<R>& d, int n) {
+static void fill_desc(FftDescTables& t, FftDesc<R>& d, int n) {
     std::vector<int> rad;
     radices_for(n, rad);
     if ((int)rad.size() > kMaxStages) throw std::runtime_error("fft: too many stages");
@@ -350,20 +435,15 @@ static void fill_desc(FftPlan<R>& p, FftDesc<R>& d, int n) {
         }
         perm[j] = pos;
     }
-    d.tw = (const cpx<R>*)upload(p, tw.data(), sizeof(cpx<R>) * n);
-    d.perm = (const int*)upload(p, perm.data(), sizeof(int) * n);
-}
-
-template <typename R>
-static void set_smem_attr() {
-    static bool done = false;
-    if (!done) {
-        check_cuda(cudaFuncSetAttribute(k_fft_smem<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes),
-                   "smem attr");
-        check_cuda(cudaFuncSetAttribute(k_fft_blue<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes),
-                   "smem attr");
-        done = true;
-    }
+    auto up = [&](const void* src, size_t bytes) {
+        void* v = nullptr;
+        check_cuda(cudaMalloc(&v, bytes), "desc table");
+        t.owned.push_back(v);
+        check_cuda(cudaMemcpy(v, src, bytes, cudaMemcpyHostToDevice), "desc upload");
+        return v;
+    };
+    d.tw = (const cpx<R>*)up(tw.data(), sizeof(cpx<R>) * n);
+    d.perm = (const int*)up(perm.data(), sizeof(int) * n);
 }
 
 static void split_four(int n, int cap, int& n1, int& n2) {
@@ -379,10 +459,7 @@ static void split_four(int n, int cap, int& n1, int& n2) {
     n2 = n / best;
 }
 
-FftEngine::FftEngine(cudaStream_t s) : stream(s) {
-    set_smem_attr<float>();
-    set_smem_attr<double>();
-}
+FftEngine::FftEngine(cudaStream_t s) : stream(s) {}
 FftEngine::~FftEngine() = default;
 
 template <typename R>
@@ -392,6 +469,82 @@ std::map<int, std::shared_ptr<FftPlan<float>>>& plan_map<float>(FftEngine& e) { 
 template <>
 std::map<int, std::shared_ptr<FftPlan<double>>>& plan_map<double>(FftEngine& e) { return e.plans64; }
 
+// w, w^2, w^4, w^8 of w = exp(sign 2 pi i num / den)
+template <typename R>
+static Tw4<R> twiddle_entry(long long num, long long den, int sign) {
+    cpx<R> w[4];
+    for (int b = 0; b < 4; ++b) {
+        double c, s;
+        unit_root(num * (1 << b), den, c, s);   // exp(-)
+        w[b] = mk((R)c, (R)(sign > 0 ? -s : s));
+    }
+    return Tw4<R>{w[0], w[1], w[2], w[3]};
+}
+
+template <typename R>
+std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad) {
+    if (rad.empty() || (int)rad.size() > kFft4Passes || sizeof(cpx<R>) * padded16_len(n) > (size_t)kFft4SmemBytes)
+        throw std::runtime_error("plan4: length " + std::to_string(n) + " not smooth/small");
+    long long prod = 1;
+    for (int r : rad) {
+        if (std::find(std::begin(kRadices), std::end(kRadices), r) == std::end(kRadices))
+            throw std::runtime_error("plan4: radix");
+        prod *= r;
+    }
+    if (prod != n) throw std::runtime_error("plan4: radices do not multiply to the length");
+    auto p = std::make_shared<Fft4PlanT<R>>();
+    Fft4DescT<R>& d = p->d;
+    d.n = n;
+    d.np = (int)rad.size();
+    d.affine = sizeof(R) == 4 && d.np >= 2 && rad.back() == 16 && fft4_end_radix(rad[0]);
+    // block g of a pass holds the input modulo x^len - exp(-2 pi i F[g] / N)
+    std::vector<long long> F{0};
+    std::vector<Tw4<R>> tab;
+    size_t fo[kFft4Passes], io[kFft4Passes];
+    long long N = 1;
+    int Ns = n;
+    for (int q = 0; q < d.np; ++q) {
+        const int r = rad[q];
+        d.radix[q] = r;
+        Ns /= r;
+        fo[q] = tab.size();
+        for (long long f : F) tab.push_back(twiddle_entry<R>(f, N * r, -1));
+        io[q] = tab.size();
+        for (int k = 0; k < Ns; ++k) tab.push_back(twiddle_entry<R>(k, (long long)Ns * r, +1));
+        std::vector<long long> G;
+        G.reserve(F.size() * r);
+        for (long long f : F)
+            for (int j = 0; j < r; ++j) G.push_back(f + j * N);
+        F.swap(G);
+        N *= r;
+    }
+    std::vector<int> pos(n);
+    p->mid.resize(n);
+    const int last = rad.back();
+    for (int i = 0; i < n; ++i) {
+        pos[F[i]] = i;
+        p->mid[F[i]] = (i % last) * (n / last) + i / last;
+    }
+    auto up = [&](const void* src, size_t bytes) {
+        void* v = nullptr;
+        check_cuda(cudaMalloc(&v, bytes), "plan4 table");
+        p->owned.push_back(v);
+        check_cuda(cudaMemcpy(v, src, bytes, cudaMemcpyHostToDevice), "plan4 upload");
+        return v;
+    };
+    const Tw4<R>* t = (const Tw4<R>*)up(tab.data(), sizeof(Tw4<R>) * tab.size());
+    for (int q = 0; q < d.np; ++q) {
+        d.fw[q] = t + fo[q];
+        d.iv[q] = t + io[q];
+    }
+    d.pos = (const int*)up(pos.data(), sizeof(int) * n);
+    d.mid = (const int*)up(p->mid.data(), sizeof(int) * n);
+    return p;
+}
+
+template std::shared_ptr<Fft4PlanT<float>> build_plan4<float>(int, const std::vector<int>&);
+template std::shared_ptr<Fft4PlanT<double>> build_plan4<double>(int, const std::vector<int>&);
+
 template <typename R>
 std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     auto& mp = plan_map<R>(*this);
@@ -399,28 +552,75 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     if (it != mp.end()) return it->second;
     auto p = std::make_shared<FftPlan<R>>();
     p->n = n;
-    const int cap = smem_capacity<R>();
-    if (is_smooth7(n) && n <= cap) {
-        p->kind = FFT_SMEM;
-        fill_desc(*p, p->d, n);
-    } else if (is_smooth7(n)) {
-        p->kind = FFT_FOUR;
-        split_four(n, cap, p->n1, p->n2);
-        p->p1 = plan<R>(p->n1);
-        p->p2 = plan<R>(p->n2);
+    const int cap = fft4_capacity<R>();
+    // convolution length of a Bluestein transform of b points: the cheapest
+    // that fits, -1 if none does
+    auto conv_len = [&](long long b) -> long long {
+        if constexpr (sizeof(R) == 4) {
+            return 2 * b - 1 <= cap ? fast_len(2 * b - 1) : -1;
+        } else {
+            long long best = -1;
+            double bc = 1e30;
+            for (long long m = 2 * b - 1; m <= cap && m <= (2 * b - 1) * 5 / 4 + 8; ++m) {
+                const auto r = fft4_order64(m);
+                if (r.empty()) continue;
+                double c = 5.0;
+                for (int x : r) c += (x & (x - 1)) == 0 ? 3.1 * std::log2((double)x) : 4.2 * std::log2((double)x);
+                if (c * m < bc) {
+                    bc = c * m;
+                    best = m;
+                }
+            }
+            return best;
+        }
+    };
+    auto core = [&](int len) {
+        if constexpr (sizeof(R) == 4) return build_plan4<R>(len, fft4_orders(len, 1).at(0));
+        else return build_plan4<R>(len, fft4_order64(len));
+    };
+    const bool fits = n >= 2 && is_smooth7(n) && n <= cap &&
+                      (sizeof(R) == 4 ? !fft4_orders(n, 1).empty() : !fft4_order64(n).empty());
+    const long long mc = fits ? 0 : conv_len(n);
+    int a = 0;   // split n = a b with b of the one-kernel kinds
+    if (!fits && mc < 0)
+        for (int x : {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16})
+            if (n % x == 0) {
+                const auto sub = plan<R>(n / x);
+                if (sub->kind == FFT_SMEM || sub->kind == FFT_BLUE) {
+                    a = x;
+                    break;
+                }
+            }
+    auto roots = [&] {
         std::vector<cpx<R>> tw(n);
         for (int i = 0; i < n; ++i) {
             double c, s;
             unit_root(i, n, c, s);
             tw[i] = mk((R)c, (R)s);
         }
-        p->tw4 = (cpx<R>*)upload(*p, tw.data(), sizeof(cpx<R>) * n);
+        return (cpx<R>*)upload(*p, tw.data(), sizeof(cpx<R>) * n);
+    };
+    if (fits) {
+        p->kind = FFT_SMEM;
+        p->core = core(n);
+    } else if (a) {
+        p->kind = FFT_SPLIT;
+        p->n1 = a;
+        p->n2 = n / a;
+        p->p2 = plan<R>(p->n2);
+        p->tw4 = roots();
+    } else if (mc < 0 && is_smooth7(n)) {
+        p->kind = FFT_FOUR;
+        split_four(n, cap, p->n1, p->n2);
+        p->p1 = plan<R>(p->n1);
+        p->p2 = plan<R>(p->n2);
+        p->tw4 = roots();
     } else {
-        const long long m = next_smooth7(2LL * n - 1);
+        const long long m = mc >= 0 ? mc : next_smooth7(2LL * n - 1);
         p->m = (int)m;
-        if (m <= cap) {
+        if (mc >= 0) {
             p->kind = FFT_BLUE;
-            fill_desc(*p, p->d, (int)m);
+            p->core = core((int)m);
         } else {
             p->kind = FFT_BLUE4;
             p->pm = plan<R>((int)m);
@@ -445,7 +645,8 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
         cpx<R>* kd = nullptr;
         check_cuda(cudaMalloc(&kd, sizeof(cpx<R>) * m), "blue kern");
         p->owned.push_back(kd);
-        note_launch(), k_cvt64<R><<<grid_for(m), 256, 0, stream>>>(d64, kd, m, 1.0 / (double)m);
+        note_launch(), k_cvt64<R><<<grid_for(m), 256, 0, stream>>>(d64, kd, m, 1.0 / (double)m,
+                                                                     p->kind == FFT_BLUE ? p->core->d.mid : nullptr);
         check_cuda(cudaStreamSynchronize(stream), "blue kern sync");
         cudaFree(d64);
         p->kern = kd;
@@ -454,83 +655,10 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     return p;
 }
 
-Fft4Plan::~Fft4Plan() {
-    for (void* p : owned) cudaFree(p);
-}
-
-// w, w^2, w^4, w^8 of w = exp(sign 2 pi i num / den)
-static void twiddle_entry(std::vector<float4>& out, long long num, long long den, int sign) {
-    double c[4], s[4];
-    for (int b = 0; b < 4; ++b) unit_root(num * (1 << b), den, c[b], s[b]);
-    const double g = sign > 0 ? -1.0 : 1.0;   // unit_root gives exp(-)
-    out.push_back(make_float4((float)c[0], (float)(g * s[0]), (float)c[1], (float)(g * s[1])));
-    out.push_back(make_float4((float)c[2], (float)(g * s[2]), (float)c[3], (float)(g * s[3])));
-}
-
-std::shared_ptr<Fft4Plan> build_plan4(int n, const std::vector<int>& rad) {
-    if (rad.empty() || (int)rad.size() > kFft4Passes || sizeof(cf32) * padded16_len(n) > (size_t)kFft4SmemBytes)
-        throw std::runtime_error("plan4: length " + std::to_string(n) + " not smooth/small");
-    long long prod = 1;
-    for (int r : rad) {
-        if (std::find(std::begin(kRadices), std::end(kRadices), r) == std::end(kRadices))
-            throw std::runtime_error("plan4: radix");
-        prod *= r;
-    }
-    if (prod != n) throw std::runtime_error("plan4: radices do not multiply to the length");
-    auto p = std::make_shared<Fft4Plan>();
-    Fft4Desc& d = p->d;
-    d.n = n;
-    d.np = (int)rad.size();
-    d.affine = d.np >= 2 && rad.back() == 16 && fft4_end_radix(rad[0]);
-    // block g of a pass holds the input modulo x^len - exp(-2 pi i F[g] / N)
-    std::vector<long long> F{0};
-    std::vector<float4> tab;
-    size_t fo[kFft4Passes], io[kFft4Passes];
-    long long N = 1;
-    int Ns = n;
-    for (int q = 0; q < d.np; ++q) {
-        const int R = rad[q];
-        d.radix[q] = R;
-        Ns /= R;
-        fo[q] = tab.size();
-        for (long long f : F) twiddle_entry(tab, f, N * R, -1);
-        io[q] = tab.size();
-        for (int k = 0; k < Ns; ++k) twiddle_entry(tab, k, (long long)Ns * R, +1);
-        std::vector<long long> G;
-        G.reserve(F.size() * R);
-        for (long long f : F)
-            for (int j = 0; j < R; ++j) G.push_back(f + j * N);
-        F.swap(G);
-        N *= R;
-    }
-    std::vector<int> pos(n);
-    p->mid.resize(n);
-    const int R = rad.back();
-    for (int i = 0; i < n; ++i) {
-        pos[F[i]] = i;
-        p->mid[F[i]] = (i % R) * (n / R) + i / R;
-    }
-    auto up = [&](const void* src, size_t bytes) {
-        void* v = nullptr;
-        check_cuda(cudaMalloc(&v, bytes), "plan4 table");
-        p->owned.push_back(v);
-        check_cuda(cudaMemcpy(v, src, bytes, cudaMemcpyHostToDevice), "plan4 upload");
-        return v;
-    };
-    const float4* t = (const float4*)up(tab.data(), sizeof(float4) * tab.size());
-    for (int q = 0; q < d.np; ++q) {
-        d.fw[q] = t + fo[q];
-        d.iv[q] = t + io[q];
-    }
-    d.pos = (const int*)up(pos.data(), sizeof(int) * n);
-    d.mid = (const int*)up(p->mid.data(), sizeof(int) * n);
-    return p;
-}
-
 std::shared_ptr<Fft4Plan> FftEngine::plan4(int n) {
     auto it = plans4.find(n);
     if (it != plans4.end()) return it->second;
-    auto p = build_plan4(n, tuned_radices(n, stream));
+    auto p = build_plan4<float>(n, tuned_radices(n, stream));
     plans4[n] = p;
     return p;
 }
@@ -539,9 +667,16 @@ long long FftEngine::tuned_len(long long minlen) { return tuned_length(minlen, s
 
 template <typename R>
 FftDesc<R> FftEngine::smem_desc(int n) {
-    auto p = plan<R>(n);
-    if (p->kind != FFT_SMEM) throw std::runtime_error("smem_desc: length not smooth/small: " + std::to_string(n));
-    return p->d;
+    if (!is_smooth7(n) || n > smem_capacity<R>())
+        throw std::runtime_error("smem_desc: length not smooth/small: " + std::to_string(n));
+    auto& t = (sizeof(R) == 4 ? descs32 : descs64)[n];
+    if (!t) {
+        t = std::make_shared<FftDescTables>();
+        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, n);
+        else fill_desc<R>(*t, t->d64, n);
+    }
+    if constexpr (sizeof(R) == 4) return t->d32;
+    else return t->d64;
 }
 
 template <typename R>
@@ -555,26 +690,42 @@ void transpose_batched(const cpx<R>* in, long long irp, long long ibp, cpx<R>* o
     note_launch(), k_transpose<R><<<grid, dim3(32, 8), 0, s>>>(in, irp, ibp, out, orp, obp, rows, cols);
 }
 
+// rows of a plan of one of the one-kernel kinds
+template <typename R>
+static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows, cudaStream_t st) {
+    const Fft4DescT<R>& d = p.core->d;
+    const size_t smem = sizeof(cpx<R>) * (size_t)padded16_len(d.n);
+    rows4_launch<R>(smem, [&](auto nt, auto mb) {
+        constexpr int NT = decltype(nt)::value, MB = decltype(mb)::value;
+        if (p.kind == FFT_SMEM) {
+            auto kernel = k_rows_smooth<R, NT, MB>;
+            check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFft4SmemBytes), "attr");
+            note_launch(), kernel<<<(unsigned)rows, NT, smem, st>>>(io, d);
+        } else {
+            auto kernel = k_rows_blue<R, NT, MB>;
+            check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFft4SmemBytes), "attr");
+            note_launch(), kernel<<<(unsigned)rows, NT, smem, st>>>(io, d, p.n, p.chirp, p.kern);
+        }
+    });
+}
+
 template <typename R>
 void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out, long long out_pitch,
                      long long batch, int dir) {
     if (batch <= 0) return;
     const int n = p.n;
     switch (p.kind) {
-        case FFT_SMEM: {
-            for (long long b0 = 0; b0 < batch; b0 += 65535LL * 16) {
-                const long long nb = std::min(batch - b0, 65535LL * 16);
-                note_launch(), k_fft_smem<R><<<(unsigned)nb, kFftThreads, sizeof(cpx<R>) * n, stream>>>(
-                    in + b0 * in_pitch, in_pitch, out + b0 * out_pitch, out_pitch, p.d, dir);
-            }
-            break;
-        }
-        case FFT_BLUE: {
-            BlueArgs<R> a{n, p.d, p.chirp, p.kern};
-            for (long long b0 = 0; b0 < batch; b0 += 65535LL * 16) {
-                const long long nb = std::min(batch - b0, 65535LL * 16);
-                note_launch(), k_fft_blue<R><<<(unsigned)nb, kFftThreads, sizeof(cpx<R>) * p.m, stream>>>(
-                    in + b0 * in_pitch, in_pitch, out + b0 * out_pitch, out_pitch, a, dir);
+        case FFT_SMEM:
+        case FFT_BLUE: launch_rows<R>(p, RowsIo<R>{in, in_pitch, out, out_pitch, 1, nullptr, dir}, batch, stream); break;
+        case FFT_SPLIT: {
+            const long long limit = (1LL << 30) / (long long)sizeof(cpx<R>);
+            const long long chunk = std::max(1LL, std::min(std::min(batch, limit / n), 65535LL));
+            cpx<R>* Y = (cpx<R>*)scratch_a.get(sizeof(cpx<R>) * chunk * n);
+            for (long long b0 = 0; b0 < batch; b0 += chunk) {
+                const long long nb = std::min(chunk, batch - b0);
+                launch_rows<R>(*p.p2, RowsIo<R>{in + b0 * in_pitch, in_pitch, Y, p.n2, p.n1, p.tw4, dir}, nb * p.n1, stream);
+                note_launch(), k_split_out<R><<<dim3((p.n2 + 255) / 256, (unsigned)nb), 256, 0, stream>>>(
+                    Y, out + b0 * out_pitch, out_pitch, p.n1, p.n2, dir);
             }
             break;
         }

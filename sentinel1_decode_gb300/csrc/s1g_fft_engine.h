@@ -2,12 +2,15 @@
 //
 // Plan kinds, chosen by length n and precision:
 //   SMEM      n is 7-smooth and fits one CTA's shared memory: one kernel, one
-//             CTA per row, in-place DIT;
+//             CTA per row, over the core of s1g_fft4.cuh;
 //   BLUE      n has a prime factor > 7: Bluestein chirp-z through a 7-smooth
 //             convolution length m >= 2n-1 that fits shared memory;
+//   SPLIT     n = a b too long for either, a <= 16 and b of the first two
+//             kinds: a kernel of the b-point transforms of every a-th element
+//             with the twiddles of the split, and one of the a-point ones;
 //   FOUR      n is 7-smooth but too long: four-step (n = n1*n2) through global
 //             memory with batched transposes;
-//   BLUE4     Bluestein whose convolution length needs the four-step path.
+//   BLUE4     Bluestein whose convolution length needs SPLIT or FOUR.
 // Every transform is unnormalised; dir=-1 forward, dir=+1 backward.
 #pragma once
 
@@ -21,7 +24,7 @@
 
 namespace s1g {
 
-enum FftKind { FFT_SMEM = 0, FFT_BLUE = 1, FFT_FOUR = 2, FFT_BLUE4 = 3 };
+enum FftKind { FFT_SMEM = 0, FFT_BLUE = 1, FFT_FOUR = 2, FFT_BLUE4 = 3, FFT_SPLIT = 4 };
 
 // Largest shared-memory buffer a CTA may use (bytes).
 constexpr int kSmemBytes = 220 * 1024;
@@ -36,6 +39,9 @@ constexpr int kFft4SmemBytes = 227 * 1024;
 long long fast_len(long long minlen);
 template <typename R>
 inline int smem_capacity() { return kSmemBytes / (int)sizeof(cpx<R>); }
+// Longest transform of the core that fits a CTA.
+template <typename R>
+inline int fft4_capacity() { return (kFft4SmemBytes / (int)sizeof(cpx<R>) - 1) * 16 / 17; }
 
 // Device memory arena owned by a processing context: grow-only scratch.
 struct DeviceArena {
@@ -45,27 +51,39 @@ struct DeviceArena {
     void* get(size_t bytes);
 };
 
+// Device tables of the core (s1g_fft4.cuh) for one length.
+template <typename R>
+struct Fft4PlanT {
+    Fft4DescT<R> d;
+    std::vector<int> mid;         // host copy of d.mid
+    std::vector<void*> owned;
+    ~Fft4PlanT() {
+        for (void* p : owned) cudaFree(p);
+    }
+};
+using Fft4Plan = Fft4PlanT<float>;
+
 template <typename R>
 struct FftPlan {
     int n = 0;
     FftKind kind = FFT_SMEM;
-    FftDesc<R> d;                 // SMEM: length n; BLUE: length m
+    std::shared_ptr<Fft4PlanT<R>> core;   // SMEM: length n; BLUE: length m
     int m = 0;                    // Bluestein convolution length
     cpx<R>* chirp = nullptr;      // w[k] = exp(-i pi k^2 / n), k < n
-    cpx<R>* kern = nullptr;       // FFT_m of conj chirp, scaled by 1/m
-    int n1 = 0, n2 = 0;           // four-step split (FOUR) of n, or of m (BLUE4)
-    std::shared_ptr<FftPlan<R>> p1, p2, pm;   // sub-plans
-    cpx<R>* tw4 = nullptr;        // four-step twiddle table, length n (or m)
+    cpx<R>* kern = nullptr;       // FFT_m of conj chirp, scaled by 1/m (BLUE: at core->d.mid)
+    int n1 = 0, n2 = 0;           // split of n: FOUR n1 x n2, SPLIT n1 = a, n2 = b
+    std::shared_ptr<FftPlan<R>> p1, p2, pm;   // sub-plans (SPLIT: p2 of length b)
+    cpx<R>* tw4 = nullptr;        // exp(-2 pi i k / n) of the split, length n
     std::vector<void*> owned;     // device allocations
     ~FftPlan();
 };
 
-// Device tables of the fused kernels' core (s1g_fft4.cuh) for one length.
-struct Fft4Plan {
-    Fft4Desc d;
-    std::vector<int> mid;         // host copy of d.mid
+// Tables of a FftDesc (s1g_fft.cuh).
+struct FftDescTables {
+    FftDesc<float> d32;
+    FftDesc<double> d64;
     std::vector<void*> owned;
-    ~Fft4Plan();
+    ~FftDescTables();
 };
 
 // One per processing context (device + stream).
@@ -75,6 +93,7 @@ struct FftEngine {
     cudaStream_t stream;
     std::map<int, std::shared_ptr<FftPlan<float>>> plans32;
     std::map<int, std::shared_ptr<FftPlan<double>>> plans64;
+    std::map<int, std::shared_ptr<FftDescTables>> descs32, descs64;   // smem_desc
     std::map<int, std::shared_ptr<Fft4Plan>> plans4;
     DeviceArena scratch_a, scratch_b, scratch_c;
 
@@ -103,9 +122,12 @@ struct FftEngine {
 // Radix orders for length n in the order of their modelled cost (at most
 // `most`; affine ones where there are any); empty if n is not 7-smooth.
 std::vector<std::vector<int>> fft4_orders(long long n, size_t most);
+// The order of the row engine's FP64 transforms (radices up to 8: registers).
+std::vector<int> fft4_order64(long long n);
 // The cheapest affine lengths >= minlen that fit shared memory.
 std::vector<long long> fft4_lengths(long long minlen, size_t most);
-std::shared_ptr<Fft4Plan> build_plan4(int n, const std::vector<int>& radices);
+template <typename R>
+std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& radices);
 // Radix order for length n: the fastest measured candidate when tuning is on
 // (S1G_AUTOTUNE unset or not "0"), else the model's.  Measurements run on
 // `st` (skipped while st is being captured) and persist in a text file

@@ -165,7 +165,6 @@ void roll_rows(const cpx<R>* in, long long in_pitch, cpx<R>* out, long long out_
 template <typename R>
 void dc_sums(const cpx<R>* rc, long long pitch, int n_a, int n_r, const cpx<R>* deramp, cf64* sums,
              cudaStream_t st);
-void dc_fit(const cf64* sums, const DcFitArgs& a, double* f_dc, cudaStream_t st);
 template <typename R>
 void fufr_prep(const cpx<R>* X, long long xpitch, int n_a, cpx<R>* y, long long ypitch, int S, int tile_len,
                const cpx<R>* deramp, long long rows, cudaStream_t st);

@@ -173,121 +173,6 @@ void dc_sums(const cpx<R>* rc, long long p, int n_a, int n_r, const cpx<R>* d, c
     note_launch(), k_dc_sums<R><<<(n_r + 127) / 128, 128, 0, st>>>(rc, p, n_a, n_r, d, sums);
 }
 
-// get_doppler_centroid after the sums: block means, get_unwrapped_estimates
-// (doppler.cpp:42-95), polyfit (signal_processing.cpp:159-214), evaluation.
-__global__ void k_dc_fit(const cf64* sums, DcFitArgs a, double* f_dc) {
-    __shared__ double fine[64];
-    __shared__ double poly[3];
-    const int n = a.n_rng;
-    const int nb = a.num_blocks;
-    // wrapped estimates into f_dc (temporary)
-    for (int j = threadIdx.x; j < n; j += blockDim.x)
-        f_dc[j] = -a.prf * atan2(sums[j].y, sums[j].x) / (2 * kPI);
-    __syncthreads();
-    const int bs = n / nb;
-    for (int b = threadIdx.x; b < nb; b += blockDim.x) {
-        const int s = b * bs;
-        const int e = (s + bs < n) ? s + bs : n - 1;
-        double acc = 0.0;
-        for (int j = s; j < e; ++j) acc += f_dc[j];
-        fine[b] = acc / ((double)e - (double)s);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        const int dense = 8;
-        const int m = nb * dense;
-        const float dt = (float)(a.rt[1] - a.rt[0]);
-        // F = floor(|exp(2 pi i dc/prf)|) for the estimates, zero padded
-        double best = -1.0;
-        int bi = 0;
-        double bre = 0.0, bim = 0.0;
-        for (int k = 0; k < m; ++k) {
-            double re = 0.0, im = 0.0;
-            for (int j = 0; j < nb; ++j) {
-                double s, c;
-                sincos((2.0 * kPI) * fine[j] / a.prf, &s, &c);
-                const double f = floor(hypot(c, s));
-                if (f == 0.0) continue;
-                double ws, wc;
-                sincospi(-2.0 * (double)((long long)j * k % m) / (double)m, &ws, &wc);
-                re += f * wc;
-                im += f * ws;
-            }
-            const double mag = hypot(re, im);
-            const double p2 = mag * mag;
-            if (p2 > best) {
-                best = p2;
-                bi = k;
-                bre = re;
-                bim = im;
-            }
-        }
-        const double val = 1.0 / (m * (double)dt);
-        const int N = (m - 1) / 2 + 1;
-        const double v = bi < N ? bi * val : (bi - m) * val;
-        const double aa = v / (double)dt;
-        const double bb = atan2(bim, bre) / (2.0 * kPI);
-        double un[64];
-        for (int j = 0; j < nb; ++j) {
-            double s1, c1, s2, c2;
-            sincos((2.0 * kPI) * fine[j] / a.prf, &s1, &c1);
-            sincos(-1.0 * (aa * a.rt[j] + bb), &s2, &c2);
-            const double pr = c1 * c2 - s1 * s2, pi_ = c1 * s2 + s1 * c2;
-            const double res = atan2(pi_, pr) / (2.0 * kPI);
-            un[j] = (aa * a.rt[j] + bb + res) * a.prf;
-        }
-        // polyfit, degree 2
-        double Sx[5] = {0, 0, 0, 0, 0}, Sy[3] = {0, 0, 0};
-        for (int i = 0; i < nb; ++i) {
-            double xi = 1.0;
-            for (int j = 0; j <= 4; ++j) {
-                if (j <= 2) Sy[j] += xi * un[i];
-                Sx[j] += xi;
-                xi *= a.rt[i];
-            }
-        }
-        double A[3][3] = {{Sx[0], Sx[1], Sx[2]}, {Sx[1], Sx[2], Sx[3]}, {Sx[2], Sx[3], Sx[4]}};
-        double B[3] = {Sy[0], Sy[1], Sy[2]};
-        for (int i = 0; i < 3; ++i) {
-            for (int k = i + 1; k < 3; ++k) {
-                if (fabs(A[k][i]) > fabs(A[i][i])) {
-                    for (int j = 0; j < 3; ++j) {
-                        const double t = A[i][j];
-                        A[i][j] = A[k][j];
-                        A[k][j] = t;
-                    }
-                    const double t = B[i];
-                    B[i] = B[k];
-                    B[k] = t;
-                }
-            }
-            for (int k = i + 1; k < 3; ++k) {
-                const double f = A[k][i] / A[i][i];
-                for (int j = i; j < 3; ++j) A[k][j] -= f * A[i][j];
-                B[k] -= f * B[i];
-            }
-        }
-        double c[3];
-        for (int i = 2; i >= 0; --i) {
-            c[i] = B[i];
-            for (int j = i + 1; j < 3; ++j) c[i] -= A[i][j] * c[j];
-            c[i] /= A[i][i];
-        }
-        poly[0] = c[0];
-        poly[1] = c[1];
-        poly[2] = c[2];
-    }
-    __syncthreads();
-    const double step = (a.far - a.near) / (n - 1);
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
-        const double t = (a.near + j * step) - a.near;
-        f_dc[j] = (poly[0] + poly[1] * t + poly[2] * t * t);
-    }
-}
-void dc_fit(const cf64* sums, const DcFitArgs& a, double* f_dc, cudaStream_t st) {
-    note_launch(), k_dc_fit<<<1, 256, 0, st>>>(sums, a, f_dc);
-}
-
 // ------------------------------------------------------------------ frequency UFR
 // y[k] = shifted_X[k mod n_a] * deramp[k] for k < tile_len (get_tiled_signal,
 // image_formation.cpp:87-122, after the azimuth fftshift, :139-140).
