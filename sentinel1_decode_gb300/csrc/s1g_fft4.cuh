@@ -338,7 +338,10 @@ __device__ __forceinline__ void pass4_r(cpx<T>* buf, int n, int Ns, const Tw4<T>
 
 // One pass with twiddles over shared memory (caller synchronises).
 template <int DIR, bool AFF, typename T>
-__device__ __noinline__ void pass4(cpx<T>* buf, int R, int n, int Ns, const Tw4<T>* tw) {
+__device__ __noinline__ void pass4(unsigned int smem, int R, int n, int Ns, const Tw4<T>* tw) {
+    // behind the call a pointer would be generic: the shared-space address
+    // keeps the accesses LDS / STS
+    cpx<T>* buf = reinterpret_cast<cpx<T>*>(__cvta_shared_to_generic(smem));
     switch (R) {
         case 2: pass4_r<2, DIR, AFF>(buf, n, Ns, tw); break;
         case 3: pass4_r<3, DIR, AFF>(buf, n, Ns, tw); break;
@@ -365,11 +368,11 @@ template <int DIR, typename T>
 __device__ __forceinline__ void pass4_any(cpx<T>* buf, const Fft4DescT<T>& d, int R, int Ns, const Tw4<T>* tw) {
     if constexpr (sizeof(T) == 4) {
         if (d.affine) {
-            pass4<DIR, true>(buf, R, d.n, Ns, tw);
+            pass4<DIR, true, T>((unsigned int)__cvta_generic_to_shared(buf), R, d.n, Ns, tw);
             return;
         }
     }
-    pass4<DIR, false>(buf, R, d.n, Ns, tw);
+    pass4<DIR, false, T>((unsigned int)__cvta_generic_to_shared(buf), R, d.n, Ns, tw);
 }
 
 template <int R, typename T, class LoadF>
@@ -474,14 +477,14 @@ __device__ __forceinline__ void fft4_mid(cpx<T>* buf, const Fft4DescT<T>& d, Mid
     if (!done) {
         // the last pass, the factor and the first inverse pass (no twiddles) apart
         const int R = d.radix[d.np - 1], nb = d.n / R;
-        pass4<-1, false>(buf, R, d.n, 1, d.fw[d.np - 1]);
+        pass4_any<-1>(buf, d, R, 1, d.fw[d.np - 1]);
         __syncthreads();
         for (int i = threadIdx.x; i < d.n; i += blockDim.x) {
             const int g = i / R;
             buf[pad16(i)] = mid((i - g * R) * nb + g, buf[pad16(i)]);
         }
         __syncthreads();
-        pass4<+1, false>(buf, R, d.n, 1, d.iv[d.np - 1]);
+        pass4_any<+1>(buf, d, R, 1, d.iv[d.np - 1]);
     }
     __syncthreads();
 }
