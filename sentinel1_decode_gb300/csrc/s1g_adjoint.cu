@@ -10,11 +10,17 @@
 //   Y = IFFT_az(Z),  L = -sum p ln p, p = |Y|^2 / sum |Y|^2
 //
 // and its adjoint carries G = dL/dRe + i dL/dIm back through the same
-// transforms.  Phases are formed in FP64 (they reach ~10^3 rad) and reduced
-// before the FP32 sine / cosine; reductions accumulate in FP64.
+// transforms.  Phases (they reach ~10^3 rad) are formed in FP64, in the FP32
+// chain as fractions of a turn in 64-bit fixed point or double-float, and
+// reduced before the FP32 sine / cosine; reductions accumulate in FP64, in the
+// FP32 chain in double-float within a thread.  GB300 does 1.9 FP64 operations
+// per clock and SM, so FP64 per element bounded these kernels: the five took
+// 1.6 of the 2.5 ms of a 1024 x 4096 evaluation's device time, now 0.42 of 1.44 ms.
 #include <algorithm>
 #include <cmath>
+#include <mutex>
 
+#include "s1g_df.cuh"
 #include "s1g_kernels.h"
 
 namespace s1g {
@@ -73,6 +79,41 @@ __global__ void k_rcmc_phase(cpx<R>* a, int n, long long rows, const double* __r
     }
 }
 
+// cos, sin of 2 pi (hi + lo) turns, |hi + lo| <= 1/2: the angle is formed to
+// 2^-46 and rounded to float once, as cis_d<float> rounds its FP64 angle, so
+// the factors are those of the FP64 phases but where 2^-46 decides the
+// rounding (under one in 10^3 elements).
+__device__ __forceinline__ cf32 cis_turn(float hi, float lo) {
+    const df p = two_prod(hi, 6.283185482025146484375f);   // 2 pi as 24 bits + the rest
+    const float r = p.hi + fmaf(hi, -1.74845560007449713e-7f, fmaf(lo, 6.28318530717958648f, p.lo));
+    float s, c;
+    __sincosf(r, &s, &c);
+    return mk(c, s);
+}
+
+// FP32: the phase is linear in the signed frequency index, so a row's step is
+// a fraction of a turn in 64-bit fixed point (2^-53 of a turn off per index)
+// and an index takes one integer product.
+__global__ void __launch_bounds__(256) k_rcmc_phase32(cf32* a, int n, const double* __restrict__ beta, double fs, int sign) {
+    __shared__ unsigned long long step;
+    const int k = blockIdx.y;
+    if (threadIdx.x == 0) {
+        const double t = (double)sign * beta[k] * fs / (double)n / 6.283185307179586476925;
+        const double f = (t - floor(t)) * 4294967296.0;
+        const double h = floor(f);
+        step = ((unsigned long long)h << 32) + (unsigned long long)((f - h) * 4294967296.0);
+    }
+    __syncthreads();
+    cf32* row = a + (long long)k * n;
+    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < n; f += gridDim.x * blockDim.x) {
+        const long long q = f < (n + 1) / 2 ? f : f - n;
+        const long long ph = (long long)((unsigned long long)q * step);
+        // the top 24 bits and the next 24, both exact as floats
+        row[f] = cmul_(row[f], cis_turn((float)(int)(ph >> 40) * 5.9604644775390625e-8f,
+                                        (float)(int)((ph >> 16) & 0xffffff) * 3.552713678800501e-15f));
+    }
+}
+
 template <typename R>
 __global__ void k_az_filter(cpx<R>* a, int n_r, long long rows, const double* __restrict__ omd,
                             const double* __restrict__ slant, double c4pl, int sign) {
@@ -83,14 +124,99 @@ __global__ void k_az_filter(cpx<R>* a, int n_r, long long rows, const double* __
     }
 }
 
+// FP32: a thread keeps one range bin's 2 R_r / lambda (turns) as a
+// double-float over the rows it takes.
+constexpr int kAzRows = 16;
+__global__ void __launch_bounds__(256) k_az_filter32(cf32* a, int n_r, int rows, const double* __restrict__ omd,
+                                                     const double* __restrict__ slant, double c4pl, int sign) {
+    __shared__ df w[kAzRows];
+    const int k0 = blockIdx.y * kAzRows;
+    const int nk = min(kAzRows, rows - k0);
+    if (threadIdx.x < nk) w[threadIdx.x] = df_from((double)sign * omd[k0 + threadIdx.x]);
+    __syncthreads();
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n_r) return;
+    const df t = df_from(c4pl * slant[r] * 0.15915494309189533577);
+    for (int k = 0; k < nk; ++k) {
+        const df u = df_mul(t, w[k]);
+        cf32* p = a + (long long)(k0 + k) * n_r + r;
+        *p = cmul_(*p, cis_turn(u.hi - rintf(u.hi), u.lo));
+    }
+}
+
+// ln x of a normal FP64 x > 0 in double-float arithmetic, error below 1e-12
+// (FP64 log takes ~40 operations of a pipe that does 1.9 per clock and SM):
+// x = 2^e m with m in [1, 2) from the bits, c = 1/m to 8 bits (table of 128 by
+// the leading bits of m), r = m c - 1 exactly by one FMA (|r| < 2^-7), ln x =
+// e ln 2 - ln c + log1p(r) (Tang, "Table-driven implementation of the
+// logarithm function", 1990), the series' first two terms in double-float.
+__device__ float c_log_c[128];     // global, not constant: lanes read different entries
+__device__ float2 c_log_t[128];    // -ln c as hi, lo
+__device__ __forceinline__ df ln_fast(double x) {
+    const unsigned int xh = (unsigned int)__double2hiint(x), xl = (unsigned int)__double2loint(x);
+    const int e = (int)(xh >> 20) - 1023;
+    // 23 leading bits of the fraction, then the other 29
+    const unsigned int f = ((xh & 0xfffffu) << 3) | (xl >> 29);
+    const float m = __int_as_float((int)(0x3f800000u | f));
+    const float ml = (float)(int)(xl & 0x1fffffffu) * 2.220446049250313e-16f;   // 2^-52
+    const int i = (int)(f >> 16);
+    const float r = __fmaf_rn(m, __ldg(c_log_c + i), -1.0f);
+    const float2 t = __ldg(c_log_t + i);
+    const df r2 = two_prod(r, r);
+    // r^3 (1/3 - r/4 + r^2/5 - r^3/6 + r^4/7), and the low part of x
+    const float p = fmaf(r, fmaf(r, fmaf(r, fmaf(r, 1.0f / 7.0f, -1.0f / 6.0f), 0.2f), -0.25f), 1.0f / 3.0f);
+    const float rest = fmaf(r2.hi * r, p, __fdividef(ml, m));
+    const float ef = (float)e;
+    // e ln 2 with ln 2 = 0x1.62e4p-1 (exact products) + 1.4286068202862268e-6
+    const df el = two_prod(ef, 1.42860677e-6f);
+    df s = quick_two_sum(ef * 0.693145751953125f, el.hi);
+    s.lo += el.lo + ef * 5.4956e-14f;
+    s = df_add_abs(s, df_make(t.x, t.y));
+    s = df_add_f(s, r);
+    s = df_add_abs(s, df_make(-0.5f * r2.hi, -0.5f * r2.lo));
+    return df_add_f(s, rest);
+}
+// tables of ln_df, once per device
+static void init_log_tables() {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "log tables");
+    std::lock_guard<std::mutex> lk(mu);
+    if (dev < 64 && done[dev]) return;
+    float c[128];
+    float2 t[128];
+    for (int i = 0; i < 128; ++i) {
+        const double mid = 1.0 + (i + 0.5) / 128.0;
+        const double q = std::rint(256.0 / mid) / 256.0;   // 8 bits after the point, exact products with m
+        c[i] = (float)q;
+        const double l = -std::log(q);
+        t[i].x = (float)l;
+        t[i].y = (float)(l - (double)t[i].x);
+    }
+    check_cuda(cudaMemcpyToSymbol(c_log_c, c, sizeof(c)), "log tables");
+    check_cuda(cudaMemcpyToSymbol(c_log_t, t, sizeof(t)), "log tables");
+    if (dev < 64) done[dev] = true;
+}
+
+// ln of |v|^2; zero gives 0 (its weight is zero)
+template <typename R>
+__device__ __forceinline__ double ln_norm(double I) {
+    if constexpr (sizeof(R) == 4) {
+        if (I >= 2.2250738585072014e-308) return df_to_double(ln_fast(I));
+    }
+    return I > 0.0 ? log(I) : 0.0;
+}
+
 // sums[0] += sum |y|^2, sums[1] += sum |y|^2 ln |y|^2
 template <typename R>
 __global__ void k_entropy_sums(const cpx<R>* __restrict__ y, long long n, double* sums) {
     double s = 0.0, t = 0.0;
     ADJ_GRID_STRIDE(i, n) {
-        const double I = (double)y[i].x * y[i].x + (double)y[i].y * y[i].y;
+        const cpx<R> v = y[i];
+        const double I = (double)v.x * v.x + (double)v.y * v.y;
         s += I;
-        if (I > 0.0) t += I * log(I);
+        t += I * ln_norm<R>(I);
     }
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_down_sync(0xffffffffu, s, o);
@@ -119,10 +245,11 @@ __global__ void k_entropy_grad(const cpx<R>* y, cpx<R>* g, long long n, const do
     const double S = sums[0];
     const double lnS = log(S);
     const double H = sums[1] / S - lnS;
+    const double off = lnS + H, k = -2.0 / S;
     ADJ_GRID_STRIDE(i, n) {
         const cpx<R> v = y[i];
         const double I = (double)v.x * v.x + (double)v.y * v.y;
-        const double d = I > 0.0 ? -2.0 * (log(I) - lnS - H) / S : 0.0;
+        const double d = I > 0.0 ? k * (ln_norm<R>(I) - off) : 0.0;
         g[i] = mk((R)(d * v.x), (R)(d * v.y));
     }
 }
@@ -136,10 +263,26 @@ __global__ void k_row_imdot(const cpx<R>* __restrict__ a, const cpx<R>* __restri
     const cpx<R>* ar = a + row * cols;
     const cpx<R>* br = b + row * cols;
     double acc = 0.0;
-    for (int c = threadIdx.x; c < cols; c += blockDim.x) {
-        const double im = (double)ar[c].x * br[c].y - (double)ar[c].y * br[c].x;
-        const double w = colw ? colw[c] : (freq_fs > 0.0 ? fft_freq(c, cols, freq_fs) : 1.0);
-        acc += w * im;
+    if constexpr (sizeof(R) == 4) {
+        // a thread's share in double-float; the frequency weight as the signed
+        // index, times fs / cols at the end
+        df s = df_make(0.f, 0.f);
+        for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+            const df p = two_prod(ar[c].x, br[c].y), q = two_prod(-ar[c].y, br[c].x);
+            df im = two_sum(p.hi, q.hi);
+            im.lo += p.lo + q.lo;
+            if (colw) im = df_mul(im, df_from(colw[c]));
+            else if (freq_fs > 0.0) im = df_mul_f(im, (float)(c < (cols + 1) / 2 ? c : c - cols));
+            s = df_add_abs(s, im);
+        }
+        acc = df_to_double(s);
+        if (!colw && freq_fs > 0.0) acc *= freq_fs / (double)cols;
+    } else {
+        for (int c = threadIdx.x; c < cols; c += blockDim.x) {
+            const double im = (double)ar[c].x * br[c].y - (double)ar[c].y * br[c].x;
+            const double w = colw ? colw[c] : (freq_fs > 0.0 ? fft_freq(c, cols, freq_fs) : 1.0);
+            acc += w * im;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
     __shared__ double wa[32];
@@ -159,15 +302,29 @@ void row_factor(cpx<R>* a, long long pitch, int cols, long long rows, const cpx<
 }
 template <typename R>
 void rcmc_phase(cpx<R>* a, int n, long long rows, const double* beta, double fs, int sign, cudaStream_t st) {
-    note_launch(), k_rcmc_phase<R><<<grid_for(rows * n), 256, 0, st>>>(a, n, rows, beta, fs, sign);
+    if constexpr (sizeof(R) == 4) {
+        // one launch per 65535 rows
+        for (long long r0 = 0; r0 < rows; r0 += 65535) {
+            const unsigned nr = (unsigned)std::min<long long>(65535, rows - r0);
+            note_launch(), k_rcmc_phase32<<<dim3((n + 1023) / 1024, nr), 256, 0, st>>>(a + r0 * n, n, beta + r0, fs, sign);
+        }
+    } else {
+        note_launch(), k_rcmc_phase<R><<<grid_for(rows * n), 256, 0, st>>>(a, n, rows, beta, fs, sign);
+    }
 }
 template <typename R>
 void az_filter(cpx<R>* a, int n_r, long long rows, const double* omd, const double* slant, double c4pl, int sign,
                cudaStream_t st) {
-    note_launch(), k_az_filter<R><<<grid_for(rows * n_r), 256, 0, st>>>(a, n_r, rows, omd, slant, c4pl, sign);
+    if constexpr (sizeof(R) == 4) {
+        note_launch(), k_az_filter32<<<dim3((n_r + 255) / 256, (unsigned)((rows + kAzRows - 1) / kAzRows)), 256, 0, st>>>(
+            a, n_r, (int)rows, omd, slant, c4pl, sign);
+    } else {
+        note_launch(), k_az_filter<R><<<grid_for(rows * n_r), 256, 0, st>>>(a, n_r, rows, omd, slant, c4pl, sign);
+    }
 }
 template <typename R>
 void entropy_sums(const cpx<R>* y, long long n, double* sums, cudaStream_t st) {
+    if constexpr (sizeof(R) == 4) init_log_tables();
     check_cuda(cudaMemsetAsync(sums, 0, 2 * sizeof(double), st), "entropy reset");
     note_launch(), k_entropy_sums<R><<<grid_for(n), 256, 0, st>>>(y, n, sums);
 }

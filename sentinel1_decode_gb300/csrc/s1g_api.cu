@@ -387,8 +387,8 @@ struct Pipe {
     }
 
     void fft_rows(int n, const cpx<R>* in, long long ip, cpx<R>* out, long long op, long long rows, int dir) {
-        auto p = fft.plan<R>(n);
-        fft.rows<R>(*p, in, ip, out, op, rows, dir);
+        if constexpr (sizeof(R) == 4) fft.rows<R>(*fft.plan8(n), in, ip, out, op, rows, dir);
+        else fft.rows<R>(*fft.plan<R>(n), in, ip, out, op, rows, dir);
     }
 
     // decode -> [n_a][n_r] in buffer A
@@ -490,7 +490,7 @@ struct Pipe {
         convert_rows<float, double>(a64, n_r, out, n_r, n_r, n_r, n_a, st);
         Pipe<float> p32(h);
         cf32* B = h->bB.as<cf32>((size_t)n_a * n_r);
-        p32.fft_rows(n_r, out, n_r, B, n_r, n_a, -1);
+        h->fft->rows<float>(*h->fft->plan<float>(n_r), out, n_r, B, n_r, n_a, -1);
         int* flags = h->bFlags.as<int>(n_a);
         eccm_detect_mixed(B, n_r, n_r, n_a, (double)h->det, a64, n_r, h->bEccmRoots.as<cf64>(n_r), flags, st);
         auto& cp = h->cffts[128];
@@ -615,7 +615,7 @@ struct Pipe {
             rate = dc_rate(g);
             h->mark("doppler");
             // FP32: formed from FP64 lines before this burst's own (run)
-            fdc = sizeof(R) == 4 ? (double*)h->bCols.p : doppler(A, g, rate);
+            fdc = doppler(A, g, rate);
             h->mark("freq_unfold");
             // azimuth_frequency_ufr (image_formation.cpp:125-219)
             nrep = std::abs(rate * g.T / g.prf);
@@ -731,16 +731,6 @@ struct Pipe {
             throw S1Error(S1G_E_UNSUPPORTED, "sinc RCMC: only the FP32 precision (S1G_PREC_FP32) has it");
         const BurstGeom g = make_geom(h->hdr, pk);
         cur_pk = &pk;
-        if constexpr (sizeof(R) == 4) {
-            // The rounding of FP32 range-compressed lines (2e-7) moves the
-            // Doppler centroid by up to 1e-5 Hz and the SLC by up to 1.3e-4:
-            // the lag-1 sums take FP64 lines.
-            if (level == S1G_AZIMUTH_COMPRESSED && tops) {
-                h->mark("doppler");
-                Pipe<double> p64(h);
-                p64.doppler(p64.range_compress(p64.decode(pk, g), g, false), g, dc_rate(g));
-            }
-        }
         h->mark("decode");
         cpx<R>* A = decode(pk, g);
         h->mark("range_compress");
@@ -1472,7 +1462,7 @@ struct FastPipe {
             cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
             cf32* Ct = h->bD.as<cf32>((size_t)n_a * n_r);
             transpose_batched<float>(rc, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
-            plain.fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, -1);
+            fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, -1);
             roll_rows<float>(Bt, n_a, Ct, n_a, n_a, n_a / 2, n_r, st);
             transpose_batched<float>(Ct, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st);
         }
@@ -1516,7 +1506,7 @@ struct FastPipe {
         h->mark("azimuth_ifft");
         cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
         transpose_batched<float>(rd, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
-        plain.fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, +1);
+        fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, +1);
         scale_rows<float>(Bt, n_a, n_a, n_r, 1.0 / n_a, st);
         transpose_batched<float>(Bt, n_a, 0, rd, n_r, 0, n_r, n_a, 1, st);
         Result r;

@@ -280,6 +280,59 @@ __global__ void __launch_bounds__(256) k_split_out(const cpx<R>* __restrict__ y,
     }
 }
 
+// The radix-8 plans' kernels (plan8): one CTA per row, digit-reversed into
+// shared memory, in-place passes.
+constexpr int kFftThreads = 512;
+__global__ void __launch_bounds__(kFftThreads) k_rows8_smooth(const cf32* __restrict__ in, long long in_pitch,
+                                                         cf32* __restrict__ out, long long out_pitch,
+                                                         FftDesc<float> d, int dir) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cf32* buf = reinterpret_cast<cf32*>(smem_raw);
+    const long long row = blockIdx.x;
+    const cf32* x = in + row * in_pitch;
+    for (int j = threadIdx.x; j < d.n; j += blockDim.x) buf[__ldg(d.perm + j)] = x[j];
+    __syncthreads();
+    fft_dit(buf, d, dir);
+    cf32* y = out + row * out_pitch;
+    for (int k = threadIdx.x; k < d.n; k += blockDim.x) y[k] = buf[k];
+}
+
+struct BlueArgs {
+    int n;
+    FftDesc<float> dm;          // length m
+    const cf32* chirp;    // n
+    const cf32* kern;     // m
+};
+
+__global__ void __launch_bounds__(kFftThreads) k_rows8_blue(const cf32* __restrict__ in, long long in_pitch,
+                                                         cf32* __restrict__ out, long long out_pitch,
+                                                         BlueArgs b, int dir) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cf32* buf = reinterpret_cast<cf32*>(smem_raw);
+    const long long row = blockIdx.x;
+    const cf32* x = in + row * in_pitch;
+    const int m = b.dm.n;
+    for (int q = threadIdx.x; q < m; q += blockDim.x) {
+        cf32 v = mk(0.0f, 0.0f);
+        if (q < b.n) {
+            cf32 xv = x[q];
+            if (dir > 0) xv = conj(xv);
+            v = xv * ldg(b.chirp + q);
+        }
+        buf[__ldg(b.dm.perm + q)] = v;
+    }
+    __syncthreads();
+    fft_dit(buf, b.dm, -1);
+    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = buf[q] * ldg(b.kern + q);
+    __syncthreads();
+    fft_dif(buf, b.dm, +1);
+    cf32* y = out + row * out_pitch;
+    for (int k = threadIdx.x; k < b.n; k += blockDim.x) {
+        cf32 v = ldg(b.chirp + k) * buf[__ldg(b.dm.perm + k)];
+        y[k] = dir > 0 ? conj(v) : v;
+    }
+}
+
 // 32x32 tiled transpose of a batch of matrices.
 template <typename R>
 __global__ void k_transpose(const cpx<R>* __restrict__ in, long long irp, long long ibp, cpx<R>* __restrict__ out,
@@ -463,13 +516,14 @@ FftEngine::FftEngine(cudaStream_t s) : stream(s) {}
 FftEngine::~FftEngine() = default;
 
 template <typename R>
-static std::map<int, std::shared_ptr<FftPlan<R>>>& plan_map(FftEngine& e);
+static std::map<int, std::shared_ptr<FftPlan<R>>>& plan_map(FftEngine& e, bool radix8);
 template <>
-std::map<int, std::shared_ptr<FftPlan<float>>>& plan_map<float>(FftEngine& e) { return e.plans32; }
+std::map<int, std::shared_ptr<FftPlan<float>>>& plan_map<float>(FftEngine& e, bool radix8) {
+    return radix8 ? e.plans8 : e.plans32;
+}
 template <>
-std::map<int, std::shared_ptr<FftPlan<double>>>& plan_map<double>(FftEngine& e) { return e.plans64; }
+std::map<int, std::shared_ptr<FftPlan<double>>>& plan_map<double>(FftEngine& e, bool) { return e.plans64; }
 
-// w, w^2, w^4, w^8 of w = exp(sign 2 pi i num / den)
 template <typename R>
 static Tw4<R> twiddle_entry(long long num, long long den, int sign) {
     cpx<R> w[4];
@@ -546,16 +600,21 @@ template std::shared_ptr<Fft4PlanT<float>> build_plan4<float>(int, const std::ve
 template std::shared_ptr<Fft4PlanT<double>> build_plan4<double>(int, const std::vector<int>&);
 
 template <typename R>
-std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
-    auto& mp = plan_map<R>(*this);
+static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
+    auto& mp = plan_map<R>(e, radix8);
     auto it = mp.find(n);
     if (it != mp.end()) return it->second;
+    cudaStream_t stream = e.stream;
     auto p = std::make_shared<FftPlan<R>>();
     p->n = n;
-    const int cap = fft4_capacity<R>();
+    const int cap = radix8 ? smem_capacity<R>() : fft4_capacity<R>();
     // convolution length of a Bluestein transform of b points: the cheapest
     // that fits, -1 if none does
     auto conv_len = [&](long long b) -> long long {
+        if (radix8) {
+            const long long m = next_smooth7(2 * b - 1);
+            return m <= cap ? m : -1;
+        }
         if constexpr (sizeof(R) == 4) {
             return 2 * b - 1 <= cap ? fast_len(2 * b - 1) : -1;
         } else {
@@ -578,14 +637,23 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
         if constexpr (sizeof(R) == 4) return build_plan4<R>(len, fft4_orders(len, 1).at(0));
         else return build_plan4<R>(len, fft4_order64(len));
     };
-    const bool fits = n >= 2 && is_smooth7(n) && n <= cap &&
+    auto desc = [&](int len) {
+        for (auto k : {(const void*)k_rows8_smooth, (const void*)k_rows8_blue})
+            check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "smem attr");
+        auto t = std::make_shared<FftDescTables>();
+        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, len);
+        else fill_desc<R>(*t, t->d64, len);
+        return t;
+    };
+    const bool fits = radix8 ? is_smooth7(n) && n <= cap :
+                      n >= 2 && is_smooth7(n) && n <= cap &&
                       (sizeof(R) == 4 ? !fft4_orders(n, 1).empty() : !fft4_order64(n).empty());
     const long long mc = fits ? 0 : conv_len(n);
     int a = 0;   // split n = a b with b of the one-kernel kinds
-    if (!fits && mc < 0)
+    if (!fits && mc < 0 && !radix8)
         for (int x : {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16})
             if (n % x == 0) {
-                const auto sub = plan<R>(n / x);
+                const auto sub = make_plan<R>(e, n / x, radix8);
                 if (sub->kind == FFT_SMEM || sub->kind == FFT_BLUE) {
                     a = x;
                     break;
@@ -602,28 +670,30 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     };
     if (fits) {
         p->kind = FFT_SMEM;
-        p->core = core(n);
+        if (radix8) p->desc = desc(n);
+        else p->core = core(n);
     } else if (a) {
         p->kind = FFT_SPLIT;
         p->n1 = a;
         p->n2 = n / a;
-        p->p2 = plan<R>(p->n2);
+        p->p2 = make_plan<R>(e, p->n2, radix8);
         p->tw4 = roots();
     } else if (mc < 0 && is_smooth7(n)) {
         p->kind = FFT_FOUR;
         split_four(n, cap, p->n1, p->n2);
-        p->p1 = plan<R>(p->n1);
-        p->p2 = plan<R>(p->n2);
+        p->p1 = make_plan<R>(e, p->n1, radix8);
+        p->p2 = make_plan<R>(e, p->n2, radix8);
         p->tw4 = roots();
     } else {
         const long long m = mc >= 0 ? mc : next_smooth7(2LL * n - 1);
         p->m = (int)m;
         if (mc >= 0) {
             p->kind = FFT_BLUE;
-            p->core = core((int)m);
+            if (radix8) p->desc = desc((int)m);
+            else p->core = core((int)m);
         } else {
             p->kind = FFT_BLUE4;
-            p->pm = plan<R>((int)m);
+            p->pm = make_plan<R>(e, (int)m, radix8);
         }
         // chirp w[k] = exp(-i pi k^2/n) = exp(-2 pi i (k^2 mod 2n)/(2n))
         std::vector<cpx<R>> w(n);
@@ -637,16 +707,16 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
         }
         p->chirp = (cpx<R>*)upload(*p, w.data(), sizeof(cpx<R>) * n);
         // kernel spectrum computed in FP64 on the device, scaled by 1/m
-        auto p64 = plan<double>((int)m);
+        auto p64 = make_plan<double>(e, (int)m, false);
         cpx<double>* d64 = nullptr;
         check_cuda(cudaMalloc(&d64, sizeof(cpx<double>) * m), "blue tmp");
         check_cuda(cudaMemcpy(d64, b.data(), sizeof(cpx<double>) * m, cudaMemcpyHostToDevice), "blue up");
-        rows<double>(*p64, d64, m, d64, m, 1, -1);
+        e.rows<double>(*p64, d64, m, d64, m, 1, -1);
         cpx<R>* kd = nullptr;
         check_cuda(cudaMalloc(&kd, sizeof(cpx<R>) * m), "blue kern");
         p->owned.push_back(kd);
         note_launch(), k_cvt64<R><<<grid_for(m), 256, 0, stream>>>(d64, kd, m, 1.0 / (double)m,
-                                                                     p->kind == FFT_BLUE ? p->core->d.mid : nullptr);
+                                                                     p->core ? p->core->d.mid : nullptr);
         check_cuda(cudaStreamSynchronize(stream), "blue kern sync");
         cudaFree(d64);
         p->kern = kd;
@@ -654,6 +724,10 @@ std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) {
     mp[n] = p;
     return p;
 }
+
+template <typename R>
+std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) { return make_plan<R>(*this, n, false); }
+std::shared_ptr<FftPlan<float>> FftEngine::plan8(int n) { return make_plan<float>(*this, n, true); }
 
 std::shared_ptr<Fft4Plan> FftEngine::plan4(int n) {
     auto it = plans4.find(n);
@@ -693,6 +767,22 @@ void transpose_batched(const cpx<R>* in, long long irp, long long ibp, cpx<R>* o
 // rows of a plan of one of the one-kernel kinds
 template <typename R>
 static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows, cudaStream_t st) {
+    if constexpr (sizeof(R) == 4) {
+        if (p.desc) {
+            for (long long b0 = 0; b0 < rows; b0 += 65535LL * 16) {
+                const unsigned nb = (unsigned)std::min(rows - b0, 65535LL * 16);
+                const cf32* in = io.in + b0 * io.ip;
+                cf32* out = io.out + b0 * io.op;
+                if (p.kind == FFT_SMEM)
+                    note_launch(), k_rows8_smooth<<<nb, kFftThreads, sizeof(cf32) * p.n, st>>>(
+                        in, io.ip, out, io.op, p.desc->d32, io.dir);
+                else
+                    note_launch(), k_rows8_blue<<<nb, kFftThreads, sizeof(cf32) * p.m, st>>>(
+                        in, io.ip, out, io.op, BlueArgs{p.n, p.desc->d32, p.chirp, p.kern}, io.dir);
+            }
+            return;
+        }
+    }
     const Fft4DescT<R>& d = p.core->d;
     const size_t smem = sizeof(cpx<R>) * (size_t)padded16_len(d.n);
     rows4_launch<R>(smem, [&](auto nt, auto mb) {

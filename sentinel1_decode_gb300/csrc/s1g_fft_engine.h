@@ -12,6 +12,14 @@
 //             memory with batched transposes;
 //   BLUE4     Bluestein whose convolution length needs SPLIT or FOUR.
 // Every transform is unnormalised; dir=-1 forward, dir=+1 backward.
+//
+// plan8 gives FP32 plans (SMEM, BLUE, FOUR, BLUE4) over the radix-8 core of
+// s1g_fft.cuh instead.  The plain FP32 pipelines and the differentiable chains
+// use them: a focus gradient is a sum that cancels to 1e-4 of its terms, so it
+// moves by up to 1e-4 with the rounding of the transforms, and so do decisions
+// of the plain pipelines at their thresholds.  Those paths keep one arithmetic
+// (a 1024 x 4096 evaluation's ten transforms: 0.71 ms, 0.42 over the other
+// core).
 #pragma once
 
 #include <map>
@@ -63,11 +71,20 @@ struct Fft4PlanT {
 };
 using Fft4Plan = Fft4PlanT<float>;
 
+// Tables of a FftDesc (s1g_fft.cuh).
+struct FftDescTables {
+    FftDesc<float> d32;
+    FftDesc<double> d64;
+    std::vector<void*> owned;
+    ~FftDescTables();
+};
+
 template <typename R>
 struct FftPlan {
     int n = 0;
     FftKind kind = FFT_SMEM;
     std::shared_ptr<Fft4PlanT<R>> core;   // SMEM: length n; BLUE: length m
+    std::shared_ptr<FftDescTables> desc;  // the same of a plan8 (no core)
     int m = 0;                    // Bluestein convolution length
     cpx<R>* chirp = nullptr;      // w[k] = exp(-i pi k^2 / n), k < n
     cpx<R>* kern = nullptr;       // FFT_m of conj chirp, scaled by 1/m (BLUE: at core->d.mid)
@@ -78,14 +95,6 @@ struct FftPlan {
     ~FftPlan();
 };
 
-// Tables of a FftDesc (s1g_fft.cuh).
-struct FftDescTables {
-    FftDesc<float> d32;
-    FftDesc<double> d64;
-    std::vector<void*> owned;
-    ~FftDescTables();
-};
-
 // One per processing context (device + stream).
 struct FftEngine {
     explicit FftEngine(cudaStream_t s);
@@ -93,12 +102,14 @@ struct FftEngine {
     cudaStream_t stream;
     std::map<int, std::shared_ptr<FftPlan<float>>> plans32;
     std::map<int, std::shared_ptr<FftPlan<double>>> plans64;
+    std::map<int, std::shared_ptr<FftPlan<float>>> plans8;
     std::map<int, std::shared_ptr<FftDescTables>> descs32, descs64;   // smem_desc
     std::map<int, std::shared_ptr<Fft4Plan>> plans4;
     DeviceArena scratch_a, scratch_b, scratch_c;
 
     template <typename R>
     std::shared_ptr<FftPlan<R>> plan(int n);
+    std::shared_ptr<FftPlan<float>> plan8(int n);
 
     // out[b*out_pitch + k] = sum_j in[b*in_pitch + j] exp(dir 2 pi i jk/n).
     // in may equal out.  Works for any n >= 1.
