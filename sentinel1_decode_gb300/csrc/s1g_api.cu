@@ -57,6 +57,14 @@ struct Buf {
     }
 };
 
+// Range reference function of the plain pipelines on the device.
+struct RangeRef {
+    int M = 0;
+    double energy = 0;
+    std::vector<double> chirp;   // re, im of the replica it belongs to
+    Buf dev;
+};
+
 struct Result {   // a product left in device memory
     const void* ptr = nullptr;
     long long rows = 0, cols = 0, pitch = 0;
@@ -95,6 +103,7 @@ struct s1g_decoder {
     IndexScratch isc;
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
+    RangeRef ref32, ref64;
     Buf bFdf, bFit, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
     Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
     Buf bTuD, bTuG, bTuI, bTuW, bTuR, bTuWt, bTuRamp, bKa0;   // time-unfolding per-burst tables and grids
@@ -117,6 +126,24 @@ struct s1g_decoder {
     std::map<std::string, std::shared_ptr<struct SwathDecode>> swath_decodes;
     Result last;
     double last_ms = 0;
+    // Status words of a product call, read back with its one synchronisation:
+    // [0] corner-turn flag, [1] time unfolding, [2..] decode status per packet
+    // (of pending's packets).  Page-locked; only while defer_status is set.
+    int* pin = nullptr;
+    size_t pin_cap = 0;
+    bool defer_status = false;
+    const std::vector<int>* pending = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    int* pinned(size_t n) {
+        if (n > pin_cap) {
+            if (pin) cudaFreeHost(pin);
+            pin = nullptr;
+            pin_cap = 0;
+            check_cuda(cudaMallocHost(&pin, sizeof(int) * n), "status words");
+            pin_cap = n;
+        }
+        return pin;
+    }
     std::string stage_text;
     bool stage_timing = false;
     double ingest_ms = 0;           // s1g_open_file: map + staged upload
@@ -164,6 +191,9 @@ struct s1g_decoder {
     ~s1g_decoder() {
         for (auto e : slot_done) cudaEventDestroy(e);
         if (copy_stream) cudaStreamDestroy(copy_stream);
+        if (ev0) cudaEventDestroy(ev0);
+        if (ev1) cudaEventDestroy(ev1);
+        if (pin) cudaFreeHost(pin);
         if (d_stream) cudaFree(d_stream);
         if (d_off) cudaFree(d_off);
         if (stream) cudaStreamDestroy(stream);
@@ -370,6 +400,17 @@ static const std::vector<int>& burst_packets(s1g_decoder* h, const std::string& 
     return it->second[burst];
 }
 
+// Throws for the first packet of pk whose decode failed.
+static void check_decode_status(const int* status, const std::vector<int>& pk) {
+    static const char* names[] = {"", "", "", "", "", "", "", "packet length", "bit read past end",
+                                  "BRC value is invalid.", "Max bit length exceeded in Huffman decoding.",
+                                  "MCode is greater than the comparison flag.", "ragged burst",
+                                  "BAQ Mode is invalid."};
+    for (size_t i = 0; i < pk.size(); ++i)
+        if (const int c = status[i])
+            throw S1Error(c, std::string("packet ") + std::to_string(pk[i]) + ": " + (c >= -13 ? names[-c] : "decode error"));
+}
+
 // ------------------------------------------------------------------ per-burst pipeline
 template <typename R>
 struct Pipe {
@@ -411,18 +452,16 @@ struct Pipe {
         if (any_fixed)
             decode_fixed_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status,
                                   h->abc_fields, st);
+        if (h->defer_status) {
+            int* pin = h->pinned((size_t)npk + 2);
+            check_cuda(cudaMemcpyAsync(pin + 2, status, sizeof(int) * npk, cudaMemcpyDeviceToHost, st), "status");
+            h->pending = &pk;
+            return A;
+        }
         std::vector<int> hs(npk);
         check_cuda(cudaMemcpyAsync(hs.data(), status, sizeof(int) * npk, cudaMemcpyDeviceToHost, st), "status");
         check_cuda(cudaStreamSynchronize(st), "decode sync");
-        for (int i = 0; i < npk; ++i)
-            if (hs[i]) {
-                static const char* names[] = {"", "", "", "", "", "", "", "packet length", "bit read past end",
-                                              "BRC value is invalid.", "Max bit length exceeded in Huffman decoding.",
-                                              "MCode is greater than the comparison flag.", "ragged burst",
-                                              "BAQ Mode is invalid."};
-                const int c = hs[i];
-                throw S1Error(c, std::string("packet ") + std::to_string(pk[i]) + ": " + (c >= -13 ? names[-c] : "decode error"));
-            }
+        check_decode_status(hs.data(), pk);
         return A;
     }
 
@@ -510,8 +549,12 @@ struct Pipe {
             }
         }
         const int M = (int)next_smooth7((long long)n_r + g.L);
-        // reference function at length M: conj(FFT_M(chirp at [0,L))) / (E * M)
-        {
+        // reference function at length M: conj(FFT_M(chirp at [0,L))) / (E * M),
+        // kept with the plans while the chirp stays
+        RangeRef& rr = sizeof(R) == 4 ? h->ref32 : h->ref64;
+        if (rr.M != M || rr.energy != g.energy || rr.chirp.size() != 2 * g.chirp.size() ||
+            std::memcmp(rr.chirp.data(), g.chirp.data(), sizeof(g.chirp[0]) * g.chirp.size()) != 0) {
+            rr.M = 0;
             std::vector<cpx<double>> c((size_t)M, mk(0.0, 0.0));
             for (int t = 0; t < g.L; ++t) c[t] = g.chirp[t];
             cf64* dc = (cf64*)h->bTab.get(sizeof(cf64) * M);
@@ -524,9 +567,13 @@ struct Pipe {
             std::vector<cpx<R>> ref(M);
             const double s = 1.0 / (g.energy * (double)M);
             for (int k = 0; k < M; ++k) ref[k] = mk((R)(spec[k].x * s), (R)(-spec[k].y * s));
-            upload(h->bRef, ref);
+            upload(rr.dev, ref);
+            check_cuda(cudaStreamSynchronize(st), "ref sync");
+            rr.chirp.assign((const double*)g.chirp.data(), (const double*)(g.chirp.data() + g.chirp.size()));
+            rr.energy = g.energy;
+            rr.M = M;
         }
-        const cpx<R>* ref = (const cpx<R>*)h->bRef.p;
+        const cpx<R>* ref = (const cpx<R>*)rr.dev.p;
         cpx<R>* B = h->bB.as<cpx<R>>((size_t)n_a * M);
         pad_rows<R>(A, n_r, n_r, B, M, M, n_a, st);
         fft_rows(M, B, M, B, M, n_a, -1);
@@ -1666,33 +1713,47 @@ static const cf32* swath_cached_decode(s1g_decoder* h, const std::vector<int>& p
 static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int level, bool tops) {
     for (auto& m : h->marks) cudaEventDestroy(m.second);
     h->marks.clear();
-    cudaEvent_t e0, e1;
-    cudaEventCreate(&e0);
-    cudaEventCreate(&e1);
-    cudaEventRecord(e0, h->stream);
+    if (!h->ev0) check_cuda(cudaEventCreate(&h->ev0), "event");
+    if (!h->ev1) check_cuda(cudaEventCreate(&h->ev1), "event");
+    cudaEventRecord(h->ev0, h->stream);
     Result r;
-    if (h->precision == S1G_PREC_FP64) r = Pipe<double>(h).run(pk, level, tops);
-    else if (h->precision == S1G_PREC_FP32_PLAIN) r = Pipe<float>(h).run(pk, level, tops);
-    else {
-        FastPipe fp(h);
-        fp.predecoded = swath_cached_decode(h, pk);
-        r = fp.run(pk, level, tops);
+    // the decode status comes back with the other status words below; where a
+    // later stage fails first, the decode's error is still the one reported
+    h->pending = nullptr;
+    h->defer_status = true;
+    auto decode_ok = [&] {
+        if (h->pending) check_decode_status(h->pin + 2, *h->pending);
+    };
+    try {
+        if (h->precision == S1G_PREC_FP64) r = Pipe<double>(h).run(pk, level, tops);
+        else if (h->precision == S1G_PREC_FP32_PLAIN) r = Pipe<float>(h).run(pk, level, tops);
+        else {
+            FastPipe fp(h);
+            fp.predecoded = swath_cached_decode(h, pk);
+            r = fp.run(pk, level, tops);
+        }
+    } catch (...) {
+        h->defer_status = false;
+        if (h->pending && cudaStreamSynchronize(h->stream) == cudaSuccess) decode_ok();
+        throw;
     }
-    cudaEventRecord(e1, h->stream);
-    check_cuda(cudaEventSynchronize(e1), "product");
+    h->defer_status = false;
+    cudaEventRecord(h->ev1, h->stream);
+    int* pin = h->pin ? h->pin : h->pinned(2);
+    tma_read_error(pin, h->stream);
+    if (r.status) check_cuda(cudaMemcpyAsync(pin + 1, r.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "tufr status");
+    check_cuda(cudaStreamSynchronize(h->stream), "product");
     float ms = 0;
-    cudaEventElapsedTime(&ms, e0, e1);
+    cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     h->last_ms = ms;
     h->close_marks();
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
     check_cuda(cudaGetLastError(), "product kernels");
-    if (tma_take_error() != 0) throw S1Error(S1G_E_TIMEOUT, "a TMA corner turn gave up waiting for its tile");
-    if (r.status) {
-        int st = 0;
-        check_cuda(cudaMemcpy(&st, r.status, sizeof(int), cudaMemcpyDeviceToHost), "tufr status");
-        if (st) throw S1Error(S1G_E_GEOMETRY, "azimuth time unfolding parameters out of range");
+    decode_ok();
+    if (pin[0] != 0) {
+        tma_take_error();
+        throw S1Error(S1G_E_TIMEOUT, "a TMA corner turn gave up waiting for its tile");
     }
+    if (r.status && pin[1]) throw S1Error(S1G_E_GEOMETRY, "azimuth time unfolding parameters out of range");
     return r;
 }
 

@@ -216,6 +216,10 @@ int tma_take_error() {
     return e;
 }
 
+void tma_read_error(int* pinned, cudaStream_t st) {
+    check_cuda(cudaMemcpyFromSymbolAsync(pinned, g_tma_error, sizeof(int), 0, cudaMemcpyDeviceToHost, st), "tma flag");
+}
+
 }  // namespace s1g
 
 using namespace s1g;

@@ -16,4 +16,8 @@ bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int ro
 // Synchronous: call it after the work has been waited for.
 int tma_take_error();
 
+// Queue a copy of the flag tma_take_error reads to page-locked host memory on
+// st, without clearing it.
+void tma_read_error(int* pinned, cudaStream_t st);
+
 }  // namespace s1g
