@@ -119,6 +119,7 @@ struct s1g_decoder {
     std::map<int, std::shared_ptr<struct FastBurst>> fast_bursts;
     std::map<std::tuple<int, int, int>, std::shared_ptr<struct CztTables>> czts;
     std::map<int, std::shared_ptr<s1g::CfftPlan>> cffts;   // compensated FFT plans by length
+    std::map<int, std::shared_ptr<s1g::DcFftPlan>> dc_plans;   // Doppler-estimator blocks by length
     std::map<std::string, std::shared_ptr<struct BatchDecode>> batch_decodes;   // by swath/level
     // every burst of a swath decoded in one launch pair for the per-burst
     // FP32 calls (built on the first such call, dropped when the stream
@@ -1144,7 +1145,7 @@ struct FastBurst {          // per-burst tables of the fast path
     // Doppler estimator: overlap-save block, its compensated FFT and filter,
     // and the lag-1 deramp products
     int dcB = 0, dcU = 0, dcNb = 0;
-    s1g::CfftDesc dcDesc;
+    s1g::DcFft dcDesc;
     float4 *dcH = nullptr, *dcG = nullptr;
     int na_smooth = 0, nr_smooth = 0;
     s1g::Fft4Desc dna, dnr;
@@ -1382,8 +1383,8 @@ struct FastPipe {
             // compensated overlap-save range compression for the lag-1 sums
             if (!choose_dc_block(n_r, g.L, fb->dcB, fb->dcU, fb->dcNb))
                 throw S1Error(S1G_E_GEOMETRY, "chirp too long for the Doppler estimator");
-            auto& cp = h->cffts[fb->dcB];
-            if (!cp) cp = make_cfft_plan(fb->dcB);
+            auto& cp = h->dc_plans[fb->dcB];
+            if (!cp) cp = make_dc_plan(fb->dcB);
             fb->dcDesc = cp->d;
             {
                 const int B = fb->dcB;
@@ -1400,7 +1401,7 @@ struct FastPipe {
                 std::vector<float4> Hb(B);
                 for (int k = 0; k < B; ++k) {
                     const df re = df_from(spec[k].x * sc), im = df_from(-spec[k].y * sc);
-                    Hb[k] = make_float4(re.hi, im.hi, re.lo, im.lo);
+                    Hb[cp->at[k]] = make_float4(re.hi, im.hi, re.lo, im.lo);
                 }
                 fb->dcH = fb->up(Hb, st);
             }

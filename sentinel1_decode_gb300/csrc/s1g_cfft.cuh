@@ -58,11 +58,11 @@ __device__ __forceinline__ cc cc_mul(const cc& a, float wx, float wy, float wlx,
     const df p1 = two_prod(a.hx, wx);
     const df p2 = two_prod(a.hy, wy);
     const df s = two_sum(p1.hi, -p2.hi);
-    const float er = s.lo + (p1.lo - p2.lo) + (a.hx * wlx - a.hy * wly) + (a.ex * wx - a.ey * wy);
+    const float er = fmaf(a.ex, wx, fmaf(-a.ey, wy, fmaf(a.hx, wlx, fmaf(-a.hy, wly, s.lo + (p1.lo - p2.lo)))));
     const df q1 = two_prod(a.hx, wy);
     const df q2 = two_prod(a.hy, wx);
     const df t = two_sum(q1.hi, q2.hi);
-    const float ei = t.lo + (q1.lo + q2.lo) + (a.hx * wly + a.hy * wlx) + (a.ex * wy + a.ey * wx);
+    const float ei = fmaf(a.ex, wy, fmaf(a.ey, wx, fmaf(a.hx, wly, fmaf(a.hy, wlx, t.lo + (q1.lo + q2.lo)))));
     return cc{s.hi, t.hi, er, ei};
 }
 
@@ -119,90 +119,82 @@ struct CBfly<3> {
     }
 };
 
-template <int P>
-__device__ __forceinline__ void cdit_stage(cf32* H, cf32* E, const CfftDesc& d, int Ns, int dir) {
-    const int n = d.n;
-    const int nb = n / P;
-    const int span = Ns * P;
-    const int step = n / span;
-    const float inv = 1.0f / (float)Ns;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-        int g, k;
-        split_idx(t, Ns, inv, g, k);
-        const int base = g * span + k;
-        cc a[P];
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const int i = pad(base + r * Ns);
-            a[r] = cc_make(H[i], E[i]);
-        }
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < P; ++r) a[r] = cc_twiddle(a[r], d.tw, r * k * step, dir);
-        }
-        CBfly<P>::run(a, dir);
-#pragma unroll
-        for (int s = 0; s < P; ++s) {
-            const int i = pad(base + s * Ns);
-            H[i] = mk(a[s].hx, a[s].hy);
-            E[i] = mk(a[s].ex, a[s].ey);
-        }
+// times exp(DIR 2 pi i NUM / 48) for the composite radices below
+template <int NUM, int DIR>
+__device__ __forceinline__ cc cc_root48(const cc& a) {
+    static_assert(NUM >= 0 && NUM < 48, "");
+    if constexpr (NUM == 0) return a;
+    else if constexpr (NUM == 24) return cc{-a.hx, -a.hy, -a.ex, -a.ey};
+    else if constexpr (NUM > 24) {
+        const cc t = cc_root48<NUM - 24, DIR>(a);
+        return cc{-t.hx, -t.hy, -t.ex, -t.ey};
+    } else if constexpr (NUM >= 12) return cc_mul_i(cc_root48<NUM - 12, DIR>(a), DIR);
+    else if constexpr (NUM == 6) {
+        // (1 + DIR i) / sqrt 2
+        const df x = two_sum(a.hx, DIR > 0 ? -a.hy : a.hy), y = two_sum(a.hy, DIR > 0 ? a.hx : -a.hx);
+        const cc z{x.hi, y.hi, x.lo + (DIR > 0 ? a.ex - a.ey : a.ex + a.ey), y.lo + (DIR > 0 ? a.ey + a.ex : a.ey - a.ex)};
+        constexpr float c = (float)0.70710678118654752440;
+        return cc_scale(z, c, (float)(0.70710678118654752440 - (double)c));
+    } else {
+        // cos, sin of 22.5, 30, 60 and 67.5 degrees
+        static_assert(NUM == 3 || NUM == 4 || NUM == 8 || NUM == 9, "");
+        constexpr double cd = NUM == 3 ? 0.92387953251128675613 : NUM == 4 ? 0.86602540378443864676
+                            : NUM == 8 ? 0.5 : 0.38268343236508977173;
+        constexpr double sd = NUM == 3 ? 0.38268343236508977173 : NUM == 4 ? 0.5
+                            : NUM == 8 ? 0.86602540378443864676 : 0.92387953251128675613;
+        constexpr float c = (float)cd, s = (float)(DIR * sd);
+        return cc_mul(a, c, s, (float)(cd - (double)c), (float)(DIR * sd - (double)s));
     }
 }
 
-template <int P>
-__device__ __forceinline__ void cdif_stage(cf32* H, cf32* E, const CfftDesc& d, int Ns, int dir) {
-    const int n = d.n;
-    const int nb = n / P;
-    const int span = Ns * P;
-    const int step = n / span;
-    const float inv = 1.0f / (float)Ns;
-    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
-        int g, k;
-        split_idx(t, Ns, inv, g, k);
-        const int base = g * span + k;
-        cc a[P];
+// A x B points in registers, j = b + B a in, s + A q out: A-point butterflies
+// over a, twiddles exp(DIR 2 pi i b s / (A B)), B-point butterflies over b.
+template <int A, int B, int DIR>
+__device__ __forceinline__ void cc_composite(cc* x) {
+    constexpr int U = 48 / (A * B);
+    cc y[A * B];   // [b][s]
 #pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const int i = pad(base + r * Ns);
-            a[r] = cc_make(H[i], E[i]);
-        }
-        CBfly<P>::run(a, dir);
-        if (Ns > 1) {
+    for (int b = 0; b < B; ++b) {
+        cc t[A];
 #pragma unroll
-            for (int s = 1; s < P; ++s) a[s] = cc_twiddle(a[s], d.tw, s * k * step, dir);
-        }
+        for (int a = 0; a < A; ++a) t[a] = x[b + B * a];
+        CBfly<A>::run(t, DIR);
 #pragma unroll
-        for (int s = 0; s < P; ++s) {
-            const int i = pad(base + s * Ns);
-            H[i] = mk(a[s].hx, a[s].hy);
-            E[i] = mk(a[s].ex, a[s].ey);
-        }
+        for (int s = 0; s < A; ++s) y[b * A + s] = t[s];
+    }
+    if constexpr (B > 1) {
+        if constexpr (A > 1) y[A + 1] = cc_root48<(U * 1) % 48, DIR>(y[A + 1]);
+        if constexpr (A > 2) y[A + 2] = cc_root48<(U * 2) % 48, DIR>(y[A + 2]);
+        if constexpr (A > 3) y[A + 3] = cc_root48<(U * 3) % 48, DIR>(y[A + 3]);
+    }
+    if constexpr (B > 2) {
+        if constexpr (A > 1) y[2 * A + 1] = cc_root48<(U * 2) % 48, DIR>(y[2 * A + 1]);
+        if constexpr (A > 2) y[2 * A + 2] = cc_root48<(U * 4) % 48, DIR>(y[2 * A + 2]);
+        if constexpr (A > 3) y[2 * A + 3] = cc_root48<(U * 6) % 48, DIR>(y[2 * A + 3]);
+    }
+    if constexpr (B > 3) {
+        if constexpr (A > 1) y[3 * A + 1] = cc_root48<(U * 3) % 48, DIR>(y[3 * A + 1]);
+        if constexpr (A > 2) y[3 * A + 2] = cc_root48<(U * 6) % 48, DIR>(y[3 * A + 2]);
+        if constexpr (A > 3) y[3 * A + 3] = cc_root48<(U * 9) % 48, DIR>(y[3 * A + 3]);
+    }
+#pragma unroll
+    for (int s = 0; s < A; ++s) {
+        cc t[B];
+#pragma unroll
+        for (int b = 0; b < B; ++b) t[b] = y[b * A + s];
+        CBfly<B>::run(t, DIR);
+#pragma unroll
+        for (int q = 0; q < B; ++q) x[s + A * q] = t[q];
     }
 }
-
-__device__ __forceinline__ void cfft_dit(cf32* H, cf32* E, const CfftDesc& d, int dir) {
-    int Ns = 1;
-    for (int st = 0; st < d.nstages; ++st) {
-        const int p = d.radix[st];
-        if (p == 4) cdit_stage<4>(H, E, d, Ns, dir);
-        else if (p == 3) cdit_stage<3>(H, E, d, Ns, dir);
-        else cdit_stage<2>(H, E, d, Ns, dir);
-        __syncthreads();
-        Ns *= p;
-    }
-}
-
-__device__ __forceinline__ void cfft_dif(cf32* H, cf32* E, const CfftDesc& d, int dir) {
-    int Ns = d.n;
-    for (int st = d.nstages - 1; st >= 0; --st) {
-        const int p = d.radix[st];
-        Ns /= p;
-        if (p == 4) cdif_stage<4>(H, E, d, Ns, dir);
-        else if (p == 3) cdif_stage<3>(H, E, d, Ns, dir);
-        else cdif_stage<2>(H, E, d, Ns, dir);
-        __syncthreads();
-    }
+template <int P, int DIR>
+__device__ __forceinline__ void cc_fft(cc* x) {
+    static_assert(P == 4 || P == 6 || P == 8 || P == 12 || P == 16, "");
+    if constexpr (P == 4) CBfly<4>::run(x, DIR);
+    else if constexpr (P == 6) cc_composite<2, 3, DIR>(x);
+    else if constexpr (P == 8) cc_composite<2, 4, DIR>(x);
+    else if constexpr (P == 12) cc_composite<4, 3, DIR>(x);
+    else cc_composite<4, 4, DIR>(x);
 }
 
 }  // namespace s1g

@@ -15,13 +15,30 @@ struct CfftPlan {
     ~CfftPlan();
 };
 
+// Transform of the overlap-save blocks: up to four passes of the radices
+// below, the last of the forward transform joined with the first of the
+// inverse one.
+struct DcFft {
+    int n = 0, np = 0;
+    int nt = 0;                  // threads of a CTA
+    int sh = 0;                  // element i of a block at i + (i >> sh) in shared memory
+    int radix[4] = {};
+    const float4* tw[3] = {};    // pass p: [s - 1][k] exp(-2 pi i s k / span) {re, im, re lo, im lo}
+};
+struct DcFftPlan {
+    DcFft d;
+    std::vector<int> at;         // where DcEstArgs::H holds frequency f
+    std::vector<void*> owned;
+    ~DcFftPlan();
+};
+
 struct DcEstArgs {
     const cf32* raw;       // [n_a][n_r] decoded (and notched) echo lines
     int n_a, n_r;
     int M, h;              // circular length and output shift of the range correlation
-    CfftDesc d;            // overlap-save block length B
+    DcFft d;               // overlap-save block length B
     int U, nb;             // outputs per block, blocks per line
-    const float4* H;       // B: conj(FFT_B(chirp)) * 2^-32 / (E B), float pairs {re, im, re lo, im lo}
+    const float4* H;       // B: conj(FFT_B(chirp)) * 2^-32 / (E B), float pairs {re, im, re lo, im lo}, at DcFftPlan::at
     float4* rcd;           // [n_a][n_r] compressed lines * 2^-32, float pairs {re, im, re lo, im lo}
     const float4* g;       // n_a - 1: deramp_t conj(deramp_t+1), float pairs
     cf64* part;            // [nchunk][n_r] partial lag-1 sums
@@ -29,6 +46,7 @@ struct DcEstArgs {
 };
 
 std::shared_ptr<CfftPlan> make_cfft_plan(int n);
+std::shared_ptr<DcFftPlan> make_dc_plan(int n);
 // Overlap-save block B = 2^a 3^b (B >= L + 32, fits shared memory) of least
 // cost for lines of n_r samples and a chirp of L samples.
 bool choose_dc_block(int n_r, int L, int& B, int& U, int& nb);
