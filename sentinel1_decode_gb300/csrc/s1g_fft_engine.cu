@@ -132,7 +132,8 @@ std::vector<int> fft4_order64(long long n) {
 std::vector<long long> fft4_lengths(long long minlen, size_t most) {
     std::vector<std::pair<double, long long>> c;
     const long long hi = std::max(64LL, (long long)(minlen * 1.25) + 16);
-    for (long long m = std::max(64LL, (minlen + 15) / 16 * 16); m <= hi; m += 16) {
+    // past hi where there is none below it (the first is 96)
+    for (long long m = std::max(64LL, (minlen + 15) / 16 * 16); m <= hi || c.empty(); m += 16) {
         if ((long long)sizeof(cf32) * padded16_len((int)m) > kFft4SmemBytes) break;
         const auto o = fft4_orders(m, 1);
         if (o.empty() || o[0].back() != 16 || !fft4_end_radix(o[0][0])) continue;
