@@ -428,9 +428,10 @@ struct Pipe {
         return d;
     }
 
-    void fft_rows(int n, const cpx<R>* in, long long ip, cpx<R>* out, long long op, long long rows, int dir) {
-        if constexpr (sizeof(R) == 4) fft.rows<R>(*fft.plan8(n), in, ip, out, op, rows, dir);
-        else fft.rows<R>(*fft.plan<R>(n), in, ip, out, op, rows, dir);
+    void fft_rows(int n, const cpx<R>* in, long long ip, cpx<R>* out, long long op, long long rows, int dir, int roll = 0,
+                  double scale = 1.0) {
+        if constexpr (sizeof(R) == 4) fft.rows<R>(*fft.plan8(n), in, ip, out, op, rows, dir, roll, scale);
+        else fft.rows<R>(*fft.plan<R>(n), in, ip, out, op, rows, dir, roll, scale);
     }
 
     // decode -> [n_a][n_r] in buffer A
@@ -584,11 +585,9 @@ struct Pipe {
         if (rd) {
             // transpose, azimuth FFT, fftshift, transpose (s1_decoder.cpp:499-505)
             cpx<R>* Bt = h->bB.as<cpx<R>>((size_t)n_a * n_r);
-            cpx<R>* Ct = h->bC.as<cpx<R>>((size_t)n_a * n_r);
             transpose_batched<R>(A, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
-            fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, -1);
-            roll_rows<R>(Bt, n_a, Ct, n_a, n_a, n_a / 2, n_r, st);
-            transpose_batched<R>(Ct, n_a, 0, A, n_r, 0, n_r, n_a, 1, st);
+            fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, -1, n_a / 2);
+            transpose_batched<R>(Bt, n_a, 0, A, n_r, 0, n_r, n_a, 1, st);
         }
         return A;
     }
@@ -727,8 +726,7 @@ struct Pipe {
         // azimuth IFFT with 1/S (s1_decoder.cpp:682)
         cpx<R>* Bt = h->bB.as<cpx<R>>((size_t)n_r * S);
         transpose_batched<R>(A, n_r, 0, Bt, S, 0, S, n_r, 1, st);
-        fft_rows(S, Bt, S, Bt, S, n_r, +1);
-        scale_rows<R>(Bt, S, S, n_r, 1.0 / S, st);
+        fft_rows(S, Bt, S, Bt, S, n_r, +1, 0, 1.0 / S);
         if (!tops) {
             transpose_batched<R>(Bt, S, 0, A, n_r, 0, n_r, S, 1, st);
             Result r;
@@ -756,8 +754,7 @@ struct Pipe {
         tufr_deramp<R>(Bt, S, S, C, shape, kaT, S, fdc, n_r, rate, q.num_tiles, q.focused_time, st);
         fft_rows(shape, C, shape, C, shape, n_r, -1);
         band_select<R>(C, shape, D, shape, shape, q.start, q.end - q.start, n_r, st);
-        fft_rows(shape, D, shape, D, shape, n_r, +1);
-        scale_rows<R>(D, shape, shape, n_r, 1.0 / shape, st);
+        fft_rows(shape, D, shape, D, shape, n_r, +1, 0, 1.0 / shape);
         cpx<R>* E = h->bE.as<cpx<R>>((size_t)n_r * down);
         tufr_resample<R>(D, shape, shape, E, down, down, kaT, S, S, fdc, n_r, rate, q.n_ref, q.focused_time, st);
         const int mid = down / 2;
@@ -897,12 +894,10 @@ static ChainResult azimuth_chain(s1g_decoder* h, const std::vector<int>& pk, con
     transpose_batched<R>(T1, n_a, 0, QM, n_r, 0, n_r, n_a, 1, st);
     p.fft_rows(n_r, QM, n_r, QM, n_r, n_a, -1);
     rcmc_phase<R>(QM, n_r, n_a, d_beta, g.fs, +1, st);
-    p.fft_rows(n_r, QM, n_r, Z, n_r, n_a, +1);
-    scale_rows<R>(Z, n_r, n_r, n_a, 1.0 / n_r, st);
+    p.fft_rows(n_r, QM, n_r, Z, n_r, n_a, +1, 0, 1.0 / n_r);
     az_filter<R>(Z, n_r, n_a, d_omd, d_slant, c4pl, -1, st);
     transpose_batched<R>(Z, n_r, 0, T2, n_a, 0, n_a, n_r, 1, st);
-    p.fft_rows(n_a, T2, n_a, T2, n_a, n_r, +1);
-    scale_rows<R>(T2, n_a, n_a, n_r, 1.0 / n_a, st);
+    p.fft_rows(n_a, T2, n_a, T2, n_a, n_r, +1, 0, 1.0 / n_a);
     entropy_sums<R>(T2, N, d_sums, st);
     double sums[2];
     check_cuda(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, st), "entropy down");
@@ -919,16 +914,14 @@ static ChainResult azimuth_chain(s1g_decoder* h, const std::vector<int>& pk, con
     if (!grads) return res;
     // adjoint
     entropy_grad<R>(T2, T2, N, d_sums, st);
-    p.fft_rows(n_a, T2, n_a, T2, n_a, n_r, -1);
-    scale_rows<R>(T2, n_a, n_a, n_r, 1.0 / n_a, st);
+    p.fft_rows(n_a, T2, n_a, T2, n_a, n_r, -1, 0, 1.0 / n_a);
     transpose_batched<R>(T2, n_a, 0, T1, n_r, 0, n_r, n_a, 1, st);   // G_Z
     row_imdot<R>(T1, Z, n_r, n_a, d_slant, 0.0, d_ak, st);
     az_filter<R>(T1, n_r, n_a, d_omd, d_slant, c4pl, +1, st);         // G_W
     p.fft_rows(n_r, T1, n_r, T1, n_r, n_a, -1);                       // F
     row_imdot<R>(T1, QM, n_r, n_a, nullptr, g.fs, d_bk, st);
     rcmc_phase<R>(T1, n_r, n_a, d_beta, g.fs, -1, st);
-    p.fft_rows(n_r, T1, n_r, T1, n_r, n_a, +1);
-    scale_rows<R>(T1, n_r, n_r, n_a, 1.0 / n_r, st);                  // G_V
+    p.fft_rows(n_r, T1, n_r, T1, n_r, n_a, +1, 0, 1.0 / n_r);                  // G_V
     transpose_batched<R>(T1, n_r, 0, T2, n_a, 0, n_a, n_r, 1, st);
     p.fft_rows(n_a, T2, n_a, T2, n_a, n_r, +1);                       // n_a IFFT_az
     transpose_batched<R>(T2, n_a, 0, T1, n_r, 0, n_r, n_a, 1, st);   // G_U
@@ -1070,8 +1063,7 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
     p.fft_rows(n_r, A, n_r, A, n_r, S, +1);
     az_filter<R>(A, n_r, S, n_r, drp, tc.slant, tc.rf, tc.fdc, tc.tcorr, tc.rscale, 1, st);
     transpose_batched<R>(A, n_r, 0, YT, S, 0, S, n_r, 1, st);
-    p.fft_rows(S, YT, S, YT, S, n_r, +1);
-    scale_rows<R>(YT, S, S, n_r, 1.0 / S, st);
+    p.fft_rows(S, YT, S, YT, S, n_r, +1, 0, 1.0 / S);
     entropy_sums<R>(YT, NS, d_sums, st);
     double sums[2];
     check_cuda(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, st), "entropy down");
@@ -1088,8 +1080,7 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
     if (!grads) return res;
     // adjoint
     entropy_grad<R>(YT, T, NS, d_sums, st);
-    p.fft_rows(S, T, S, T, S, n_r, -1);
-    scale_rows<R>(T, S, S, n_r, 1.0 / S, st);                        // G_Z^T
+    p.fft_rows(S, T, S, T, S, n_r, -1, 0, 1.0 / S);                        // G_Z^T
     transpose_batched<R>(T, S, 0, C, n_r, 0, n_r, S, 1, st);         // G_Z
     tops_dpsi<R>(C, A, n_r, S, n_r, drp, tc, 1, d_dz, st);
     tops_factor_adj<R>(C, n_r, S, n_r, drp, tc, 1, st);
@@ -1508,11 +1499,9 @@ struct FastPipe {
         const bool rd = (level == S1G_RANGE_DOPPLER) || (az && !tops);
         if (rd) {
             cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
-            cf32* Ct = h->bD.as<cf32>((size_t)n_a * n_r);
             transpose_batched<float>(rc, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
-            fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, -1);
-            roll_rows<float>(Bt, n_a, Ct, n_a, n_a, n_a / 2, n_r, st);
-            transpose_batched<float>(Ct, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st);
+            fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, -1, n_a / 2);
+            transpose_batched<float>(Bt, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st);
         }
         if (!az) {
             r.ptr = rc;
@@ -1554,8 +1543,7 @@ struct FastPipe {
         h->mark("azimuth_ifft");
         cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
         transpose_batched<float>(rd, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
-        fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, +1);
-        scale_rows<float>(Bt, n_a, n_a, n_r, 1.0 / n_a, st);
+        fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, +1, 0, 1.0 / n_a);
         transpose_batched<float>(Bt, n_a, 0, rd, n_r, 0, n_r, n_a, 1, st);
         Result r;
         r.ptr = rd;

@@ -195,6 +195,8 @@ struct RowsIo {
     int a;               // 1: plain rows
     const cpx<R>* tw;
     int dir;
+    int n, roll;         // points of a row, where output 0 goes
+    R scale;
 };
 template <typename R>
 __device__ __forceinline__ void rows_put(const RowsIo<R>& io, cpx<R>* y, int k, int off, cpx<R> v) {
@@ -204,7 +206,8 @@ __device__ __forceinline__ void rows_put(const RowsIo<R>& io, cpx<R>* y, int k, 
         if (io.dir > 0) w = conj(w);
         v = cmul4(v, w);
     }
-    y[k] = v;
+    k += io.roll;
+    y[k < io.n ? k : k - io.n] = v * io.scale;
 }
 
 // Rows of a 7-smooth length: out[k] = sum_j in[j] exp(dir 2 pi i j k / n).
@@ -249,88 +252,186 @@ __global__ void __launch_bounds__(NT, MB) k_rows_blue(RowsIo<R> io, Fft4DescT<R>
 
 // a-point transforms across the a split rows of a line: out[k + b k1].
 template <typename R, int A>
-__device__ __forceinline__ void split_out(const cpx<R>* y, cpx<R>* out, int b, int k, int dir) {
+__device__ __forceinline__ void split_out(const cpx<R>* y, cpx<R>* out, int b, int k, int dir, int roll, R scale) {
     cpx<R> v[A];
 #pragma unroll
     for (int r = 0; r < A; ++r) v[r] = y[(long long)r * b + k];
     if (dir > 0) Dft<R, A, +1>::run(v);
     else Dft<R, A, -1>::run(v);
 #pragma unroll
-    for (int j = 0; j < A; ++j) out[k + (long long)j * b] = v[j];
+    for (int j = 0; j < A; ++j) {
+        const int i = k + j * b + roll;
+        out[i < A * b ? i : i - A * b] = v[j] * scale;
+    }
 }
 template <typename R>
 __global__ void __launch_bounds__(256) k_split_out(const cpx<R>* __restrict__ y, cpx<R>* __restrict__ out,
-                                                   long long op, int a, int b, int dir) {
+                                                   long long op, int a, int b, int dir, int roll, R scale) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= b) return;
     y += (long long)blockIdx.y * a * b;
     out += (long long)blockIdx.y * op;
     switch (a) {
-        case 2: split_out<R, 2>(y, out, b, k, dir); break;
-        case 3: split_out<R, 3>(y, out, b, k, dir); break;
-        case 4: split_out<R, 4>(y, out, b, k, dir); break;
-        case 5: split_out<R, 5>(y, out, b, k, dir); break;
-        case 6: split_out<R, 6>(y, out, b, k, dir); break;
-        case 7: split_out<R, 7>(y, out, b, k, dir); break;
-        case 8: split_out<R, 8>(y, out, b, k, dir); break;
-        case 9: split_out<R, 9>(y, out, b, k, dir); break;
-        case 10: split_out<R, 10>(y, out, b, k, dir); break;
-        case 12: split_out<R, 12>(y, out, b, k, dir); break;
-        case 15: split_out<R, 15>(y, out, b, k, dir); break;
-        default: split_out<R, 16>(y, out, b, k, dir); break;
+        case 2: split_out<R, 2>(y, out, b, k, dir, roll, scale); break;
+        case 3: split_out<R, 3>(y, out, b, k, dir, roll, scale); break;
+        case 4: split_out<R, 4>(y, out, b, k, dir, roll, scale); break;
+        case 5: split_out<R, 5>(y, out, b, k, dir, roll, scale); break;
+        case 6: split_out<R, 6>(y, out, b, k, dir, roll, scale); break;
+        case 7: split_out<R, 7>(y, out, b, k, dir, roll, scale); break;
+        case 8: split_out<R, 8>(y, out, b, k, dir, roll, scale); break;
+        case 9: split_out<R, 9>(y, out, b, k, dir, roll, scale); break;
+        case 10: split_out<R, 10>(y, out, b, k, dir, roll, scale); break;
+        case 12: split_out<R, 12>(y, out, b, k, dir, roll, scale); break;
+        case 15: split_out<R, 15>(y, out, b, k, dir, roll, scale); break;
+        default: split_out<R, 16>(y, out, b, k, dir, roll, scale); break;
     }
 }
 
-// The radix-8 plans' kernels (plan8): one CTA per row, digit-reversed into
-// shared memory, in-place passes.
+// The radix-8 plans' kernels (plan8), one CTA per row, decimation in time from
+// digit-reversed positions.  The first and the last stage take and give the
+// row itself: consecutive threads read elements j, j + n / P, ... that the
+// first butterfly wants.  The arithmetic and its order are those of fft_dit
+// (s1g_fft.cuh).  4.2 M points in rows of 1024 or 4096: 38 us (71 with separate
+// loops for loading and storing, unpadded shared memory and 512 threads at
+// every length): a chain of dependent shared-memory stages.
+// The chirp-z rows stay with separate loops: joined in the same manner they
+// fuse other products and sums, and the gradients move (see plan8).
 constexpr int kFftThreads = 512;
-__global__ void __launch_bounds__(kFftThreads) k_rows8_smooth(const cf32* __restrict__ in, long long in_pitch,
-                                                         cf32* __restrict__ out, long long out_pitch,
-                                                         FftDesc<float> d, int dir) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    cf32* buf = reinterpret_cast<cf32*>(smem_raw);
-    const long long row = blockIdx.x;
-    const cf32* x = in + row * in_pitch;
-    for (int j = threadIdx.x; j < d.n; j += blockDim.x) buf[__ldg(d.perm + j)] = x[j];
-    __syncthreads();
-    fft_dit(buf, d, dir);
-    cf32* y = out + row * out_pitch;
-    for (int k = threadIdx.x; k < d.n; k += blockDim.x) y[k] = buf[k];
+struct Rows8 {
+    const cf32* in;
+    long long ip;
+    cf32* out;
+    long long op;
+    int n, roll;             // points of a row, where output 0 goes
+    float scale;
+    int dir;
+    int mask;                // -1: padded shared memory, 0: not
+    FftDesc<float> d;        // length n, or of the chirp-z convolution
+    const cf32* chirp;       // n
+    const cf32* kern;        // d.n
+};
+__host__ __device__ __forceinline__ int pad8(int i, int mask) { return i + (((i >> 3) + (i >> 6) + (i >> 9)) & mask); }
+// t = g Ns + k
+__device__ __forceinline__ int rows8_base(int t, int Ns, int P, float inv, int& k) {
+    int g = __float2int_rz((float)t * inv);
+    k = t - g * Ns;
+    if (k < 0) {
+        --g;
+        k += Ns;
+    } else if (k >= Ns) {
+        ++g;
+        k -= Ns;
+    }
+    return g * Ns * P + k;
+}
+template <int P, class Load>
+__device__ __forceinline__ void rows8_in(cf32* buf, const FftDesc<float>& d, int dir, int mask, Load load) {
+    const int nb = d.n / P;
+    for (int j = threadIdx.x; j < nb; j += blockDim.x) {
+        cf32 a[P];
+#pragma unroll
+        for (int r = 0; r < P; ++r) a[r] = load(j + r * nb);
+        Bfly<float, P>::run(a, dir);
+        const int pos = __ldg(d.perm + j);
+#pragma unroll
+        for (int s = 0; s < P; ++s) buf[pad8(pos + s, mask)] = a[s];
+    }
+}
+template <int P>
+__device__ __forceinline__ void rows8_dit(cf32* buf, const FftDesc<float>& d, int Ns, int dir, int mask) {
+    const int nb = d.n / P, step = nb / Ns;
+    const float inv = 1.0f / (float)Ns;
+    for (int t = threadIdx.x; t < nb; t += blockDim.x) {
+        int k;
+        const int base = rows8_base(t, Ns, P, inv, k);
+        cf32 a[P];
+        a[0] = buf[pad8(base, mask)];
+#pragma unroll
+        for (int r = 1; r < P; ++r) a[r] = buf[pad8(base + r * Ns, mask)] * twid(d, r * k * step, dir);
+        Bfly<float, P>::run(a, dir);
+#pragma unroll
+        for (int s = 0; s < P; ++s) buf[pad8(base + s * Ns, mask)] = a[s];
+    }
+}
+template <int P, class Store>
+__device__ __forceinline__ void rows8_out(const cf32* buf, const FftDesc<float>& d, int dir, int mask, Store store) {
+    const int nb = d.n / P;
+    for (int k = threadIdx.x; k < nb; k += blockDim.x) {
+        cf32 a[P];
+        a[0] = buf[pad8(k, mask)];
+#pragma unroll
+        for (int r = 1; r < P; ++r) a[r] = buf[pad8(k + r * nb, mask)] * twid(d, r * k, dir);
+        Bfly<float, P>::run(a, dir);
+#pragma unroll
+        for (int s = 0; s < P; ++s) store(k + s * nb, a[s]);
+    }
+}
+#define ROWS8_RADIX(r, CALL)                              \
+    switch (r) {                                          \
+        case 2: { constexpr int P = 2; CALL; break; }     \
+        case 3: { constexpr int P = 3; CALL; break; }     \
+        case 4: { constexpr int P = 4; CALL; break; }     \
+        case 5: { constexpr int P = 5; CALL; break; }     \
+        case 7: { constexpr int P = 7; CALL; break; }     \
+        default: { constexpr int P = 8; CALL; break; }    \
+    }
+__device__ __forceinline__ void rows8_put(const Rows8& a, cf32* y, int k, cf32 v) {
+    k += a.roll;
+    y[k < a.n ? k : k - a.n] = v * a.scale;
 }
 
-struct BlueArgs {
-    int n;
-    FftDesc<float> dm;          // length m
-    const cf32* chirp;    // n
-    const cf32* kern;     // m
-};
+__global__ void __launch_bounds__(kFftThreads, 2) k_rows8_smooth(const __grid_constant__ Rows8 a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cf32* buf = reinterpret_cast<cf32*>(smem_raw);
+    const FftDesc<float>& d = a.d;
+    const cf32* x = a.in + (long long)blockIdx.x * a.ip;
+    cf32* y = a.out + (long long)blockIdx.x * a.op;
+    auto put = [&](int k, cf32 v) { rows8_put(a, y, k, v); };
+    if (d.nstages < 2) {
+        // n is 1 or a radix: one thread
+        if (threadIdx.x > 0) return;
+        cf32 v[8];
+        for (int j = 0; j < d.n; ++j) v[j] = x[j];
+        if (d.nstages == 1) ROWS8_RADIX(d.radix[0], (Bfly<float, P>::run(v, a.dir)));
+        for (int j = 0; j < d.n; ++j) put(j, v[j]);
+        return;
+    }
+    ROWS8_RADIX(d.radix[0], (rows8_in<P>(buf, d, a.dir, a.mask, [&](int j) { return x[j]; })));
+    __syncthreads();
+    int Ns = d.radix[0];
+    for (int st = 1; st + 1 < d.nstages; ++st) {
+        const int p = d.radix[st];
+        ROWS8_RADIX(p, (rows8_dit<P>(buf, d, Ns, a.dir, a.mask)));
+        __syncthreads();
+        Ns *= p;
+    }
+    ROWS8_RADIX(d.radix[d.nstages - 1], (rows8_out<P>(buf, d, a.dir, a.mask, put)));
+}
 
-__global__ void __launch_bounds__(kFftThreads) k_rows8_blue(const cf32* __restrict__ in, long long in_pitch,
-                                                         cf32* __restrict__ out, long long out_pitch,
-                                                         BlueArgs b, int dir) {
+__global__ void __launch_bounds__(kFftThreads) k_rows8_blue(const __grid_constant__ Rows8 a) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cf32* buf = reinterpret_cast<cf32*>(smem_raw);
     const long long row = blockIdx.x;
-    const cf32* x = in + row * in_pitch;
-    const int m = b.dm.n;
+    const cf32* x = a.in + row * a.ip;
+    const int m = a.d.n;
     for (int q = threadIdx.x; q < m; q += blockDim.x) {
         cf32 v = mk(0.0f, 0.0f);
-        if (q < b.n) {
+        if (q < a.n) {
             cf32 xv = x[q];
-            if (dir > 0) xv = conj(xv);
-            v = xv * ldg(b.chirp + q);
+            if (a.dir > 0) xv = conj(xv);
+            v = xv * ldg(a.chirp + q);
         }
-        buf[__ldg(b.dm.perm + q)] = v;
+        buf[__ldg(a.d.perm + q)] = v;
     }
     __syncthreads();
-    fft_dit(buf, b.dm, -1);
-    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = buf[q] * ldg(b.kern + q);
+    fft_dit(buf, a.d, -1);
+    for (int q = threadIdx.x; q < m; q += blockDim.x) buf[q] = buf[q] * ldg(a.kern + q);
     __syncthreads();
-    fft_dif(buf, b.dm, +1);
-    cf32* y = out + row * out_pitch;
-    for (int k = threadIdx.x; k < b.n; k += blockDim.x) {
-        cf32 v = ldg(b.chirp + k) * buf[__ldg(b.dm.perm + k)];
-        y[k] = dir > 0 ? conj(v) : v;
+    fft_dif(buf, a.d, +1);
+    cf32* y = a.out + row * a.op;
+    for (int k = threadIdx.x; k < a.n; k += blockDim.x) {
+        cf32 v = ldg(a.chirp + k) * buf[__ldg(a.d.perm + k)];
+        rows8_put(a, y, k, a.dir > 0 ? conj(v) : v);
     }
 }
 
@@ -413,6 +514,16 @@ __global__ void k_cvt64(const cpx<double>* __restrict__ in, cpx<R>* __restrict__
                         const int* __restrict__ at) {
     for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x)
         out[at ? at[i] : i] = mk((R)(in[i].x * scale), (R)(in[i].y * scale));
+}
+
+template <typename R>
+__global__ void k_roll_scale(const cpx<R>* __restrict__ in, cpx<R>* __restrict__ out, long long op, int n, long long rows,
+                             int roll, R scale) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rows * n; i += (long long)gridDim.x * blockDim.x) {
+        const long long r = i / n;
+        const int k = (int)(i - r * n) + roll;
+        out[r * op + (k < n ? k : k - n)] = in[i] * scale;
+    }
 }
 
 static int grid_for(long long total, int threads = 256) {
@@ -770,17 +881,14 @@ template <typename R>
 static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows, cudaStream_t st) {
     if constexpr (sizeof(R) == 4) {
         if (p.desc) {
-            for (long long b0 = 0; b0 < rows; b0 += 65535LL * 16) {
-                const unsigned nb = (unsigned)std::min(rows - b0, 65535LL * 16);
-                const cf32* in = io.in + b0 * io.ip;
-                cf32* out = io.out + b0 * io.op;
-                if (p.kind == FFT_SMEM)
-                    note_launch(), k_rows8_smooth<<<nb, kFftThreads, sizeof(cf32) * p.n, st>>>(
-                        in, io.ip, out, io.op, p.desc->d32, io.dir);
-                else
-                    note_launch(), k_rows8_blue<<<nb, kFftThreads, sizeof(cf32) * p.m, st>>>(
-                        in, io.ip, out, io.op, BlueArgs{p.n, p.desc->d32, p.chirp, p.kern}, io.dir);
-            }
+            const FftDesc<float>& d = p.desc->d32;
+            const int padded = pad8(d.n, -1);
+            const bool smooth = p.kind == FFT_SMEM, fits = smooth && sizeof(cf32) * (size_t)padded <= (size_t)kSmemBytes;
+            const int nt = smooth ? std::min(kFftThreads, std::max(64, (d.n / 8 + 31) / 32 * 32)) : kFftThreads;
+            const size_t smem = sizeof(cf32) * (size_t)(fits ? padded : d.n);
+            const Rows8 q{io.in, io.ip, io.out, io.op, p.n, io.roll, io.scale, io.dir, fits ? -1 : 0, d, p.chirp, p.kern};
+            if (smooth) note_launch(), k_rows8_smooth<<<(unsigned)rows, nt, smem, st>>>(q);
+            else note_launch(), k_rows8_blue<<<(unsigned)rows, nt, smem, st>>>(q);
             return;
         }
     }
@@ -802,23 +910,26 @@ static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows
 
 template <typename R>
 void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out, long long out_pitch,
-                     long long batch, int dir) {
+                     long long batch, int dir, int roll, double scale) {
     if (batch <= 0) return;
     const int n = p.n;
     switch (p.kind) {
         case FFT_SMEM:
-        case FFT_BLUE: launch_rows<R>(p, RowsIo<R>{in, in_pitch, out, out_pitch, 1, nullptr, dir}, batch, stream); break;
+        case FFT_BLUE: launch_rows<R>(p, RowsIo<R>{in, in_pitch, out, out_pitch, 1, nullptr, dir, n, roll, (R)scale}, batch,
+                                      stream);
+            return;
         case FFT_SPLIT: {
             const long long limit = (1LL << 30) / (long long)sizeof(cpx<R>);
             const long long chunk = std::max(1LL, std::min(std::min(batch, limit / n), 65535LL));
             cpx<R>* Y = (cpx<R>*)scratch_a.get(sizeof(cpx<R>) * chunk * n);
             for (long long b0 = 0; b0 < batch; b0 += chunk) {
                 const long long nb = std::min(chunk, batch - b0);
-                launch_rows<R>(*p.p2, RowsIo<R>{in + b0 * in_pitch, in_pitch, Y, p.n2, p.n1, p.tw4, dir}, nb * p.n1, stream);
+                launch_rows<R>(*p.p2, RowsIo<R>{in + b0 * in_pitch, in_pitch, Y, p.n2, p.n1, p.tw4, dir, p.n2, 0, (R)1}, nb * p.n1,
+                               stream);
                 note_launch(), k_split_out<R><<<dim3((p.n2 + 255) / 256, (unsigned)nb), 256, 0, stream>>>(
-                    Y, out + b0 * out_pitch, out_pitch, p.n1, p.n2, dir);
+                    Y, out + b0 * out_pitch, out_pitch, p.n1, p.n2, dir, roll, (R)scale);
             }
-            break;
+            return;
         }
         case FFT_FOUR: {
             const int n1 = p.n1, n2 = p.n2;
@@ -859,15 +970,27 @@ void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, 
             break;
         }
     }
+    // lengths over one CTA: roll and scale are passes of their own
+    if (roll || scale != 1.0) {
+        const long long chunk = std::max(1LL, std::min(batch, (256LL << 20) / (long long)sizeof(cpx<R>) / n));
+        cpx<R>* A = (cpx<R>*)scratch_a.get(sizeof(cpx<R>) * chunk * n);
+        for (long long b0 = 0; b0 < batch; b0 += chunk) {
+            const long long nb = std::min(chunk, batch - b0);
+            check_cuda(cudaMemcpy2DAsync(A, sizeof(cpx<R>) * n, out + b0 * out_pitch, sizeof(cpx<R>) * out_pitch,
+                                         sizeof(cpx<R>) * n, nb, cudaMemcpyDeviceToDevice, stream), "fft copy");
+            note_launch(), k_roll_scale<R><<<grid_for(nb * n), 256, 0, stream>>>(A, out + b0 * out_pitch, out_pitch, n, nb,
+                                                                                 roll, (R)scale);
+        }
+    }
     check_cuda(cudaGetLastError(), "fft launch");
 }
 
 template std::shared_ptr<FftPlan<float>> FftEngine::plan<float>(int);
 template std::shared_ptr<FftPlan<double>> FftEngine::plan<double>(int);
 template void FftEngine::rows<float>(const FftPlan<float>&, const cpx<float>*, long long, cpx<float>*, long long,
-                                     long long, int);
+                                     long long, int, int, double);
 template void FftEngine::rows<double>(const FftPlan<double>&, const cpx<double>*, long long, cpx<double>*, long long,
-                                      long long, int);
+                                      long long, int, int, double);
 template FftDesc<float> FftEngine::smem_desc<float>(int);
 template FftDesc<double> FftEngine::smem_desc<double>(int);
 template void transpose_batched<float>(const cpx<float>*, long long, long long, cpx<float>*, long long, long long,

@@ -18,7 +18,7 @@
 // use them: a focus gradient is a sum that cancels to 1e-4 of its terms, so it
 // moves by up to 1e-4 with the rounding of the transforms, and so do decisions
 // of the plain pipelines at their thresholds.  Those paths keep one arithmetic
-// (a 1024 x 4096 evaluation's ten transforms: 0.71 ms, 0.42 over the other
+// (a 1024 x 4096 evaluation's ten transforms: 0.38 ms, 0.42 over the other
 // core).
 #pragma once
 
@@ -111,11 +111,11 @@ struct FftEngine {
     std::shared_ptr<FftPlan<R>> plan(int n);
     std::shared_ptr<FftPlan<float>> plan8(int n);
 
-    // out[b*out_pitch + k] = sum_j in[b*in_pitch + j] exp(dir 2 pi i jk/n).
-    // in may equal out.  Works for any n >= 1.
+    // out[b*out_pitch + (k + roll) % n] = scale sum_j in[b*in_pitch + j] exp(dir 2 pi i jk/n),
+    // 0 <= roll < n.  in may equal out.  Works for any n >= 1.
     template <typename R>
     void rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out,
-              long long out_pitch, long long batch, int dir);
+              long long out_pitch, long long batch, int dir, int roll = 0, double scale = 1.0);
 
     // Smooth descriptor for device-side fused kernels (throws if n is not
     // 7-smooth or does not fit shared memory).

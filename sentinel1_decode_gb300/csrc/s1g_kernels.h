@@ -160,9 +160,6 @@ template <typename R>
 void rc_crop(const cpx<R>* in, long long in_pitch, int m, cpx<R>* out, long long out_pitch, int n_r, int h,
              long long rows, cudaStream_t st);
 template <typename R>
-void roll_rows(const cpx<R>* in, long long in_pitch, cpx<R>* out, long long out_pitch, int n, int shift,
-               long long rows, cudaStream_t st);
-template <typename R>
 void dc_sums(const cpx<R>* rc, long long pitch, int n_a, int n_r, const cpx<R>* deramp, cf64* sums,
              cudaStream_t st);
 template <typename R>
@@ -174,8 +171,6 @@ void band_select(const cpx<R>* Y, long long ypitch, cpx<R>* Z, long long zpitch,
 template <typename R>
 void scale_mul_vec(cpx<R>* a, long long pitch, int n, long long rows, const cpx<R>* vec, double scale,
                    cudaStream_t st);
-template <typename R>
-void scale_rows(cpx<R>* a, long long pitch, int n, long long rows, double scale, cudaStream_t st);
 template <typename R>
 void src_filter(cpx<R>* data, long long pitch, int S, int n_r, const RowParam* rows, const double* slant,
                 const double* range_freq, const double* f_dc, double c3, cudaStream_t st);

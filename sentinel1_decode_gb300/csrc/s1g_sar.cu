@@ -79,22 +79,6 @@ void rc_crop(const cpx<R>* in, long long ip, int m, cpx<R>* out, long long op, i
 
 // out[k] = in[(k - shift) mod n] (std::rotate right by shift)
 template <typename R>
-__global__ void k_roll_rows(const cpx<R>* in, long long ip, cpx<R>* out, long long op, int n, int shift, long long rows) {
-    GRID_STRIDE(i, rows * n) {
-        const long long r = i / n;
-        const int k = (int)(i % n);
-        int src = k - shift;
-        if (src < 0) src += n;
-        out[r * op + k] = in[r * ip + src];
-    }
-}
-template <typename R>
-void roll_rows(const cpx<R>* in, long long ip, cpx<R>* out, long long op, int n, int shift, long long rows,
-               cudaStream_t st) {
-    note_launch(), k_roll_rows<R><<<grid1(rows * n), 256, 0, st>>>(in, ip, out, op, n, shift, rows);
-}
-
-template <typename R>
 __global__ void k_scale_mul_vec(cpx<R>* a, long long p, int n, long long rows, const cpx<R>* v, double scale) {
     GRID_STRIDE(i, rows * n) {
         const long long r = i / n;
@@ -106,19 +90,6 @@ __global__ void k_scale_mul_vec(cpx<R>* a, long long p, int n, long long rows, c
 template <typename R>
 void scale_mul_vec(cpx<R>* a, long long p, int n, long long rows, const cpx<R>* v, double scale, cudaStream_t st) {
     note_launch(), k_scale_mul_vec<R><<<grid1(rows * n), 256, 0, st>>>(a, p, n, rows, v, scale);
-}
-
-template <typename R>
-__global__ void k_scale_rows(cpx<R>* a, long long p, int n, long long rows, double scale) {
-    GRID_STRIDE(i, rows * n) {
-        const long long r = i / n;
-        const int q = (int)(i % n);
-        a[r * p + q] = a[r * p + q] * (R)scale;
-    }
-}
-template <typename R>
-void scale_rows(cpx<R>* a, long long p, int n, long long rows, double scale, cudaStream_t st) {
-    note_launch(), k_scale_rows<R><<<grid1(rows * n), 256, 0, st>>>(a, p, n, rows, scale);
 }
 
 template <typename R>
@@ -524,9 +495,7 @@ void eccm_notch(cpx<R>* data, long long p, int n_r, long long rows, const int* f
     template void pad_rows<R>(const cpx<R>*, long long, int, cpx<R>*, long long, int, long long, cudaStream_t);  \
     template void mul_rows_by_vec<R>(cpx<R>*, long long, int, long long, const cpx<R>*, cudaStream_t);             \
     template void rc_crop<R>(const cpx<R>*, long long, int, cpx<R>*, long long, int, int, long long, cudaStream_t); \
-    template void roll_rows<R>(const cpx<R>*, long long, cpx<R>*, long long, int, int, long long, cudaStream_t);   \
     template void scale_mul_vec<R>(cpx<R>*, long long, int, long long, const cpx<R>*, double, cudaStream_t);       \
-    template void scale_rows<R>(cpx<R>*, long long, int, long long, double, cudaStream_t);                         \
     template void band_select<R>(const cpx<R>*, long long, cpx<R>*, long long, int, int, int, long long,           \
                                  cudaStream_t);                                                                  \
     template void dc_sums<R>(const cpx<R>*, long long, int, int, const cpx<R>*, cf64*, cudaStream_t);              \
