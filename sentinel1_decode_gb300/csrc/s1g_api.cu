@@ -65,6 +65,16 @@ struct RangeRef {
     Buf dev;
 };
 
+// The caller's device buffer for a complex<float> product of this shape: the
+// last kernel of a chain writes there instead of into a buffer that is copied.
+struct Dest {
+    cf32* p = nullptr;
+    long long rows = 0, cols = 0;
+    cf32* take(long long r, long long c) const {
+        return r == rows && c == cols && !(reinterpret_cast<uintptr_t>(p) & 15) ? p : nullptr;
+    }
+};
+
 struct Result {   // a product left in device memory
     const void* ptr = nullptr;
     long long rows = 0, cols = 0, pitch = 0;
@@ -125,7 +135,6 @@ struct s1g_decoder {
     // FP32 calls (built on the first such call, dropped when the stream
     // content or the A/B/C decode mode changes)
     std::map<std::string, std::shared_ptr<struct SwathDecode>> swath_decodes;
-    Result last;
     double last_ms = 0;
     // Status words of a product call, read back with its one synchronisation:
     // [0] corner-turn flag, [1] time unfolding, [2..] decode status per packet
@@ -1239,6 +1248,7 @@ struct FastPipe {
     FftEngine& fft;
     const cf32* predecoded = nullptr;   // burst already decoded (batched decode)
     cf64* predecoded64 = nullptr;       // ... and its FP64 samples (for the ECCM notch), or null
+    Dest dest;                          // caller's buffer for the product
     cf32* final_out = nullptr;          // write the SLC here ([N_out][N_r]) instead of a work buffer
     int* tufr_status = nullptr;         // per-burst time-unfolding status slot
     explicit FastPipe(s1g_decoder* hh) : h(hh), st(hh->stream), fft(*hh->fft) {}
@@ -1494,20 +1504,23 @@ struct FastPipe {
             plain.eccm_fp64(pk, g, w, predecoded64);
             raw = w;
         }
-        cf32* rc = h->bB.as<cf32>((size_t)n_a * n_r);
+        cf32* fin = dest.take(n_a, n_r);
+        cf32* rc = fin && level == S1G_RANGE_COMPRESSED ? fin : h->bB.as<cf32>((size_t)n_a * n_r);
         rc_fused(raw, rc, n_a, n_r, g.h, fb.dM, fb.ref, st);
         const bool rd = (level == S1G_RANGE_DOPPLER) || (az && !tops);
         if (rd) {
             cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
             transpose_batched<float>(rc, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
             fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, -1, n_a / 2);
+            if (fin && !az) rc = fin;
             transpose_batched<float>(Bt, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st);
         }
         if (!az) {
             r.ptr = rc;
             return r;
         }
-        if (!tops) return stripmap(rc, fb, plain);
+        if (!tops) return stripmap(rc, fb, fin ? fin : rc);
+        if (!final_out) final_out = dest.take(fb.n_out, n_r);
         return tops_chain(rc, raw, fb);
     }
 
@@ -1536,7 +1549,7 @@ struct FastPipe {
         return ra;
     }
 
-    Result stripmap(cf32* rd, const FastBurst& fb, Pipe<float>& plain) {
+    Result stripmap(cf32* rd, const FastBurst& fb, cf32* out) {
         const int n_a = fb.g.n_a, n_r = fb.g.n_r;
         h->mark("row_pass");
         rowpass_fused(row_args(rd, fb, 0, fb.zero_df), st);
@@ -1544,9 +1557,9 @@ struct FastPipe {
         cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
         transpose_batched<float>(rd, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
         fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, +1, 0, 1.0 / n_a);
-        transpose_batched<float>(Bt, n_a, 0, rd, n_r, 0, n_r, n_a, 1, st);
+        transpose_batched<float>(Bt, n_a, 0, out, n_r, 0, n_r, n_a, 1, st);
         Result r;
-        r.ptr = rd;
+        r.ptr = out;
         r.rows = n_a;
         r.cols = n_r;
         r.pitch = n_r;
@@ -1699,7 +1712,7 @@ struct FastPipe {
 
 static const cf32* swath_cached_decode(s1g_decoder* h, const std::vector<int>& pk);
 
-static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int level, bool tops) {
+static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int level, bool tops, Dest dest = {}) {
     for (auto& m : h->marks) cudaEventDestroy(m.second);
     h->marks.clear();
     if (!h->ev0) check_cuda(cudaEventCreate(&h->ev0), "event");
@@ -1719,6 +1732,7 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
         else {
             FastPipe fp(h);
             fp.predecoded = swath_cached_decode(h, pk);
+            fp.dest = dest;
             r = fp.run(pk, level, tops);
         }
     } catch (...) {
@@ -1753,6 +1767,7 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
 // buffer row is zero-filled on the right.
 static void deliver(s1g_decoder* h, const Result& r, long long row0, void* out, long long cols, int out_type,
                     int on_device, long long rows_to_copy, long long dst_row0, long long col0 = 0) {
+    if (r.ptr == (char*)out + (size_t)dst_row0 * cols * sizeof(cf32)) return;   // written there (Dest)
     const size_t esz = out_type == S1G_CF32 ? 8 : 16;
     void* dst = nullptr;
     void* stage = nullptr;
@@ -2252,13 +2267,14 @@ int s1g_burst_product(s1g_decoder* h, const char* swath, int burst, int level, v
     if (!swath || !out || !level_ok(level) || (out_type != S1G_CF32 && out_type != S1G_CF64))
         return S1G_E_INVALID_ARGUMENT;
     const auto& pk = burst_packets(h, swath, burst);
-    const Result r = compute_burst(h, pk, level, true);
+    Dest dest;
+    if (out_on_device && out_type == S1G_CF32) dest = {(cf32*)out, rows, cols};
+    const Result r = compute_burst(h, pk, level, true, dest);
     if (r.rows != rows || r.cols != cols) {
         h->err = "output buffer shape " + std::to_string(rows) + "x" + std::to_string(cols) + " != product " +
                  std::to_string(r.rows) + "x" + std::to_string(r.cols);
         return S1G_E_BUFFER;
     }
-    h->last = r;
     deliver(h, r, 0, out, cols, out_type, out_on_device, rows, 0);
     API_END(h)
 }
@@ -2374,7 +2390,9 @@ int s1g_swath_product(s1g_decoder* h, const char* swath, int level, void* out, i
     const bool tops = tops_for(swath);
     long long row = 0;
     for (const auto& e : plan) {
-        const Result r = compute_burst(h, e.pk, level, tops);
+        Dest dest;
+        if (out_on_device && out_type == S1G_CF32 && e.col0 == 0) dest = {(cf32*)out + row * cols, e.rows, cols};
+        const Result r = compute_burst(h, e.pk, level, tops, dest);
         deliver(h, r, 0, out, cols, out_type, out_on_device, r.rows, row, e.col0);
         row += r.rows;
         if (e.pad_rows) {
