@@ -15,7 +15,7 @@
 // reduced before the FP32 sine / cosine; reductions accumulate in FP64, in the
 // FP32 chain in double-float within a thread.  GB300 does 1.9 FP64 operations
 // per clock and SM, so FP64 per element bounded these kernels: the five took
-// 1.6 of the 2.5 ms of a 1024 x 4096 evaluation's device time, now 0.42 of 1.44 ms.
+// 1.6 of the 2.5 ms of a 1024 x 4096 evaluation's device time, now 0.27 of 0.89 ms.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -144,28 +144,56 @@ __global__ void __launch_bounds__(256) k_az_filter32(cf32* a, int n_r, int rows,
     }
 }
 
-// ln x of a normal FP64 x > 0 in double-float arithmetic, error below 1e-12
-// (FP64 log takes ~40 operations of a pipe that does 1.9 per clock and SM):
-// x = 2^e m with m in [1, 2) from the bits, c = 1/m to 8 bits (table of 128 by
-// the leading bits of m), r = m c - 1 exactly by one FMA (|r| < 2^-7), ln x =
-// e ln 2 - ln c + log1p(r) (Tang, "Table-driven implementation of the
-// logarithm function", 1990), the series' first two terms in double-float.
+// |v|^2 2^(-2 e) as a float pair in [1, 32), v's larger part of order 2^e; zero
+// gives zero.  Exact to 2^-47 for every float, whose squares leave the float
+// range.
+struct Norm32 {
+    df I;
+    int e;
+};
+__device__ __forceinline__ float pow2(int e) { return __int_as_float((e + 127) << 23); }   // |e| <= 126
+__device__ __forceinline__ Norm32 norm32(cf32& v) {
+    Norm32 r;
+    float m = fmaxf(fabsf(v.x), fabsf(v.y));
+    r.e = 0;
+    if (m < 5.421010862427522e-20f) {   // 2^-64
+        v.x *= 1.2676506002282294e30f;  // 2^100
+        v.y *= 1.2676506002282294e30f;
+        m *= 1.2676506002282294e30f;
+        r.e = -100;
+    }
+    const int e = m > 0.0f ? min((__float_as_int(m) >> 23) - 127, 126) : 0;
+    const float u = pow2(-e);
+    v.x *= u;
+    v.y *= u;
+    r.e += e;
+    const df a = two_prod(v.x, v.x), b = two_prod(v.y, v.y);
+    r.I = two_sum(a.hi, b.hi);
+    r.I.lo += a.lo + b.lo;
+    r.I = quick_two_sum(r.I.hi, r.I.lo);
+    return r;
+}
+
+// ln (x 2^k) of a float pair x in [1, 32) in double-float, error below 1e-12
+// (an FP64 log takes ~40 operations of a pipe that does 1.9 per clock and SM):
+// x = 2^e m with m in [1, 2), c = 1/m to 8 bits (table of 128 by the leading
+// bits of m), r = m c - 1 exactly by one FMA (|r| < 2^-7), ln x = e ln 2 -
+// ln c + log1p(r) (Tang, "Table-driven implementation of the logarithm
+// function", 1990), the series' first two terms in double-float.
 __device__ float c_log_c[128];     // global, not constant: lanes read different entries
 __device__ float2 c_log_t[128];    // -ln c as hi, lo
-__device__ __forceinline__ df ln_fast(double x) {
-    const unsigned int xh = (unsigned int)__double2hiint(x), xl = (unsigned int)__double2loint(x);
-    const int e = (int)(xh >> 20) - 1023;
-    // 23 leading bits of the fraction, then the other 29
-    const unsigned int f = ((xh & 0xfffffu) << 3) | (xl >> 29);
+__device__ __forceinline__ df ln32(df x, int k) {
+    const unsigned int bits = (unsigned int)__float_as_int(x.hi);
+    const unsigned int f = bits & 0x7fffffu;
+    const int e = (int)(bits >> 23) - 127 + k;
     const float m = __int_as_float((int)(0x3f800000u | f));
-    const float ml = (float)(int)(xl & 0x1fffffffu) * 2.220446049250313e-16f;   // 2^-52
     const int i = (int)(f >> 16);
     const float r = __fmaf_rn(m, __ldg(c_log_c + i), -1.0f);
     const float2 t = __ldg(c_log_t + i);
     const df r2 = two_prod(r, r);
     // r^3 (1/3 - r/4 + r^2/5 - r^3/6 + r^4/7), and the low part of x
     const float p = fmaf(r, fmaf(r, fmaf(r, fmaf(r, 1.0f / 7.0f, -1.0f / 6.0f), 0.2f), -0.25f), 1.0f / 3.0f);
-    const float rest = fmaf(r2.hi * r, p, __fdividef(ml, m));
+    const float rest = fmaf(r2.hi * r, p, __fdividef(x.lo, x.hi));
     const float ef = (float)e;
     // e ln 2 with ln 2 = 0x1.62e4p-1 (exact products) + 1.4286068202862268e-6
     const df el = two_prod(ef, 1.42860677e-6f);
@@ -176,7 +204,7 @@ __device__ __forceinline__ df ln_fast(double x) {
     s = df_add_abs(s, df_make(-0.5f * r2.hi, -0.5f * r2.lo));
     return df_add_f(s, rest);
 }
-// tables of ln_df, once per device
+// tables of ln32, once per device
 static void init_log_tables() {
     static std::mutex mu;
     static bool done[64] = {};
@@ -199,24 +227,37 @@ static void init_log_tables() {
     if (dev < 64) done[dev] = true;
 }
 
-// ln of |v|^2; zero gives 0 (its weight is zero)
-template <typename R>
-__device__ __forceinline__ double ln_norm(double I) {
-    if constexpr (sizeof(R) == 4) {
-        if (I >= 2.2250738585072014e-308) return df_to_double(ln_fast(I));
-    }
-    return I > 0.0 ? log(I) : 0.0;
-}
-
 // sums[0] += sum |y|^2, sums[1] += sum |y|^2 ln |y|^2
 template <typename R>
 __global__ void k_entropy_sums(const cpx<R>* __restrict__ y, long long n, double* sums) {
     double s = 0.0, t = 0.0;
-    ADJ_GRID_STRIDE(i, n) {
-        const cpx<R> v = y[i];
-        const double I = (double)v.x * v.x + (double)v.y * v.y;
-        s += I;
-        t += I * ln_norm<R>(I);
+    if constexpr (sizeof(R) == 4) {
+        // double-float in units of 2^(2 E) with E the largest exponent so far
+        df sd = df_make(0.f, 0.f), td = sd;
+        int E = -1000;
+        ADJ_GRID_STRIDE(i, n) {
+            cf32 v = y[i];
+            const Norm32 q = norm32(v);
+            if (q.I.hi == 0.0f) continue;
+            if (q.e > E) {
+                const float u = 2 * (E - q.e) < -126 ? 0.0f : pow2(2 * (E - q.e));
+                sd = df_make(sd.hi * u, sd.lo * u);
+                td = df_make(td.hi * u, td.lo * u);
+                E = q.e;
+            }
+            const float u = 2 * (q.e - E) < -126 ? 0.0f : pow2(2 * (q.e - E));
+            const df I = df_make(q.I.hi * u, q.I.lo * u);
+            sd = df_add_abs(sd, I);
+            td = df_add_abs(td, df_mul(I, ln32(q.I, 2 * q.e)));
+        }
+        s = scalbn(df_to_double(sd), 2 * E);
+        t = scalbn(df_to_double(td), 2 * E);
+    } else {
+        ADJ_GRID_STRIDE(i, n) {
+            const double I = (double)y[i].x * y[i].x + (double)y[i].y * y[i].y;
+            s += I;
+            if (I > 0.0) t += I * log(I);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         s += __shfl_down_sync(0xffffffffu, s, o);
@@ -246,11 +287,27 @@ __global__ void k_entropy_grad(const cpx<R>* y, cpx<R>* g, long long n, const do
     const double lnS = log(S);
     const double H = sums[1] / S - lnS;
     const double off = lnS + H, k = -2.0 / S;
-    ADJ_GRID_STRIDE(i, n) {
-        const cpx<R> v = y[i];
-        const double I = (double)v.x * v.x + (double)v.y * v.y;
-        const double d = I > 0.0 ? k * (ln_norm<R>(I) - off) : 0.0;
-        g[i] = mk((R)(d * v.x), (R)(d * v.y));
+    if constexpr (sizeof(R) == 4) {
+        const df od = df_from(-off);
+        int ke;
+        const df km = df_from(frexp(k, &ke));
+        ADJ_GRID_STRIDE(i, n) {
+            cf32 v = y[i];
+            const Norm32 q = norm32(v);
+            const df d = df_mul(km, df_add_abs(ln32(q.I, 2 * q.e), od));
+            // v d 2^(e + ke) in two exact steps
+            const int x = max(-252, min(252, q.e + ke)), h = x / 2;
+            const float u = pow2(h), w = pow2(x - h);
+            const bool some = q.I.hi > 0.0f;
+            g[i] = mk(some ? df_mul_f(d, v.x).hi * u * w : 0.0f, some ? df_mul_f(d, v.y).hi * u * w : 0.0f);
+        }
+    } else {
+        ADJ_GRID_STRIDE(i, n) {
+            const cpx<R> v = y[i];
+            const double I = (double)v.x * v.x + (double)v.y * v.y;
+            const double d = I > 0.0 ? k * (log(I) - off) : 0.0;
+            g[i] = mk((R)(d * v.x), (R)(d * v.y));
+        }
     }
 }
 
