@@ -114,7 +114,7 @@ struct s1g_decoder {
     DecodeTables tabs;
     Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
     RangeRef ref32, ref64;
-    Buf bFdf, bFit, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
+    Buf bBand, bFdf, bFit, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
     Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
     Buf bTuD, bTuG, bTuI, bTuW, bTuR, bTuWt, bTuRamp, bKa0;   // time-unfolding per-burst tables and grids
     Buf bImgIn, bImgOut, bImgMax;        // image epilogue
@@ -443,6 +443,26 @@ struct Pipe {
         else fft.rows<R>(*fft.plan<R>(n), in, ip, out, op, rows, dir, roll, scale);
     }
 
+    // out = scale IFFT(band of FFT(in)), rows of n points, the bins [start,
+    // start + width) moved to [0, width) (image_formation.cpp:160-200,315-345).
+    // in is scratch afterwards.
+    void through_band(cpx<R>* in, cpx<R>* out, int n, int start, int width, long long rows, double scale) {
+        if constexpr (sizeof(R) == 8) {
+            if (width > 0 && start >= 0 && start + width <= n) {
+                const auto f = fft.band_plan(n, start, width, false), b = fft.band_plan(n, 0, width, true);
+                if (f->nb && b->nb) {
+                    cf64* band = h->bBand.as<cf64>((size_t)rows * width);
+                    fft.to_band(*f, in, n, band, width, rows);
+                    fft.from_band(*b, band, width, out, n, rows, scale);
+                    return;
+                }
+            }
+        }
+        fft_rows(n, in, n, in, n, rows, -1);
+        band_select<R>(in, n, out, n, n, start, width, rows, st);
+        fft_rows(n, out, n, out, n, rows, +1, 0, scale);
+    }
+
     // decode -> [n_a][n_r] in buffer A
     cpx<R>* decode(const std::vector<int>& pk, const BurstGeom& g) {
         const int npk = (int)pk.size();
@@ -699,9 +719,7 @@ struct Pipe {
             transpose_batched<R>(A, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
             fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, -1);
             fufr_prep<R>(Bt, n_a, n_a, Ct, S, S, tile_len, dder, n_r, st);
-            fft_rows(S, Ct, S, Ct, S, n_r, -1);
-            band_select<R>(Ct, S, Bt, S, S, start, end - start, n_r, st);
-            fft_rows(S, Bt, S, Bt, S, n_r, +1);
+            through_band(Ct, Bt, S, start, end - start, n_r, 1.0);
             cpx<R>* drer = upload(h->bRef, rer);
             scale_mul_vec<R>(Bt, S, S, n_r, drer, 1.0 / S, st);
             A = h->bA.as<cpx<R>>((size_t)S * n_r);
@@ -761,9 +779,7 @@ struct Pipe {
         cpx<R>* D = h->bD.as<cpx<R>>((size_t)n_r * shape);
         // bD held the column tables; they are no longer needed after the row pass
         tufr_deramp<R>(Bt, S, S, C, shape, kaT, S, fdc, n_r, rate, q.num_tiles, q.focused_time, st);
-        fft_rows(shape, C, shape, C, shape, n_r, -1);
-        band_select<R>(C, shape, D, shape, shape, q.start, q.end - q.start, n_r, st);
-        fft_rows(shape, D, shape, D, shape, n_r, +1, 0, 1.0 / shape);
+        through_band(C, D, shape, q.start, q.end - q.start, n_r, 1.0 / shape);
         cpx<R>* E = h->bE.as<cpx<R>>((size_t)n_r * down);
         tufr_resample<R>(D, shape, shape, E, down, down, kaT, S, S, fdc, n_r, rate, q.n_ref, q.focused_time, st);
         const int mid = down / 2;

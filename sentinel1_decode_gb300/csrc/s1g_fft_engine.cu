@@ -170,8 +170,9 @@ void* DeviceArena::get(size_t bytes) {
 
 // ------------------------------------------------------------------ kernels
 // Launch shape of the row kernels.  FP64 is bound by its pipe (1.9 FMAs per
-// clock and SM): a few warps keep it busy, and 256 threads leave radix 8 its
-// registers.
+// clock and SM): 512 threads per SM keep it busy and leave radix 8 its
+// registers (256 where one CTA fits: 6.09 ms for 3002 rows of 10k points, 5.86
+// with 512).
 template <typename R, class F>
 static void rows4_launch(size_t smem, F f) {
     using std::integral_constant;
@@ -179,7 +180,7 @@ static void rows4_launch(size_t smem, F f) {
         fft4_launch(smem, f);
     } else {
         if (2 * (smem + 1024) <= 228 * 1024) f(integral_constant<int, 256>(), integral_constant<int, 2>());
-        else f(integral_constant<int, 256>(), integral_constant<int, 1>());
+        else f(integral_constant<int, 512>(), integral_constant<int, 1>());
     }
 }
 
@@ -248,6 +249,97 @@ __global__ void __launch_bounds__(NT, MB) k_rows_blue(RowsIo<R> io, Fft4DescT<R>
     fft4_tail(buf, d, [&](int k, cpx<R> v) {
         if (k < n) rows_put(io, y, k, off, cmul4(v, ldg(chirp + k)));
     });
+}
+
+// Band transforms (FftEngine::to_band, from_band), FP64, a CTA for several rows.
+// n (k0 + k) = n k0 + (n^2 + k^2 - (k - n)^2) / 2 makes them convolutions with
+// a chirp.  The side with all P points goes through shared memory in nb runs
+// of L points, each against its own shift of the chirp; the other side is one
+// run, so the products of all runs add up as spectra (in W, a few hundred KB
+// per CTA that stay in L2) before one inverse transform, or are formed from
+// one spectrum.  FP64 arithmetic bounds it (1.9 FMAs per clock and SM), so
+// what counts is the sum of the transform lengths: nb + 1 of L + width - 1
+// points against 2 of 2 P - 1, or 12 of 2 (P / 6) - 1 where those split.  3002
+// rows of 4987 points, a band of 600: 2.5 ms forward and 2.4 back, whole
+// transforms 6.1 each way; of 29922 = 6 x 4987 points: 28.9 and 28.3, 36.1
+// split.
+struct BandArgs {
+    const cf64* in;
+    long long ip;
+    cf64* out;
+    long long op;
+    long long rows;
+    Fft4DescT<double> d;
+    int P, width, L, nb;
+    const cf64 *pre, *chirp, *H;
+    cf64* W;
+    double scale;
+};
+template <int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_to_band(const __grid_constant__ BandArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cf64* buf = reinterpret_cast<cf64*>(smem_raw);
+    const Fft4DescT<double>& d = a.d;
+    const int last = d.radix[d.np - 1];
+    cf64* W = a.W + (long long)blockIdx.x * d.n;
+    for (long long row = blockIdx.x; row < a.rows; row += gridDim.x) {
+        const cf64* x = a.in + row * a.ip;
+        cf64* y = a.out + row * a.op;
+        for (int b = 0; b < a.nb; ++b) {
+            const int n0 = b * a.L;
+            fft4_head(buf, d, [&](int j) {
+                if (j >= a.L || n0 + j >= a.P) return mk(0.0, 0.0);
+                return cmul4(x[n0 + j], ldg(a.pre + n0 + j));
+            });
+            pass4_any<-1>(buf, d, last, 1, d.fw[d.np - 1]);
+            __syncthreads();
+            const cf64* H = a.H + (long long)b * d.n;
+            for (int i = threadIdx.x; i < d.n; i += NT) {
+                cf64 v = cmul4(buf[pad16(i)], ldg(H + i));
+                if (b > 0) v = v + W[i];
+                if (b + 1 < a.nb) W[i] = v;
+                else buf[pad16(i)] = v;
+            }
+            __syncthreads();
+        }
+        pass4_any<+1>(buf, d, last, 1, d.iv[d.np - 1]);
+        __syncthreads();
+        fft4_tail(buf, d, [&](int k, cf64 v) {
+            if (k < a.width) y[k] = cmul4(v, ldg(a.chirp + k));
+        });
+        __syncthreads();
+    }
+}
+template <int NT, int MB>
+__global__ void __launch_bounds__(NT, MB) k_from_band(const __grid_constant__ BandArgs a) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    cf64* buf = reinterpret_cast<cf64*>(smem_raw);
+    const Fft4DescT<double>& d = a.d;
+    const int last = d.radix[d.np - 1];
+    cf64* W = a.W + (long long)blockIdx.x * d.n;
+    for (long long row = blockIdx.x; row < a.rows; row += gridDim.x) {
+        const cf64* x = a.in + row * a.ip;
+        cf64* y = a.out + row * a.op;
+        fft4_head(buf, d, [&](int k) { return k < a.width ? cmul4(conj(x[k]), ldg(a.chirp + k)) : mk(0.0, 0.0); });
+        pass4_any<-1>(buf, d, last, 1, d.fw[d.np - 1]);
+        __syncthreads();
+        for (int b = 0; b < a.nb; ++b) {
+            const int n0 = b * a.L;
+            const cf64* H = a.H + (long long)b * d.n;
+            for (int i = threadIdx.x; i < d.n; i += NT) {
+                const cf64 v = b > 0 ? W[i] : buf[pad16(i)];
+                if (b == 0 && a.nb > 1) W[i] = v;
+                buf[pad16(i)] = cmul4(v, ldg(H + i));
+            }
+            __syncthreads();
+            pass4_any<+1>(buf, d, last, 1, d.iv[d.np - 1]);
+            __syncthreads();
+            fft4_tail(buf, d, [&](int j, cf64 v) {
+                if (j < a.L && n0 + j < a.P) y[n0 + j] = conj(cmul4(v, ldg(a.pre + n0 + j))) * a.scale;
+            });
+            __syncthreads();
+        }
+    }
 }
 
 // a-point transforms across the a split rows of a line: out[k + b k1].
@@ -526,6 +618,30 @@ __global__ void k_roll_scale(const cpx<R>* __restrict__ in, cpx<R>* __restrict__
     }
 }
 
+// exp(-pi i t / P), t reduced mod 2 P exactly
+__device__ __forceinline__ cf64 half_root(long long t, int P) {
+    t %= 2LL * P;
+    if (t < 0) t += 2LL * P;
+    double c, s;
+    sincospi((double)t / (double)P, &s, &c);
+    return mk(c, -s);
+}
+// Tables of a BandPlan; h: nb rows of m, the conjugate chirp at t + step b for
+// t in (-before, after), the negative ones at the row's end.
+__global__ void k_band_tables(int P, int k0, int width, int m, int nb, int step, int before, int after,
+                              cf64* __restrict__ pre, cf64* __restrict__ chirp, cf64* __restrict__ h) {
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < max((long long)P, (long long)m * nb);
+         i += (long long)gridDim.x * blockDim.x) {
+        if (i < P) pre[i] = half_root(2 * i * k0 + i * i, P);
+        if (i < width) chirp[i] = half_root(i * i, P);
+        if (i < (long long)m * nb) {
+            const int b = (int)(i / m), q = (int)(i - (long long)b * m);
+            const long long t = q < after ? q : q - m, u = t + (long long)step * b;
+            h[i] = q < after || q - m > -before ? conj(half_root(u * u, P)) : mk(0.0, 0.0);
+        }
+    }
+}
+
 static int grid_for(long long total, int threads = 256) {
     long long g = (total + threads - 1) / threads;
     if (g > 152 * 32) g = 152 * 32;
@@ -711,6 +827,43 @@ std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad) {
 template std::shared_ptr<Fft4PlanT<float>> build_plan4<float>(int, const std::vector<int>&);
 template std::shared_ptr<Fft4PlanT<double>> build_plan4<double>(int, const std::vector<int>&);
 
+// Factors of SPLIT (k_split_out).
+static const int kSplits[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16};
+
+// Lengths of the core in FP64 with their modelled instructions, ascending.
+static const std::vector<std::pair<int, double>>& lengths64() {
+    static const auto all = [] {
+        std::vector<std::pair<int, double>> v;
+        for (int n = 2; n <= fft4_capacity<double>(); ++n) {
+            const auto r = fft4_order64(n);
+            if (r.empty()) continue;
+            double c = 5.0;
+            for (int x : r) c += (x & (x - 1)) == 0 ? 3.1 * std::log2((double)x) : 4.2 * std::log2((double)x);
+            v.push_back({n, c * n});
+        }
+        return v;
+    }();
+    return all;
+}
+static double cost64(long long n) {
+    const auto& v = lengths64();
+    const auto it = std::lower_bound(v.begin(), v.end(), std::make_pair((int)n, 0.0));
+    return it != v.end() && it->first == n ? it->second : 1e30;
+}
+// The cheapest length >= least of the core in FP64, -1 if none fits.
+static long long length64(long long least) {
+    const auto& v = lengths64();
+    long long best = -1;
+    double bc = 1e30;
+    for (auto it = std::lower_bound(v.begin(), v.end(), std::make_pair((int)std::min(least, 1LL << 30), 0.0));
+         it != v.end() && it->first <= least * 5 / 4 + 8; ++it)
+        if (it->second < bc) {
+            bc = it->second;
+            best = it->first;
+        }
+    return best;
+}
+
 template <typename R>
 static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
     auto& mp = plan_map<R>(e, radix8);
@@ -730,19 +883,7 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
         if constexpr (sizeof(R) == 4) {
             return 2 * b - 1 <= cap ? fast_len(2 * b - 1) : -1;
         } else {
-            long long best = -1;
-            double bc = 1e30;
-            for (long long m = 2 * b - 1; m <= cap && m <= (2 * b - 1) * 5 / 4 + 8; ++m) {
-                const auto r = fft4_order64(m);
-                if (r.empty()) continue;
-                double c = 5.0;
-                for (int x : r) c += (x & (x - 1)) == 0 ? 3.1 * std::log2((double)x) : 4.2 * std::log2((double)x);
-                if (c * m < bc) {
-                    bc = c * m;
-                    best = m;
-                }
-            }
-            return best;
+            return length64(2 * b - 1);
         }
     };
     auto core = [&](int len) {
@@ -763,7 +904,7 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
     const long long mc = fits ? 0 : conv_len(n);
     int a = 0;   // split n = a b with b of the one-kernel kinds
     if (!fits && mc < 0 && !radix8)
-        for (int x : {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16})
+        for (int x : kSplits)
             if (n % x == 0) {
                 const auto sub = make_plan<R>(e, n / x, radix8);
                 if (sub->kind == FFT_SMEM || sub->kind == FFT_BLUE) {
@@ -840,6 +981,123 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
 template <typename R>
 std::shared_ptr<FftPlan<R>> FftEngine::plan(int n) { return make_plan<R>(*this, n, false); }
 std::shared_ptr<FftPlan<float>> FftEngine::plan8(int n) { return make_plan<float>(*this, n, true); }
+
+// The same of a row transform of n points as make_plan chooses it.
+static double row_cost64(long long n) {
+    const double c = cost64(n);
+    if (c < 1e29) return c;
+    const long long m = length64(2 * n - 1);
+    if (m >= 0) return 2 * cost64(m);
+    for (int x : kSplits)
+        if (n % x == 0 && (cost64(n / x) < 1e29 || length64(2 * (n / x) - 1) >= 0)) return x * row_cost64(n / x) + 4.0 * n;
+    return 1e29;
+}
+
+BandPlan::~BandPlan() {
+    for (void* q : owned) cudaFree(q);
+}
+
+// Bands follow the scene's Doppler rate, so their plans are few but not fixed.
+constexpr size_t kBandPlans = 8;
+
+std::shared_ptr<BandPlan> FftEngine::band_plan(int P, int k0, int width, bool inverse) {
+    const std::vector<int> key{P, k0, width, (int)inverse};
+    const auto it = bands.find(key);
+    if (it != bands.end()) return it->second;
+    auto p = std::make_shared<BandPlan>();
+    p->P = P;
+    p->k0 = k0;
+    p->width = width;
+    p->inverse = inverse;
+    // runs of L points: nb + 1 transforms, against the plain one of P
+    double best = P > 0 && width > 0 ? row_cost64(P) : 0.0;
+    long long m = 0;
+    for (int nb = 1; nb <= 16; ++nb) {
+        const int L = (P + nb - 1) / nb;
+        const long long q = length64((long long)L + width - 1);
+        if (q < 0) continue;
+        const double c = (nb + 1) * cost64(q);
+        if (c < 0.95 * best) {
+            best = c;
+            m = q;
+            p->nb = nb;
+            p->L = L;
+        }
+    }
+    if (p->nb) {
+        p->core = build_plan4<double>((int)m, fft4_order64(m));
+        auto table = [&](size_t n) {
+            void* q = nullptr;
+            check_cuda(cudaMalloc(&q, sizeof(cf64) * n), "band table");
+            p->owned.push_back(q);
+            return (cf64*)q;
+        };
+        p->pre = table(P);
+        p->chirp = table(width);
+        p->H = table((size_t)m * p->nb);
+        cf64* tmp = (cf64*)scratch_band.get(sizeof(cf64) * (size_t)m * p->nb);
+        const int before = inverse ? width : p->L, after = inverse ? p->L : width;
+        note_launch(), k_band_tables<<<grid_for(std::max<long long>(P, m * p->nb)), 256, 0, stream>>>(
+            P, k0, width, (int)m, p->nb, inverse ? p->L : -p->L, before, after, p->pre, p->chirp, tmp);
+        rows<double>(*plan<double>((int)m), tmp, m, tmp, m, p->nb, -1);
+        for (int b = 0; b < p->nb; ++b)
+            note_launch(), k_cvt64<double><<<grid_for(m), 256, 0, stream>>>(tmp + b * m, p->H + b * m, m, 1.0 / (double)m,
+                                                                            p->core->d.pos);
+    }
+    if (bands.size() >= kBandPlans) bands.clear();
+    bands[key] = p;
+    return p;
+}
+
+static void launch_band(FftEngine& e, const BandPlan& p, BandArgs a) {
+    if (a.rows <= 0) return;
+    static int sms[64] = {};
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "band");
+    int n = dev < 64 ? sms[dev] : 0;
+    if (!n) {
+        check_cuda(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "band");
+        if (dev < 64) sms[dev] = n;
+    }
+    a.d = p.core->d;
+    a.P = p.P;
+    a.width = p.width;
+    a.L = p.L;
+    a.nb = p.nb;
+    a.pre = p.pre;
+    a.chirp = p.chirp;
+    a.H = p.H;
+    const size_t smem = sizeof(cf64) * (size_t)padded16_len(a.d.n);
+    rows4_launch<double>(smem, [&](auto nt, auto mb) {
+        constexpr int NT = decltype(nt)::value, MB = decltype(mb)::value;
+        const int grid = (int)std::min<long long>(a.rows, (long long)n * MB);
+        a.W = (cf64*)e.scratch_band.get(sizeof(cf64) * (size_t)grid * a.d.n);
+        auto kernel = p.inverse ? k_from_band<NT, MB> : k_to_band<NT, MB>;
+        check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFft4SmemBytes), "attr");
+        note_launch(), kernel<<<grid, NT, smem, e.stream>>>(a);
+    });
+    check_cuda(cudaGetLastError(), "band launch");
+}
+void FftEngine::to_band(const BandPlan& p, const cf64* in, long long ip, cf64* out, long long op, long long rows) {
+    BandArgs a{};
+    a.in = in;
+    a.ip = ip;
+    a.out = out;
+    a.op = op;
+    a.rows = rows;
+    launch_band(*this, p, a);
+}
+void FftEngine::from_band(const BandPlan& p, const cf64* in, long long ip, cf64* out, long long op, long long rows,
+                          double scale) {
+    BandArgs a{};
+    a.in = in;
+    a.ip = ip;
+    a.out = out;
+    a.op = op;
+    a.rows = rows;
+    a.scale = scale;
+    launch_band(*this, p, a);
+}
 
 std::shared_ptr<Fft4Plan> FftEngine::plan4(int n) {
     auto it = plans4.find(n);

@@ -95,6 +95,20 @@ struct FftPlan {
     ~FftPlan();
 };
 
+// FP64 transforms of P points of which only a band of the spectrum is wanted
+// or given (to_band, from_band), as chirp-z transforms of runs of L points
+// that share one transform of length m on the band's side: nb + 1 of them.
+struct BandPlan {
+    int P = 0, k0 = 0, width = 0, L = 0, nb = 0;   // nb = 0: the plain transform is cheaper
+    bool inverse = false;
+    std::shared_ptr<Fft4PlanT<double>> core;       // length m
+    cf64* pre = nullptr;    // P: exp(-2 pi i n k0 / P - pi i n^2 / P)
+    cf64* chirp = nullptr;  // width: exp(-pi i k^2 / P)
+    cf64* H = nullptr;      // nb x m: spectra of the shifted conjugate chirps, at core->d.pos
+    std::vector<void*> owned;
+    ~BandPlan();
+};
+
 // One per processing context (device + stream).
 struct FftEngine {
     explicit FftEngine(cudaStream_t s);
@@ -103,9 +117,10 @@ struct FftEngine {
     std::map<int, std::shared_ptr<FftPlan<float>>> plans32;
     std::map<int, std::shared_ptr<FftPlan<double>>> plans64;
     std::map<int, std::shared_ptr<FftPlan<float>>> plans8;
+    std::map<std::vector<int>, std::shared_ptr<BandPlan>> bands;   // at most kBandPlans
     std::map<int, std::shared_ptr<FftDescTables>> descs32, descs64;   // smem_desc
     std::map<int, std::shared_ptr<Fft4Plan>> plans4;
-    DeviceArena scratch_a, scratch_b, scratch_c;
+    DeviceArena scratch_a, scratch_b, scratch_c, scratch_band;
 
     template <typename R>
     std::shared_ptr<FftPlan<R>> plan(int n);
@@ -116,6 +131,13 @@ struct FftEngine {
     template <typename R>
     void rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out,
               long long out_pitch, long long batch, int dir, int roll = 0, double scale = 1.0);
+
+    // to_band: out[k] = sum_n in[n] exp(-2 pi i n (k0 + k) / P), k < width, rows
+    // of P points; from_band: out[n] = scale sum_k in[k] exp(2 pi i n k / P),
+    // n < P, rows of width points (k0 = 0).  in and out are different.
+    std::shared_ptr<BandPlan> band_plan(int P, int k0, int width, bool inverse);
+    void to_band(const BandPlan& p, const cf64* in, long long ip, cf64* out, long long op, long long rows);
+    void from_band(const BandPlan& p, const cf64* in, long long ip, cf64* out, long long op, long long rows, double scale);
 
     // Smooth descriptor for device-side fused kernels (throws if n is not
     // 7-smooth or does not fit shared memory).

@@ -87,3 +87,18 @@ def test_interval_and_step_in_32_bits(S, T):
     want = np.minimum(u * (S - 1) // (TS - 1), S - 2)
     np.testing.assert_array_equal(q, want)
     np.testing.assert_array_equal(d, u + (-want * (TS - 1) // (S - 1)))
+
+
+# FP64 products do not depend on whether the unfolding's transforms run over
+# the band alone: the oracle's transforms are whole ones.  1e-8 is the bound of
+# the FP64 products.
+@pytest.mark.gpu
+@pytest.mark.parametrize("lines,quads", [(601, 300), (640, 257), (433, 500), (1000, 200)])
+def test_fp64_band_transforms_vs_oracle(lib_path, lines, quads):
+    import s1_oracle as O
+    data = burst(lines, quads, pulse=5.0, seed=11)
+    ref = O.S1Decoder(data).get_azimuth_compressed_burst("IW2", 0)
+    d = S1Decoder(data, precision="fp64")
+    out = d.get_azimuth_compressed_burst("IW2", 0)
+    d.close()
+    assert rel_l2(out, ref) < 1e-8
