@@ -2591,10 +2591,9 @@ int s1g_eccm_mask(s1g_decoder* h, const char* swath, int burst, uint8_t* out, in
 // two convolution FFTs of length m plus 3 complex multiplications per point
 // (6 flops each); the compensated Doppler transforms counted as plain FFTs
 // (a lower bound: compensated arithmetic costs several times more); the time
-// unfolding's gather as 7 flops per (sample, grid point) pair and range bin
-// (one complex multiply-add by a real weight plus half of the weight, shared
-// by two range bins) over ~(W T S + M) pairs, its two grid FFTs and a
-// 15-tap complex stencil per output row.
+// unfolding's gather as 4 flops per (sample, grid point) pair and range bin
+// (a complex multiply-add by a real weight from a table) over ~(W T S + M)
+// pairs, its two grid FFTs and a 15-tap complex stencil per output row.
 static double fft_flops(double n) { return n > 1 ? 5.0 * n * std::log2(n) : 0.0; }
 static double czt_flops(const CztDev& c) { return 2.0 * fft_flops(c.dm.n) + 18.0 * c.dm.n; }
 
@@ -2621,7 +2620,7 @@ int s1g_burst_stage_flops(s1g_decoder* h, const char* swath, int burst, char* bu
         const double dnr = fb.nr_smooth ? 2.0 * fft_flops(n_r) : 2.0 * czt_flops(fb.cnr);
         o << "row_pass " << S * (dnr + 60.0 * n_r) << "\n";
         o << "azimuth_ifft " << n_r * czt_flops(fb.cS) << "\n";
-        o << "time_unfold " << n_r * (7.0 * (kNuW * T * S + M) + 2.0 * fft_flops(M) + 6.0 * M +
+        o << "time_unfold " << n_r * (4.0 * (kNuW * T * S + M) + 2.0 * fft_flops(M) + 6.0 * M +
                                       8.0 * kNuTaps * n_out) << "\n";
         o << "tiles " << T << "\n";
     } else {

@@ -12,15 +12,30 @@
 // six times the arithmetic.  Twiddles are exp(-2 pi i k/n) split into float
 // pairs from FP64.
 //
-// Layout: two padded arrays H[pad(i)], E[pad(i)] (s1g_fft2.cuh padding).
-// Radices 2, 3 and 4 only (transform lengths 2^a 3^b).  dit: input at
-// pad(perm[j]), output natural; dif: natural input, output at pad(perm[j]).
+// Butterflies of radix 2, 3 and 4 and composites of them up to 16, for the
+// Doppler estimator (s1g_dcest.cu) and the ECCM notch (s1g_eccm.cu: two padded
+// arrays H[pad(i)], E[pad(i)], digit-reversed positions by perm).
 #pragma once
 
 #include "s1g_df.cuh"
-#include "s1g_fft2.cuh"
+#include "s1g_fft.cuh"
 
 namespace s1g {
+
+__device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
+
+// t = g * ns + k with 0 <= k < ns (t < 2^24)
+__device__ __forceinline__ void split_idx(int t, int ns, float inv_ns, int& g, int& k) {
+    g = __float2int_rz((float)t * inv_ns);
+    k = t - g * ns;
+    if (k < 0) {
+        --g;
+        k += ns;
+    } else if (k >= ns) {
+        ++g;
+        k -= ns;
+    }
+}
 
 struct CfftDesc {
     int n = 0;

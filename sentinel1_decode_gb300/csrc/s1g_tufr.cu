@@ -399,15 +399,6 @@ __device__ __forceinline__ double nu_kernel(double t, double beta) {
     return fabs(z) < 1.0 ? exp(beta * (sqrt(1.0 - z * z) - 1.0)) : 0.0;
 }
 
-__device__ double nu_kernel_ft(double xi, double beta, const double* gx, const double* gw) {
-    double acc = 0.0;
-    for (int q = 0; q < kNuQuad; ++q) {
-        const double t = 0.5 * kNuW * gx[q];
-        acc += gw[q] * nu_kernel(t, beta) * cospi(2.0 * xi * t);
-    }
-    return 0.5 * kNuW * acc;
-}
-
 // Per-burst tables of the time unfolding (see TufrTables), one thread per entry.
 // Band mask / Phi(p / M)^2 at the grid bins, a warp per bin: Phi by the
 // Gauss-Legendre rule, whose nodes come in pairs +-x (two pairs per lane).
