@@ -13,16 +13,13 @@
 // pairs from FP64.
 //
 // Butterflies of radix 2, 3 and 4 and composites of them up to 16, for the
-// Doppler estimator (s1g_dcest.cu) and the ECCM notch (s1g_eccm.cu: two padded
-// arrays H[pad(i)], E[pad(i)], digit-reversed positions by perm).
+// Doppler estimator (s1g_dcest.cu) and the ECCM notch (s1g_eccm.cu).
 #pragma once
 
 #include "s1g_df.cuh"
 #include "s1g_fft.cuh"
 
 namespace s1g {
-
-__device__ __forceinline__ int pad(int i) { return i + (i >> 5); }
 
 // t = g * ns + k with 0 <= k < ns (t < 2^24)
 __device__ __forceinline__ void split_idx(int t, int ns, float inv_ns, int& g, int& k) {
@@ -39,10 +36,7 @@ __device__ __forceinline__ void split_idx(int t, int ns, float inv_ns, int& g, i
 
 struct CfftDesc {
     int n = 0;
-    int nstages = 0;
-    int8_t radix[kMaxStages] = {};
     const float4* tw = nullptr;  // {cos hi, -sin hi, cos lo, -sin lo} of exp(-2 pi i k / n)
-    const int* perm = nullptr;
 };
 
 struct cc {

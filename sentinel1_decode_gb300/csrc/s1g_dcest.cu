@@ -218,53 +218,20 @@ CfftPlan::~CfftPlan() {
     for (void* p : owned) cudaFree(p);
 }
 
-static bool only_23(int n) {
-    while (n % 2 == 0) n /= 2;
-    while (n % 3 == 0) n /= 3;
-    return n == 1;
-}
-
 std::shared_ptr<CfftPlan> make_cfft_plan(int n) {
-    if (n < 2 || !only_23(n)) throw std::runtime_error("compensated FFT: length must be 2^a 3^b");
     auto p = std::make_shared<CfftPlan>();
-    std::vector<int> rad;
-    int m = n, c2 = 0, c3 = 0;
-    while (m % 2 == 0) { m /= 2; ++c2; }
-    while (m % 3 == 0) { m /= 3; ++c3; }
-    while (c2 >= 2) { rad.push_back(4); c2 -= 2; }
-    if (c2) rad.push_back(2);
-    for (int i = 0; i < c3; ++i) rad.push_back(3);
-    if ((int)rad.size() > kMaxStages) throw std::runtime_error("compensated FFT: too many stages");
-    CfftDesc& d = p->d;
-    d.n = n;
-    d.nstages = (int)rad.size();
-    for (size_t i = 0; i < rad.size(); ++i) d.radix[i] = (int8_t)rad[i];
+    p->d.n = n;
     std::vector<float4> tw(n);
     for (int i = 0; i < n; ++i) {
         const double ang = 2.0 * M_PI * ((double)i / (double)n);
         const df c = df_from(std::cos(ang)), s = df_from(-std::sin(ang));
         tw[i] = make_float4(c.hi, s.hi, c.lo, s.lo);
     }
-    std::vector<int> perm(n);
-    for (int j = 0; j < n; ++j) {
-        int jj = j, size = n, pos = 0;
-        for (int st = d.nstages - 1; st >= 0; --st) {
-            const int r = jj % rad[st];
-            jj /= rad[st];
-            size /= rad[st];
-            pos += r * size;
-        }
-        perm[j] = pos;
-    }
-    void *dt = nullptr, *dp = nullptr;
+    void* dt = nullptr;
     check_cuda(cudaMalloc(&dt, sizeof(float4) * n), "cfft tw");
     p->owned.push_back(dt);
-    check_cuda(cudaMalloc(&dp, sizeof(int) * n), "cfft perm");
-    p->owned.push_back(dp);
     check_cuda(cudaMemcpy(dt, tw.data(), sizeof(float4) * n, cudaMemcpyHostToDevice), "cfft tw up");
-    check_cuda(cudaMemcpy(dp, perm.data(), sizeof(int) * n, cudaMemcpyHostToDevice), "cfft perm up");
-    d.tw = (const float4*)dt;
-    d.perm = (const int*)dp;
+    p->d.tw = (const float4*)dt;
     return p;
 }
 

@@ -34,6 +34,23 @@ __host__ __device__ __forceinline__ df df_from(double x) {
 __host__ __device__ __forceinline__ double df_to_double(df a) { return (double)a.hi + (double)a.lo; }
 
 #ifdef __CUDACC__
+// v as a float pair without the FP64 pipe: the leading 24 bits of the
+// significand (truncated) and the other 29 rounded to 24.  Zero, and what has
+// no such pair (below 2^-62, above 2^127), by conversions.
+__device__ __forceinline__ df df_split(double v) {
+    const unsigned int h = (unsigned int)__double2hiint(v), l = (unsigned int)__double2loint(v);
+    const int e = (int)((h >> 20) & 0x7ff) - 1023;
+    if (e < -62 || e > 126) {
+        const float f = (float)v;
+        return df_make(f, (float)(v - (double)f));
+    }
+    const unsigned int s = h & 0x80000000u;
+    const float hi = __uint_as_float(s | (unsigned int)(e + 127) << 23 | (h & 0xfffffu) << 3 | l >> 29);
+    // low 29 bits in units of 2^(e - 52)
+    const float unit = __uint_as_float(s | (unsigned int)(e - 52 + 127) << 23);
+    return df_make(hi, (float)(int)(l & 0x1fffffffu) * unit);
+}
+
 __device__ __forceinline__ df quick_two_sum(float a, float b) {
     const float s = __fadd_rn(a, b);
     const float e = __fsub_rn(b, __fsub_rn(s, a));

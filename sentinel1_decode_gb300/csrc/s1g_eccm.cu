@@ -14,13 +14,13 @@
 // conversions per clock and SM, so what runs per value stays off that pipe:
 // the samples are split by their bits, a gradient is formed in FP32 and in
 // FP64 only within 1e-5 of the threshold.  1500 lines of 12000 samples: the
-// notch 1.32 ms (3.70 with FP64 splits, gradients and output sums), the
-// detection 0.06 ms (0.56 with FP64 magnitudes).
+// notch 0.90 ms (1.32 with a trip through shared memory per radix-4 stage, 3.70
+// with FP64 splits, gradients and output sums too), the detection 0.06 ms (0.56
+// with FP64 magnitudes).
 //
 // One block per flagged line (flags from k_eccm_detect_mixed below), windows
-// of 128 samples at stride 64 in batches of kEccmBatch, forward transform
-// from digit-reversed positions, gradient and decision from h + e,
-// zeroing, inverse transform back to digit-reversed positions, 1/128, and
+// of 128 samples at stride 64 in batches of kEccmBatch: forward transform,
+// gradient and decision from h + e, zeroing, inverse transform, 1/128, and
 // each sample written from the last window that covers it (later windows
 // overwrite earlier ones).
 #include <stdexcept>
@@ -34,122 +34,29 @@ namespace s1g {
 namespace {
 
 constexpr int kEccmFft = 128;
-constexpr int kEccmBatch = 16;   // windows per pass
+constexpr int kEccmBatch = 16;                       // windows per pass
+constexpr int kEccmThreads = 128;
+constexpr int kEccmRow = kEccmFft + kEccmFft / 8;    // float4 of a window, one of padding in 8
 
-template <int P>
-__device__ __forceinline__ void cdit_stage_b(cf32* H, cf32* E, const CfftDesc& d, int Ns, int dir, int nwin) {
-    const int n = d.n;
-    const int nb = n / P;
-    const int span = Ns * P;
-    const int step = n / span;
-    for (int t = threadIdx.x; t < nwin * nb; t += blockDim.x) {
-        const int w = t / nb, tt = t - w * nb;
-        const int g = tt / Ns, k = tt - g * Ns;
-        const int base = w * n + g * span + k;
-        cc a[P];
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const int i = pad(base + r * Ns);
-            a[r] = cc_make(H[i], E[i]);
-        }
-        if (Ns > 1) {
-#pragma unroll
-            for (int r = 1; r < P; ++r) a[r] = cc_twiddle(a[r], d.tw, r * k * step, dir);
-        }
-        CBfly<P>::run(a, dir);
-#pragma unroll
-        for (int s = 0; s < P; ++s) {
-            const int i = pad(base + s * Ns);
-            H[i] = mk(a[s].hx, a[s].hy);
-            E[i] = mk(a[s].ex, a[s].ey);
-        }
-    }
+__device__ __forceinline__ cc at_cc(const float4* S, int i) {
+    const float4 v = S[i];
+    return cc{v.x, v.y, v.z, v.w};
 }
-
-template <int P>
-__device__ __forceinline__ void cdif_stage_b(cf32* H, cf32* E, const CfftDesc& d, int Ns, int dir, int nwin) {
-    const int n = d.n;
-    const int nb = n / P;
-    const int span = Ns * P;
-    const int step = n / span;
-    for (int t = threadIdx.x; t < nwin * nb; t += blockDim.x) {
-        const int w = t / nb, tt = t - w * nb;
-        const int g = tt / Ns, k = tt - g * Ns;
-        const int base = w * n + g * span + k;
-        cc a[P];
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            const int i = pad(base + r * Ns);
-            a[r] = cc_make(H[i], E[i]);
-        }
-        CBfly<P>::run(a, dir);
-        if (Ns > 1) {
-#pragma unroll
-            for (int s = 1; s < P; ++s) a[s] = cc_twiddle(a[s], d.tw, s * k * step, dir);
-        }
-#pragma unroll
-        for (int s = 0; s < P; ++s) {
-            const int i = pad(base + s * Ns);
-            H[i] = mk(a[s].hx, a[s].hy);
-            E[i] = mk(a[s].ex, a[s].ey);
-        }
-    }
-}
-
-// digit-reversed input -> natural output (every window of the batch)
-__device__ void cfft_dit_b(cf32* H, cf32* E, const CfftDesc& d, int dir, int nwin) {
-    int Ns = 1;
-    for (int st = 0; st < d.nstages; ++st) {
-        const int p = d.radix[st];
-        if (p == 4) cdit_stage_b<4>(H, E, d, Ns, dir, nwin);
-        else if (p == 3) cdit_stage_b<3>(H, E, d, Ns, dir, nwin);
-        else cdit_stage_b<2>(H, E, d, Ns, dir, nwin);
-        __syncthreads();
-        Ns *= p;
-    }
-}
-
-// natural input -> digit-reversed output
-__device__ void cfft_dif_b(cf32* H, cf32* E, const CfftDesc& d, int dir, int nwin) {
-    int Ns = d.n;
-    for (int st = d.nstages - 1; st >= 0; --st) {
-        const int p = d.radix[st];
-        Ns /= p;
-        if (p == 4) cdif_stage_b<4>(H, E, d, Ns, dir, nwin);
-        else if (p == 3) cdif_stage_b<3>(H, E, d, Ns, dir, nwin);
-        else cdif_stage_b<2>(H, E, d, Ns, dir, nwin);
-        __syncthreads();
-    }
-}
-
-// v as a float pair without the FP64 pipe: the leading 24 bits of the
-// significand (truncated) and the other 29 rounded to 24.  Zero, and what has
-// no such pair (below 2^-62, above 2^127), by conversions.
-__device__ __forceinline__ df split_bits(double v) {
-    const unsigned int h = (unsigned int)__double2hiint(v), l = (unsigned int)__double2loint(v);
-    const int e = (int)((h >> 20) & 0x7ff) - 1023;
-    if (e < -62 || e > 126) {
-        const float f = (float)v;
-        return df_make(f, (float)(v - (double)f));
-    }
-    const unsigned int s = h & 0x80000000u;
-    const float hi = __uint_as_float(s | (unsigned int)(e + 127) << 23 | (h & 0xfffffu) << 3 | l >> 29);
-    // low 29 bits in units of 2^(e - 52)
-    const float unit = __uint_as_float(s | (unsigned int)(e - 52 + 127) << 23);
-    return df_make(hi, (float)(int)(l & 0x1fffffffu) * unit);
-}
-
-__device__ __forceinline__ double2 cc_value(const cf32* H, const cf32* E, int i) {
-    return make_double2((double)H[i].x + (double)E[i].x, (double)H[i].y + (double)E[i].y);
+__device__ __forceinline__ double2 cc_value(const cc& v) {
+    return make_double2((double)v.hx + (double)v.ex, (double)v.hy + (double)v.ey);
 }
 
 }  // namespace
 
-__global__ void __launch_bounds__(256) k_eccm_notch_cc(const cf64* __restrict__ in, long long ip, cf32* __restrict__ out,
-                                                       long long op, int n_r, const int* __restrict__ flags,
-                                                       double mit, CfftDesc d, int num_ffts) {
-    __shared__ cf32 H[kEccmBatch * kEccmFft + (kEccmBatch * kEccmFft) / 32 + 1];
-    __shared__ cf32 E[kEccmBatch * kEccmFft + (kEccmBatch * kEccmFft) / 32 + 1];
+// A window is 16 x 8 points: radix-16 butterflies (one per thread) over the
+// samples k + 8 r, read from the line and written to it by the same passes,
+// and radix-8 ones over positions 8 s0 + s1, which then hold frequency
+// s0 + 16 s1.
+__global__ void __launch_bounds__(kEccmThreads, 4) k_eccm_notch_cc(const cf64* __restrict__ in, long long ip,
+                                                                   cf32* __restrict__ out, long long op, int n_r,
+                                                                   const int* __restrict__ flags, double mit, CfftDesc d,
+                                                                   int num_ffts) {
+    __shared__ float4 S[kEccmBatch * kEccmRow];
     __shared__ unsigned char zero[kEccmBatch * kEccmFft];
     const long long row = blockIdx.x;
     if (!flags[row]) return;
@@ -159,77 +66,101 @@ __global__ void __launch_bounds__(256) k_eccm_notch_cc(const cf64* __restrict__ 
     // float range; big_max < 0 sends every bin to FP64
     const float mit2 = (float)(mit * mit);
     const float big_max = mit > 1e-9 && mit < 1e12 ? (float)mit * 1e5f : -1.0f;
+    const int wa = threadIdx.x >> 3, k = threadIdx.x & 7;
+    float4* Sa = S + wa * kEccmRow + k;
     for (int w0 = 0; w0 < num_ffts; w0 += kEccmBatch) {
         const int nw = min(kEccmBatch, num_ffts - w0);
-        // windows of the original line, zero-filled past their (cut) end
-        for (int t = threadIdx.x; t < nw * kEccmFft; t += blockDim.x) {
-            const int w = t >> 7, q = t & 127;
-            const int s = (w0 + w) * 64;
-            int e = s + kEccmFft;
-            if (e > n_r) e = n_r - 1;
-            df x = df_make(0.f, 0.f), y = x;
-            if (s + q < e) {
-                const double2 v = __ldg(reinterpret_cast<const double2*>(line) + s + q);
-                x = split_bits(v.x);
-                y = split_bits(v.y);
+        // the original line's window, zero-filled past its (cut) end
+        const int s0 = (w0 + wa) * 64;
+        int end = s0 + kEccmFft;
+        if (end > n_r) end = n_r - 1;
+        if (wa < nw) {
+            cc v[16];
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                df x = df_make(0.f, 0.f), y = x;
+                const int j = s0 + k + 8 * r;
+                if (j < end) {
+                    const double2 z = __ldg(reinterpret_cast<const double2*>(line) + j);
+                    x = df_split(z.x);
+                    y = df_split(z.y);
+                }
+                v[r] = cc{x.hi, y.hi, x.lo, y.lo};
             }
-            const int i = pad(w * kEccmFft + __ldg(d.perm + q));
-            H[i] = mk(x.hi, y.hi);
-            E[i] = mk(x.lo, y.lo);
+            cc_fft<16, -1>(v);
+#pragma unroll
+            for (int s = 0; s < 16; ++s) {
+                if (s > 0) v[s] = cc_twiddle(v[s], d.tw, s * k, -1);
+                Sa[9 * s] = make_float4(v[s].hx, v[s].hy, v[s].ex, v[s].ey);
+            }
         }
         __syncthreads();
-        cfft_dit_b(H, E, d, -1, nw);
+        for (int t = threadIdx.x; t < nw * 16; t += kEccmThreads) {
+            float4* b = S + (t >> 4) * kEccmRow + 9 * (t & 15);
+            cc v[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) v[r] = at_cc(b, r);
+            cc_fft<8, -1>(v);
+#pragma unroll
+            for (int s = 0; s < 8; ++s) b[s] = make_float4(v[s].hx, v[s].hy, v[s].ex, v[s].ey);
+        }
+        __syncthreads();
         // central-difference gradient along frequency (one-sided at the ends)
-        for (int t = threadIdx.x; t < nw * kEccmFft; t += blockDim.x) {
+        for (int t = threadIdx.x; t < nw * kEccmFft; t += kEccmThreads) {
             const int w = t >> 7, q = t & 127;
-            const int b = w * kEccmFft;
+            const float4* b = S + w * kEccmRow;
             // (X[up] - X[dn]) scale; in FP32 where that decides: its error is
             // below 2^-22 of itself and 2^-40 of the values
-            const int up = pad(b + min(q + 1, kEccmFft - 1)), dn = pad(b + max(q - 1, 0));
+            const int up = min(q + 1, kEccmFft - 1), dn = max(q - 1, 0);
             const float scale = q != 0 && q != kEccmFft - 1 ? 0.5f : 1.0f;
-            const cf32 hu = H[up], hd = H[dn], eu = E[up], ed = E[dn];
-            const float gx = scale * ((hu.x - hd.x) + (eu.x - ed.x)), gy = scale * ((hu.y - hd.y) + (eu.y - ed.y));
+            const cc u = at_cc(b, 9 * (up & 15) + (up >> 4)), v = at_cc(b, 9 * (dn & 15) + (dn >> 4));
+            const float gx = scale * ((u.hx - v.hx) + (u.ex - v.ex)), gy = scale * ((u.hy - v.hy) + (u.ey - v.ey));
             const float g2 = fmaf(gx, gx, gy * gy);
-            const float big = fmaxf(fmaxf(fabsf(hu.x), fabsf(hu.y)), fmaxf(fabsf(hd.x), fabsf(hd.y)));
+            const float big = fmaxf(fmaxf(fabsf(u.hx), fabsf(u.hy)), fmaxf(fabsf(v.hx), fabsf(v.hy)));
             if (fabsf(g2 - mit2) > 1e-5f * mit2 && big < big_max) {
                 zero[t] = g2 < mit2 ? 0 : 1;
             } else {
-                const double2 a = cc_value(H, E, up), c = cc_value(H, E, dn);
+                const double2 a = cc_value(u), c = cc_value(v);
                 const double x = (a.x - c.x) * scale, y = (a.y - c.y) * scale;
                 zero[t] = (hypot(x, y) < mit) ? 0 : 1;
             }
         }
         __syncthreads();
-        for (int t = threadIdx.x; t < nw * kEccmFft; t += blockDim.x)
-            if (zero[t]) {
-                const int i = pad(t);
-                H[i] = mk(0.f, 0.f);
-                E[i] = mk(0.f, 0.f);
+        for (int t = threadIdx.x; t < nw * 16; t += kEccmThreads) {
+            const int w = t >> 4, s = t & 15;
+            float4* b = S + w * kEccmRow + 9 * s;
+            cc v[8];
+#pragma unroll
+            for (int r = 0; r < 8; ++r) {
+                v[r] = at_cc(b, r);
+                if (zero[w * kEccmFft + s + 16 * r]) v[r] = cc{0.f, 0.f, 0.f, 0.f};
             }
+            cc_fft<8, 1>(v);
+#pragma unroll
+            for (int r = 0; r < 8; ++r) b[r] = make_float4(v[r].hx, v[r].hy, v[r].ex, v[r].ey);
+        }
         __syncthreads();
-        cfft_dif_b(H, E, d, +1, nw);
-        for (int t = threadIdx.x; t < nw * kEccmFft; t += blockDim.x) {
-            const int w = t >> 7, q = t & 127;
-            const int wi = w0 + w;
-            const int s = wi * 64;
-            int e = s + kEccmFft;
-            if (e > n_r) e = n_r - 1;
-            const int j = s + q;
-            if (j >= e) continue;
-            // owner of j: the later of the (at most two) windows covering it
-            int owner = -1;
-            for (int c = j / 64; c >= j / 64 - 1 && c >= 0; --c) {
-                if (c >= num_ffts) continue;
-                int ce = c * 64 + kEccmFft;
-                if (ce > n_r) ce = n_r - 1;
-                if (j < ce) {
-                    owner = c;
-                    break;
-                }
+        if (wa < nw) {
+            cc v[16];
+#pragma unroll
+            for (int s = 0; s < 16; ++s) {
+                v[s] = at_cc(Sa, 9 * s);
+                if (s > 0) v[s] = cc_twiddle(v[s], d.tw, s * k, +1);
             }
-            if (owner != wi) continue;
-            const int i = pad(w * kEccmFft + __ldg(d.perm + q));
-            o[j] = mk((H[i].x + E[i].x) * (1.0f / 128.0f), (H[i].y + E[i].y) * (1.0f / 128.0f));
+            cc_fft<16, 1>(v);
+#pragma unroll
+            for (int r = 0; r < 16; ++r) {
+                const int wi = w0 + wa, j = s0 + k + 8 * r;
+                if (j >= end) continue;
+                // a later window that covers j overwrites it: the next one
+                // covers the second half of this one
+                if (8 * r + k >= 64 && wi + 1 < num_ffts) {
+                    int ce = (wi + 1) * 64 + kEccmFft;
+                    if (ce > n_r) ce = n_r - 1;
+                    if (j < ce) continue;
+                }
+                o[j] = mk((v[r].hx + v[r].ex) * (1.0f / 128.0f), (v[r].hy + v[r].ey) * (1.0f / 128.0f));
+            }
         }
         __syncthreads();
     }
@@ -340,10 +271,10 @@ void eccm_detect_mixed(const cf32* X32, long long xp, int n, long long rows, dou
 
 void eccm_notch_cc(const cf64* in, long long ip, cf32* out, long long op, int n_r, long long rows, const int* flags,
                    double mit, const CfftDesc& d128, cudaStream_t st) {
-    if (d128.n != kEccmFft) throw std::runtime_error("eccm: the compensated transform must have 128 points");
+    if (d128.n != kEccmFft) throw std::runtime_error("eccm: the twiddles must be those of 128 points");
     const int num_ffts = eccm_num_windows(n_r);
     if (rows > 0 && num_ffts > 0)
-        note_launch(), k_eccm_notch_cc<<<(unsigned)rows, 256, 0, st>>>(in, ip, out, op, n_r, flags, mit, d128,
+        note_launch(), k_eccm_notch_cc<<<(unsigned)rows, kEccmThreads, 0, st>>>(in, ip, out, op, n_r, flags, mit, d128,
                                                                         num_ffts);
 }
 
