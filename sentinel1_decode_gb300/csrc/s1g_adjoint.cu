@@ -15,7 +15,7 @@
 // reduced before the FP32 sine / cosine; reductions accumulate in FP64, in the
 // FP32 chain in double-float within a thread.  GB300 does 1.9 FP64 operations
 // per clock and SM, so FP64 per element bounded these kernels: the five took
-// 1.6 of the 2.5 ms of a 1024 x 4096 evaluation's device time, now 0.27 of 0.89 ms.
+// 1.6 of the 2.5 ms of a 1024 x 4096 evaluation's device time, now 0.27 of 0.84 ms.
 #include <algorithm>
 #include <cmath>
 #include <mutex>
@@ -82,7 +82,7 @@ __global__ void k_rcmc_phase(cpx<R>* a, int n, long long rows, const double* __r
 // cos, sin of 2 pi (hi + lo) turns, |hi + lo| <= 1/2: the angle is formed to
 // 2^-46 and rounded to float once, as cis_d<float> rounds its FP64 angle, so
 // the factors are those of the FP64 phases but where 2^-46 decides the
-// rounding (under one in 10^3 elements).
+// rounding (one in 10^6 elements).
 __device__ __forceinline__ cf32 cis_turn(float hi, float lo) {
     const df p = two_prod(hi, 6.283185482025146484375f);   // 2 pi as 24 bits + the rest
     const float r = p.hi + fmaf(hi, -1.74845560007449713e-7f, fmaf(lo, 6.28318530717958648f, p.lo));
@@ -124,23 +124,42 @@ __global__ void k_az_filter(cpx<R>* a, int n_r, long long rows, const double* __
     }
 }
 
-// FP32: a thread keeps one range bin's 2 R_r / lambda (turns) as a
-// double-float over the rows it takes.
+// An FP64 value as three floats.
+struct tf {
+    float a, b, c;
+};
+__device__ __forceinline__ tf tf_from(double x) {
+    tf r;
+    r.a = (float)x;
+    const double y = x - (double)r.a;
+    r.b = (float)y;
+    r.c = (float)(y - (double)r.b);
+    return r;
+}
+
+// FP32: a thread keeps one range bin's 2 R_r / lambda (turns) over the rows it
+// takes; the product with 1 - D (10^3 turns) is reduced to a fraction of a turn
+// that is good to 2^-48, as the FP64 phase is.
 constexpr int kAzRows = 16;
 __global__ void __launch_bounds__(256) k_az_filter32(cf32* a, int n_r, int rows, const double* __restrict__ omd,
                                                      const double* __restrict__ slant, double c4pl, int sign) {
-    __shared__ df w[kAzRows];
+    __shared__ tf w[kAzRows];
     const int k0 = blockIdx.y * kAzRows;
     const int nk = min(kAzRows, rows - k0);
-    if (threadIdx.x < nk) w[threadIdx.x] = df_from((double)sign * omd[k0 + threadIdx.x]);
+    if (threadIdx.x < nk) w[threadIdx.x] = tf_from((double)sign * omd[k0 + threadIdx.x]);
     __syncthreads();
     const int r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= n_r) return;
-    const df t = df_from(c4pl * slant[r] * 0.15915494309189533577);
+    const tf t = tf_from(c4pl * slant[r] * 0.15915494309189533577);
     for (int k = 0; k < nk; ++k) {
-        const df u = df_mul(t, w[k]);
-        cf32* p = a + (long long)(k0 + k) * n_r + r;
-        *p = cmul_(*p, cis_turn(u.hi - rintf(u.hi), u.lo));
+        const tf m = w[k];
+        const df p = two_prod(t.a, m.a), q = two_prod(t.a, m.b), u = two_prod(t.b, m.a);
+        const df s0 = two_sum(p.hi - rintf(p.hi), p.lo);
+        const df s1 = two_sum(s0.hi, q.hi);
+        const df s2 = two_sum(s1.hi, u.hi);
+        const float rest = fmaf(t.b, m.b, fmaf(t.a, m.c, fmaf(t.c, m.a, q.lo + u.lo)));
+        cf32* x = a + (long long)(k0 + k) * n_r + r;
+        *x = cmul_(*x, cis_turn(s2.hi, (s0.lo + s1.lo) + (s2.lo + rest)));
     }
 }
 
@@ -328,7 +347,7 @@ __global__ void k_row_imdot(const cpx<R>* __restrict__ a, const cpx<R>* __restri
             const df p = two_prod(ar[c].x, br[c].y), q = two_prod(-ar[c].y, br[c].x);
             df im = two_sum(p.hi, q.hi);
             im.lo += p.lo + q.lo;
-            if (colw) im = df_mul(im, df_from(colw[c]));
+            if (colw) im = df_mul(im, df_split(colw[c]));
             else if (freq_fs > 0.0) im = df_mul_f(im, (float)(c < (cols + 1) / 2 ? c : c - cols));
             s = df_add_abs(s, im);
         }

@@ -437,10 +437,13 @@ struct Pipe {
         return d;
     }
 
+    std::shared_ptr<FftPlan<R>> row_plan(int n) {
+        if constexpr (sizeof(R) == 4) return fft.plan8(n);
+        else return fft.plan<R>(n);
+    }
     void fft_rows(int n, const cpx<R>* in, long long ip, cpx<R>* out, long long op, long long rows, int dir, int roll = 0,
                   double scale = 1.0) {
-        if constexpr (sizeof(R) == 4) fft.rows<R>(*fft.plan8(n), in, ip, out, op, rows, dir, roll, scale);
-        else fft.rows<R>(*fft.plan<R>(n), in, ip, out, op, rows, dir, roll, scale);
+        fft.rows<R>(*row_plan(n), in, ip, out, op, rows, dir, roll, scale);
     }
 
     // out = scale IFFT(band of FFT(in)), rows of n points, the bins [start,
@@ -606,11 +609,19 @@ struct Pipe {
         }
         const cpx<R>* ref = (const cpx<R>*)rr.dev.p;
         cpx<R>* B = h->bB.as<cpx<R>>((size_t)n_a * M);
-        pad_rows<R>(A, n_r, n_r, B, M, M, n_a, st);
-        fft_rows(M, B, M, B, M, n_a, -1);
-        mul_rows_by_vec<R>(B, M, M, n_a, ref, st);
-        fft_rows(M, B, M, B, M, n_a, +1);
-        rc_crop<R>(B, M, M, A, n_r, n_r, g.h, n_a, st);
+        const auto plan = row_plan(M);
+        if (fft.one_kernel(*plan)) {
+            // zero padding, filter, shift and crop in the transforms' ends
+            const RowEnds<R> fwd{n_r, M, ref}, inv{M, n_r, nullptr};
+            fft.rows<R>(*plan, A, n_r, B, M, n_a, -1, 0, 1.0, &fwd);
+            fft.rows<R>(*plan, B, M, A, n_r, n_a, +1, g.h % M, 1.0, &inv);
+        } else {
+            pad_rows<R>(A, n_r, n_r, B, M, M, n_a, st);
+            fft_rows(M, B, M, B, M, n_a, -1);
+            mul_rows_by_vec<R>(B, M, M, n_a, ref, st);
+            fft_rows(M, B, M, B, M, n_a, +1);
+            rc_crop<R>(B, M, M, A, n_r, n_r, g.h, n_a, st);
+        }
         if (rd) {
             // transpose, azimuth FFT, fftshift, transpose (s1_decoder.cpp:499-505)
             cpx<R>* Bt = h->bB.as<cpx<R>>((size_t)n_a * n_r);

@@ -6,8 +6,8 @@
 //                   the two length-S DFTs done as band-limited chirp-z transforms
 //   k_czt_rows      azimuth IFFT (length S, chirp-z) per range bin
 // here, k_rowpass_fused (range FFT, SRC, range IFFT, scaling, RCMC, azimuth
-// filter) in s1g_rowpass.cu and k_tufr_fused (time unfolding, resampling and
-// re-ramp) in s1g_tufr.cu.  The Doppler lag-1 sums come from s1g_dcest.cu.
+// filter) in s1g_rowpass.cu and the k_tufr_* kernels (time unfolding, resampling
+// and re-ramp) in s1g_tufr.cu.  The Doppler lag-1 sums come from s1g_dcest.cu.
 // Phase arguments are formed in double-float (s1g_df.cuh); no FP64
 // arithmetic runs per sample.
 #include <algorithm>

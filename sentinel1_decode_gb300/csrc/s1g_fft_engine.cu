@@ -198,6 +198,8 @@ struct RowsIo {
     int dir;
     int n, roll;         // points of a row, where output 0 goes
     R scale;
+    int valid, count;    // inputs given (zeros follow), outputs wanted (of the rolled row)
+    const cpx<R>* mul;   // factor of output k (before the roll), or null
 };
 template <typename R>
 __device__ __forceinline__ void rows_put(const RowsIo<R>& io, cpx<R>* y, int k, int off, cpx<R> v) {
@@ -207,8 +209,11 @@ __device__ __forceinline__ void rows_put(const RowsIo<R>& io, cpx<R>* y, int k, 
         if (io.dir > 0) w = conj(w);
         v = cmul4(v, w);
     }
+    v = v * io.scale;
+    if (io.mul) v = v * ldg(io.mul + k);
     k += io.roll;
-    y[k < io.n ? k : k - io.n] = v * io.scale;
+    if (k >= io.n) k -= io.n;
+    if (k < io.count) y[k] = v;
 }
 
 // Rows of a 7-smooth length: out[k] = sum_j in[j] exp(dir 2 pi i j k / n).
@@ -222,6 +227,7 @@ __global__ void __launch_bounds__(NT, MB) k_rows_smooth(RowsIo<R> io, Fft4DescT<
     const cpx<R>* x = io.in + line * io.ip + off;
     cpx<R>* y = io.out + (long long)blockIdx.x * io.op;
     fft4_head(buf, d, [&](int j) {
+        if (j >= io.valid) return mk((R)0, (R)0);
         const cpx<R> v = x[(long long)j * io.a];
         return io.dir > 0 ? conj(v) : v;
     });
@@ -241,7 +247,7 @@ __global__ void __launch_bounds__(NT, MB) k_rows_blue(RowsIo<R> io, Fft4DescT<R>
     const cpx<R>* x = io.in + line * io.ip + off;
     cpx<R>* y = io.out + (long long)blockIdx.x * io.op;
     fft4_head(buf, d, [&](int j) {
-        if (j >= n) return mk((R)0, (R)0);
+        if (j >= io.valid) return mk((R)0, (R)0);
         const cpx<R> v = x[(long long)j * io.a];
         return cmul4(io.dir > 0 ? conj(v) : v, ldg(chirp + j));
     });
@@ -394,8 +400,10 @@ struct Rows8 {
     long long ip;
     cf32* out;
     long long op;
-    int n, roll;             // points of a row, where output 0 goes
+    int n, roll;             // as RowsIo
     float scale;
+    int valid, count;
+    const cf32* mul;
     int dir;
     int mask;                // -1: padded shared memory, 0: not
     FftDesc<float> d;        // length n, or of the chirp-z convolution
@@ -468,8 +476,15 @@ __device__ __forceinline__ void rows8_out(const cf32* buf, const FftDesc<float>&
         default: { constexpr int P = 8; CALL; break; }    \
     }
 __device__ __forceinline__ void rows8_put(const Rows8& a, cf32* y, int k, cf32 v) {
+    v = v * a.scale;
+    if (a.mul) {
+        // rounded as the product of a pass of its own
+        const cf32 m = ldg(a.mul + k);
+        v = mk(__fmaf_rn(v.x, m.x, -__fmul_rn(v.y, m.y)), __fmaf_rn(v.y, m.x, __fmul_rn(v.x, m.y)));
+    }
     k += a.roll;
-    y[k < a.n ? k : k - a.n] = v * a.scale;
+    if (k >= a.n) k -= a.n;
+    if (k < a.count) y[k] = v;
 }
 
 __global__ void __launch_bounds__(kFftThreads, 2) k_rows8_smooth(const __grid_constant__ Rows8 a) {
@@ -483,12 +498,12 @@ __global__ void __launch_bounds__(kFftThreads, 2) k_rows8_smooth(const __grid_co
         // n is 1 or a radix: one thread
         if (threadIdx.x > 0) return;
         cf32 v[8];
-        for (int j = 0; j < d.n; ++j) v[j] = x[j];
+        for (int j = 0; j < d.n; ++j) v[j] = j < a.valid ? x[j] : mk(0.0f, 0.0f);
         if (d.nstages == 1) ROWS8_RADIX(d.radix[0], (Bfly<float, P>::run(v, a.dir)));
         for (int j = 0; j < d.n; ++j) put(j, v[j]);
         return;
     }
-    ROWS8_RADIX(d.radix[0], (rows8_in<P>(buf, d, a.dir, a.mask, [&](int j) { return x[j]; })));
+    ROWS8_RADIX(d.radix[0], (rows8_in<P>(buf, d, a.dir, a.mask, [&](int j) { return j < a.valid ? x[j] : mk(0.0f, 0.0f); })));
     __syncthreads();
     int Ns = d.radix[0];
     for (int st = 1; st + 1 < d.nstages; ++st) {
@@ -508,7 +523,7 @@ __global__ void __launch_bounds__(kFftThreads) k_rows8_blue(const __grid_constan
     const int m = a.d.n;
     for (int q = threadIdx.x; q < m; q += blockDim.x) {
         cf32 v = mk(0.0f, 0.0f);
-        if (q < a.n) {
+        if (q < a.valid) {
             cf32 xv = x[q];
             if (a.dir > 0) xv = conj(xv);
             v = xv * ldg(a.chirp + q);
@@ -1144,7 +1159,7 @@ static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows
             const bool smooth = p.kind == FFT_SMEM, fits = smooth && sizeof(cf32) * (size_t)padded <= (size_t)kSmemBytes;
             const int nt = smooth ? std::min(kFftThreads, std::max(64, (d.n / 8 + 31) / 32 * 32)) : kFftThreads;
             const size_t smem = sizeof(cf32) * (size_t)(fits ? padded : d.n);
-            const Rows8 q{io.in, io.ip, io.out, io.op, p.n, io.roll, io.scale, io.dir, fits ? -1 : 0, d, p.chirp, p.kern};
+            const Rows8 q{io.in, io.ip, io.out, io.op, p.n, io.roll, io.scale, io.valid, io.count, io.mul, io.dir, fits ? -1 : 0, d, p.chirp, p.kern};
             if (smooth) note_launch(), k_rows8_smooth<<<(unsigned)rows, nt, smem, st>>>(q);
             else note_launch(), k_rows8_blue<<<(unsigned)rows, nt, smem, st>>>(q);
             return;
@@ -1168,13 +1183,15 @@ static void launch_rows(const FftPlan<R>& p, const RowsIo<R>& io, long long rows
 
 template <typename R>
 void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out, long long out_pitch,
-                     long long batch, int dir, int roll, double scale) {
+                     long long batch, int dir, int roll, double scale, const RowEnds<R>* ends) {
     if (batch <= 0) return;
     const int n = p.n;
+    if (ends && !one_kernel(p)) throw std::runtime_error("fft: partial rows of a length over one CTA");
     switch (p.kind) {
         case FFT_SMEM:
-        case FFT_BLUE: launch_rows<R>(p, RowsIo<R>{in, in_pitch, out, out_pitch, 1, nullptr, dir, n, roll, (R)scale}, batch,
-                                      stream);
+        case FFT_BLUE: launch_rows<R>(p, RowsIo<R>{in, in_pitch, out, out_pitch, 1, nullptr, dir, n, roll, (R)scale,
+                                                ends ? ends->valid : n, ends ? ends->count : n,
+                                                ends ? ends->mul : nullptr}, batch, stream);
             return;
         case FFT_SPLIT: {
             const long long limit = (1LL << 30) / (long long)sizeof(cpx<R>);
@@ -1182,8 +1199,8 @@ void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, 
             cpx<R>* Y = (cpx<R>*)scratch_a.get(sizeof(cpx<R>) * chunk * n);
             for (long long b0 = 0; b0 < batch; b0 += chunk) {
                 const long long nb = std::min(chunk, batch - b0);
-                launch_rows<R>(*p.p2, RowsIo<R>{in + b0 * in_pitch, in_pitch, Y, p.n2, p.n1, p.tw4, dir, p.n2, 0, (R)1}, nb * p.n1,
-                               stream);
+                launch_rows<R>(*p.p2, RowsIo<R>{in + b0 * in_pitch, in_pitch, Y, p.n2, p.n1, p.tw4, dir, p.n2, 0, (R)1, p.n2, p.n2,
+                                                   nullptr}, nb * p.n1, stream);
                 note_launch(), k_split_out<R><<<dim3((p.n2 + 255) / 256, (unsigned)nb), 256, 0, stream>>>(
                     Y, out + b0 * out_pitch, out_pitch, p.n1, p.n2, dir, roll, (R)scale);
             }
@@ -1246,9 +1263,9 @@ void FftEngine::rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, 
 template std::shared_ptr<FftPlan<float>> FftEngine::plan<float>(int);
 template std::shared_ptr<FftPlan<double>> FftEngine::plan<double>(int);
 template void FftEngine::rows<float>(const FftPlan<float>&, const cpx<float>*, long long, cpx<float>*, long long,
-                                     long long, int, int, double);
+                                     long long, int, int, double, const RowEnds<float>*);
 template void FftEngine::rows<double>(const FftPlan<double>&, const cpx<double>*, long long, cpx<double>*, long long,
-                                      long long, int, int, double);
+                                      long long, int, int, double, const RowEnds<double>*);
 template FftDesc<float> FftEngine::smem_desc<float>(int);
 template FftDesc<double> FftEngine::smem_desc<double>(int);
 template void transpose_batched<float>(const cpx<float>*, long long, long long, cpx<float>*, long long, long long,

@@ -95,6 +95,15 @@ struct FftPlan {
     ~FftPlan();
 };
 
+// A row transform of which part is given or wanted: inputs from `valid` on are
+// zero and not read, output k is multiplied by mul[k] (null: not) before the
+// roll, rolled outputs from `count` on are not written.
+template <typename R>
+struct RowEnds {
+    int valid, count;
+    const cpx<R>* mul;
+};
+
 // FP64 transforms of P points of which only a band of the spectrum is wanted
 // or given (to_band, from_band), as chirp-z transforms of runs of L points
 // that share one transform of length m on the band's side: nb + 1 of them.
@@ -130,7 +139,11 @@ struct FftEngine {
     // 0 <= roll < n.  in may equal out.  Works for any n >= 1.
     template <typename R>
     void rows(const FftPlan<R>& p, const cpx<R>* in, long long in_pitch, cpx<R>* out,
-              long long out_pitch, long long batch, int dir, int roll = 0, double scale = 1.0);
+              long long out_pitch, long long batch, int dir, int roll = 0, double scale = 1.0,
+              const RowEnds<R>* ends = nullptr);
+    // whether a plan takes RowEnds
+    template <typename R>
+    static bool one_kernel(const FftPlan<R>& p) { return p.kind == FFT_SMEM || p.kind == FFT_BLUE; }
 
     // to_band: out[k] = sum_n in[n] exp(-2 pi i n (k0 + k) / P), k < width, rows
     // of P points; from_band: out[n] = scale sum_k in[k] exp(2 pi i n k / P),
