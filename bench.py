@@ -437,14 +437,14 @@ def main():
         for k, v in per.items():
             alg[k] = alg.get(k, 0) + v
     hbm, peak_kind = peaks()
-    # dominant kernel: the time unfolding (k_tufr_fused, one launch per burst)
-    # of the TOPS chain; for stripmap the slowest stage
+    # dominant stage: the time unfolding (its largest kernel k_tufr_spread, one
+    # launch per burst) of the TOPS chain; for stripmap the slowest stage
     dom = "time_unfold" if tops else max((k for k in alg if k != "total"), key=lambda k: stages.get(k, 0.0))
-    dom_kernel = {"time_unfold": "k_tufr_fused", "row_pass": "k_rowpass_fused", "azimuth_ifft": "k_czt_rows",
-                  "range_compress": "k_rc_fused", "batch_decode": "k_decode_symbols"}[dom]
+    dom_kernel = {"time_unfold": "k_tufr_spread", "row_pass": "k_rowpass_fused", "azimuth_ifft": "k_czt_rows",
+                  "range_compress": "k_rc_fused", "batch_decode": "k_decode_fdbaq"}[dom]
     dom_ms = stages.get(dom, 0.0) / nbursts
     achieved = (alg[dom] / nbursts) / (dom_ms / 1e3) / 1e9 if dom_ms > 0 else 0.0
-    tpu = profiled_value("k_tufr_fused") if tops else None
+    tpu = profiled_value("k_tufr_spread") if tops else None
     traffic = tpu * sum(n_r * S for (_, n_r, S, _) in geo) / nbursts if tpu else None
     roofline = {"bound": "hbm", "kernel": dom_kernel, "achieved": achieved, "peak": hbm, "unit": "GB/s",
                 "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
@@ -452,9 +452,9 @@ def main():
                 "stage_ms_per_burst": {k: v / nbursts for k, v in sorted(stages.items())},
                 "pipeline_alg_bytes_per_step": alg["total"],
                 "pipeline_achieved_gbs": alg["total"] / (dev_ms / args.steps / 1e3) / 1e9,
-                "note": ("instruction-issue and special-function bound: deramp staging (per-interval phase "
-                         "polynomials), type-1 NUFFT gather (~58 samples per grid point, two range bins per "
-                         "weight), forward and inverse ~9k grid FFT per range bin"
+                "note": ("L1 and instruction-issue bound: knots, re-ramp, type-1 NUFFT gather (~53 samples per "
+                         "grid point, four range bins per weight), forward and inverse ~10k grid FFT per range "
+                         "bin; the figures are those of the stage's four kernels"
                          if tops else "shared-memory FFT bound (stripmap range-Doppler chain)")}
 
     # the compute roof: nominal FP32 flops of each stage (FFTs as 5 N log2 N,
@@ -488,7 +488,7 @@ def main():
 
     # the roof this kernel meets: instruction issue (4 warp instructions per
     # SM per clock), at the SM clock sampled during the timed region
-    ipu = profiled_value("k_tufr_fused", "warp_inst_per_unit") if tops else None
+    ipu = profiled_value("k_tufr_spread", "warp_inst_per_unit") if tops else None
     if ipu and dom_ms > 0 and clk.get("sm_mhz"):
         sms = ctypes.c_int()
         rt.cudaDeviceGetAttribute(ctypes.byref(sms), 16, local)
