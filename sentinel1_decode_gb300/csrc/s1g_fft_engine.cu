@@ -1012,8 +1012,8 @@ BandPlan::~BandPlan() {
     for (void* q : owned) cudaFree(q);
 }
 
-// Bands follow the scene's Doppler rate, so their plans are few but not fixed.
-constexpr size_t kBandPlans = 8;
+// Bands follow a burst's Doppler rate: four plans a burst, up to 2 MB each.
+constexpr size_t kBandPlans = 40;
 
 std::shared_ptr<BandPlan> FftEngine::band_plan(int P, int k0, int width, bool inverse) {
     const std::vector<int> key{P, k0, width, (int)inverse};
@@ -1040,7 +1040,8 @@ std::shared_ptr<BandPlan> FftEngine::band_plan(int P, int k0, int width, bool in
         }
     }
     if (p->nb) {
-        p->core = build_plan4<double>((int)m, fft4_order64(m));
+        const auto pm = plan<double>((int)m);   // a length of the core
+        p->core = pm->core;
         auto table = [&](size_t n) {
             void* q = nullptr;
             check_cuda(cudaMalloc(&q, sizeof(cf64) * n), "band table");
@@ -1054,7 +1055,7 @@ std::shared_ptr<BandPlan> FftEngine::band_plan(int P, int k0, int width, bool in
         const int before = inverse ? width : p->L, after = inverse ? p->L : width;
         note_launch(), k_band_tables<<<grid_for(std::max<long long>(P, m * p->nb)), 256, 0, stream>>>(
             P, k0, width, (int)m, p->nb, inverse ? p->L : -p->L, before, after, p->pre, p->chirp, tmp);
-        rows<double>(*plan<double>((int)m), tmp, m, tmp, m, p->nb, -1);
+        rows<double>(*pm, tmp, m, tmp, m, p->nb, -1);
         for (int b = 0; b < p->nb; ++b)
             note_launch(), k_cvt64<double><<<grid_for(m), 256, 0, stream>>>(tmp + b * m, p->H + b * m, m, 1.0 / (double)m,
                                                                             p->core->d.pos);
