@@ -314,28 +314,64 @@ __device__ __forceinline__ double lin_resample_at(const double* arr, int n_in, i
     return y0 + ((x - x0) * (y1 - y0) / (x1 - x0));
 }
 
+// Where linear_resample(arr, n_out)[k] reads: arr[i] + w (arr[i + 1] - arr[i]).
+struct LinAt {
+    int i;
+    double w;
+};
+__device__ __forceinline__ LinAt lin_resample_pos(int n_in, int n_out, int k) {
+    if (n_in == n_out) return {k < n_in - 1 ? k : n_in - 2, k < n_in - 1 ? 0.0 : 1.0};
+    if (k == n_out - 1) return {n_in - 2, 1.0};
+    const double dx_in = 1.0 / (n_in - 1);
+    const double x = k * (1.0 / (n_out - 1));
+    int i = (int)(x / dx_in);
+    if (i > n_in - 2) i = n_in - 2;
+    if (i < n_in - 2 && (i + 1 + 1) * dx_in <= x) ++i;
+    if (i > 0 && (i + 1) * dx_in <= x) ++i;
+    while (i > 0 && x < i * dx_in) --i;
+    const double x0 = i * dx_in, x1 = (i + 1) * dx_in;
+    return {i, (x - x0) / (x1 - x0)};
+}
+
+// Deramped tiled line of every range bin.  FP64 arithmetic bounds it: two
+// divisions and a sine / cosine per sample; a thread takes one sample of
+// kDerampBins bins, whose place between the knots is the same.  3002 bins of
+// 29922 samples: 9.9 ms (15.0 with the place per sample).
+constexpr int kDerampBins = 32;
 template <typename R>
-__global__ void k_tufr_deramp(const cpx<R>* a, long long ap, int S, cpx<R>* y, long long yp, const double* kaT,
-                              long long kp, const double* f_dc, int n_r, double dc_rate, int num_tiles, double ft) {
+__global__ void __launch_bounds__(256) k_tufr_deramp(const cpx<R>* a, long long ap, int S, cpx<R>* y, long long yp,
+                                                     const double* kaT, long long kp, const double* f_dc, int n_r,
+                                                     double dc_rate, int num_tiles, double ft) {
     const int shape = num_tiles * S;
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= shape) return;
     const double start = -ft / 2, end = ft / 2;
     const double step = (end - start) / (shape - 1);
-    GRID_STRIDE(i, (long long)n_r * shape) {
-        const int j = (int)(i / shape), k = (int)(i % shape);
-        const double ka = lin_resample_at(kaT + (long long)j * kp, S, shape, k);
+    const double tau = start + k * step;
+    const LinAt at = lin_resample_pos(S, shape, k);
+    const int src = k % S;
+    const int j1 = min(n_r, ((int)blockIdx.y + 1) * kDerampBins);
+    for (int j = blockIdx.y * kDerampBins; j < j1; ++j) {
+        const double* arr = kaT + (long long)j * kp;
+        const double y0 = arr[at.i], y1 = arr[at.i + 1];
+        const double ka = at.w == 1.0 ? y1 : y0 + at.w * (y1 - y0);
         const double kt = -ka * dc_rate / (dc_rate - ka);
         const double dct = -f_dc[j] / ka;
-        const double t = dct + (start + k * step);
+        const double t = dct + tau;
         const double th1 = ((-kPI) * kt) * (t * t);
         const double th2 = (((2.0 * kPI) * (kt + ka)) * dct) * t;
-        y[(long long)j * yp + k] = a[(long long)j * ap + (k % S)] * expi<R>(th1 + th2);
+        y[(long long)j * yp + k] = a[(long long)j * ap + src] * expi<R>(th1 + th2);
     }
 }
 template <typename R>
 void tufr_deramp(const cpx<R>* a, long long ap, int S, cpx<R>* y, long long yp, const double* kaT, long long kp,
                  const double* f_dc, int n_r, double dc_rate, int num_tiles, double ft, cudaStream_t st) {
-    note_launch(), k_tufr_deramp<R><<<grid1((long long)n_r * num_tiles * S), 256, 0, st>>>(a, ap, S, y, yp, kaT, kp, f_dc, n_r,
-                                                                            dc_rate, num_tiles, ft);
+    // bins beyond one grid's second dimension in further launches
+    const int shape = num_tiles * S, most = 65535 * kDerampBins;
+    for (int j = 0; j < n_r; j += most)
+        note_launch(), k_tufr_deramp<R><<<dim3((shape + 255) / 256, (std::min(n_r - j, most) + kDerampBins - 1) / kDerampBins), 256,
+                                          0, st>>>(a + j * ap, ap, S, y + j * yp, yp, kaT + j * kp, kp, f_dc + j, n_r - j,
+                                                   dc_rate, num_tiles, ft);
 }
 
 // quadratic_resample (signal_processing.cpp:109-155) + re-ramp
