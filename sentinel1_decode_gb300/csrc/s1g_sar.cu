@@ -3,6 +3,7 @@
 // azimuth filter, ECCM).  Arithmetic follows the reference function named
 // at each kernel; phases are generated in FP64 and wrapped before the
 // complex exponential, so the FP32 instantiations only round the result.
+#include <algorithm>
 #include <cmath>
 #include <stdexcept>
 
