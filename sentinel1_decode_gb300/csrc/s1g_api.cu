@@ -132,9 +132,10 @@ struct s1g_decoder {
     std::map<int, std::shared_ptr<s1g::DcFftPlan>> dc_plans;   // Doppler-estimator blocks by length
     std::map<std::string, std::shared_ptr<struct BatchDecode>> batch_decodes;   // by swath/level
     // every burst of a swath decoded in one launch pair for the per-burst
-    // FP32 calls (built on the first such call, dropped when the stream
-    // content or the A/B/C decode mode changes)
+    // FP32 calls (built on the first such call, decoded again after every load,
+    // dropped when the packet layout or the A/B/C decode mode changes)
     std::map<std::string, std::shared_ptr<struct SwathDecode>> swath_decodes;
+    uint64_t loads = 0;           // streams loaded so far: which one decoded samples are of
     double last_ms = 0;
     // Status words of a product call, read back with its one synchronisation:
     // [0] corner-turn flag, [1] time unfolding, [2..] decode status per packet
@@ -304,8 +305,10 @@ static void upload_staged(uint8_t* dst, const uint8_t* src, size_t n, cudaStream
 // s1_decoder.cpp:13-34), build the state vectors.  Plans derived from the
 // content (per-burst tables, batch decode jobs, the captured batch graph)
 // are kept only when the new stream's headers and packet layout hash to the
-// same value as the previous stream's and no buffer moved.
+// same value as the previous stream's and no buffer moved.  Decoded samples
+// are of one load: the hash says nothing about the user data.
 static void ingest(s1g_decoder* h, const uint8_t* bytes, size_t n, bool staged) {
+    ++h->loads;
     const size_t need = std::max<size_t>(n, 1) + 64;
     bool moved = false;
     if (!h->d_stream || need > h->stream_cap) {
@@ -2708,13 +2711,15 @@ struct BatchRun {
     int* tstat = nullptr;
 };
 
-// Per-burst FP32 calls decode the whole swath once: one thread per packet
-// walks its bitstream, so a single burst (~1500 packets) occupies few SMs
-// and waits on the walk's latency, while a swath's packets fill the GPU.
+// Per-burst FP32 calls decode the whole swath once a load: one warp per packet
+// walks its bitstream, so a single burst (~1500 packets) leaves most of the
+// GPU's warp slots empty and waits on the walk's latency, while a swath's
+// packets fill it.
 // A burst whose packets failed to decode is not served from the cache (its
 // own decode reports the error as usual).
 struct SwathDecode {
     std::shared_ptr<BatchDecode> plan;
+    uint64_t load = 0;                        // s1g_decoder::loads the samples are of (0: none yet)
     Buf raw;
     std::vector<int> status;                  // per job
     std::map<int, size_t> burst_of_first;     // first packet index -> burst
@@ -2730,36 +2735,39 @@ static const cf32* swath_cached_decode(s1g_decoder* h, const std::vector<int>& p
     if (bit == h->bursts.end() || bit->second.size() < 2) return nullptr;
     auto& slot = h->swath_decodes[sw];
     if (!slot) {
-        auto sd = std::make_shared<SwathDecode>();
+        auto made = std::make_shared<SwathDecode>();
         std::vector<const std::vector<int>*> lists;
         size_t j = 0;
         for (size_t k = 0; k < bit->second.size(); ++k) {
             lists.push_back(&bit->second[k]);
-            sd->burst_of_first[bit->second[k].front()] = k;
-            sd->job0.push_back(j);
+            made->burst_of_first[bit->second[k].front()] = k;
+            made->job0.push_back(j);
             j += bit->second[k].size();
         }
         try {
-            sd->plan = batch_decode_plan(h, lists);
+            made->plan = batch_decode_plan(h, lists);
         } catch (const S1Error&) {
             return nullptr;   // a format the decoder rejects: leave it to the burst's own decode
         }
-        cf32* raw = sd->raw.as<cf32>((size_t)std::max<long long>(sd->plan->raw_elems, 1));
-        int* st = h->bDecStatus.as<int>((size_t)std::max(sd->plan->njobs, 1));
-        if (sd->plan->any_d)
-            decode_jobs(h->d_stream, h->nbytes, h->d_off, sd->plan->d_jobs, sd->plan->njobs, sd->plan->nq_max, raw,
+        slot = made;
+    }
+    SwathDecode& sd = *slot;
+    if (sd.load != h->loads) {
+        cf32* raw = sd.raw.as<cf32>((size_t)std::max<long long>(sd.plan->raw_elems, 1));
+        int* st = h->bDecStatus.as<int>((size_t)std::max(sd.plan->njobs, 1));
+        if (sd.plan->any_d)
+            decode_jobs(h->d_stream, h->nbytes, h->d_off, sd.plan->d_jobs, sd.plan->njobs, sd.plan->nq_max, raw,
                         nullptr, st, h->tabs, h->stream);
-        if (sd->plan->any_fixed)
-            decode_fixed_jobs<float>(h->d_stream, h->nbytes, h->d_off, sd->plan->d_jobs, sd->plan->njobs, raw, st,
+        if (sd.plan->any_fixed)
+            decode_fixed_jobs<float>(h->d_stream, h->nbytes, h->d_off, sd.plan->d_jobs, sd.plan->njobs, raw, st,
                                      h->abc_fields, h->stream);
-        sd->status.resize(sd->plan->njobs);
-        check_cuda(cudaMemcpyAsync(sd->status.data(), st, sizeof(int) * sd->status.size(), cudaMemcpyDeviceToHost,
+        sd.status.resize(sd.plan->njobs);
+        check_cuda(cudaMemcpyAsync(sd.status.data(), st, sizeof(int) * sd.status.size(), cudaMemcpyDeviceToHost,
                                    h->stream),
                    "swath decode status");
         check_cuda(cudaStreamSynchronize(h->stream), "swath decode");
-        slot = sd;
+        sd.load = h->loads;
     }
-    const SwathDecode& sd = *slot;
     auto it = sd.burst_of_first.find(pk.front());
     if (it == sd.burst_of_first.end()) return nullptr;
     const size_t k = it->second;
