@@ -7,6 +7,7 @@
 // the reference's _range_compress / _azimuth_compress (s1_decoder.cpp:448-701)
 // as GPU kernels on the handle's stream.
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstring>
@@ -37,12 +38,18 @@ struct S1Error : std::runtime_error {
     S1Error(int c, const std::string& m) : std::runtime_error(m), code(c) {}
 };
 
+// A work buffer that grows.  moves: the owner's count of buffers given up for
+// larger ones (their addresses may be in a captured batch), or null.
 struct Buf {
+    uint64_t* moves = nullptr;
     void* p = nullptr;
     size_t n = 0;
     void* get(size_t bytes) {
         if (bytes > n) {
-            if (p) cudaFree(p);
+            if (p) {
+                cudaFree(p);
+                if (moves) ++*moves;
+            }
             p = nullptr;
             n = 0;
             check_cuda(cudaMalloc(&p, bytes), "work buffer cudaMalloc");
@@ -88,6 +95,12 @@ using namespace s1g;
 
 struct s1g_decoder {
     int device = 0;
+    const uint64_t id = new_id();   // of this handle alone, as its address is not
+    uint64_t moves = 0;             // device buffers of this handle given up so far (Buf)
+    static uint64_t new_id() {
+        static std::atomic<uint64_t> n{0};
+        return ++n;
+    }
     cudaStream_t stream = nullptr;
     std::unique_ptr<FftEngine> fft;
     uint8_t* d_stream = nullptr;
@@ -112,18 +125,24 @@ struct s1g_decoder {
     std::string err;
     IndexScratch isc;
     DecodeTables tabs;
-    Buf bA, bB, bC, bD, bE, bKa, bOut, bStage, bSmall, bRows, bCols, bStatus, bFlags, bRef, bTab, bPk;
+    Buf bA{&moves}, bB{&moves}, bC{&moves}, bD{&moves}, bE{&moves}, bKa{&moves}, bOut{&moves}, bStage{&moves},
+        bSmall{&moves}, bRows{&moves}, bCols{&moves}, bStatus{&moves}, bFlags{&moves}, bRef{&moves}, bTab{&moves},
+        bPk{&moves};
     RangeRef ref32, ref64;
-    Buf bBand, bFdf, bFit, bTd, bTstat, bDc, bDcPart, bRawAll, bDecStatus, bBatchStatus;
-    Buf bSrc, bSrcLo;                         // SRC table of the direct row pass
-    Buf bTuD, bTuG, bTuI, bTuW, bTuR, bTuWt, bTuRamp, bKa0;   // time-unfolding per-burst tables and grids
-    Buf bImgIn, bImgOut, bImgMax;        // image epilogue
-    Buf bJ0, bJ1, bJ2, bJ3, bJ4, bJ5, bJe, bJd;   // differentiable azimuth chains
-    Buf bRawW;                               // decoded rows after the FP64 ECCM notch (FP32 paths)
-    Buf bEccm, bEccmSt;                      // FP64 decode of the ECCM notch
-    Buf bEccmRoots;                          // FP64 roots of unity of the ECCM detection
-    Buf bRawAll64;                           // FP64 samples of a batch decode (ECCM)
-    Buf bEccmMask;                           // s1g_eccm_mask output staging
+    Buf bBand{&moves}, bFdf{&moves}, bFit{&moves}, bTd{&moves}, bTstat{&moves}, bDc{&moves}, bDcPart{&moves},
+        bRawAll{&moves}, bDecStatus{&moves}, bBatchStatus{&moves};
+    Buf bSrc{&moves}, bSrcLo{&moves};   // SRC table of the direct row pass
+    // time-unfolding per-burst tables and grids
+    Buf bTuD{&moves}, bTuG{&moves}, bTuI{&moves}, bTuW{&moves}, bTuR{&moves}, bTuWt{&moves}, bTuRamp{&moves},
+        bKa0{&moves};
+    Buf bImgIn{&moves}, bImgOut{&moves}, bImgMax{&moves};   // image epilogue
+    // differentiable azimuth chains
+    Buf bJ0{&moves}, bJ1{&moves}, bJ2{&moves}, bJ3{&moves}, bJ4{&moves}, bJ5{&moves}, bJe{&moves}, bJd{&moves};
+    Buf bRawW{&moves};   // decoded rows after the FP64 ECCM notch (FP32 paths)
+    Buf bEccm{&moves}, bEccmSt{&moves};   // FP64 decode of the ECCM notch
+    Buf bEccmRoots{&moves};   // FP64 roots of unity of the ECCM detection
+    Buf bRawAll64{&moves};   // FP64 samples of a batch decode (ECCM)
+    Buf bEccmMask{&moves};   // s1g_eccm_mask output staging
     // fast-path caches: per-burst tables (keyed by first packet index) and
     // chirp-z transform tables (keyed by period, nin, nout)
     std::map<int, std::shared_ptr<struct FastBurst>> fast_bursts;
@@ -312,7 +331,7 @@ static void ingest(s1g_decoder* h, const uint8_t* bytes, size_t n, bool staged) 
     const size_t need = std::max<size_t>(n, 1) + 64;
     bool moved = false;
     if (!h->d_stream || need > h->stream_cap) {
-        if (h->d_stream) cudaFree(h->d_stream);
+        if (h->d_stream) cudaFree(h->d_stream), ++h->moves;
         h->d_stream = nullptr;
         h->stream_cap = 0;
         check_cuda(cudaMalloc(&h->d_stream, need), "stream alloc");
@@ -330,7 +349,7 @@ static void ingest(s1g_decoder* h, const uint8_t* bytes, size_t n, bool staged) 
     // upper bound on packets: every packet is at least 7 bytes
     const int maxp = (int)std::min<long long>(h->nbytes / 7 + 1, 1LL << 30);
     if (!h->d_off || maxp > h->off_cap) {
-        if (h->d_off) cudaFree(h->d_off);
+        if (h->d_off) cudaFree(h->d_off), ++h->moves;
         h->d_off = nullptr;
         h->off_cap = 0;
         check_cuda(cudaMalloc(&h->d_off, sizeof(long long) * (size_t)maxp), "offsets");
@@ -2850,7 +2869,7 @@ static void enqueue_batch(s1g_decoder** hs, int n_streams, const char* swath, in
     size_t slot = 0;
     for (int s = 0; s < n_streams; ++s)
         for (size_t k = 0; k < lists[s].size(); ++k) slot_of[s].push_back(slot++);
-    for (size_t i = h0->batch_bufs.size(); i < nslots; ++i) h0->batch_bufs.emplace_back(new Buf());
+    for (size_t i = h0->batch_bufs.size(); i < nslots; ++i) h0->batch_bufs.emplace_back(new Buf{&h0->moves});
     h0->batch_out.assign(nslots, Result());
     size_t kmax = 0;
     for (int s = 0; s < n_streams; ++s) kmax = std::max(kmax, lists[s].size());
@@ -2937,7 +2956,9 @@ static void check_batch(const BatchRun& br, int n_streams) {
 
 // A batch captured into a CUDA graph (second call with the same handles,
 // swath, level and settings; the first call runs eagerly and leaves every
-// buffer and table at its final size).
+// buffer and table at its final size).  It holds the addresses of the handles'
+// buffers, so its key also counts the buffers they gave up: another swath or a
+// per-burst call that needs larger ones has the batch run and captured anew.
 struct BatchGraph {
     std::string key;
     cudaGraphExec_t exec = nullptr;
@@ -2953,9 +2974,9 @@ static std::string batch_key(s1g_decoder** hs, int n, const char* swath, int lev
     std::ostringstream o;
     o << swath << "/" << level;
     for (int s = 0; s < n; ++s)
-        o << "/" << (const void*)hs[s] << ":" << hs[s]->precision << ":" << hs[s]->use_eccm << ":" << hs[s]->det << ":"
-          << hs[s]->mit << ":" << hs[s]->abc_fields << ":" << hs[s]->epoch << ":" << hs[s]->rcmc << ":"
-          << hs[s]->rcmc_L;
+        o << "/" << hs[s]->id << ":" << hs[s]->moves << ":" << hs[s]->fft->moves << ":" << hs[s]->precision << ":"
+          << hs[s]->use_eccm << ":" << hs[s]->det << ":" << hs[s]->mit << ":" << hs[s]->abc_fields << ":"
+          << hs[s]->epoch << ":" << hs[s]->rcmc << ":" << hs[s]->rcmc_L;
     for (int s = 0; s < n; ++s) {
         o << "/sel" << s << (hs[s]->batch_sel_on ? ":" : "-");
         for (int b : hs[s]->batch_sel) o << b << ",";
@@ -3029,7 +3050,8 @@ int s1g_process_swath_batch(s1g_decoder** hs, int n_streams, const char* swath, 
             enqueue_batch(hs, n_streams, swath, level, eager);
             check_cuda(cudaEventRecord(b1, h0->stream), "b1");
             run = &eager;
-            if (graph) h0->graph_warm = key;
+            // the key of the buffers as the call leaves them
+            if (graph) h0->graph_warm = batch_key(hs, n_streams, swath, level);
         }
         check_cuda(cudaEventSynchronize(b1), "batch end");
         float ms = 0;

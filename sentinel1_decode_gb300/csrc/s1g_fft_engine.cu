@@ -159,6 +159,7 @@ void* DeviceArena::get(size_t bytes) {
         if (ptr) {
             cudaDeviceSynchronize();
             cudaFree(ptr);
+            if (moves) ++*moves;
         }
         ptr = nullptr;
         size = 0;

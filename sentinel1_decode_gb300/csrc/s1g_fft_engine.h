@@ -22,6 +22,7 @@
 // core).
 #pragma once
 
+#include <cstdint>
 #include <map>
 #include <memory>
 #include <string>
@@ -52,7 +53,9 @@ template <typename R>
 inline int fft4_capacity() { return (kFft4SmemBytes / (int)sizeof(cpx<R>) - 1) * 16 / 17; }
 
 // Device memory arena owned by a processing context: grow-only scratch.
+// moves: the owner's count of arenas given up for larger ones.
 struct DeviceArena {
+    uint64_t* moves = nullptr;
     void* ptr = nullptr;
     size_t size = 0;
     ~DeviceArena();
@@ -129,7 +132,8 @@ struct FftEngine {
     std::map<std::vector<int>, std::shared_ptr<BandPlan>> bands;   // at most kBandPlans
     std::map<int, std::shared_ptr<FftDescTables>> descs32, descs64;   // smem_desc
     std::map<int, std::shared_ptr<Fft4Plan>> plans4;
-    DeviceArena scratch_a, scratch_b, scratch_c, scratch_band;
+    uint64_t moves = 0;
+    DeviceArena scratch_a{&moves}, scratch_b{&moves}, scratch_c{&moves}, scratch_band{&moves};
 
     template <typename R>
     std::shared_ptr<FftPlan<R>> plan(int n);

@@ -90,3 +90,97 @@ def test_reload_of_the_same_layout_gives_its_own_samples(lib_path):
     assert not np.array_equal(got, before)
     d.close()
     fresh.close()
+
+
+GROWTH = """
+data = stream(*bursts((1000, 24), (1003, 24)), *bursts((1000, 40), (1001, 44), swath="IW3"))
+d = S1Decoder(data)
+for _ in range(3):                                      # eager, capture, replay
+    process_swath_batch([d], "IW2")
+assert (count("capture"), count("replay")) == (1, 2)
+"""
+
+
+@pytest.mark.parametrize("grow", [
+    'process_swath_batch([d], "IW3")',                                     # longer lines, same handle
+    'd.get_range_compressed_burst("IW3", 1)',                              # a per-burst call
+    'd.set_precision("fp64"); d.get_range_compressed_burst("IW3", 1); d.set_precision("fp32")',
+])
+def test_no_replay_over_buffers_that_moved(fake, grow):
+    """A captured batch holds the addresses of the handle's buffers: once one of
+    them has been replaced by a larger one, the batch is run and captured anew."""
+    fake(GROWTH + grow + """
+captured, replayed = count("capture"), count("replay")
+process_swath_batch([d], "IW2")
+assert (count("capture"), count("replay")) == (captured, replayed)      # eager
+process_swath_batch([d], "IW2")
+process_swath_batch([d], "IW2")
+assert (count("capture"), count("replay")) == (captured + 1, replayed + 2)
+""")
+
+
+def test_no_replay_for_another_handle_at_the_same_address(fake):
+    """The key of a captured batch tells handles apart by more than their address."""
+    fake("""
+data = stream(*bursts((1000, 24)))
+a = S1Decoder(data)
+for _ in range(40):
+    b = S1Decoder(data)
+    for _ in range(2):
+        process_swath_batch([a, b], "IW2")
+    at = b.handle.value
+    b.close()
+    c = S1Decoder(data)
+    if c.handle.value == at:
+        break
+    c.close()
+else:
+    sys.exit("no handle at the same address")
+captured, replayed = count("capture"), count("replay")
+process_swath_batch([a, c], "IW2")
+assert (count("capture"), count("replay")) == (captured, replayed)
+""")
+
+
+def test_replay_goes_on_while_nothing_moves(fake):
+    """Smaller products in between and reloads of the same bytes cost no capture."""
+    fake("""
+data = stream(*bursts((1000, 24), (1003, 24)))
+d = S1Decoder(data)
+for _ in range(2):
+    process_swath_batch([d], "IW2")
+d.get_range_compressed_burst("IW2", 0)
+d.get_burst("IW2", 0)
+d.reload(data)
+for _ in range(3):
+    process_swath_batch([d], "IW2")
+assert (count("capture"), count("replay")) == (1, 4), (count("capture"), count("replay"))
+""")
+
+
+@pytest.mark.gpu
+def test_batch_after_growth_equals_a_fresh_handle(lib_path):
+    """Batches of two swaths in turn, the second of longer lines, and per-burst
+    products in between: every SLC is a fresh handle's."""
+    import numpy as np
+    from sentinel1_decode_gb300 import S1Decoder, batch_outputs, process_swath_batch, synth
+    from test_batch import fetch
+    spec = [synth.BurstSpec(num_lines=n, num_quads=q, swath=sw, num_targets=2, gap_lines=200)
+            for sw, n, q in (("IW2", 1000, 96), ("IW2", 1003, 96), ("IW3", 1010, 130), ("IW3", 1031, 136))]
+    data = synth.generate(synth.StreamSpec(spec, seed=4))
+    want = {}
+    for sw in ("IW2", "IW3"):
+        f = S1Decoder(data, precision="fp32")
+        want[sw] = [f.get_azimuth_compressed_burst(sw, b, dtype=np.complex64) for b in range(2)]
+        f.close()
+    d = S1Decoder(data, precision="fp32")
+    for sw in ("IW2", "IW2", "IW2", "IW3", "IW2", "IW2", "product", "IW2", "IW3", "IW3", "IW2", "IW2"):
+        if sw == "product":
+            d.set_precision("fp64")
+            d.get_range_compressed_burst("IW3", 1)
+            d.set_precision("fp32")
+            continue
+        process_swath_batch([d], sw)
+        for got, ref in zip([fetch(*o) for o in batch_outputs(d)], want[sw]):
+            np.testing.assert_array_equal(got, ref)
+    d.close()
