@@ -16,6 +16,18 @@ void check_cuda(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw std::runtime_error(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+int device_sms() {
+    static std::atomic<int> known[64];
+    int dev = 0, n = 0;
+    check_cuda(cudaGetDevice(&dev), "device");
+    if (dev < 64) n = known[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        check_cuda(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "device");
+        if (dev < 64) known[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
 static std::atomic<long long> g_launches{0};
 void note_launch() { g_launches.fetch_add(1, std::memory_order_relaxed); }
 long long launch_count() { return g_launches.load(); }
@@ -1068,14 +1080,6 @@ std::shared_ptr<BandPlan> FftEngine::band_plan(int P, int k0, int width, bool in
 
 static void launch_band(FftEngine& e, const BandPlan& p, BandArgs a) {
     if (a.rows <= 0) return;
-    static int sms[64] = {};
-    int dev = 0;
-    check_cuda(cudaGetDevice(&dev), "band");
-    int n = dev < 64 ? sms[dev] : 0;
-    if (!n) {
-        check_cuda(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev), "band");
-        if (dev < 64) sms[dev] = n;
-    }
     a.d = p.core->d;
     a.P = p.P;
     a.width = p.width;
@@ -1087,7 +1091,7 @@ static void launch_band(FftEngine& e, const BandPlan& p, BandArgs a) {
     const size_t smem = sizeof(cf64) * (size_t)padded16_len(a.d.n);
     rows4_launch<double>(smem, [&](auto nt, auto mb) {
         constexpr int NT = decltype(nt)::value, MB = decltype(mb)::value;
-        const int grid = (int)std::min<long long>(a.rows, (long long)n * MB);
+        const int grid = (int)std::min<long long>(a.rows, (long long)device_sms() * MB);
         a.W = (cf64*)e.scratch_band.get(sizeof(cf64) * (size_t)grid * a.d.n);
         auto kernel = p.inverse ? k_from_band<NT, MB> : k_to_band<NT, MB>;
         check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFft4SmemBytes), "attr");

@@ -195,6 +195,14 @@ void transpose_batched(const cpx<R>* in, long long in_row_pitch, long long in_ba
                        cudaStream_t s);
 
 void check_cuda(cudaError_t e, const char* what);
+// Multiprocessors of the current device.
+int device_sms();
+// Allow a kernel `bytes` of dynamic shared memory.  The limit belongs to the
+// current device, so it is set at every launch, not once a process.
+template <class K>
+inline void allow_dynamic_smem(K kernel, int bytes) {
+    check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "attr");
+}
 
 // Count of kernels this library has launched (reported by the benchmark).
 void note_launch();

@@ -186,22 +186,10 @@ bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int ro
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
         return false;
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms <= 0) sms = 1;
-    }
     const long long tiles = (long long)((cols + kTileCols - 1) / kTileCols) * ((rows + kTileRows - 1) / kTileRows);
-    const int grid = (int)std::min<long long>(tiles, 4LL * sms);
+    const int grid = (int)std::min<long long>(tiles, 4LL * device_sms());
     const size_t smem = 2 * kTileBytes + 1024;
-    static bool attr = false;
-    if (!attr) {
-        check_cuda(cudaFuncSetAttribute(k_transpose_tma, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem),
-                   "tma transpose attr");
-        attr = true;
-    }
+    allow_dynamic_smem(k_transpose_tma, (int)smem);
     note_launch(), k_transpose_tma<<<grid, 256, smem, st>>>(map, out, op, rows, cols);
     return true;
 }

@@ -184,3 +184,21 @@ def test_batch_after_growth_equals_a_fresh_handle(lib_path):
         for got, ref in zip([fetch(*o) for o in batch_outputs(d)], want[sw]):
             np.testing.assert_array_equal(got, ref)
     d.close()
+
+
+def test_kernels_get_their_shared_memory_on_every_device(fake):
+    """The limit of dynamic shared memory belongs to a kernel and a device: one
+    process with handles on two of them."""
+    fake("""
+data = stream(*bursts((300, 1000)))
+for device in (0, 1):
+    for precision in ("fp32", "fp32_plain", "fp64"):
+        d = S1Decoder(data, device=device, precision=precision)
+        d.apply_eccm(1000, 10)
+        if precision == "fp32":
+            d.get_azimuth_compressed_burst("IW2", 0, dtype=np.complex64)
+        d.get_range_compressed_burst("IW2", 0, range_doppler=True, dtype=np.complex64)
+        d.close()
+    assert count("refused") == 0, device
+assert count("launch:k_rc_dc") and count("launch:k_transpose_tma") and count("launch:k_eccm_notch")
+""")
