@@ -241,8 +241,8 @@ static void init_log_tables() {
         t[i].x = (float)l;
         t[i].y = (float)(l - (double)t[i].x);
     }
-    check_cuda(cudaMemcpyToSymbol(c_log_c, c, sizeof(c)), "log tables");
-    check_cuda(cudaMemcpyToSymbol(c_log_t, t, sizeof(t)), "log tables");
+    upload_symbol(c_log_c, c, sizeof(c), "log tables");
+    upload_symbol(c_log_t, t, sizeof(t), "log tables");
     if (dev < 64) done[dev] = true;
 }
 

@@ -418,7 +418,7 @@ static void open_stream(s1g_decoder* h, const uint8_t* bytes, size_t n, bool sta
     check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
     check_cuda(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
     h->fft.reset(new FftEngine(h->stream));
-    h->tabs.init();
+    h->tabs.init(h->stream);
     ingest(h, bytes, n, staged);
 }
 
@@ -559,8 +559,7 @@ struct Pipe {
             std::unique_ptr<Buf>& b = h->burst_idx[pk];
             if (!b) {
                 b = std::make_unique<Buf>();
-                check_cuda(cudaMemcpy(b->as<int>(pk.size()), pk.data(), sizeof(int) * pk.size(), cudaMemcpyHostToDevice),
-                           "burst index upload");
+                upload_table(b->as<int>(pk.size()), pk.data(), sizeof(int) * pk.size(), st, "burst index upload");
             }
             d_idx = (const int*)b->p;
         }
@@ -589,7 +588,7 @@ struct Pipe {
         int* flags = h->bFlags.as<int>(n_a);
         eccm_detect_mixed(B, n_r, n_r, n_a, (double)h->det, a64, n_r, h->bEccmRoots.as<cf64>(n_r), flags, st);
         auto& cp = h->cffts[128];
-        if (!cp) cp = make_cfft_plan(128);
+        if (!cp) cp = make_cfft_plan(128, st);
         eccm_notch_cc(a64, n_r, out, n_r, n_r, n_a, flags, (double)h->mit, cp->d, st);
     }
 
@@ -1274,8 +1273,8 @@ static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     check_cuda(cudaMalloc(&db, sizeof(cpx<double>) * m), "czt tmp");
     check_cuda(cudaMalloc(&dk, sizeof(cf32) * m), "czt kern");
     t->owned = {dw, dk};
-    check_cuda(cudaMemcpy(dw, w.data(), sizeof(cf32) * nw, cudaMemcpyHostToDevice), "czt up");
-    check_cuda(cudaMemcpy(db, b.data(), sizeof(cpx<double>) * m, cudaMemcpyHostToDevice), "czt up");
+    upload_table(dw, w.data(), sizeof(cf32) * nw, h->stream, "czt up");
+    upload_table(db, b.data(), sizeof(cpx<double>) * m, h->stream, "czt up");
     auto p64 = h->fft->plan<double>(m);
     h->fft->rows<double>(*p64, (cpx<double>*)db, m, (cpx<double>*)db, m, 1, -1);
     check_cuda(cudaStreamSynchronize(h->stream), "czt fft");
@@ -1284,7 +1283,7 @@ static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     cudaFree(db);
     std::vector<cf32> K(m);
     for (int q = 0; q < m; ++q) K[plan->mid[q]] = mk((float)(B[q].x / m), (float)(B[q].y / m));
-    check_cuda(cudaMemcpy(dk, K.data(), sizeof(cf32) * m, cudaMemcpyHostToDevice), "czt up");
+    upload_table(dk, K.data(), sizeof(cf32) * m, h->stream, "czt up");
     t->dev.chirp = (const cf32*)dw;
     t->dev.kern = (const cf32*)dk;
     h->czts[key] = t;
@@ -1434,7 +1433,7 @@ struct FastPipe {
             if (!choose_dc_block(n_r, g.L, fb->dcB, fb->dcU, fb->dcNb))
                 throw S1Error(S1G_E_GEOMETRY, "chirp too long for the Doppler estimator");
             auto& cp = h->dc_plans[fb->dcB];
-            if (!cp) cp = make_dc_plan(fb->dcB);
+            if (!cp) cp = make_dc_plan(fb->dcB, st);
             fb->dcDesc = cp->d;
             {
                 const int B = fb->dcB;
@@ -2214,10 +2213,12 @@ int s1g_packet_samples(s1g_decoder* h, int64_t packet, void* out, int64_t n, int
         src = line32.data();
         bytes = sizeof(cf32) * g.n_r;
     }
-    if (out_on_device)
-        check_cuda(cudaMemcpy(out, src, bytes, cudaMemcpyHostToDevice), "samples up");
-    else
+    if (out_on_device) {
+        upload_table(out, src, bytes, h->stream, "samples up");
+        check_cuda(cudaStreamSynchronize(h->stream), "samples up");
+    } else {
         std::memcpy(out, src, bytes);
+    }
     API_END(h)
 }
 
@@ -2716,8 +2717,7 @@ static std::shared_ptr<BatchDecode> batch_decode_plan(s1g_decoder* h, const std:
     bd->raw_elems = out;
     bd->njobs = (int)jobs.size();
     check_cuda(cudaMalloc(&bd->d_jobs, sizeof(DecodeJob) * std::max<size_t>(jobs.size(), 1)), "decode jobs");
-    check_cuda(cudaMemcpy(bd->d_jobs, jobs.data(), sizeof(DecodeJob) * jobs.size(), cudaMemcpyHostToDevice),
-               "decode jobs up");
+    upload_table(bd->d_jobs, jobs.data(), sizeof(DecodeJob) * jobs.size(), h->stream, "decode jobs up");
     return bd;
 }
 

@@ -214,7 +214,7 @@ CfftPlan::~CfftPlan() {
     for (void* p : owned) cudaFree(p);
 }
 
-std::shared_ptr<CfftPlan> make_cfft_plan(int n) {
+std::shared_ptr<CfftPlan> make_cfft_plan(int n, cudaStream_t st) {
     auto p = std::make_shared<CfftPlan>();
     p->d.n = n;
     std::vector<float4> tw(n);
@@ -226,7 +226,7 @@ std::shared_ptr<CfftPlan> make_cfft_plan(int n) {
     void* dt = nullptr;
     check_cuda(cudaMalloc(&dt, sizeof(float4) * n), "cfft tw");
     p->owned.push_back(dt);
-    check_cuda(cudaMemcpy(dt, tw.data(), sizeof(float4) * n, cudaMemcpyHostToDevice), "cfft tw up");
+    upload_table(dt, tw.data(), sizeof(float4) * n, st, "cfft tw up");
     p->d.tw = (const float4*)dt;
     return p;
 }
@@ -281,7 +281,7 @@ DcFftPlan::~DcFftPlan() {
     for (void* p : owned) cudaFree(p);
 }
 
-std::shared_ptr<DcFftPlan> make_dc_plan(int n) {
+std::shared_ptr<DcFftPlan> make_dc_plan(int n, cudaStream_t st) {
     auto plan = std::make_shared<DcFftPlan>();
     DcFft& d = plan->d;
     d = dc_passes(n);
@@ -299,7 +299,7 @@ std::shared_ptr<DcFftPlan> make_dc_plan(int n) {
         void* v = nullptr;
         check_cuda(cudaMalloc(&v, sizeof(float4) * tw.size()), "dc twiddles");
         plan->owned.push_back(v);
-        check_cuda(cudaMemcpy(v, tw.data(), sizeof(float4) * tw.size(), cudaMemcpyHostToDevice), "dc twiddles up");
+        upload_table(v, tw.data(), sizeof(float4) * tw.size(), st, "dc twiddles up");
         d.tw[p] = (const float4*)v;
         span = Ns;
     }

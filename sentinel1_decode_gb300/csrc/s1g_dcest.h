@@ -46,8 +46,8 @@ struct DcEstArgs {
 };
 
 // Twiddles of n points.
-std::shared_ptr<CfftPlan> make_cfft_plan(int n);
-std::shared_ptr<DcFftPlan> make_dc_plan(int n);
+std::shared_ptr<CfftPlan> make_cfft_plan(int n, cudaStream_t st);
+std::shared_ptr<DcFftPlan> make_dc_plan(int n, cudaStream_t st);
 // Overlap-save block B = 2^a 3^b (B >= L + 32, fits shared memory) of least
 // cost for lines of n_r samples and a chirp of L samples.
 bool choose_dc_block(int n_r, int L, int& B, int& U, int& nb);
@@ -57,7 +57,7 @@ void dc_lag1_sums(const DcEstArgs& a, cudaStream_t st);
 // (s1g_eccm.cu): the lines with flags[row] set, read from the FP64 decoded
 // samples `in`, notched (fft 128, stride 64, mitigation threshold mit) into
 // the complex<float> rows of `out`; other rows of `out` are left as they are.
-// d128: the 128-point twiddles (make_cfft_plan(128)).
+// d128: the 128-point twiddles (make_cfft_plan of 128).
 void eccm_notch_cc(const cf64* in, long long ip, cf32* out, long long op, int n_r, long long rows, const int* flags,
                    double mit, const CfftDesc& d128, cudaStream_t st);
 // The ECCM line detection flags[row] = (max_k |FFT(line)_k| >= det) from the

@@ -821,12 +821,12 @@ DecodeTables::~DecodeTables() {
     if (lut) cudaFree(lut);
 }
 
-void DecodeTables::init() {
+void DecodeTables::init(cudaStream_t st) {
     if (lut) return;
     std::vector<HuffEntry> h;
     build_lut(h);
     check_cuda(cudaMalloc(&lut, sizeof(HuffEntry) * h.size()), "lut");
-    check_cuda(cudaMemcpy(lut, h.data(), sizeof(HuffEntry) * h.size(), cudaMemcpyHostToDevice), "lut up");
+    upload_table(lut, h.data(), sizeof(HuffEntry) * h.size(), st, "lut up");
 }
 
 template <typename R>

@@ -177,7 +177,7 @@ std::vector<int> fft4_order64(long long n);
 // The cheapest affine lengths >= minlen that fit shared memory.
 std::vector<long long> fft4_lengths(long long minlen, size_t most);
 template <typename R>
-std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& radices);
+std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& radices, cudaStream_t st);
 // Radix order for length n: the fastest measured candidate when tuning is on
 // (S1G_AUTOTUNE unset or not "0"), else the model's.  Measurements run on
 // `st` (skipped while st is being captured) and persist in a text file
@@ -195,6 +195,18 @@ void transpose_batched(const cpx<R>* in, long long in_row_pitch, long long in_ba
                        cudaStream_t s);
 
 void check_cuda(cudaError_t e, const char* what);
+// Copy a host table (which may go when the call returns) to device memory in
+// the order of st.  A plain cudaMemcpy of pageable memory may return before the
+// device has it, and the handles' streams do not wait for the legacy stream.
+inline void upload_table(void* dst, const void* src, size_t bytes, cudaStream_t st, const char* what) {
+    check_cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), what);
+}
+// Copy a host table to a device variable that every stream may read from now on.
+template <class T>
+inline void upload_symbol(T& symbol, const void* src, size_t bytes, const char* what) {
+    check_cuda(cudaMemcpyToSymbol(symbol, src, bytes), what);
+    check_cuda(cudaStreamSynchronize(cudaStreamLegacy), what);
+}
 // Multiprocessors of the current device.
 int device_sms();
 // Allow a kernel `bytes` of dynamic shared memory.  The limit belongs to the

@@ -15,6 +15,7 @@
 // address is looked up with cudaGetSymbolAddress once per device, with that
 // device current, and passed to the kernel.
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
 
@@ -57,9 +58,10 @@ static int setup_device(int dev, std::string& err) {
     }
     uint8_t host[sizeof(g_noalloc_lut)];
     huffman_lut_fill(host);
-    e = cudaMemcpyToSymbol(g_noalloc_lut, host, sizeof(host));
-    if (e != cudaSuccess) {
-        err = std::string("cudaMemcpyToSymbol(lut): ") + cudaGetErrorString(e);
+    try {
+        upload_symbol(g_noalloc_lut, host, sizeof(host), "Huffman table");
+    } catch (const std::exception& x) {
+        err = x.what();
         return S1G_E_CUDA;
     }
     d.ready = true;

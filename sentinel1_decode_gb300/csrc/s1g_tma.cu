@@ -199,7 +199,11 @@ int tma_take_error() {
     if (cudaMemcpyFromSymbol(&e, g_tma_error, sizeof(int)) != cudaSuccess) return -1;
     if (e) {
         const int zero = 0;
-        cudaMemcpyToSymbol(g_tma_error, &zero, sizeof(int));
+        try {
+            upload_symbol(g_tma_error, &zero, sizeof(int), "tma flag");
+        } catch (const std::exception&) {
+            return -1;
+        }
     }
     return e;
 }

@@ -4,8 +4,9 @@
 // those of the packet indexer and the header gather, so that streams open.
 // Two devices.  What it watches is read back with fake_count:
 //   launch:<text>   launches of kernels whose (mangled) name holds the text
-//   unordered       launches on another stream than the legacy one after a copy
-//                   of pageable memory on that one that nothing waited for
+//   pending         1 after a copy of pageable memory or a memset on the legacy
+//                   stream that nothing waited for
+//   unordered       launches on another stream while that is so
 //   refused         launches with more dynamic shared memory than the kernel may
 //                   have on the current device (they fail, as on a GPU)
 //   capture, replay graphs captured and launched
@@ -104,6 +105,7 @@ extern "C" {
 long long fake_count(const char* what) {
     Lock lk(mu);
     const std::string w = what;
+    if (w == "pending") return legacy_copy;
     if (w.rfind("launch:", 0) != 0) return counts[w];
     long long n = 0;
     for (const auto& kv : launches)
@@ -208,11 +210,13 @@ cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size
     for (size_t r = 0; r < h; ++r) std::memcpy((char*)d + r * dp, (const char*)s + r * sp, w);
     return cudaSuccess;
 }
-cudaError_t cudaMemset(void* d, int v, size_t n) {
+cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t stream) {
+    Lock lk(mu);
     std::memset(d, v, n);
+    if (legacy(stream)) legacy_copy = true;
     return cudaSuccess;
 }
-cudaError_t cudaMemsetAsync(void* d, int v, size_t n, cudaStream_t) { return cudaMemset(d, v, n); }
+cudaError_t cudaMemset(void* d, int v, size_t n) { return cudaMemsetAsync(d, v, n, nullptr); }
 cudaError_t cudaMemcpyToSymbol(const void* symbol, const void* s, size_t n, size_t off, cudaMemcpyKind) {
     Lock lk(mu);
     std::memcpy((char*)var_memory(symbol) + off, s, n);

@@ -202,3 +202,61 @@ for device in (0, 1):
     assert count("refused") == 0, device
 assert count("launch:k_rc_dc") and count("launch:k_transpose_tma") and count("launch:k_eccm_notch")
 """)
+
+
+ORDER = {
+    "products": """
+for precision in ("fp32", "fp32_plain", "fp64"):
+    d = S1Decoder(stream(*bursts((1000, 31), (1003, 31))), precision=precision)
+    for eccm in (False, True):
+        d.get_range_compressed_burst("IW2", 0, range_doppler=True, dtype=np.complex64)
+        if precision == "fp32":         # the others read their tile counts back from kernels
+            d.get_azimuth_compressed_burst("IW2", 1, dtype=np.complex64)
+        d.apply_eccm(1000, 10)
+    if precision == "fp32":
+        for _ in range(2):
+            process_swath_batch([d], "IW2")
+""",
+    # one 20-line group of a stripmap among others: packets that are not in a row
+    "scattered": """
+d = S1Decoder(stream(*[x for k in range(6) for x in bursts((40, 40 + k), swath="S%d" % (k % 2 + 1))]))
+d.apply_eccm(1000, 10)
+for precision in ("fp32", "fp64"):
+    d.set_precision(precision)
+    for level in ("raw", "range"):
+        try:
+            (d.get_swath if level == "raw" else d.get_range_compressed_swath)("S1", dtype=np.complex64)
+        except S1GError:
+            pass
+""",
+    "adjoint": """
+d = S1Decoder(stream(*bursts((300, 40), swath="S1", beam_start=512, beam_sweep=0)))
+try:
+    d.azimuth_adjoint("S1", 0, [1.0], 0.0)
+except S1GError as e:
+    assert "zero" in str(e) or "empty" in str(e), e       # kernels do nothing: the image is 0
+assert count("launch:k_entropy_sums") == 1
+""",
+    "noalloc": """
+lib = load_library()
+x = np.zeros(4096, np.uint8)
+p = x.ctypes.data
+assert lib.s1g_decode_fdbaq_noalloc(p, 1000, p + 2048, 2, 8, p, 16, p + 3000, 0x1000) == 0
+assert count("launch:k_decode_fdbaq") == 1
+""",
+    "packet": """
+d = S1Decoder(stream(*bursts((300, 40))))
+x = np.zeros(80, np.complex64)
+assert d._lib.s1g_packet_samples(d.handle, 3, x.ctypes.data, 80, 0, 1) == 0
+""",
+}
+
+
+@pytest.mark.parametrize("what", sorted(ORDER))
+def test_tables_reach_the_device_before_their_readers(fake, what):
+    """The handles' streams do not wait for the legacy stream, and a copy from
+    pageable memory on that one may return before the device has the data."""
+    fake(ORDER[what] + """
+assert count("unordered") == 0, (count("unordered"), rt.fake_last_unordered())
+assert count("pending") == 0
+""")
