@@ -2447,8 +2447,12 @@ int s1g_swath_product(s1g_decoder* h, const char* swath, int level, void* out, i
         row += r.rows;
         if (e.pad_rows) {
             const size_t nb = (size_t)e.pad_rows * cols * esz;
-            if (out_on_device) check_cuda(cudaMemset((char*)out + (size_t)row * cols * esz, 0, nb), "pad");
-            else memset((char*)out + (size_t)row * cols * esz, 0, nb);
+            if (out_on_device) {
+                check_cuda(cudaMemsetAsync((char*)out + (size_t)row * cols * esz, 0, nb, h->stream), "pad");
+                check_cuda(cudaStreamSynchronize(h->stream), "pad");
+            } else {
+                memset((char*)out + (size_t)row * cols * esz, 0, nb);
+            }
             row += e.pad_rows;
         }
     }

@@ -260,3 +260,17 @@ def test_tables_reach_the_device_before_their_readers(fake, what):
 assert count("unordered") == 0, (count("unordered"), rt.fake_last_unordered())
 assert count("pending") == 0
 """)
+
+
+def test_swath_padding_is_done_when_the_call_returns(fake):
+    """The rows of zeros between the bursts of a focused IW swath, in the caller's
+    device buffer."""
+    fake("""
+d = S1Decoder(stream(*bursts((1000, 24), (1003, 24), (1001, 24))))
+for level in range(4):
+    rows, cols = ctypes.c_int64(), ctypes.c_int64()
+    assert d._lib.s1g_swath_shape(d.handle, b"IW2", level, ctypes.byref(rows), ctypes.byref(cols)) == 0
+    out = np.zeros((rows.value, cols.value), np.complex64)
+    assert d._lib.s1g_swath_product(d.handle, b"IW2", level, out.ctypes.data, *out.shape, 0, 1) == 0
+    assert count("pending") == 0, level
+""")
