@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(128) k_dc_lag1(DcEstArgs a) {
 static size_t dc_smem(int n, int sh) { return sizeof(float4) * (size_t)(n + (n >> sh)); }
 
 void dc_lag1_sums(const DcEstArgs& a, cudaStream_t st) {
-    allow_dynamic_smem(k_rc_dc, kSmemBytes);
+    allow_dynamic_smem<k_rc_dc>(kSmemBytes);
     const size_t smem = dc_smem(a.d.n, a.d.sh);
     if (smem > (size_t)kSmemBytes) throw std::runtime_error("Doppler estimator: shared memory");
     const long long blocks = (long long)a.n_a * a.nb;

@@ -22,6 +22,7 @@
 // core).
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <map>
 #include <memory>
@@ -209,11 +210,17 @@ inline void upload_symbol(T& symbol, const void* src, size_t bytes, const char* 
 }
 // Multiprocessors of the current device.
 int device_sms();
-// Allow a kernel `bytes` of dynamic shared memory.  The limit belongs to the
-// current device, so it is set at every launch, not once a process.
-template <class K>
-inline void allow_dynamic_smem(K kernel, int bytes) {
+// Allow a kernel `bytes` (the same at every call) of dynamic shared memory on
+// the current device: the limit belongs to a device, so one flag per process
+// would leave the second device without it.
+template <auto kernel>
+inline void allow_dynamic_smem(int bytes) {
+    static std::atomic<bool> done[64];
+    int dev = 0;
+    check_cuda(cudaGetDevice(&dev), "attr");
+    if (dev < 64 && done[dev].load(std::memory_order_relaxed)) return;
     check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "attr");
+    if (dev < 64) done[dev].store(true, std::memory_order_relaxed);
 }
 
 // Count of kernels this library has launched (reported by the benchmark).

@@ -516,7 +516,7 @@ void eccm_notch(cpx<R>* data, long long p, int n_r, long long rows, const int* f
     const int num_ffts = eccm_num_windows(n_r);
     constexpr int WB = sizeof(R) == 4 ? 32 : 8;
     const size_t smem = sizeof(cpx<R>) * ((size_t)n_r + WB * 128) + WB * 128;
-    allow_dynamic_smem(k_eccm_notch<R, WB>, kSmemBytes);
+    allow_dynamic_smem<k_eccm_notch<R, WB>>(kSmemBytes);
     if (smem > (size_t)kSmemBytes) throw std::runtime_error("eccm: line too long for shared memory");
     if (rows > 0)
         note_launch(), k_eccm_notch<R, WB><<<(unsigned)rows, 256, smem, st>>>(data, p, n_r, flags, mit, d128, mask_out, num_ffts);

@@ -189,7 +189,7 @@ bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int ro
     const long long tiles = (long long)((cols + kTileCols - 1) / kTileCols) * ((rows + kTileRows - 1) / kTileRows);
     const int grid = (int)std::min<long long>(tiles, 4LL * device_sms());
     const size_t smem = 2 * kTileBytes + 1024;
-    allow_dynamic_smem(k_transpose_tma, (int)smem);
+    allow_dynamic_smem<k_transpose_tma>((int)smem);
     note_launch(), k_transpose_tma<<<grid, 256, smem, st>>>(map, out, op, rows, cols);
     return true;
 }
