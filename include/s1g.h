@@ -36,9 +36,11 @@
  * first with the *_shape calls.
  *
  * Errors: every call returns S1G_OK or a negative code; s1g_last_error()
- * gives the message; after an error other than S1G_E_BUFFER the contents of an
- * output buffer are undefined.  A decoder handle is not thread-safe: use one handle per
- * host thread.  All GPU work of a handle runs on its own CUDA stream.
+ * gives the message.  A product call that fails leaves the output buffer as it
+ * was (a swath call may have written its earlier bursts); after S1G_E_CUDA and
+ * S1G_E_TIMEOUT the contents of a device buffer are undefined.  A decoder
+ * handle is not thread-safe: use one handle per host thread.  All GPU work of a
+ * handle runs on its own CUDA stream.
  */
 #ifndef S1G_H
 #define S1G_H

@@ -73,7 +73,8 @@ struct RangeRef {
 };
 
 // The caller's device buffer for a complex<float> product of this shape: the
-// last kernel of a chain writes there instead of into a buffer that is copied.
+// last kernel of a chain writes there instead of into a buffer that is copied
+// (unless the chain has failed: see Failed).
 struct Dest {
     cf32* p = nullptr;
     long long rows = 0, cols = 0;
@@ -163,6 +164,10 @@ struct s1g_decoder {
     size_t pin_cap = 0;
     bool defer_status = false;
     const std::vector<int>* pending = nullptr;
+    // device word a failed decode sets (0 otherwise), while the product of the
+    // call is formed in the caller's buffer: its last kernel then writes nothing
+    Buf bFailed{&moves};
+    int* failed = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     int* pinned(size_t n) {
         if (n > pin_cap) {
@@ -504,10 +509,14 @@ struct Pipe {
         cpx<R>* A = h->bA.as<cpx<R>>((size_t)npk * g.n_r);
         int* status = h->bStatus.as<int>(npk);
         if (any_d)
-            decode_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status, h->tabs, st);
-        if (any_fixed)
+            decode_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status, h->tabs,
+                            st, any_fixed ? nullptr : h->failed);
+        if (any_fixed) {
             decode_fixed_burst<R>(h->d_stream, h->nbytes, h->d_off, d_idx, pk.front(), npk, g.nq, A, g.n_r, status,
                                   h->abc_fields, st);
+            // the FDBAQ decoder's status of the other packets is overwritten
+            if (h->failed) any_status(status, npk, h->failed, st);
+        }
         if (h->defer_status) {
             int* pin = h->pinned((size_t)npk + 2);
             check_cuda(cudaMemcpyAsync(pin + 2, status, sizeof(int) * npk, cudaMemcpyDeviceToHost, st), "status");
@@ -1297,6 +1306,9 @@ struct FastPipe {
     const cf32* predecoded = nullptr;   // burst already decoded (batched decode)
     cf64* predecoded64 = nullptr;       // ... and its FP64 samples (for the ECCM notch), or null
     Dest dest;                          // caller's buffer for the product
+    Failed failed(const int* unfold = nullptr) const {   // what its last kernel looks at; none without it
+        return dest.p ? Failed{h->failed, unfold} : Failed{};
+    }
     cf32* final_out = nullptr;          // write the SLC here ([N_out][N_r]) instead of a work buffer
     int* tufr_status = nullptr;         // per-burst time-unfolding status slot
     explicit FastPipe(s1g_decoder* hh) : h(hh), st(hh->stream), fft(*hh->fft) {}
@@ -1554,14 +1566,14 @@ struct FastPipe {
         }
         cf32* fin = dest.take(n_a, n_r);
         cf32* rc = fin && level == S1G_RANGE_COMPRESSED ? fin : h->bB.as<cf32>((size_t)n_a * n_r);
-        rc_fused(raw, rc, n_a, n_r, g.h, fb.dM, fb.ref, st);
+        rc_fused(raw, rc, n_a, n_r, g.h, fb.dM, fb.ref, st, rc == fin ? failed() : Failed{});
         const bool rd = (level == S1G_RANGE_DOPPLER) || (az && !tops);
         if (rd) {
             cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
             transpose_batched<float>(rc, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
             fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, -1, n_a / 2);
             if (fin && !az) rc = fin;
-            transpose_batched<float>(Bt, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st);
+            transpose_batched<float>(Bt, n_a, 0, rc, n_r, 0, n_r, n_a, 1, st, rc == fin ? failed() : Failed{});
         }
         if (!az) {
             r.ptr = rc;
@@ -1605,7 +1617,7 @@ struct FastPipe {
         cf32* Bt = h->bC.as<cf32>((size_t)n_a * n_r);
         transpose_batched<float>(rd, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
         fft.rows<float>(*fft.plan<float>(n_a), Bt, n_a, Bt, n_a, n_r, +1, 0, 1.0 / n_a);
-        transpose_batched<float>(Bt, n_a, 0, out, n_r, 0, n_r, n_a, 1, st);
+        transpose_batched<float>(Bt, n_a, 0, out, n_r, 0, n_r, n_a, 1, st, failed());
         Result r;
         r.ptr = out;
         r.rows = n_a;
@@ -1746,7 +1758,7 @@ struct FastPipe {
         tufr_fused(ta, tl, st);
         h->mark("corner_turn");
         cf32* O = final_out ? final_out : h->bA.as<cf32>((size_t)ta.n_out * n_r);
-        transpose_batched<float>(outT, ta.n_out, 0, O, n_r, 0, n_r, ta.n_out, 1, st);
+        transpose_batched<float>(outT, ta.n_out, 0, O, n_r, 0, n_r, ta.n_out, 1, st, failed(stat));
         Result r;
         r.ptr = O;
         r.rows = ta.n_out;
@@ -1774,6 +1786,19 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
     auto decode_ok = [&] {
         if (h->pending) check_decode_status(h->pin + 2, *h->pending);
     };
+    h->failed = nullptr;
+    if (dest.p && !h->bFailed.p)
+        check_cuda(cudaMemsetAsync(h->bFailed.as<int>(1), 0, sizeof(int), h->stream), "failure word");
+    if (dest.p) h->failed = (int*)h->bFailed.p;
+    // it stays 0 but for a decode error, whose call clears it
+    struct Clear {
+        s1g_decoder* h;
+        bool done = false;
+        ~Clear() {
+            if (!done && h->failed) cudaMemsetAsync(h->failed, 0, sizeof(int), h->stream);
+            h->failed = nullptr;
+        }
+    } clear{h};
     try {
         if (h->precision == S1G_PREC_FP64) r = Pipe<double>(h).run(pk, level, tops);
         else if (h->precision == S1G_PREC_FP32_PLAIN) r = Pipe<float>(h).run(pk, level, tops);
@@ -1805,6 +1830,7 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
         throw S1Error(S1G_E_TIMEOUT, "a TMA corner turn gave up waiting for its tile");
     }
     if (r.status && pin[1]) throw S1Error(S1G_E_GEOMETRY, "azimuth time unfolding parameters out of range");
+    clear.done = true;
     return r;
 }
 

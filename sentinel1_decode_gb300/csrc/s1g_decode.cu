@@ -425,7 +425,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
                                                         const long long* __restrict__ offsets, DecodeSpec spec,
                                                         cf32* __restrict__ out32, cf64* __restrict__ out64,
                                                         int* __restrict__ status, int nq_max,
-                                                        const HuffEntry* __restrict__ lut_g) {
+                                                        const HuffEntry* __restrict__ lut_g, int* __restrict__ any) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     DecodeShared& sh = *reinterpret_cast<DecodeShared*>(smem_raw);
     for (int i = threadIdx.x; i < 5 * kHuffWindow / 2; i += blockDim.x)
@@ -606,11 +606,15 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
             if (F32) out32[jb.out + k] = mk(0.f, 0.f);
             if (F64) out64[jb.out + k] = mk(0.0, 0.0);
         }
-    if (lane == 0) status[j] = st;
+    if (lane == 0) {
+        status[j] = st;
+        if (st && any) *any = 1;
+    }
 }
 
 static void launch_fdbaq(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeSpec& spec,
-                         cf32* out32, cf64* out64, int* d_status, int nq_max, const void* d_lut, cudaStream_t st) {
+                         cf32* out32, cf64* out64, int* d_status, int nq_max, const void* d_lut, cudaStream_t st,
+                         int* any = nullptr) {
     // one warp per CTA where two packets' symbols do not fit (nq above ~25000)
     const int warps = decode_smem(nq_max, kDecodeWarps) <= (size_t)kSmemBytes ? kDecodeWarps : 1;
     const size_t smem = decode_smem(nq_max, warps);
@@ -618,7 +622,7 @@ static void launch_fdbaq(const uint8_t* d_stream, long long n, const long long* 
         if (smem > 48 * 1024)
             check_cuda(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "attr");
         note_launch(), kernel<<<(spec.njobs + warps - 1) / warps, 32 * warps, smem, st>>>(
-            d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, (const HuffEntry*)d_lut);
+            d_stream, n, d_offsets, spec, out32, out64, d_status, nq_max, (const HuffEntry*)d_lut, any);
     };
     if (out32 && out64) go(k_decode_fdbaq<true, true>);
     else if (out64) go(k_decode_fdbaq<false, true>);
@@ -832,10 +836,18 @@ void DecodeTables::init(cudaStream_t st) {
 template <typename R>
 void decode_burst(const uint8_t* d_stream, long long n, const long long* d_offsets, const int* d_pkidx, int p0,
                   int npk, int nq, cpx<R>* out, long long pitch, int* d_status, const DecodeTables& tabs,
-                  cudaStream_t st) {
+                  cudaStream_t st, int* any) {
     const DecodeSpec spec{nullptr, npk, d_pkidx, p0, nq, pitch};
-    if constexpr (sizeof(R) == 4) launch_fdbaq(d_stream, n, d_offsets, spec, out, nullptr, d_status, nq, tabs.lut, st);
-    else launch_fdbaq(d_stream, n, d_offsets, spec, nullptr, out, d_status, nq, tabs.lut, st);
+    if constexpr (sizeof(R) == 4) launch_fdbaq(d_stream, n, d_offsets, spec, out, nullptr, d_status, nq, tabs.lut, st, any);
+    else launch_fdbaq(d_stream, n, d_offsets, spec, nullptr, out, d_status, nq, tabs.lut, st, any);
+}
+
+__global__ void k_any_status(const int* __restrict__ status, int n, int* __restrict__ any) {
+    for (int i = threadIdx.x; i < n; i += blockDim.x)
+        if (status[i]) *any = 1;
+}
+void any_status(const int* d_status, int n, int* any, cudaStream_t st) {
+    note_launch(), k_any_status<<<1, 256, 0, st>>>(d_status, n, any);
 }
 
 void decode_jobs(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeJob* d_jobs, int njobs,
@@ -871,8 +883,8 @@ template void decode_fixed_jobs<double>(const uint8_t*, long long, const long lo
                                         cpx<double>*, int*, int, cudaStream_t);
 
 template void decode_burst<float>(const uint8_t*, long long, const long long*, const int*, int, int, int, cpx<float>*,
-                                  long long, int*, const DecodeTables&, cudaStream_t);
+                                  long long, int*, const DecodeTables&, cudaStream_t, int*);
 template void decode_burst<double>(const uint8_t*, long long, const long long*, const int*, int, int, int,
-                                   cpx<double>*, long long, int*, const DecodeTables&, cudaStream_t);
+                                   cpx<double>*, long long, int*, const DecodeTables&, cudaStream_t, int*);
 
 }  // namespace s1g

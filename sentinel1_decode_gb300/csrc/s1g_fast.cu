@@ -49,9 +49,10 @@ void czt_rows(const cf32* in, long long ip, cf32* out, long long op, long long r
 template <int NT, int MB>
 __global__ void __launch_bounds__(NT, MB)
     k_rc_fused(const cf32* __restrict__ raw, cf32* __restrict__ rc, int n_r, int h, Fft4Desc d,
-               const cf32* __restrict__ ref) {
+               const cf32* __restrict__ ref, Failed failed) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     cf32* buf = reinterpret_cast<cf32*>(smem_raw);
+    const int bad = failed.first();
     const cf32* x = raw + (long long)blockIdx.x * n_r;
     cf32* y = rc + (long long)blockIdx.x * n_r;
     fft4_head(buf, d, [&](int q) { return q < n_r ? x[q] : mk(0.f, 0.f); });
@@ -59,17 +60,17 @@ __global__ void __launch_bounds__(NT, MB)
     fft4_tail(buf, d, [&](int q, cf32 v) {
         int k = q + h;
         if (k >= d.n) k -= d.n;
-        if (k < n_r) y[k] = v;
+        if (k < n_r && !bad) y[k] = v;
     });
 }
 
 void rc_fused(const cf32* raw, cf32* rc, int n_a, int n_r, int h, const Fft4Desc& d, const cf32* ref,
-              cudaStream_t st) {
+              cudaStream_t st, Failed failed) {
     const size_t smem = fft4_smem(d.n);
     fft4_launch(smem, [&](auto nt, auto mb) {
         auto kernel = k_rc_fused<decltype(nt)::value, decltype(mb)::value>;
         allow_smem(kernel);
-        note_launch(), kernel<<<n_a, decltype(nt)::value, smem, st>>>(raw, rc, n_r, h, d, ref);
+        note_launch(), kernel<<<n_a, decltype(nt)::value, smem, st>>>(raw, rc, n_r, h, d, ref, failed);
     });
 }
 

@@ -149,7 +149,7 @@ struct TufrArgs {
 };
 
 void rc_fused(const cf32* raw, cf32* rc, int n_a, int n_r, int h, const Fft4Desc& d, const cf32* ref,
-              cudaStream_t st);
+              cudaStream_t st, Failed failed = {});
 void fufr_fused(const FufrArgs& a, cudaStream_t st);
 // Doppler centroid of every range bin (f_dc, and as float pairs in f_dc_df
 // unless it is null) from nchunk partial lag-1 sums [nchunk][n_r]; poly: device

@@ -558,8 +558,9 @@ __global__ void __launch_bounds__(kFftThreads) k_rows8_blue(const __grid_constan
 // 32x32 tiled transpose of a batch of matrices.
 template <typename R>
 __global__ void k_transpose(const cpx<R>* __restrict__ in, long long irp, long long ibp, cpx<R>* __restrict__ out,
-                            long long orp, long long obp, int rows, int cols) {
+                            long long orp, long long obp, int rows, int cols, Failed failed) {
     __shared__ cpx<R> tile[32][33];
+    if (failed.first() | failed.second()) return;
     const long long b = blockIdx.z;
     const int c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
     const cpx<R>* src = in + b * ibp;
@@ -1146,13 +1147,13 @@ FftDesc<R> FftEngine::smem_desc(int n) {
 
 template <typename R>
 void transpose_batched(const cpx<R>* in, long long irp, long long ibp, cpx<R>* out, long long orp, long long obp,
-                       int rows, int cols, long long batch, cudaStream_t s) {
+                       int rows, int cols, long long batch, cudaStream_t s, Failed failed) {
     if constexpr (sizeof(R) == 4) {
         // single complex<float> matrices go through the TMA-staged corner turn
-        if (batch == 1 && transpose_tma(in, irp, out, orp, rows, cols, s)) return;
+        if (batch == 1 && transpose_tma(in, irp, out, orp, rows, cols, s, failed)) return;
     }
     dim3 grid((cols + 31) / 32, (rows + 31) / 32, (unsigned)batch);
-    note_launch(), k_transpose<R><<<grid, dim3(32, 8), 0, s>>>(in, irp, ibp, out, orp, obp, rows, cols);
+    note_launch(), k_transpose<R><<<grid, dim3(32, 8), 0, s>>>(in, irp, ibp, out, orp, obp, rows, cols, failed);
 }
 
 // rows of a plan of one of the one-kernel kinds
@@ -1275,9 +1276,9 @@ template void FftEngine::rows<double>(const FftPlan<double>&, const cpx<double>*
 template FftDesc<float> FftEngine::smem_desc<float>(int);
 template FftDesc<double> FftEngine::smem_desc<double>(int);
 template void transpose_batched<float>(const cpx<float>*, long long, long long, cpx<float>*, long long, long long,
-                                       int, int, long long, cudaStream_t);
+                                       int, int, long long, cudaStream_t, Failed);
 template void transpose_batched<double>(const cpx<double>*, long long, long long, cpx<double>*, long long,
-                                        long long, int, int, long long, cudaStream_t);
+                                        long long, int, int, long long, cudaStream_t, Failed);
 template struct FftPlan<float>;
 template struct FftPlan<double>;
 

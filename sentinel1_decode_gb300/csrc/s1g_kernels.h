@@ -72,9 +72,13 @@ void spectrogram(const cf64* line, int n, int fft, int stride, cf64* out, cudaSt
 // BigTIFF float32 writer, bottom-up rows (host).
 int write_bigtiff(const char* path, const float* img, long long rows, long long cols, std::string& err);
 
+// any (null: not wanted): a device word set to 1 where a packet fails.
 template <typename R>
 void decode_burst(const uint8_t* d_stream, long long n, const long long* d_offsets, const int* d_pkidx, int p0,
-                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, const DecodeTables& tabs, cudaStream_t st);
+                  int npk, int nq, cpx<R>* out, long long pitch, int* d_status, const DecodeTables& tabs,
+                  cudaStream_t st, int* any = nullptr);
+// The same word from the status of n packets.
+void any_status(const int* d_status, int n, int* any, cudaStream_t st);
 
 // Data formats A/B (bypass) and C (BAQ): rows of packets whose baq_mode is
 // 0 or 3..5 (FDBAQ rows are skipped).  fields = 0: the reference's output;

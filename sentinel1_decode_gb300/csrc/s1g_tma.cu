@@ -81,8 +81,9 @@ __device__ __forceinline__ void tma_load_2d(void* dst, const CUtensorMap* map, i
 }  // namespace
 
 __global__ void __launch_bounds__(256) k_transpose_tma(const __grid_constant__ CUtensorMap src, cf32* __restrict__ out,
-                                                       long long op, int rows, int cols) {
+                                                       long long op, int rows, int cols, Failed failed) {
     extern __shared__ unsigned char smem_raw[];
+    const int bad0 = failed.first(), bad1 = failed.second(), bad2 = failed.a ? g_tma_error : 0;
     __shared__ uint64_t bar[2];
     __shared__ int s_fail;
     // the 128-byte swizzle repeats every 1024 bytes: tile buffers 1024-aligned
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(256) k_transpose_tma(const __grid_constant__ C
 #pragma unroll
             for (int q = 0; q < kTileRows / 32; ++q) {
                 const int r = 32 * q + lane;
-                if (r0 + r >= rows) continue;
+                if (r0 + r >= rows || (bad0 | bad1 | bad2)) continue;
                 const int off = r * 128 + ((((c >> 1) ^ (r & 7))) << 4) + ((c & 1) << 3);
                 orow[r] = *reinterpret_cast<const cf32*>(tile + off);
             }
@@ -171,7 +172,8 @@ static PFN_cuTensorMapEncodeTiled_v12000 encode_tiled() {
     return fn;
 }
 
-bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int rows, int cols, cudaStream_t st) {
+bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int rows, int cols, cudaStream_t st,
+                   Failed failed) {
     PFN_cuTensorMapEncodeTiled_v12000 enc = encode_tiled();
     // a tiled TMA copy needs a 16-byte aligned base and a row pitch that is a
     // multiple of 16 bytes (an even number of complex<float>)
@@ -190,7 +192,7 @@ bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int ro
     const int grid = (int)std::min<long long>(tiles, 4LL * device_sms());
     const size_t smem = 2 * kTileBytes + 1024;
     allow_dynamic_smem<k_transpose_tma>((int)smem);
-    note_launch(), k_transpose_tma<<<grid, 256, smem, st>>>(map, out, op, rows, cols);
+    note_launch(), k_transpose_tma<<<grid, 256, smem, st>>>(map, out, op, rows, cols, failed);
     return true;
 }
 

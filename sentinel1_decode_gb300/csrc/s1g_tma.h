@@ -9,7 +9,8 @@ namespace s1g {
 // tensor-memory-accelerator tile loads.  Returns false, launching nothing,
 // where a tiled TMA copy cannot read the source (odd pitch, base not 16-byte
 // aligned, no driver entry point); the caller then transposes another way.
-bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int rows, int cols, cudaStream_t st);
+bool transpose_tma(const cf32* in, long long ip, cf32* out, long long op, int rows, int cols, cudaStream_t st,
+                   Failed failed = {});
 
 // 1 if a TMA corner turn gave up waiting for its tile since the last call
 // (and clears the flag), 0 otherwise, -1 if the flag cannot be read.
