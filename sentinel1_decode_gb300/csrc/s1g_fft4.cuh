@@ -500,10 +500,9 @@ __device__ __forceinline__ void fft4_back(cpx<T>* buf, const Fft4DescT<T>& d) {
     }
 }
 
-// The other inverse passes: store(i, v) gets output i.  No barrier at the end.
+// The last inverse pass: store(i, v) gets output i.  No barrier at the end.
 template <bool ROLL = false, typename T, class StoreF>
-__device__ __forceinline__ void fft4_tail(cpx<T>* buf, const Fft4DescT<T>& d, StoreF store) {
-    fft4_back(buf, d);
+__device__ __forceinline__ void fft4_last(cpx<T>* buf, const Fft4DescT<T>& d, StoreF store) {
     bool done = false;
     if constexpr (sizeof(T) == 4) if (d.affine) {
         done = true;
@@ -518,6 +517,13 @@ __device__ __forceinline__ void fft4_tail(cpx<T>* buf, const Fft4DescT<T>& d, St
     if (!done) {
         for (int i = threadIdx.x; i < d.n; i += blockDim.x) store(i, buf[pad16(i)]);
     }
+}
+
+// The inverse passes after fft4_mid.
+template <bool ROLL = false, typename T, class StoreF>
+__device__ __forceinline__ void fft4_tail(cpx<T>* buf, const Fft4DescT<T>& d, StoreF store) {
+    fft4_back(buf, d);
+    fft4_last<ROLL>(buf, d, store);
 }
 
 // fft4_tail and fft4_head of the next transform of the same plan in one:
