@@ -731,7 +731,6 @@ struct Pipe {
         if (tops) {
             rate = dc_rate(g);
             h->mark("doppler");
-            // FP32: formed from FP64 lines before this burst's own (run)
             fdc = doppler(A, g, rate);
             h->mark("freq_unfold");
             // azimuth_frequency_ufr (image_formation.cpp:125-219)

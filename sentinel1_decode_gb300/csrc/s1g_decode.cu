@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(32 * kDecodeWarps) k_decode_fdbaq(const uint8_
 static void launch_fdbaq(const uint8_t* d_stream, long long n, const long long* d_offsets, const DecodeSpec& spec,
                          cf32* out32, cf64* out64, int* d_status, int nq_max, const void* d_lut, cudaStream_t st,
                          int* any = nullptr) {
-    // one warp per CTA where two packets' symbols do not fit (nq above ~25000)
+    // one warp per CTA where the symbols of kDecodeWarps packets do not fit (nq above ~25000)
     const int warps = decode_smem(nq_max, kDecodeWarps) <= (size_t)kSmemBytes ? kDecodeWarps : 1;
     const size_t smem = decode_smem(nq_max, warps);
     auto go = [&](auto kernel) {

@@ -170,8 +170,9 @@ __global__ void k_dc_wrapped(const cf64* __restrict__ part, int nchunk, int n, d
 // Block means, unwrap (doppler.cpp:42-95) and the quadratic fit's three
 // coefficients: a warp per block mean, a thread per bin of the dense DFT (its
 // roots from a table: one SM does 1.9 FP64 operations a clock) and per block
-// of the unwrap.  20 us, where 256 threads with serial means and one thread
-// for the unwrap took 288 (and the FP64 pipeline's all-serial fit 19.8 ms).
+// of the unwrap.  69 us (84 with the kernels before and after it), where 256
+// threads with serial means and one thread for the unwrap took 288 (and the FP64
+// pipeline's all-serial fit 19.8 ms).
 __global__ void __launch_bounds__(1024) k_dc_fit(const double* __restrict__ f_dc, DcFitArgs a, double* __restrict__ poly) {
     __shared__ double fine[kFitBlocks], fval[kFitBlocks], un[kFitBlocks];
     __shared__ double mag2[8 * kFitBlocks], fre[8 * kFitBlocks], fim[8 * kFitBlocks];

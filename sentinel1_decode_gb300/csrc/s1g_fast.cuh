@@ -187,7 +187,7 @@ struct TufrLaunch {
 };
 TufrLaunch tufr_launch(int S, int tmax, int M);
 void tufr_fused(const TufrArgs& a, const TufrLaunch& L, cudaStream_t st);
-// Fill a.tab for the burst whose parameters are at a.P (tables sized for a.tmax tiles).
+// Fill a.tab for the burst whose parameters are at a.P (a.tab.wt sized by tufr_launch).
 void tufr_tables(const TufrArgs& a, cudaStream_t st);
 void czt_rows(const cf32* in, long long ip, cf32* out, long long op, long long rows, const CztDev& c, int dir,
               float scale, cudaStream_t st);

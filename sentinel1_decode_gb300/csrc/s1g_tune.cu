@@ -2,7 +2,7 @@
 // length the fused kernels need, it times the modelled cheapest radix orders
 // and, where the length is free (chirp-z convolutions, zero-padded range
 // lines, the non-uniform FFT grid), the cheapest affine lengths, on this GPU
-// with the kernels' own launch shape (fft4_shape), and keeps the fastest.
+// with the kernels' own launch shape (fft4_launch), and keeps the fastest.
 //
 // A measurement is a launch of one CTA per slot of every SM, each running a
 // forward transform, a factor and an inverse transform four times; the
