@@ -179,6 +179,19 @@ struct s1g_decoder {
         }
         return pin;
     }
+    // Host tables of queued uploads: a copy from pageable memory may read it after
+    // the call that queues it.  Let go once the stream has been waited for.
+    std::vector<std::shared_ptr<const void>> held;
+    template <typename T>
+    const std::vector<T>& hold(std::vector<T> v) {
+        if (held.size() >= 64) {
+            check_cuda(cudaStreamSynchronize(stream), "uploads");
+            held.clear();
+        }
+        auto p = std::make_shared<const std::vector<T>>(std::move(v));
+        held.push_back(p);
+        return *p;
+    }
     std::string stage_text;
     bool stage_timing = false;
     double ingest_ms = 0;           // s1g_open_file: map + staged upload
@@ -423,7 +436,7 @@ static void open_stream(s1g_decoder* h, const uint8_t* bytes, size_t n, bool sta
     check_cuda(cudaSetDevice(h->device), "cudaSetDevice");
     check_cuda(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking), "stream");
     h->fft.reset(new FftEngine(h->stream));
-    h->tabs.init(h->stream);
+    h->tabs.init();
     ingest(h, bytes, n, staged);
 }
 
@@ -457,10 +470,16 @@ struct Pipe {
     const std::vector<int>* cur_pk = nullptr;   // packets of the burst being processed
     explicit Pipe(s1g_decoder* hh) : h(hh), st(hh->stream), fft(*hh->fft) {}
 
+    // queue a copy of v, which the handle holds until the stream is waited for
     template <typename T>
-    T* upload(Buf& b, const std::vector<T>& v) {
+    void put(T* d, std::vector<T> v, const char* what) {
+        const std::vector<T>& kept = h->hold(std::move(v));
+        check_cuda(cudaMemcpyAsync(d, kept.data(), sizeof(T) * kept.size(), cudaMemcpyHostToDevice, st), what);
+    }
+    template <typename T>
+    T* upload(Buf& b, std::vector<T> v) {
         T* d = b.as<T>(v.size());
-        check_cuda(cudaMemcpyAsync(d, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice, st), "upload");
+        put(d, std::move(v), "upload");
         return d;
     }
 
@@ -568,7 +587,7 @@ struct Pipe {
             std::unique_ptr<Buf>& b = h->burst_idx[pk];
             if (!b) {
                 b = std::make_unique<Buf>();
-                upload_table(b->as<int>(pk.size()), pk.data(), sizeof(int) * pk.size(), st, "burst index upload");
+                upload_table(b->as<int>(pk.size()), pk.data(), sizeof(int) * pk.size(), "burst index upload");
             }
             d_idx = (const int*)b->p;
         }
@@ -597,7 +616,7 @@ struct Pipe {
         int* flags = h->bFlags.as<int>(n_a);
         eccm_detect_mixed(B, n_r, n_r, n_a, (double)h->det, a64, n_r, h->bEccmRoots.as<cf64>(n_r), flags, st);
         auto& cp = h->cffts[128];
-        if (!cp) cp = make_cfft_plan(128, st);
+        if (!cp) cp = make_cfft_plan(128);
         eccm_notch_cc(a64, n_r, out, n_r, n_r, n_a, flags, (double)h->mit, cp->d, st);
     }
 
@@ -702,7 +721,7 @@ struct Pipe {
             const double th = kPI_ * rate * std::pow(t[a] - (0.5 * 1.06), 2.0);
             d[a] = mk((R)std::cos(th), (R)std::sin(th));
         }
-        cpx<R>* dd = upload(h->bTab, d);
+        cpx<R>* dd = upload(h->bTab, std::move(d));
         cf64* sums = (cf64*)h->bSmall.get(sizeof(cf64) * n_r);
         dc_sums<R>(rc, n_r, n_a, n_r, dd, sums, st);
         DcFitArgs fa{};
@@ -753,32 +772,31 @@ struct Pipe {
                 der[k] = mk((R)std::cos(th), (R)std::sin(th));
                 rer[k] = mk((R)std::cos(th2), (R)std::sin(th2));
             }
-            cpx<R>* dder = upload(h->bTab, der);
+            cpx<R>* dder = upload(h->bTab, std::move(der));
             cpx<R>* Bt = h->bB.as<cpx<R>>((size_t)n_r * std::max(n_a, S));
             cpx<R>* Ct = h->bC.as<cpx<R>>((size_t)n_r * S);
             transpose_batched<R>(A, n_r, 0, Bt, n_a, 0, n_a, n_r, 1, st);
             fft_rows(n_a, Bt, n_a, Bt, n_a, n_r, -1);
             fufr_prep<R>(Bt, n_a, n_a, Ct, S, S, tile_len, dder, n_r, st);
             through_band(Ct, Bt, S, start, end - start, n_r, 1.0);
-            cpx<R>* drer = upload(h->bRef, rer);
+            cpx<R>* drer = upload(h->bRef, std::move(rer));
             scale_mul_vec<R>(Bt, S, S, n_r, drer, 1.0 / S, st);
             A = h->bA.as<cpx<R>>((size_t)S * n_r);
             transpose_batched<R>(Bt, S, 0, A, n_r, 0, n_r, S, 1, st);
             time_delta /= double(S) / double(n_a);
         } else {
-            std::vector<double> z(n_r, 0.0);
             fdc = h->bCols.as<double>(n_r);
-            check_cuda(cudaMemcpyAsync(fdc, z.data(), sizeof(double) * n_r, cudaMemcpyHostToDevice, st), "dc0");
+            check_cuda(cudaMemsetAsync(fdc, 0, sizeof(double) * n_r, st), "dc0");
         }
         const std::vector<double> az_freqs =
             tops ? linspace(-nrep * g.prf / 2, nrep * g.prf / 2, S) : linspace(-g.prf / 2, g.prf / 2, S);
-        const std::vector<RowParam> rp = row_params(g, S, time_delta, az_freqs);
-        RowParam* drp = upload(h->bRows, rp);
+        RowParam* drp = upload(h->bRows, row_params(g, S, time_delta, az_freqs));
         double* cols = h->bD.as<double>((size_t)4 * n_r);
-        check_cuda(cudaMemcpyAsync(cols, g.slant.data(), sizeof(double) * n_r, cudaMemcpyHostToDevice, st), "cols");
-        check_cuda(cudaMemcpyAsync(cols + n_r, g.range_freq.data(), sizeof(double) * n_r, cudaMemcpyHostToDevice, st), "cols");
-        check_cuda(cudaMemcpyAsync(cols + 2 * n_r, g.tcorr.data(), sizeof(double) * n_r, cudaMemcpyHostToDevice, st), "cols");
-        check_cuda(cudaMemcpyAsync(cols + 3 * n_r, g.rscale.data(), sizeof(double) * n_r, cudaMemcpyHostToDevice, st), "cols");
+        std::vector<double> hcols;
+        hcols.reserve((size_t)4 * n_r);
+        for (const std::vector<double>* v : {&g.slant, &g.range_freq, &g.tcorr, &g.rscale})
+            hcols.insert(hcols.end(), v->begin(), v->begin() + n_r);
+        put(cols, std::move(hcols), "cols");
         const double* slant = cols;
         const double* rf = cols + n_r;
         const double* tcorr = cols + 2 * n_r;
@@ -936,7 +954,8 @@ static ChainResult azimuth_chain(s1g_decoder* h, const std::vector<int>& pk, con
         e[a] = mk((R)std::cos(-ph), (R)std::sin(-ph));
     }
     double* dd = (double*)h->bJd.get(sizeof(double) * hostd.size());
-    check_cuda(cudaMemcpyAsync(dd, hostd.data(), sizeof(double) * (3 * n_a + n_r), cudaMemcpyHostToDevice, st),
+    const std::vector<double>& geometry = h->hold(std::move(hostd));
+    check_cuda(cudaMemcpyAsync(dd, geometry.data(), sizeof(double) * (3 * n_a + n_r), cudaMemcpyHostToDevice, st),
                "chain geometry");
     const double* d_beta = dd;
     const double* d_omd = dd + n_a;
@@ -945,7 +964,7 @@ static ChainResult azimuth_chain(s1g_decoder* h, const std::vector<int>& pk, con
     double* d_bk = d_ak + n_a;
     double* d_dphi = d_bk + n_a;
     double* d_sums = d_dphi + n_a;
-    cpx<R>* d_e = p.upload(h->bJe, e);
+    cpx<R>* d_e = p.upload(h->bJe, std::move(e));
     cpx<R>* U = h->bJ0.as<cpx<R>>((size_t)N);
     cpx<R>* T1 = h->bJ1.as<cpx<R>>((size_t)N);
     cpx<R>* QM = h->bJ2.as<cpx<R>>((size_t)N);
@@ -967,6 +986,7 @@ static ChainResult azimuth_chain(s1g_decoder* h, const std::vector<int>& pk, con
     double sums[2];
     check_cuda(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, st), "entropy down");
     check_cuda(cudaStreamSynchronize(st), "chain sync");
+    h->held.clear();
     ChainResult res;
     res.rows = n_a;
     res.cols = n_r;
@@ -1067,7 +1087,6 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
         rer_c[k] = mk((R)std::cos(th2), (R)(-std::sin(th2)));
     }
     const double time_delta = g.T / g.prf / (double(S) / double(n_a));
-    const std::vector<RowParam> rp = p.row_params(g, S, time_delta, f);
     // device tables: [der | rer | conj rer] complex, then the per-range-bin
     // columns and the reductions in FP64
     std::vector<cpx<R>> vecs;
@@ -1082,7 +1101,7 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
         for (int j = 0; j < nt; ++j, xp *= xa[a]) ph += theta[j] * xp;
         vecs.push_back(mk((R)std::cos(-ph), (R)std::sin(-ph)));
     }
-    cpx<R>* dv = p.upload(h->bJe, vecs);
+    cpx<R>* dv = p.upload(h->bJe, std::move(vecs));
     const cpx<R>* d_der = dv;
     const cpx<R>* d_rer = dv + S;
     const cpx<R>* d_rerc = dv + 2 * S;
@@ -1096,13 +1115,14 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
         cols[4 * n_r + j] = g.rscale[j];
     }
     double* dd = (double*)h->bJd.get(sizeof(double) * cols.size());
-    check_cuda(cudaMemcpyAsync(dd, cols.data(), sizeof(double) * 5 * n_r, cudaMemcpyHostToDevice, st), "tops columns");
+    const std::vector<double>& columns = h->hold(std::move(cols));
+    check_cuda(cudaMemcpyAsync(dd, columns.data(), sizeof(double) * 5 * n_r, cudaMemcpyHostToDevice, st), "tops columns");
     TopsCols tc{dd, dd + n_r, dd + 2 * n_r, dd + 3 * n_r, dd + 4 * n_r};
     double* d_dz = dd + 5 * n_r;      // per azimuth row: centroid derivative through the post factor
     double* d_ds = d_dz + S;          // ... through SRC
     double* d_dphi = d_ds + S;        // per line: d L / d phi_a
     double* d_sums = d_dphi + n_a;    // entropy sums
-    RowParam* drp = p.upload(h->bRows, rp);
+    RowParam* drp = p.upload(h->bRows, p.row_params(g, S, time_delta, f));
     const long long NA = (long long)n_a * n_r, NS = (long long)S * n_r;
     const int wmax = std::max(n_a, S);
     cpx<R>* U = h->bJ0.as<cpx<R>>((size_t)NA);
@@ -1133,6 +1153,7 @@ static ChainResult tops_chain(s1g_decoder* h, const std::vector<int>& pk, const 
     double sums[2];
     check_cuda(cudaMemcpyAsync(sums, d_sums, sizeof(sums), cudaMemcpyDeviceToHost, st), "entropy down");
     check_cuda(cudaStreamSynchronize(st), "chain sync");
+    h->held.clear();
     ChainResult res;
     res.rows = S;
     res.cols = n_r;
@@ -1281,8 +1302,10 @@ static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     check_cuda(cudaMalloc(&db, sizeof(cpx<double>) * m), "czt tmp");
     check_cuda(cudaMalloc(&dk, sizeof(cf32) * m), "czt kern");
     t->owned = {dw, dk};
-    upload_table(dw, w.data(), sizeof(cf32) * nw, h->stream, "czt up");
-    upload_table(db, b.data(), sizeof(cpx<double>) * m, h->stream, "czt up");
+    Uploads up;
+    up.table(dw, w.data(), sizeof(cf32) * nw, "czt up");
+    up.table(db, b.data(), sizeof(cpx<double>) * m, "czt up");
+    up.done();
     auto p64 = h->fft->plan<double>(m);
     h->fft->rows<double>(*p64, (cpx<double>*)db, m, (cpx<double>*)db, m, 1, -1);
     check_cuda(cudaStreamSynchronize(h->stream), "czt fft");
@@ -1291,7 +1314,7 @@ static CztDev get_czt(s1g_decoder* h, int P, int nin, int nout) {
     cudaFree(db);
     std::vector<cf32> K(m);
     for (int q = 0; q < m; ++q) K[plan->mid[q]] = mk((float)(B[q].x / m), (float)(B[q].y / m));
-    upload_table(dk, K.data(), sizeof(cf32) * m, h->stream, "czt up");
+    upload_table(dk, K.data(), sizeof(cf32) * m, "czt up");
     t->dev.chirp = (const cf32*)dw;
     t->dev.kern = (const cf32*)dk;
     h->czts[key] = t;
@@ -1444,7 +1467,7 @@ struct FastPipe {
             if (!choose_dc_block(n_r, g.L, fb->dcB, fb->dcU, fb->dcNb))
                 throw S1Error(S1G_E_GEOMETRY, "chirp too long for the Doppler estimator");
             auto& cp = h->dc_plans[fb->dcB];
-            if (!cp) cp = make_dc_plan(fb->dcB, st);
+            if (!cp) cp = make_dc_plan(fb->dcB);
             fb->dcDesc = cp->d;
             {
                 const int B = fb->dcB;
@@ -1809,7 +1832,10 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
         }
     } catch (...) {
         h->defer_status = false;
-        if (h->pending && cudaStreamSynchronize(h->stream) == cudaSuccess) decode_ok();
+        if (cudaStreamSynchronize(h->stream) == cudaSuccess) {
+            h->held.clear();
+            decode_ok();
+        }
         throw;
     }
     h->defer_status = false;
@@ -1818,6 +1844,7 @@ static Result compute_burst(s1g_decoder* h, const std::vector<int>& pk, int leve
     tma_read_error(pin, h->stream);
     if (r.status) check_cuda(cudaMemcpyAsync(pin + 1, r.status, sizeof(int), cudaMemcpyDeviceToHost, h->stream), "tufr status");
     check_cuda(cudaStreamSynchronize(h->stream), "product");
+    h->held.clear();
     float ms = 0;
     cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     h->last_ms = ms;
@@ -2239,8 +2266,7 @@ int s1g_packet_samples(s1g_decoder* h, int64_t packet, void* out, int64_t n, int
         bytes = sizeof(cf32) * g.n_r;
     }
     if (out_on_device) {
-        upload_table(out, src, bytes, h->stream, "samples up");
-        check_cuda(cudaStreamSynchronize(h->stream), "samples up");
+        upload_table(out, src, bytes, "samples up");
     } else {
         std::memcpy(out, src, bytes);
     }
@@ -2746,7 +2772,7 @@ static std::shared_ptr<BatchDecode> batch_decode_plan(s1g_decoder* h, const std:
     bd->raw_elems = out;
     bd->njobs = (int)jobs.size();
     check_cuda(cudaMalloc(&bd->d_jobs, sizeof(DecodeJob) * std::max<size_t>(jobs.size(), 1)), "decode jobs");
-    upload_table(bd->d_jobs, jobs.data(), sizeof(DecodeJob) * jobs.size(), h->stream, "decode jobs up");
+    upload_table(bd->d_jobs, jobs.data(), sizeof(DecodeJob) * jobs.size(), "decode jobs up");
     return bd;
 }
 
@@ -3088,7 +3114,10 @@ int s1g_process_swath_batch(s1g_decoder** hs, int n_streams, const char* swath, 
         h0->last_ms = ms;
         cudaEventDestroy(b0);
         cudaEventDestroy(b1);
-        for (int s = 0; s < n_streams; ++s) hs[s]->close_marks();
+        for (int s = 0; s < n_streams; ++s) {
+            hs[s]->close_marks();
+            hs[s]->held.clear();
+        }
         check_cuda(cudaGetLastError(), "batch kernels");
         check_batch(*run, n_streams);
         *samples = run->total;

@@ -214,7 +214,7 @@ CfftPlan::~CfftPlan() {
     for (void* p : owned) cudaFree(p);
 }
 
-std::shared_ptr<CfftPlan> make_cfft_plan(int n, cudaStream_t st) {
+std::shared_ptr<CfftPlan> make_cfft_plan(int n) {
     auto p = std::make_shared<CfftPlan>();
     p->d.n = n;
     std::vector<float4> tw(n);
@@ -226,7 +226,7 @@ std::shared_ptr<CfftPlan> make_cfft_plan(int n, cudaStream_t st) {
     void* dt = nullptr;
     check_cuda(cudaMalloc(&dt, sizeof(float4) * n), "cfft tw");
     p->owned.push_back(dt);
-    upload_table(dt, tw.data(), sizeof(float4) * n, st, "cfft tw up");
+    upload_table(dt, tw.data(), sizeof(float4) * n, "cfft tw up");
     p->d.tw = (const float4*)dt;
     return p;
 }
@@ -281,12 +281,13 @@ DcFftPlan::~DcFftPlan() {
     for (void* p : owned) cudaFree(p);
 }
 
-std::shared_ptr<DcFftPlan> make_dc_plan(int n, cudaStream_t st) {
+std::shared_ptr<DcFftPlan> make_dc_plan(int n) {
     auto plan = std::make_shared<DcFftPlan>();
     DcFft& d = plan->d;
     d = dc_passes(n);
     if (d.n != n) throw std::runtime_error("Doppler estimator: block length");
     int span = n;
+    Uploads uploads;
     for (int p = 0; p + 1 < d.np; ++p) {
         const int P = d.radix[p], Ns = span / P;
         std::vector<float4> tw((size_t)(P - 1) * Ns);
@@ -299,7 +300,7 @@ std::shared_ptr<DcFftPlan> make_dc_plan(int n, cudaStream_t st) {
         void* v = nullptr;
         check_cuda(cudaMalloc(&v, sizeof(float4) * tw.size()), "dc twiddles");
         plan->owned.push_back(v);
-        upload_table(v, tw.data(), sizeof(float4) * tw.size(), st, "dc twiddles up");
+        uploads.table(v, tw.data(), sizeof(float4) * tw.size(), "dc twiddles up");
         d.tw[p] = (const float4*)v;
         span = Ns;
     }

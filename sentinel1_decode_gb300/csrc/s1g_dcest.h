@@ -46,8 +46,8 @@ struct DcEstArgs {
 };
 
 // Twiddles of n points.
-std::shared_ptr<CfftPlan> make_cfft_plan(int n, cudaStream_t st);
-std::shared_ptr<DcFftPlan> make_dc_plan(int n, cudaStream_t st);
+std::shared_ptr<CfftPlan> make_cfft_plan(int n);
+std::shared_ptr<DcFftPlan> make_dc_plan(int n);
 // Overlap-save block B = 2^a 3^b (B >= L + 32, fits shared memory) of least
 // cost for lines of n_r samples and a chirp of L samples.
 bool choose_dc_block(int n_r, int L, int& B, int& U, int& nb);

@@ -825,12 +825,12 @@ DecodeTables::~DecodeTables() {
     if (lut) cudaFree(lut);
 }
 
-void DecodeTables::init(cudaStream_t st) {
+void DecodeTables::init() {
     if (lut) return;
     std::vector<HuffEntry> h;
     build_lut(h);
     check_cuda(cudaMalloc(&lut, sizeof(HuffEntry) * h.size()), "lut");
-    upload_table(lut, h.data(), sizeof(HuffEntry) * h.size(), st, "lut up");
+    upload_table(lut, h.data(), sizeof(HuffEntry) * h.size(), "lut up");
 }
 
 template <typename R>

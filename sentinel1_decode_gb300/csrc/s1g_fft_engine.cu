@@ -700,11 +700,11 @@ static void radices_for(int n, std::vector<int>& out) {
 }
 
 template <typename R>
-static void* upload(FftPlan<R>& p, const void* host, size_t bytes, cudaStream_t st) {
+static void* upload(FftPlan<R>& p, const void* host, size_t bytes, Uploads& up) {
     void* d = nullptr;
     check_cuda(cudaMalloc(&d, bytes), "plan cudaMalloc");
     p.owned.push_back(d);
-    upload_table(d, host, bytes, st, "plan upload");
+    up.table(d, host, bytes, "plan upload");
     return d;
 }
 
@@ -722,7 +722,7 @@ FftDescTables::~FftDescTables() {
 }
 
 template <typename R>
-static void fill_desc(FftDescTables& t, FftDesc<R>& d, int n, cudaStream_t st) {
+static void fill_desc(FftDescTables& t, FftDesc<R>& d, int n) {
     std::vector<int> rad;
     radices_for(n, rad);
     if ((int)rad.size() > kMaxStages) throw std::runtime_error("fft: too many stages");
@@ -746,11 +746,12 @@ static void fill_desc(FftDescTables& t, FftDesc<R>& d, int n, cudaStream_t st) {
         }
         perm[j] = pos;
     }
+    Uploads uploads;
     auto up = [&](const void* src, size_t bytes) {
         void* v = nullptr;
         check_cuda(cudaMalloc(&v, bytes), "desc table");
         t.owned.push_back(v);
-        upload_table(v, src, bytes, st, "desc upload");
+        uploads.table(v, src, bytes, "desc upload");
         return v;
     };
     d.tw = (const cpx<R>*)up(tw.data(), sizeof(cpx<R>) * n);
@@ -794,7 +795,7 @@ static Tw4<R> twiddle_entry(long long num, long long den, int sign) {
 }
 
 template <typename R>
-std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad, cudaStream_t st) {
+std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad) {
     if (rad.empty() || (int)rad.size() > kFft4Passes || sizeof(cpx<R>) * padded16_len(n) > (size_t)kFft4SmemBytes)
         throw std::runtime_error("plan4: length " + std::to_string(n) + " not smooth/small");
     long long prod = 1;
@@ -837,11 +838,12 @@ std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad, cu
         pos[F[i]] = i;
         p->mid[F[i]] = (i % last) * (n / last) + i / last;
     }
+    Uploads uploads;
     auto up = [&](const void* src, size_t bytes) {
         void* v = nullptr;
         check_cuda(cudaMalloc(&v, bytes), "plan4 table");
         p->owned.push_back(v);
-        upload_table(v, src, bytes, st, "plan4 upload");
+        uploads.table(v, src, bytes, "plan4 upload");
         return v;
     };
     const Tw4<R>* t = (const Tw4<R>*)up(tab.data(), sizeof(Tw4<R>) * tab.size());
@@ -854,8 +856,8 @@ std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& rad, cu
     return p;
 }
 
-template std::shared_ptr<Fft4PlanT<float>> build_plan4<float>(int, const std::vector<int>&, cudaStream_t);
-template std::shared_ptr<Fft4PlanT<double>> build_plan4<double>(int, const std::vector<int>&, cudaStream_t);
+template std::shared_ptr<Fft4PlanT<float>> build_plan4<float>(int, const std::vector<int>&);
+template std::shared_ptr<Fft4PlanT<double>> build_plan4<double>(int, const std::vector<int>&);
 
 // Factors of SPLIT (k_split_out).
 static const int kSplits[] = {2, 3, 4, 5, 6, 7, 8, 9, 10, 12, 15, 16};
@@ -917,15 +919,15 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
         }
     };
     auto core = [&](int len) {
-        if constexpr (sizeof(R) == 4) return build_plan4<R>(len, fft4_orders(len, 1).at(0), stream);
-        else return build_plan4<R>(len, fft4_order64(len), stream);
+        if constexpr (sizeof(R) == 4) return build_plan4<R>(len, fft4_orders(len, 1).at(0));
+        else return build_plan4<R>(len, fft4_order64(len));
     };
     auto desc = [&](int len) {
         for (auto k : {(const void*)k_rows8_smooth, (const void*)k_rows8_blue})
             check_cuda(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes), "smem attr");
         auto t = std::make_shared<FftDescTables>();
-        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, len, stream);
-        else fill_desc<R>(*t, t->d64, len, stream);
+        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, len);
+        else fill_desc<R>(*t, t->d64, len);
         return t;
     };
     const bool fits = radix8 ? is_smooth7(n) && n <= cap :
@@ -949,7 +951,8 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
             unit_root(i, n, c, s);
             tw[i] = mk((R)c, (R)s);
         }
-        return (cpx<R>*)upload(*p, tw.data(), sizeof(cpx<R>) * n, stream);
+        Uploads up;
+        return (cpx<R>*)upload(*p, tw.data(), sizeof(cpx<R>) * n, up);
     };
     if (fits) {
         p->kind = FFT_SMEM;
@@ -988,12 +991,14 @@ static std::shared_ptr<FftPlan<R>> make_plan(FftEngine& e, int n, bool radix8) {
             b[k] = mk(c, -s);  // conj(w)
             if (k > 0) b[m - k] = mk(c, -s);
         }
-        p->chirp = (cpx<R>*)upload(*p, w.data(), sizeof(cpx<R>) * n, stream);
+        Uploads up;
+        p->chirp = (cpx<R>*)upload(*p, w.data(), sizeof(cpx<R>) * n, up);
         // kernel spectrum computed in FP64 on the device, scaled by 1/m
         auto p64 = make_plan<double>(e, (int)m, false);
         cpx<double>* d64 = nullptr;
         check_cuda(cudaMalloc(&d64, sizeof(cpx<double>) * m), "blue tmp");
-        upload_table(d64, b.data(), sizeof(cpx<double>) * m, stream, "blue up");
+        up.table(d64, b.data(), sizeof(cpx<double>) * m, "blue up");
+        up.done();
         e.rows<double>(*p64, d64, m, d64, m, 1, -1);
         cpx<R>* kd = nullptr;
         check_cuda(cudaMalloc(&kd, sizeof(cpx<R>) * m), "blue kern");
@@ -1125,7 +1130,7 @@ void FftEngine::from_band(const BandPlan& p, const cf64* in, long long ip, cf64*
 std::shared_ptr<Fft4Plan> FftEngine::plan4(int n) {
     auto it = plans4.find(n);
     if (it != plans4.end()) return it->second;
-    auto p = build_plan4<float>(n, tuned_radices(n, stream), stream);
+    auto p = build_plan4<float>(n, tuned_radices(n, stream));
     plans4[n] = p;
     return p;
 }
@@ -1139,8 +1144,8 @@ FftDesc<R> FftEngine::smem_desc(int n) {
     auto& t = (sizeof(R) == 4 ? descs32 : descs64)[n];
     if (!t) {
         t = std::make_shared<FftDescTables>();
-        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, n, stream);
-        else fill_desc<R>(*t, t->d64, n, stream);
+        if constexpr (sizeof(R) == 4) fill_desc<R>(*t, t->d32, n);
+        else fill_desc<R>(*t, t->d64, n);
     }
     if constexpr (sizeof(R) == 4) return t->d32;
     else return t->d64;

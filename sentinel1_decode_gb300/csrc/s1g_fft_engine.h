@@ -178,7 +178,7 @@ std::vector<int> fft4_order64(long long n);
 // The cheapest affine lengths >= minlen that fit shared memory.
 std::vector<long long> fft4_lengths(long long minlen, size_t most);
 template <typename R>
-std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& radices, cudaStream_t st);
+std::shared_ptr<Fft4PlanT<R>> build_plan4(int n, const std::vector<int>& radices);
 // Radix order for length n: the fastest measured candidate when tuning is on
 // (S1G_AUTOTUNE unset or not "0"), else the model's.  Measurements run on
 // `st` (skipped while st is being captured) and persist in a text file
@@ -205,11 +205,32 @@ void transpose_batched(const cpx<R>* in, long long in_row_pitch, long long in_ba
                        cudaStream_t s, Failed failed = {});
 
 void check_cuda(cudaError_t e, const char* what);
-// Copy a host table (which may go when the call returns) to device memory in
-// the order of st.  A plain cudaMemcpy of pageable memory may return before the
-// device has it, and the handles' streams do not wait for the legacy stream.
-inline void upload_table(void* dst, const void* src, size_t bytes, cudaStream_t st, const char* what) {
-    check_cuda(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st), what);
+// Copies of host tables to device memory, there for every stream when this goes.
+// A copy of pageable memory by cudaMemcpy may return before the device has it,
+// and the handles' streams do not wait for the legacy stream, so that one is
+// waited for (not the handle's, whose kernels may run on meanwhile); an
+// asynchronous copy might read the host's memory after it has returned.
+struct Uploads {
+    bool open = false;
+    Uploads() = default;
+    Uploads(const Uploads&) = delete;
+    void table(void* dst, const void* src, size_t bytes, const char* what) {
+        open = true;
+        check_cuda(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
+    }
+    void done() {
+        if (open) check_cuda(cudaStreamSynchronize(cudaStreamLegacy), "uploads");
+        open = false;
+    }
+    ~Uploads() {
+        if (open) cudaStreamSynchronize(cudaStreamLegacy);
+    }
+};
+// One of them.
+inline void upload_table(void* dst, const void* src, size_t bytes, const char* what) {
+    Uploads u;
+    u.table(dst, src, bytes, what);
+    u.done();
 }
 // Copy a host table to a device variable that every stream may read from now on.
 template <class T>

@@ -37,7 +37,7 @@ void gather_headers(const uint8_t* d_stream, long long n, const long long* d_off
 // ------------------------------------------------------------------ decode
 struct DecodeTables {
     void* lut = nullptr;
-    void init(cudaStream_t st);
+    void init();
     ~DecodeTables();
 };
 

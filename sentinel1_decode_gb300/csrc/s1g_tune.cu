@@ -176,7 +176,7 @@ struct Tuner {
         std::vector<int> best;
         double bt = 1e30;
         for (const auto& c : cand) {
-            auto plan = build_plan4<float>(n, c, st);
+            auto plan = build_plan4<float>(n, c);
             const double t = time_plan(plan->d, st);
             if (best.empty() || t < bt * 0.98) {
                 bt = t;
@@ -216,7 +216,7 @@ long long tuned_length(long long minlen, cudaStream_t st) {
     long long best = c[0];
     double bt = 1e30;
     for (const long long m : c) {
-        auto plan = build_plan4<float>((int)m, t.radices_locked((int)m, st), st);
+        auto plan = build_plan4<float>((int)m, t.radices_locked((int)m, st));
         const double us = t.time_plan(plan->d, st);
         if (us < bt * 0.98) {
             bt = us;

@@ -7,6 +7,8 @@
 //   pending         1 after a copy of pageable memory or a memset on the legacy
 //                   stream that nothing waited for
 //   unordered       launches on another stream while that is so
+//   stale           copies queued on a stream whose pageable source had changed or
+//                   gone by the time the stream was waited for
 //   refused         launches with more dynamic shared memory than the kernel may
 //                   have on the current device (they fail, as on a GPU)
 //   capture, replay graphs captured and launched
@@ -20,6 +22,7 @@
 #include <set>
 #include <string>
 #include <utility>
+#include <vector>
 
 namespace {
 
@@ -41,6 +44,14 @@ std::map<std::pair<const void*, int>, int> smem_limit;
 std::set<void*> page_locked;
 std::string last_unordered;
 bool legacy_copy = false;
+// queued copies from pageable memory: what the device may read as late as when
+// the stream is waited for, and what it has to read
+struct Queued {
+    cudaStream_t stream;
+    const void* src;
+    std::string data;
+};
+std::vector<Queued> queued;
 cudaStream_t capturing = nullptr;
 thread_local Config config;
 thread_local int device = 0;
@@ -55,6 +66,14 @@ cudaError_t fail(cudaError_t e) {
 bool legacy(cudaStream_t s) { return s == nullptr || s == cudaStreamLegacy; }
 bool pageable(const void* p) { return page_locked.empty() || !page_locked.count(const_cast<void*>(p)); }
 void* handle() { return std::calloc(1, 16); }
+void waited(cudaStream_t stream, bool all) {
+    std::vector<Queued> rest;
+    for (Queued& q : queued) {
+        if (!all && q.stream != stream) rest.push_back(std::move(q));
+        else if (std::memcmp(q.src, q.data.data(), q.data.size()) != 0) ++counts["stale"];
+    }
+    queued.swap(rest);
+}
 
 // parameter i of a launch
 template <typename T>
@@ -203,7 +222,10 @@ cudaError_t cudaMemcpy(void* d, const void* s, size_t n, cudaMemcpyKind kind) {
 cudaError_t cudaMemcpyAsync(void* d, const void* s, size_t n, cudaMemcpyKind kind, cudaStream_t stream) {
     Lock lk(mu);
     std::memcpy(d, s, n);
-    if (legacy(stream) && kind == cudaMemcpyHostToDevice && pageable(s)) legacy_copy = true;
+    if (kind == cudaMemcpyHostToDevice && pageable(s)) {
+        if (legacy(stream)) legacy_copy = true;
+        else queued.push_back({stream, s, std::string((const char*)s, n)});
+    }
     return cudaSuccess;
 }
 cudaError_t cudaMemcpy2DAsync(void* d, size_t dp, const void* s, size_t sp, size_t w, size_t h, cudaMemcpyKind, cudaStream_t) {
@@ -266,11 +288,13 @@ cudaError_t cudaStreamSynchronize(cudaStream_t s) {
     Lock lk(mu);
     if (capturing) return fail(cudaErrorStreamCaptureUnsupported);
     if (legacy(s)) legacy_copy = false;
+    waited(s, false);
     return cudaSuccess;
 }
 cudaError_t cudaDeviceSynchronize() {
     Lock lk(mu);
     legacy_copy = false;
+    waited(nullptr, true);
     return capturing ? fail(cudaErrorStreamCaptureUnsupported) : cudaSuccess;
 }
 cudaError_t cudaStreamWaitEvent(cudaStream_t, cudaEvent_t, unsigned) { return cudaSuccess; }
